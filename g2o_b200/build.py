@@ -11,7 +11,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libg2o_b200.so")
 CLI = os.path.join(HERE, "g2o_cuda_cli")
 CLI_SOURCE = "g2o_cuda_cli.cpp"
-SOURCES = ["g2oc_api.cu", "noalloc.cu", "structure.cpp", "g2o_io.cpp"]
+SOURCES = ["g2oc_api.cu", "noalloc.cu", "structure.cpp", "chol_plan.cpp", "g2o_io.cpp"]
 HEADERS = sorted(f for f in os.listdir(CSRC) if f.endswith((".h", ".cuh")))
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

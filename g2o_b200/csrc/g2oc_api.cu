@@ -1194,7 +1194,7 @@ struct Engine final : EngineBase {
       const long long total = (long long)P.np * P.np;
       G2OC_K(K_TC_EXPAND) tc_expand_tiles<<<cdiv(total, 256), 256, 0, st>>>(tiles.p, P.tile_index.p, P.nbt, P.n,
                                                                            P.np, P.A.p);
-      G2OC_K(K_TC_EXPAND) chol_pivot_floor<float><<<1, 1024, 0, st>>>(P.A.p, P.np, P.n, P.floor.p);
+      G2OC_K(K_TC_EXPAND) tc_pivot_floor<<<1, 1024, 0, st>>>(P.A.p, P.np, P.n, P.floor.p);
       for (int k = 0; k < P.nt; ++k) {
         float* Wk = P.W.p + (size_t)k * kTc * kTc;
         G2OC_K(K_TC_POTRF) tc_potrf<<<1, 256, kTcPotrfSmem, st>>>(P.A.p, P.np, k, Wk, P.floor.p, P.info.p);
@@ -1266,21 +1266,27 @@ struct Engine final : EngineBase {
     return G2OC_OK;
   }
 
-  int chol_solve(const Real* val, const double* rhs, double* xout, int* ok) {
+  int ensure_chol() {
+    if (c->chol) return G2OC_OK;
     const Structure& S = c->S;
-    if (!c->chol) {
-      const std::vector<int32_t>& rc = S.ba && S.schur ? S.schur_rc : S.hpp_rc;
-      std::unique_ptr<CholPlan> P(new CholPlan());
-      G2OC_TRY(chol_plan_build(*P, S.sys_nb, S.pd, rc, !S.ba, c->stream));
-      c->chol = std::move(P);
-    }
-    return g2oc::chol_solve<Real>(*c->chol, c->stream, sys(val), rhs, xout, ok, &c->kcount[K_CHOLESKY]);
+    std::unique_ptr<CholPlan> P(new CholPlan());
+    G2OC_TRY(chol_plan_build(*P, S.sys_nb, S.pd, S.sys_brow, S.sys_rcol, !S.ba, c->stream));
+    P->extra = c->barrier_extra;
+    c->chol = std::move(P);
+    return G2OC_OK;
+  }
+
+  // the outcome (positive definite or not) stays on the device, c->chol->state
+  int chol_solve(const Real* val, const double* rhs, double* xout) {
+    G2OC_TRY(ensure_chol());
+    return chol_solve_async<Real>(*c->chol, c->stream, sys(val), rhs, xout, &c->kcount[K_CHOLESKY]);
   }
 
   int solve(double lambda) override {
     const Structure& S = c->S;
     cudaStream_t st = c->stream;
     int ok = 1;
+    const CholState* outcome = nullptr;
     const bool use_chol = c->prm.linear_solver == G2OC_LINEAR_CHOLESKY ||
                           (c->prm.linear_solver == 2 && !S.ba);
     if (S.Cf == 0) {
@@ -1318,7 +1324,8 @@ struct Engine final : EngineBase {
         G2OC_TRY(tc_factor(&ok));
         G2OC_TRY(tc_resolve(c->rhs.p, c->xs.p));
       } else if (use_chol) {
-        G2OC_TRY(chol_solve(Sval.p, c->rhs.p, c->xs.p, &ok));
+        G2OC_TRY(chol_solve(Sval.p, c->rhs.p, c->xs.p));
+        outcome = c->chol->state.p;
       } else {
         G2OC_TRY(pcg_solve(Sval.p, c->rhs.p, c->xs.p, false));
       }
@@ -1413,12 +1420,18 @@ struct Engine final : EngineBase {
         G2OC_K(K_DAMP) sys_gather_damped<Real, 6><<<cdiv(nel, 256), 256, 0, st>>>(
             hpp.p, c->sys_perm.p, c->sys_brow.p, c->sys_rptr.p, c->sys_rcol.p, nnzb, lambda, sysval.p);
       G2OC_LAUNCH_CHECK();
-      if (use_chol) G2OC_TRY(chol_solve(sysval.p, c->b.p, c->x.p, &ok));
-      else G2OC_TRY(pcg_solve(sysval.p, c->b.p, c->x.p, false));
-      if (sizeof(Real) == 4 && ok && use_chol && !S.ba && c->prm.refine_max_iterations >= 0)
-        G2OC_TRY(refine_pose_graph(lambda));
+      if (use_chol) {
+        G2OC_TRY(chol_solve(sysval.p, c->b.p, c->x.p));
+        outcome = c->chol->state.p;
+        if (sizeof(Real) == 4 && !S.ba && c->prm.refine_max_iterations >= 0) {
+          G2OC_TRY(chol_outcome(*c->chol, st, &ok));
+          if (ok) G2OC_TRY(refine_pose_graph(lambda));
+        }
+      } else {
+        G2OC_TRY(pcg_solve(sysval.p, c->b.p, c->x.p, false));
+      }
     }
-    G2OC_K(K_LM_CONTROL) set_solve_ok<<<1, 32, 0, st>>>(c->sc.p, ok);
+    G2OC_K(K_LM_CONTROL) set_solve_ok<<<1, 32, 0, st>>>(c->sc.p, ok, outcome);
     G2OC_LAUNCH_CHECK();
     return G2OC_OK;
   }
@@ -1660,7 +1673,8 @@ struct Engine final : EngineBase {
     G2OC_TRY(schur_rhs_from(rp, rl, c->rhs.p));
     int ok = 1;
     if (use_chol) {
-      G2OC_TRY(chol_solve(Sval.p, c->rhs.p, c->xs.p, &ok));
+      G2OC_TRY(chol_solve(Sval.p, c->rhs.p, c->xs.p));
+      G2OC_TRY(chol_outcome(*c->chol, st, &ok));
       if (!ok) {
         set_error("adjoint solve: the reduced system is not positive definite");
         return G2OC_ERR_NOT_PD;
@@ -1892,7 +1906,7 @@ struct BalEngine final : EngineBase {
   int solve(double lambda) override {
     const Structure& S = c->S;
     cudaStream_t st = c->stream;
-    int ok = 1;
+    const CholState* outcome = nullptr;
     const double* bl = c->b.p + (size_t)S.Cf * 9;
     if (S.Cf == 0) {
       // every camera fixed: x_l = (H_ll + lambda I)^-1 b_l
@@ -1907,10 +1921,12 @@ struct BalEngine final : EngineBase {
       if (c->prm.linear_solver == G2OC_LINEAR_CHOLESKY) {
         if (!c->chol) {
           std::unique_ptr<CholPlan> P(new CholPlan());
-          G2OC_TRY(chol_plan_build(*P, S.sys_nb, 9, S.schur ? S.schur_rc : S.hpp_rc, false, st));
+          G2OC_TRY(chol_plan_build(*P, S.sys_nb, 9, S.sys_brow, S.sys_rcol, false, st));
+          P->extra = c->barrier_extra;
           c->chol = std::move(P);
         }
-        G2OC_TRY(g2oc::chol_solve<double>(*c->chol, st, A, c->rhs.p, c->xs.p, &ok, &c->kcount[K_CHOLESKY]));
+        G2OC_TRY(chol_solve_async<double>(*c->chol, st, A, c->rhs.p, c->xs.p, &c->kcount[K_CHOLESKY]));
+        outcome = c->chol->state.p;
       } else {
         G2OC_K(K_PCG_DIAG_INV) pcg_diag_inv_lanes<double, 9><<<cdiv(A.nb, 3 * 4), 128, 0, st>>>(A, minv.p,
                                                                                              c->flag.p);
@@ -1923,7 +1939,7 @@ struct BalEngine final : EngineBase {
                                     st));
       G2OC_TRY(backsub(bl, c->xs.p, c->x.p + (size_t)S.Cf * 9));
     }
-    G2OC_K(K_LM_CONTROL) set_solve_ok<<<1, 32, 0, st>>>(c->sc.p, ok);
+    G2OC_K(K_LM_CONTROL) set_solve_ok<<<1, 32, 0, st>>>(c->sc.p, 1, outcome);
     G2OC_LAUNCH_CHECK();
     return G2OC_OK;
   }
@@ -2076,6 +2092,11 @@ static int read_state(g2oc_ctx* c, DevScalars* h, g2oc_iteration_stats* stv) {
   if (ps.sync_error) {
     G2OC_TRY(reset_pcg(c));
     set_error("PCG: a grid barrier wait ran out");
+    return G2OC_ERR_TIMEOUT;
+  }
+  if (h->chol_error) {
+    G2OC_CUDA_TRY(cudaMemsetAsync(&c->sc.p->chol_error, 0, sizeof(int), c->stream));
+    set_error("cholesky: a wait for a tile ran out");
     return G2OC_ERR_TIMEOUT;
   }
   if (stv) stv->iterations_linear_solver += (int)(ps.total_iterations - c->pcg_seen);
@@ -3945,7 +3966,7 @@ int g2oc_solve_block_system(g2oc_ctx* c, int32_t linear_solver, int32_t nb, cons
   int it = 0, ok = 1;
   if (linear_solver == G2OC_LINEAR_CHOLESKY) {
     CholPlan P;
-    G2OC_TRY(chol_plan_build(P, nb, bs, cs.rcv, true, st));
+    G2OC_TRY(chol_plan_build(P, nb, bs, cs.tmp.sys_brow, cs.tmp.sys_rcol, true, st));
     G2OC_TRY(chol_solve<double>(P, st, A, rhs.p, xo.p, &ok, &c->kcount[K_CHOLESKY]));
   } else {
     G2OC_TRY(mi.alloc((size_t)nb * bs * bs));
@@ -3989,7 +4010,7 @@ static int solve_pattern(g2oc_ctx* c, CallerSystem& cs, int32_t nb, int32_t nreq
   }
   cudaStream_t st = c->stream;
   CholPlan P;
-  G2OC_TRY(chol_plan_build(P, nb, cs.bs, cs.rcv, true, st, &extra));
+  G2OC_TRY(chol_plan_build(P, nb, cs.bs, cs.tmp.sys_brow, cs.tmp.sys_rcol, true, st, &extra));
   DBuf<int2> d_req;
   DBuf<double> d_out;
   G2OC_TRY(d_req.upload(pairs, st));

@@ -179,7 +179,8 @@ struct DevScalars {
   int solve_ok;
   int accept;            // last trial accepted
   int nonfinite;         // a non-finite value was met
-  int pad[3];
+  int chol_error;        // a wait of the tiled Cholesky ran out
+  int pad[2];
 };
 
 }  // namespace g2oc

@@ -264,6 +264,23 @@ static __global__ void __launch_bounds__(128, 1)
 //   W21 = -W22 (L21 W11)                   two products
 // A non-positive pivot sets *info (the pivot is replaced by 1 so the
 // arithmetic stays finite).
+// the pivot floor of a factorization: 4 n eps (FP64) times the largest
+// diagonal entry of the expanded matrix, one CTA of 1024 threads (fixed tree)
+static __global__ void __launch_bounds__(1024) tc_pivot_floor(const float* A, int np, int n, double* floor) {
+  __shared__ double red[32];
+  double m = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) m = fmax(m, fabs((double)A[(size_t)i * np + i]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double r = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r = fmax(r, red[w]);
+    *floor = 4.0 * (double)n * 2.220446049250313e-16 * r;
+  }
+}
+
 constexpr int kTcLd = 68;                    // operand blocks, as tile_dmma64 reads them
 constexpr int kTcBlk = 64 * kTcLd;           // doubles per operand block
 constexpr int kTcTri = 64 * 65;              // doubles per diagonal block (leading dimension 65)

@@ -207,5 +207,140 @@ __device__ __forceinline__ void tile_potrf_inv_blk64(double* T, int ld, double* 
   }
 }
 
+// ------------------------------------------------- 64 x 64 tile, blocked by 8
+constexpr int kLd = 68;  // leading dimension of the tiles in shared memory: the
+                         // fragment loads (eight rows x four k of a warp
+                         // instruction) fall in distinct bank pairs
+
+// Factorization and inverse of the tile of a sparse plan, where the time of
+// one tile is the time of a step of the elimination tree's chain: W = L^-1 of
+// the leading width x width part (the rest of W is zero). T (shared memory,
+// row-major, kLd): the lower triangle of A in, L's strictly lower 8 x 8 blocks
+// out (padding up to the next multiple of 8 must be the identity); Ws (same
+// layout): W; S: 8 x kLd doubles of scratch. 256 threads. *info is set and the
+// pivot replaced by 1 where a pivot is not above floor.
+//
+// Bound by the chain of pivots (64 dependent rsqrt of ~75 cycles with two FP64
+// operations each) and kept short around it, per block column p of 8:
+//   A  every lane of the warps 0..2 factors the 8 x 8 diagonal block
+//      redundantly in its own registers, so no value passes between lanes
+//      inside the chain; warps 0 and 1 then solve one row of the panel below
+//      per thread against that factor, still in registers, and warp 2 forms
+//      W_pp. Meanwhile warps 3..7 take step p - 1's rank-8 update of the block
+//      columns beyond p, and the sums L_(p-1),: W of W's block row p - 1.
+//   B  the update of block column p + 1, one fragment per warp (all that the
+//      next A waits for), and block row p - 1 of W, -W_(p-1)(p-1) times its sums.
+// Products are FP64 tensor-core fragments; every sum has a fixed order.
+__device__ __forceinline__ void tile_trail_frag(double* T, int o, int fi, int fj) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const double* X = T + (o + 8) * kLd + o;
+  double c[2];
+  dmma_frag<false, false>(X, kLd, X, kLd, fi, fj, 8, c);
+  double* D = T + (o + 8 + 8 * fi + g) * kLd + o + 8 + 8 * fj + 2 * t4;
+  if (fi != fj || g >= 2 * t4) D[0] -= c[0];
+  if (fi != fj || g >= 2 * t4 + 1) D[1] -= c[1];
+}
+
+// columns 8 f .. of the sums L_p,: W (W is lower triangular: k from 8 f on)
+__device__ __forceinline__ void tile_w_sum(const double* T, const double* Ws, double* S, int p, int f) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  double c[2];
+  dmma_frag<false, true>(T + 8 * p * kLd + 8 * f, kLd, Ws + 8 * f * kLd + 8 * f, kLd, 0, 0, 8 * (p - f), c);
+  S[g * kLd + 8 * f + 2 * t4] = c[0];
+  S[g * kLd + 8 * f + 2 * t4 + 1] = c[1];
+}
+__device__ __forceinline__ void tile_w_row(double* Ws, const double* S, int p, int f) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  double c[2];
+  dmma_frag<false, true>(Ws + 8 * p * kLd + 8 * p, kLd, S + 8 * f, kLd, 0, 0, 8, c);
+  Ws[(8 * p + g) * kLd + 8 * f + 2 * t4] = -c[0];
+  Ws[(8 * p + g) * kLd + 8 * f + 2 * t4 + 1] = -c[1];
+}
+
+__device__ __forceinline__ void tile_potrf_inv64(double* T, double* Ws, double* S, int width, double floor,
+                                                 int* info) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int e = tid; e < 64 * 64; e += 256) Ws[(e >> 6) * kLd + (e & 63)] = 0.0;
+  __syncthreads();
+  const int nst = (width + 7) >> 3;
+  for (int p = 0; p < nst; ++p) {
+    const int o = 8 * p;
+    if (warp <= 2) {
+      double d[8][8], rs[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) d[i][j] = T[(o + i) * kLd + o + j];
+      const int row = o + 8 + tid;
+      const bool mine = warp < 2 && row < 8 * nst;
+      double x[8];
+      if (mine)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) x[c] = T[row * kLd + o + c];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        double v = d[j][j];
+        if (!(v > floor)) {
+          if (tid == 0) *info = 1;
+          v = 1.0;
+        }
+        rs[j] = rsqrt(v);
+#pragma unroll
+        for (int i = j + 1; i < 8; ++i) d[i][j] *= rs[j];
+#pragma unroll
+        for (int c = j + 1; c < 8; ++c)
+#pragma unroll
+          for (int i = c; i < 8; ++i) d[i][c] -= d[i][j] * d[c][j];
+      }
+      if (mine) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          x[c] *= rs[c];
+#pragma unroll
+          for (int q = c + 1; q < 8; ++q) x[q] -= x[c] * d[q][c];
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) T[row * kLd + o + c] = x[c];
+      } else if (warp == 2 && lane < 8) {
+        // column `lane` of W_pp
+        double w[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) w[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          w[c] *= rs[c];
+#pragma unroll
+          for (int q = c + 1; q < 8; ++q) w[q] -= w[c] * d[q][c];
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) Ws[(o + i) * kLd + o + lane] = w[i];
+      }
+    } else if (p > 0) {
+      const int nw = p - 1, nf = nst - 1 - p, n = nw + nf * (nf + 1) / 2;
+      for (int f = warp - 3; f < n; f += 5) {
+        if (f < nw) {
+          tile_w_sum(T, Ws, S, p - 1, f);
+        } else {
+          const int q = f - nw;
+          int fi = 0;
+          while ((fi + 1) * (fi + 2) / 2 <= q) ++fi;
+          tile_trail_frag(T, o - 8, 1 + fi, 1 + q - fi * (fi + 1) / 2);
+        }
+      }
+    }
+    __syncthreads();
+    if (warp < nst - 1 - p) tile_trail_frag(T, o, warp, 0);
+    if (p > 1 && 7 - warp < p - 1) tile_w_row(Ws, S, p - 1, 7 - warp);
+    __syncthreads();
+  }
+  if (nst > 1) {
+    for (int f = warp; f < nst - 1; f += 8) {
+      tile_w_sum(T, Ws, S, nst - 1, f);
+      __syncwarp();
+      tile_w_row(Ws, S, nst - 1, f);
+    }
+    __syncthreads();
+  }
+}
 
 }  // namespace g2oc
