@@ -10,6 +10,8 @@
 // bit-identical run to run; no floating-point atomics.
 #pragma once
 
+#include <type_traits>
+
 #include "g2o_math.cuh"
 #include "g2oc_internal.h"
 #include "reduce.cuh"
@@ -236,6 +238,11 @@ static __global__ void ba_jacobians_kernel(BAEdges E, BAVertices V, double* jp, 
   for (int i = 0; i < 12; ++i) jc[12 * k + i] = Jc[i];
 }
 
+// place of entry (r, c) of a 6 x 3 Hpl block in its 18 stored values: the
+// first two components of every row in pairs, then the third ones, as
+// schur_rows reads them
+__host__ __device__ constexpr int hpl_at(int r, int c) { return c < 2 ? 2 * r + c : 12 + r; }
+
 // Landmark pass of BlockSolver::buildSystem (block_solver.hpp:492-565) for the
 // landmark side: one thread per free landmark walks its edges (contiguous in
 // the point-major order), accumulates H_ll = sum Jp^T Om' Jp and
@@ -298,7 +305,7 @@ __global__ void ba_landmark_pass(BAEdges E, BAVertices V, const int* l_ptr, int 
 #pragma unroll
       for (int r = 0; r < 6; ++r)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) B[r * 3 + c] += Jc[r] * A0[c] + Jc[6 + r] * A1[c];
+        for (int c = 0; c < 3; ++c) B[hpl_at(r, c)] += Jc[r] * A0[c] + Jc[6 + r] * A1[c];
     }
   }
   if (cur >= 0) {
@@ -372,7 +379,7 @@ __global__ void __launch_bounds__(256) ba_landmark_warp(BAEdges E, BAVertices V,
 #pragma unroll
       for (int r = 0; r < 6; ++r)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) hb[r * 3 + c] = Jc[r] * A0[c] + Jc[6 + r] * A1[c];
+        for (int c = 0; c < 3; ++c) hb[hpl_at(r, c)] = Jc[r] * A0[c] + Jc[6 + r] * A1[c];
       R2* o = &stage[wid][(blk - blk0) * 9];
 #pragma unroll
       for (int q = 0; q < 9; ++q) {
@@ -491,12 +498,10 @@ __global__ void __launch_bounds__(THREADS) ba_camera_pass(BACamEdges CE, BAVerti
 
 // ---------------------------------------------------------------- Schur
 // Landmark step of the Schur loop (block_solver.hpp:359-378):
-// Dinv = (H_ll + lambda I)^-1 and BD_a = B_a Dinv for every Hpl block a of
-// the landmark, written in camera-major order (bdc[hc_index[a]]) so a camera
-// row's blocks are contiguous for the Schur row kernel.
+// Dinv = (H_ll + lambda I)^-1 of every landmark.
 template <typename Real>
-__global__ void schur_landmark(const Real* hll, const Real* hpl, const int* hb_ptr, const int* hc_index, int Pf,
-                               double lambda_all, const double* lambda_of, Real* dinv, Real* bdc, int* nonfinite) {
+__global__ void schur_landmark(const Real* hll, int Pf, double lambda_all, const double* lambda_of, Real* dinv,
+                               int* nonfinite) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= Pf) return;
   const double lambda = lambda_of ? lambda_of[l] : lambda_all;  // per landmark (batched windows)
@@ -506,55 +511,29 @@ __global__ void schur_landmark(const Real* hll, const Real* hpl, const int* hb_p
                  (double)h[2], (double)h[4], (double)h[5] + lambda};
   double Di[9];
   if (!inverse3(A, Di)) *nonfinite = 1;
-  Real D[9];
 #pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    D[i] = (Real)Di[i];
-    dinv[(size_t)l * 9 + i] = D[i];
-  }
-  if (!bdc) return;
-  const int b1 = hb_ptr[l + 1];
-  for (int a = hb_ptr[l]; a < b1; ++a) {
-    const Real* B = hpl + (size_t)a * 18;
-    Real* o = bdc + (size_t)hc_index[a] * 18;
-#pragma unroll
-    for (int r = 0; r < 6; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) o[r * 3 + c] = B[r * 3] * D[c] + B[r * 3 + 1] * D[3 + c] + B[r * 3 + 2] * D[6 + c];
-  }
+  for (int i = 0; i < 9; ++i) dinv[(size_t)l * 9 + i] = (Real)Di[i];
 }
 
-// One 6 x 3 Hpl block (18 values, row-major) into registers. FP32 blocks are
+// One 6 x 3 Hpl block (18 values, hpl_at order) into registers. FP32 blocks are
 // 72 bytes at a 72-byte stride: a block starts on a 16-byte boundary when its
 // index is even (four 16-byte loads, then 8 bytes) and on an 8-byte one when
 // odd (8 bytes, then four 16-byte loads): five loads instead of nine. FP64
 // blocks (144 bytes) are nine 16-byte loads.
-template <bool VEC>
 __device__ __forceinline__ void ldg_block18(const float* hpl, int blk, float (&b)[18]) {
   const float* base = hpl + (size_t)blk * 18;
-  if (VEC) {
-    const bool odd = blk & 1;
-    const int o4 = odd ? 2 : 0;
-    const float4 u0 = __ldg(reinterpret_cast<const float4*>(base + o4));
-    const float4 u1 = __ldg(reinterpret_cast<const float4*>(base + o4 + 4));
-    const float4 u2 = __ldg(reinterpret_cast<const float4*>(base + o4 + 8));
-    const float4 u3 = __ldg(reinterpret_cast<const float4*>(base + o4 + 12));
-    const float2 w = __ldg(reinterpret_cast<const float2*>(base + (odd ? 0 : 16)));
-    const float q[18] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w, u2.x,
-                         u2.y, u2.z, u2.w, u3.x, u3.y, u3.z, u3.w, w.x,  w.y};
+  const bool odd = blk & 1;
+  const int o4 = odd ? 2 : 0;
+  const float4 u0 = __ldg(reinterpret_cast<const float4*>(base + o4));
+  const float4 u1 = __ldg(reinterpret_cast<const float4*>(base + o4 + 4));
+  const float4 u2 = __ldg(reinterpret_cast<const float4*>(base + o4 + 8));
+  const float4 u3 = __ldg(reinterpret_cast<const float4*>(base + o4 + 12));
+  const float2 w = __ldg(reinterpret_cast<const float2*>(base + (odd ? 0 : 16)));
+  const float q[18] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w, u2.x,
+                       u2.y, u2.z, u2.w, u3.x, u3.y, u3.z, u3.w, w.x,  w.y};
 #pragma unroll
-    for (int t = 0; t < 18; ++t) b[t] = odd ? (t < 2 ? q[16 + t] : q[t - 2]) : q[t];
-  } else {
-    const float2* B2 = reinterpret_cast<const float2*>(base);
-#pragma unroll
-    for (int t = 0; t < 9; ++t) {
-      const float2 v = __ldg(B2 + t);
-      b[2 * t] = v.x;
-      b[2 * t + 1] = v.y;
-    }
-  }
+  for (int t = 0; t < 18; ++t) b[t] = odd ? (t < 2 ? q[16 + t] : q[t - 2]) : q[t];
 }
-template <bool VEC>
 __device__ __forceinline__ void ldg_block18(const double* hpl, int blk, double (&b)[18]) {
   const double2* B2 = reinterpret_cast<const double2*>(hpl + (size_t)blk * 18);
 #pragma unroll
@@ -578,63 +557,35 @@ struct DenseOut {
 };
 
 
-// Schur complement by camera rows (block_solver.hpp:343-433): one CTA per
-// free camera r stages the camera's BD_a blocks (contiguous in bdc) in shared
-// memory with coalesced loads. The diagonal block S(r, r) = Hpp(r) + lambda I
-// - sum_a BD_a B_a^T over all of the camera's landmarks is reduced by the
-// whole CTA (fixed assignment and tree); each off-diagonal block (r, c) is
-// summed by two lanes (lane parity = rows 0-2 or 3-5, 18 FP64 accumulators
-// each) over its co-observing pairs in landmark order, with B_b from L1/L2.
-// With bs != nullptr the reduced right-hand side bs_r = b_r - sum_a BD_a
-// b_l(a) is formed from the same staged blocks. S is written in the row-SoA
-// layout of sys_offset.
-// G = lanes per off-diagonal block: lane pairs split the block's 6 rows in two
-// halves and the G / 2 pairs of a group split its pair list (partial sums
-// combined by a fixed xor tree). rows: the camera rows of this launch (or
-// nullptr: row = blockIdx.x); the row's G is chosen from its pair-list lengths.
-// tiles != nullptr: S is written straight into the dense tiles of the tile PCG
-// (block k at tile_off[k], scalar rows 96 apart; an off-diagonal block inside
-// a diagonal tile also into its transposed place) instead of the row-SoA;
-// dn.M != nullptr: into the windows' dense matrices (DenseOut) instead.
-// block_order (or nullptr: storage order): per row, the off-diagonal block j
-// that the q-th lane group of a round takes, block_order[rptr[r] + q].
-template <typename Real, int THREADS, bool STAGE, int G = 2, bool VEC = false>
-__global__ void __launch_bounds__(THREADS, sizeof(Real) == 4 ? 2 : 1)
-    schur_rows(const int* rows, const int* hc_ptr, const int* hc_blk, const int* hc_col, const Real* hpl,
-               const Real* dinv, const Real* bdc, const int* rptr, const int* rcol, const int* pair_ptr,
-               const int2* pairs, const int* block_order, const int* s_hpp, const Real* hpp, double lambda_all, const double* lambda_of, Real* S,
-               Real* tiles, const int* tile_off, DenseOut dn, const double* b_p, const double* b_l, double* bs,
-               int bds) {
+// Where the Schur complement goes: the row-SoA layout of sys_offset (S);
+// tiles != nullptr: straight into the dense tiles of the tile PCG (block k at
+// tile_off[k], scalar rows 96 apart; an off-diagonal block inside a diagonal
+// tile also into its transposed place); dn.M != nullptr: into the windows'
+// dense matrices.
+template <typename Real>
+struct SchurOut {
+  Real* S;
+  Real* tiles;
+  const int* tile_off;
+  DenseOut dn;
+};
+
+// The camera's part of a Schur row, by the CTA that has the row: BD_a =
+// B_a Dinv_l of the camera's Hpl blocks, one thread per block, into BDw (shared
+// memory, or the camera's part of the scratch); with B_a still in registers,
+// its diagonal-block term BD_a B_a^T (upper 21 entries) and its
+// right-hand-side term BD_a b_l. The sums over the CTA (warp sums, then the
+// warps in order: a fixed order) give S(r, r) = Hpp(r) + lambda I -
+// sum_a BD_a B_a^T and, with bs != nullptr, bs_r = b_r - sum_a BD_a b_l(a).
+// Ends with a barrier that publishes BDw.
+template <typename Real, int THREADS>
+__device__ __forceinline__ void schur_camera(int r, const int* hc_ptr, const int* hc_blk, const int* hc_col,
+                                             const Real* hpl, const Real* dinv, Real* BDw, const int* rptr,
+                                             const int* s_hpp, const Real* hpp, double lambda,
+                                             const SchurOut<Real>& out, const double* b_p, const double* b_l,
+                                             double* bs, double (*red)[36]) {
   constexpr int TS = kTileBlocks * 6;  // scalar row stride of a tile
-  static_assert(G >= 2 && G <= 32 && (G & (G - 1)) == 0, "lanes per block: a power of two in [2, 32]");
-  using R2 = typename Vec2<Real>::T;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ double red[THREADS / 32][27];
-  const int r = rows ? rows[blockIdx.x] : blockIdx.x;
-  const double lambda = lambda_of ? lambda_of[r] : lambda_all;  // per camera row (batched windows)
   const int a0 = hc_ptr[r], na = hc_ptr[r + 1] - a0;
-  const int rb = rptr[r], nblk = rptr[r + 1] - rb;
-  Real* Sr = S + (size_t)rb * 36;
-  // dense output: the window's matrix, its row length and this row's first index
-  double* Md = nullptr;
-  int dn_n = 0, dn_h0 = 0;
-  if (dn.M) {
-    const int w = dn.win_of_cam[r];
-    dn_h0 = dn.cam[w];
-    dn_n = 6 * (dn.cam[w + 1] - dn_h0);
-    Md = dn.M + dn.mat[w];
-  }
-  // One pass over the camera's Hpl blocks B_a, one thread per block: BD_a =
-  // B_a Dinv_l, staged in shared memory (or, for cameras with more blocks
-  // than shared memory holds, written to the camera-major scratch bdc and read
-  // back in place); with B_a still in registers, its diagonal-block term
-  // BD_a B_a^T (upper 21 entries) and its right-hand-side term BD_a b_l.
-  // staged BD blocks: bds entries apart, rows 0-2 at 0 and rows 3-5 at bds / 2
-  // (bds = 24 in FP32: each half starts on a 16-byte boundary, read with two
-  // 16-byte loads and one 4-byte load; else 18, packed)
-  if (!STAGE) bds = 18;
-  const int bhalf = bds / 2;
-  Real* BDw = STAGE ? reinterpret_cast<Real*>(smem_raw) : const_cast<Real*>(bdc) + (size_t)a0 * 18;
   Real dacc[21];
   double racc[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
@@ -653,197 +604,399 @@ __global__ void __launch_bounds__(THREADS, sizeof(Real) == 4 ? 2 : 1)
     }
     const Real* Dl = dinv + (size_t)l * 9;
     Real b[18], D[9], bd[18];
-    ldg_block18<VEC>(hpl, a, b);
+    ldg_block18(hpl, a, b);
 #pragma unroll
     for (int q = 0; q < 9; ++q) D[q] = Dl[q];
-    Real* o = BDw + (size_t)t * bds;
+    Real* o = BDw + (size_t)t * 18;
 #pragma unroll
     for (int i = 0; i < 6; ++i)
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        bd[i * 3 + c] = b[i * 3] * D[c] + b[i * 3 + 1] * D[3 + c] + b[i * 3 + 2] * D[6 + c];
-        o[(i / 3) * bhalf + (i % 3) * 3 + c] = bd[i * 3 + c];
+        bd[hpl_at(i, c)] = b[hpl_at(i, 0)] * D[c] + b[hpl_at(i, 1)] * D[3 + c] + b[hpl_at(i, 2)] * D[6 + c];
+        o[hpl_at(i, c)] = bd[hpl_at(i, c)];
       }
     int u = 0;
 #pragma unroll
     for (int i = 0; i < 6; ++i)
 #pragma unroll
       for (int c = i; c < 6; ++c, ++u)
-        dacc[u] += bd[i * 3] * b[c * 3] + bd[i * 3 + 1] * b[c * 3 + 1] + bd[i * 3 + 2] * b[c * 3 + 2];
+        dacc[u] += bd[hpl_at(i, 0)] * b[hpl_at(c, 0)] + bd[hpl_at(i, 1)] * b[hpl_at(c, 1)] +
+                   bd[hpl_at(i, 2)] * b[hpl_at(c, 2)];
     if (bs) {
       const double* bl = b_l + (size_t)l * 3;
 #pragma unroll
       for (int q = 0; q < 6; ++q)
-        racc[q] += (double)bd[q * 3] * bl[0] + (double)bd[q * 3 + 1] * bl[1] + (double)bd[q * 3 + 2] * bl[2];
+        racc[q] += (double)bd[hpl_at(q, 0)] * bl[0] + (double)bd[hpl_at(q, 1)] * bl[1] +
+                   (double)bd[hpl_at(q, 2)] * bl[2];
     }
   }
-  if (!STAGE) __threadfence_block();
-  // fixed-order CTA sum of the 21 diagonal-block and 6 right-hand-side terms:
-  // warp sums, then term u summed over the warps in order by thread u, which
-  // writes its entry (and its mirror) of the diagonal block or of bs. The
-  // barrier also publishes the staged BD.
-  {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double acc[27];
+  __threadfence_block();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double acc[27];
 #pragma unroll
-    for (int u = 0; u < 21; ++u) acc[u] = (double)dacc[u];
+  for (int u = 0; u < 21; ++u) acc[u] = (double)dacc[u];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) acc[21 + q] = racc[q];
+  for (int q = 0; q < 6; ++q) acc[21 + q] = racc[q];
 #pragma unroll
-    for (int u = 0; u < 27; ++u) acc[u] = warp_sum(acc[u]);
-    if (lane == 0) {
+  for (int u = 0; u < 27; ++u) acc[u] = warp_sum(acc[u]);
+  if (lane == 0) {
 #pragma unroll
-      for (int u = 0; u < 27; ++u) red[warp][u] = acc[u];
+    for (int u = 0; u < 27; ++u) red[warp][u] = acc[u];
+  }
+  __syncthreads();
+  const int u = threadIdx.x;
+  if (u >= 27) return;
+  double sum = red[0][u];
+#pragma unroll
+  for (int w = 1; w < THREADS / 32; ++w) sum += red[w][u];
+  if (u >= 21) {
+    if (bs) bs[(size_t)r * 6 + (u - 21)] = b_p[(size_t)r * 6 + (u - 21)] - sum;
+    return;
+  }
+  int i = 0, c = u;  // u -> (i, c), i <= c, row by row
+  while (c >= 6 - i) {
+    c -= 6 - i;
+    ++i;
+  }
+  c += i;
+  const int rb = rptr[r], nblk = rptr[r + 1] - rb, hb = s_hpp[rb];
+  double v = -sum + (i == c ? lambda : 0.0), w = -sum;
+  if (hb >= 0) {
+    v += (double)hpp[(size_t)hb * 36 + i * 6 + c];
+    w += (double)hpp[(size_t)hb * 36 + c * 6 + i];
+  }
+  if (out.tiles) {
+    Real* Td = out.tiles + out.tile_off[rb];
+    Td[i * TS + c] = (Real)v;
+    if (c != i) Td[c * TS + i] = (Real)w;
+  } else if (out.dn.M) {
+    const int wi = out.dn.win_of_cam[r], h0 = out.dn.cam[wi], n = 6 * (out.dn.cam[wi + 1] - h0);
+    double* Dd = out.dn.M + out.dn.mat[wi] + (size_t)(r - h0) * 6 * n + (r - h0) * 6;
+    Dd[(size_t)i * n + c] = (double)(Real)v;
+    if (c != i) Dd[(size_t)c * n + i] = (double)(Real)w;
+  } else {
+    Real* Sr = out.S + (size_t)rb * 36;
+    Sr[(size_t)(i * 6 + c) * nblk] = (Real)v;
+    if (c != i) Sr[(size_t)(c * 6 + i) * nblk] = (Real)w;
+  }
+}
+
+// Schur complement by camera rows (block_solver.hpp:343-433): one CTA per
+// free camera r of `rows` (the ones with the most pairs first). schur_camera
+// stages the camera's BD_a blocks and forms the diagonal block and the reduced
+// right-hand side; each off-diagonal block S(r, c) = [Hpp(r, c)] -
+// sum BD_a B_b^T is summed by a warp over its co-observing pairs.
+// pose_blocks: some off-diagonal blocks have an Hpp part (a pose edge set).
+//
+// A warp takes four pairs per FP64 tensor-core step (m8n8k4): the product
+// sum over pairs of BD_a B_b^T is one over k = (pair, component), and the
+// components of a pair can go into different steps, so lane (g, t) holds row
+// g of pair t and step m takes component m: two loads per four pairs for each
+// operand, of runs of 96 and 48 bytes (hpl_at). Sums are FP64 for both storage
+// types, in the order of the pair list by fours: a fixed order. Rows with
+// fewer blocks than a CTA has warps cut each block's pairs over two or four
+// warps (sums in warp order).
+//
+// Bound by latency: the gathers (one Hpl block per pair, from L2 and DRAM),
+// the chain of a step, and the camera's part, during which no gather is under
+// way. On the 1000-camera graph in FP64 (3.7 M pairs, 7.5 per block) it takes
+// 0.33 ms (0.35 with vector FMAs, two lanes per block); on windows of 10 to 60
+// cameras (longer lists, few rows) 96 windows take 342 against 431 us, and one
+// launch serves every list length, where the lanes per block had to be chosen
+// by it (123 cameras: 42 us in one launch against 109 in three).
+template <typename Real, int THREADS, bool STAGE>
+__global__ void __launch_bounds__(THREADS, sizeof(Real) == 4 ? 2 : 1)
+    schur_rows(const int* rows, const int* hc_ptr, const int* hc_blk, const int* hc_col, const Real* hpl,
+               const Real* dinv, Real* bdc, const int* rptr, const int* rcol, const int* pair_ptr,
+               const int2* pairs, const int* s_hpp, const Real* hpp, double lambda_all, const double* lambda_of,
+               SchurOut<Real> out, const double* b_p, const double* b_l, double* bs, bool pose_blocks) {
+  constexpr int TS = kTileBlocks * 6;  // scalar row stride of a tile
+  constexpr int WARPS = THREADS / 32;
+  using R2 = typename Vec2<Real>::T;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[WARPS][36];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int r = rows[blockIdx.x];
+  const int rb = rptr[r], nblk = rptr[r + 1] - rb, noff = nblk - 1;
+  // the row's pair list comes into L2 while the camera's blocks are staged
+  if (noff > 0) {
+    const char* p0 = reinterpret_cast<const char*>(pairs + pair_ptr[rb + 1]);
+    const char* p1 = reinterpret_cast<const char*>(pairs + pair_ptr[rb + nblk]);
+    for (const char* p = p0 + 128 * threadIdx.x; p < p1; p += 128 * THREADS)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+  }
+  Real* const BDw = STAGE ? reinterpret_cast<Real*>(smem_raw) : bdc + (size_t)hc_ptr[r] * 18;
+  schur_camera<Real, THREADS>(r, hc_ptr, hc_blk, hc_col, hpl, dinv, BDw, rptr, s_hpp, hpp,
+                              lambda_of ? lambda_of[r] : lambda_all, out, b_p, b_l, bs, red);
+  const int g = lane >> 2, t = lane & 3;
+  const bool in = g < 6;  // the fragment's rows 6 and 7 are empty
+  auto gather = [&](int blk, bool valid, Real (&b)[3]) {
+    const Real* B = hpl + (size_t)blk * 18;
+    R2 u;
+    u.x = u.y = Real(0);
+    b[2] = Real(0);
+    if (valid && in) {
+      u = __ldg(reinterpret_cast<const R2*>(B) + g);
+      b[2] = __ldg(B + 12 + g);
+    }
+    b[0] = u.x;
+    b[1] = u.y;
+  };
+  auto product = [&](int a, const Real (&b)[3], double (&acc)[2]) {
+    double x[3] = {0.0, 0.0, 0.0};
+    if (a >= 0 && in) {
+      const Real* D = BDw + (size_t)a * 18;
+      const R2 u = *(reinterpret_cast<const R2*>(D) + g);
+      x[0] = (double)u.x;
+      x[1] = (double)u.y;
+      x[2] = (double)D[12 + g];
+    }
+#pragma unroll
+    for (int m = 2; m >= 0; --m)
+      asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                   : "+d"(acc[0]), "+d"(acc[1])
+                   : "d"(x[m]), "d"((double)b[m]));
+  };
+  // entries (g, 2 t) and (g, 2 t + 1) of block j (acc: the sum of its products)
+  auto store = [&](int j, double acc0, double acc1, int hb, int off, int cc) {
+    if (!in || t > 2) return;
+    double w0 = -acc0, w1 = -acc1;
+    if (hb >= 0) {
+      w0 += (double)hpp[(size_t)hb * 36 + g * 6 + 2 * t];
+      w1 += (double)hpp[(size_t)hb * 36 + g * 6 + 2 * t + 1];
+    }
+    if (out.tiles) {
+      R2 pr;
+      pr.x = (Real)w0;
+      pr.y = (Real)w1;
+      __stcs(reinterpret_cast<R2*>(out.tiles + off + g * TS + 2 * t), pr);
+      if (r / kTileBlocks == cc / kTileBlocks) {
+        Real* base = out.tiles + (size_t)(off / (TS * TS)) * (TS * TS);
+        Real* m = base + ((cc % kTileBlocks) * 6 + 2 * t) * TS + (r % kTileBlocks) * 6 + g;
+        __stcs(m, pr.x);
+        __stcs(m + TS, pr.y);
+      }
+    } else if (out.dn.M) {
+      // block (r, cc) transposed into the lower triangle of the window's matrix
+      const int wi = out.dn.win_of_cam[r], h0 = out.dn.cam[wi], n = 6 * (out.dn.cam[wi + 1] - h0);
+      double* D = out.dn.M + out.dn.mat[wi] + ((size_t)(cc - h0) * 6 + 2 * t) * n + (r - h0) * 6 + g;
+      D[0] = (double)(Real)w0;
+      D[n] = (double)(Real)w1;
+    } else {
+      Real* Sr = out.S + (size_t)rb * 36;
+      __stcs(Sr + (size_t)(g * 6 + 2 * t) * nblk + j, (Real)w0);
+      __stcs(Sr + (size_t)(g * 6 + 2 * t + 1) * nblk + j, (Real)w1);
+    }
+  };
+  const int split = noff * 4 <= WARPS ? 4 : noff * 2 <= WARPS ? 2 : 1;
+  if (split > 1) {
+    const int j = 1 + warp / split, sub = warp % split;
+    double acc[2] = {0.0, 0.0};
+    if (j < nblk) {
+      const int p1 = pair_ptr[rb + j + 1];
+      int p = pair_ptr[rb + j] + 4 * sub + t;
+      int2 nx = p < p1 ? __ldcs(pairs + p) : make_int2(-1, 0);
+      for (; p - t < p1; p += 4 * split) {
+        const bool valid = p < p1;
+        const int2 pr = nx;
+        if (p + 4 * split < p1) nx = __ldcs(pairs + p + 4 * split);
+        Real b[3];
+        gather(pr.y, valid, b);
+        product(valid ? pr.x : -1, b, acc);
+      }
+    }
+    __syncthreads();  // red is read above
+    if (in && t < 3) {
+      red[warp][g * 6 + 2 * t] = acc[0];
+      red[warp][g * 6 + 2 * t + 1] = acc[1];
     }
     __syncthreads();
-    const int u = threadIdx.x;
-    if (u < 27) {
-      double sum = red[0][u];
-#pragma unroll
-      for (int w = 1; w < THREADS / 32; ++w) sum += red[w][u];
-      if (u < 21) {
-        int i = 0, c = u;  // u -> (i, c), i <= c, row by row
-        while (c >= 6 - i) {
-          c -= 6 - i;
-          ++i;
-        }
-        c += i;
-        const int hb = s_hpp[rb];
-        Real* Td = tiles ? tiles + tile_off[rb] : nullptr;
-        double* Dd = Md ? Md + (size_t)(r - dn_h0) * 6 * dn_n + (r - dn_h0) * 6 : nullptr;
-        double v = -sum + (i == c ? lambda : 0.0);
-        if (hb >= 0) v += (double)hpp[(size_t)hb * 36 + i * 6 + c];
-        if (Td) Td[i * TS + c] = (Real)v;
-        else if (Dd) Dd[(size_t)i * dn_n + c] = (double)(Real)v;
-        else Sr[(size_t)(i * 6 + c) * nblk] = (Real)v;
-        if (c != i) {
-          double w = -sum;
-          if (hb >= 0) w += (double)hpp[(size_t)hb * 36 + c * 6 + i];
-          if (Td) Td[c * TS + i] = (Real)w;
-          else if (Dd) Dd[(size_t)c * dn_n + i] = (double)(Real)w;
-          else Sr[(size_t)(c * 6 + i) * nblk] = (Real)w;
-        }
-      } else if (bs) {
-        bs[(size_t)r * 6 + (u - 21)] = b_p[(size_t)r * 6 + (u - 21)] - sum;
+    if (j < nblk && sub == 0 && in && t < 3) {
+      for (int w = 1; w < split; ++w) {
+        acc[0] += red[warp + w][g * 6 + 2 * t];
+        acc[1] += red[warp + w][g * 6 + 2 * t + 1];
       }
+      const int k = rb + j;
+      store(j, acc[0], acc[1], pose_blocks ? s_hpp[k] : -1, out.tiles ? out.tile_off[k] : 0, rcol[k]);
+    }
+    return;
+  }
+  // This warp's blocks are j = 1 + warp + WARPS i; lane i % 32 loads what
+  // belongs to block i (its pairs' range, its column and place), so that a
+  // warp waits for it once in 32 blocks and not at each. A step is up to
+  // eight pairs of one block; the pair indices of step n + 3 and the blocks of
+  // step n + 2 are on their way while step n is multiplied (four stages,
+  // unrolled so that no register waiting for a load is moved).
+  struct Step {
+    int i, p, p1;  // block of the batch (>= mine: none), first pair, the block's end
+  };
+  for (int i0 = 0; 1 + warp + WARPS * i0 < nblk; i0 += 32) {
+    const int mine = min(32, (nblk - 2 - warp - WARPS * i0) / WARPS + 1);
+    const int jl = 1 + warp + WARPS * (i0 + lane);
+    int m_p0 = 0, m_p1 = 0, m_col = 0, m_off = 0, m_hb = -1;
+    if (lane < mine) {
+      m_p0 = pair_ptr[rb + jl];
+      m_p1 = pair_ptr[rb + jl + 1];
+      m_col = rcol[rb + jl];
+      if (out.tiles) m_off = out.tile_off[rb + jl];
+      if (pose_blocks) m_hb = s_hpp[rb + jl];
+    }
+    auto open = [&](int i) {
+      return Step{i, __shfl_sync(0xffffffffu, m_p0, i & 31), __shfl_sync(0xffffffffu, m_p1, i & 31)};
+    };
+    auto after = [&](const Step& st) {
+      if (st.i < mine && st.p + 8 < st.p1) return Step{st.i, st.p + 8, st.p1};
+      return open(st.i + 1);
+    };
+    auto index = [&](const Step& st, int2 (&pr)[2]) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int p = st.p + 4 * h + t;
+        pr[h] = st.i < mine && p < st.p1 ? __ldcs(pairs + p) : make_int2(-1, -1);
+      }
+    };
+    auto blocks = [&](const int2 (&pr)[2], Real (&b)[2][3]) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) gather(max(pr[h].y, 0), pr[h].y >= 0, b[h]);
+    };
+    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};  // the two halves of the steps: independent chains of products
+    int2 ix[4][2];
+    Real bv[4][2][3];
+    Step s0 = open(0);
+    index(s0, ix[0]);
+    Step s1 = after(s0);
+    index(s1, ix[1]);
+    Step s2 = after(s1);
+    index(s2, ix[2]);
+    blocks(ix[0], bv[0]);
+    blocks(ix[1], bv[1]);
+    auto stage = [&](auto cur) {
+      constexpr int C = decltype(cur)::value;
+      if (s0.i >= mine) return false;
+      const Step s3 = after(s2);
+      index(s3, ix[(C + 3) & 3]);
+      blocks(ix[(C + 2) & 3], bv[(C + 2) & 3]);
+      product(ix[C][0].x, bv[C][0], acc[0]);
+      if (s0.p + 4 < s0.p1) product(ix[C][1].x, bv[C][1], acc[1]);
+      if (s1.i != s0.i) {
+        const int hb = __shfl_sync(0xffffffffu, m_hb, s0.i), off = __shfl_sync(0xffffffffu, m_off, s0.i);
+        const int cc = __shfl_sync(0xffffffffu, m_col, s0.i);
+        store(1 + warp + WARPS * (i0 + s0.i), acc[0][0] + acc[1][0], acc[0][1] + acc[1][1], hb, off, cc);
+        acc[0][0] = acc[0][1] = acc[1][0] = acc[1][1] = 0.0;
+      }
+      s0 = s1;
+      s1 = s2;
+      s2 = s3;
+      return true;
+    };
+    while (stage(std::integral_constant<int, 0>()) && stage(std::integral_constant<int, 1>()) &&
+           stage(std::integral_constant<int, 2>()) && stage(std::integral_constant<int, 3>())) {
     }
   }
-  const Real* BDa = BDw;
-  // off-diagonal blocks (the row's diagonal is its first block); the loop
-  // runs the same number of times in every lane, so the group reduction's
-  // shuffles see full warps
-  const int half = threadIdx.x & 1, sub = (threadIdx.x % G) >> 1;
-  for (int j0 = 1; j0 < nblk; j0 += THREADS / G) {
-    const int q = j0 + (int)threadIdx.x / G;
-    const bool valid = q < nblk;
-    const int j = (valid && block_order) ? block_order[rb + q] : q;
+}
+
+// FP32 rows with short pair lists: the off-diagonal blocks by two lanes each
+// (lane parity = rows 0-2 or 3-5, 18 FP32 accumulators each) over their pairs
+// in landmark order, two gathers in flight per lane. FP32 FMAs need no
+// conversion to FP64 fragments: 228 us per pass of the 1000-camera graph (7.5
+// pairs per block) against 245 for schur_rows; lists of 12 and more pairs
+// leave too few lanes busy here.
+template <int THREADS, bool STAGE>
+__global__ void __launch_bounds__(THREADS, 2)
+    schur_rows_short(const int* rows, const int* hc_ptr, const int* hc_blk, const int* hc_col, const float* hpl,
+                     const float* dinv, float* bdc, const int* rptr, const int* rcol, const int* pair_ptr,
+                     const int2* pairs, const int* s_hpp, const float* hpp, double lambda_all,
+                     const double* lambda_of, SchurOut<float> out, const double* b_p, const double* b_l, double* bs,
+                     bool pose_blocks) {
+  constexpr int TS = kTileBlocks * 6;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[THREADS / 32][36];
+  const int r = rows[blockIdx.x];
+  const int rb = rptr[r], nblk = rptr[r + 1] - rb;
+  float* const BDw = STAGE ? reinterpret_cast<float*>(smem_raw) : bdc + (size_t)hc_ptr[r] * 18;
+  schur_camera<float, THREADS>(r, hc_ptr, hc_blk, hc_col, hpl, dinv, BDw, rptr, s_hpp, hpp,
+                               lambda_of ? lambda_of[r] : lambda_all, out, b_p, b_l, bs, red);
+  const int half = threadIdx.x & 1;
+  for (int j = 1 + (int)threadIdx.x / 2; j < nblk; j += THREADS / 2) {
     const int k = rb + j;
-    // pair products summed in the storage type (FP64 on the FP64 path; FP32
-    // on the mixed path, whose S is stored in FP32), added to Hpp in FP64
-    Real acc[18];
+    float acc[18];
 #pragma unroll
-    for (int t = 0; t < 18; ++t) acc[t] = 0;
-    // two pairs per step: their index and Hpl loads are independent, so two
-    // gathers are in flight per thread; accumulation stays in pair order.
-    // The pair list and S are touched once per pass: streamed (evict-first
-    // loads and stores), so the L2 lines go to the Hpl blocks gathered again
-    auto load_b = [&](int blk, Real (&b)[18]) { ldg_block18<VEC>(hpl, blk, b); };
-    auto accum = [&](int a, const Real (&b)[18]) {
-      const Real* D = BDa + (size_t)a * bds + half * bhalf;
-      Real d[9];
-      if (sizeof(Real) == 4 && bds == 24) {
-        const float4 d0 = *reinterpret_cast<const float4*>(D);
-        const float4 d1 = *reinterpret_cast<const float4*>(D + 4);
-        d[0] = d0.x; d[1] = d0.y; d[2] = d0.z; d[3] = d0.w;
-        d[4] = d1.x; d[5] = d1.y; d[6] = d1.z; d[7] = d1.w;
-        d[8] = D[8];
-      } else {
+    for (int t = 0; t < 18; ++t) acc[t] = 0.f;
+    // two pairs per step: their index and Hpl loads are independent;
+    // accumulation stays in pair order. The pair list and S are touched once
+    // per pass: streamed, so the L2 lines go to the Hpl blocks gathered again
+    auto accum = [&](int a, const float (&b)[18]) {
+      const float* D = BDw + (size_t)a * 18;
 #pragma unroll
-        for (int t = 0; t < 9; ++t) d[t] = D[t];
-      }
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
+      for (int i = 0; i < 3; ++i) {
+        const int q = half * 3 + i;
+        const float d0 = D[2 * q], d1 = D[2 * q + 1], d2 = D[12 + q];
 #pragma unroll
         for (int c = 0; c < 6; ++c)
-          acc[i * 6 + c] += d[i * 3] * b[c * 3] + d[i * 3 + 1] * b[c * 3 + 1] + d[i * 3 + 2] * b[c * 3 + 2];
+          acc[i * 6 + c] += d0 * b[hpl_at(c, 0)] + d1 * b[hpl_at(c, 1)] + d2 * b[hpl_at(c, 2)];
+      }
     };
-    constexpr int STEP = G / 2;  // this lane's pairs: p0 + sub, p0 + sub + STEP, ...
-    int p = valid ? pair_ptr[k] + sub : 0;
-    const int p1 = valid ? pair_ptr[k + 1] : 0;
+    int p = pair_ptr[k];
+    const int p1 = pair_ptr[k + 1];
     // the next step's pair indices are loaded while this step's blocks are
     int2 na2 = make_int2(0, 0), nb2 = make_int2(0, 0);
     if (p < p1) na2 = __ldcs(pairs + p);
-    if (p + STEP < p1) nb2 = __ldcs(pairs + p + STEP);
-    for (; p + STEP < p1; p += 2 * STEP) {
+    if (p + 1 < p1) nb2 = __ldcs(pairs + p + 1);
+    for (; p + 1 < p1; p += 2) {
       const int2 pa = na2, pb = nb2;
-      if (p + 2 * STEP < p1) na2 = __ldcs(pairs + p + 2 * STEP);
-      if (p + 3 * STEP < p1) nb2 = __ldcs(pairs + p + 3 * STEP);
-      Real ba[18], bb[18];
-      load_b(pa.y, ba);
-      load_b(pb.y, bb);
+      if (p + 2 < p1) na2 = __ldcs(pairs + p + 2);
+      if (p + 3 < p1) nb2 = __ldcs(pairs + p + 3);
+      float ba[18], bb[18];
+      ldg_block18(hpl, pa.y, ba);
+      ldg_block18(hpl, pb.y, bb);
       accum(pa.x, ba);
       accum(pb.x, bb);
     }
     if (p < p1) {
-      const int2 pa = na2;
-      Real ba[18];
-      load_b(pa.y, ba);
-      accum(pa.x, ba);
+      float ba[18];
+      ldg_block18(hpl, na2.y, ba);
+      accum(na2.x, ba);
     }
+    const int hb = pose_blocks ? s_hpp[k] : -1, cc = rcol[k];
+    float v[18];
 #pragma unroll
-    for (int off = 2; off < G; off <<= 1)
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-      for (int t = 0; t < 18; ++t) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], off);
-    if (valid && sub == 0) {
-      const int hb = s_hpp[k];
-      Real v[18];
+      for (int c = 0; c < 6; ++c) {
+        double w = -(double)acc[i * 6 + c];
+        if (hb >= 0) w += (double)hpp[(size_t)hb * 36 + (half * 3 + i) * 6 + c];
+        v[i * 6 + c] = (float)w;
+      }
+    if (out.tiles) {
+      // this lane's three scalar rows of the block, in pairs (8-byte aligned)
+      const int off = out.tile_off[k];
+      float* T = out.tiles + off + half * 3 * TS;
 #pragma unroll
       for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int c = 0; c < 6; ++c) {
-          const int e = (half * 3 + i) * 6 + c;
-          double w = -(double)acc[i * 6 + c];
-          if (hb >= 0) w += (double)hpp[(size_t)hb * 36 + e];
-          v[i * 6 + c] = (Real)w;
-        }
-      if (tiles) {
-        // this lane's three scalar rows of the block: six contiguous entries each
-        const int off = tile_off[k];
-        Real* T = tiles + off + half * 3 * TS;
-        // (six entries of a row start on an 8-byte boundary in FP32: pairs)
+        for (int c = 0; c < 6; c += 2)
+          __stcs(reinterpret_cast<float2*>(T + i * TS + c), make_float2(v[i * 6 + c], v[i * 6 + c + 1]));
+      if (r / kTileBlocks == cc / kTileBlocks) {
+        float* base = out.tiles + (size_t)(off / (TS * TS)) * (TS * TS);
+        const int lr = (r % kTileBlocks) * 6 + half * 3, lc = (cc % kTileBlocks) * 6;
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
-          for (int c = 0; c < 6; c += 2) {
-            R2 pr;
-            pr.x = v[i * 6 + c];
-            pr.y = v[i * 6 + c + 1];
-            __stcs(reinterpret_cast<R2*>(T + i * TS + c), pr);
-          }
-        const int cc = rcol[k];
-        if (r / kTileBlocks == cc / kTileBlocks) {
-          Real* base = tiles + (size_t)(off / (TS * TS)) * (TS * TS);
-          const int lr = (r % kTileBlocks) * 6 + half * 3, lc = (cc % kTileBlocks) * 6;
-#pragma unroll
-          for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int c = 0; c < 6; ++c) __stcs(base + (lc + c) * TS + lr + i, v[i * 6 + c]);
-        }
-      } else if (Md) {
-        // block (r, cc) transposed into the lower triangle: entry (3h + i, c)
-        // at row (cc - h0) * 6 + c, column (r - h0) * 6 + 3h + i
-        const int cc = rcol[k];
-        double* D = Md + (size_t)(cc - dn_h0) * 6 * dn_n + (r - dn_h0) * 6 + half * 3;
-#pragma unroll
-        for (int c = 0; c < 6; ++c)
-#pragma unroll
-          for (int i = 0; i < 3; ++i) D[(size_t)c * dn_n + i] = (double)v[i * 6 + c];
-      } else {
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int c = 0; c < 6; ++c) __stcs(Sr + (size_t)((half * 3 + i) * 6 + c) * nblk + j, v[i * 6 + c]);
+          for (int c = 0; c < 6; ++c) __stcs(base + (lc + c) * TS + lr + i, v[i * 6 + c]);
       }
+    } else if (out.dn.M) {
+      const int wi = out.dn.win_of_cam[r], h0 = out.dn.cam[wi], n = 6 * (out.dn.cam[wi + 1] - h0);
+      double* D = out.dn.M + out.dn.mat[wi] + (size_t)(cc - h0) * 6 * n + (r - h0) * 6 + half * 3;
+#pragma unroll
+      for (int c = 0; c < 6; ++c)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) D[(size_t)c * n + i] = (double)v[i * 6 + c];
+    } else {
+      float* Sr = out.S + (size_t)rb * 36;
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) __stcs(Sr + (size_t)((half * 3 + i) * 6 + c) * nblk + j, v[i * 6 + c]);
     }
   }
 }
@@ -871,11 +1024,11 @@ __global__ void __launch_bounds__(THREADS) schur_rhs(const int* hc_ptr, const in
   double acc[6] = {0, 0, 0, 0, 0, 0};
   const int e1 = hc_ptr[h + 1];
   for (int p = hc_ptr[h] + threadIdx.x; p < e1; p += THREADS) {
-    const int a = hc_blk[p];
     const double* d = db + (size_t)hc_col[p] * 3;
-    const Real* B = hpl + (size_t)a * 18;
+    const Real* B = hpl + (size_t)hc_blk[p] * 18;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) acc[q] += (double)B[q * 3] * d[0] + (double)B[q * 3 + 1] * d[1] + (double)B[q * 3 + 2] * d[2];
+    for (int q = 0; q < 6; ++q)
+      acc[q] += (double)B[hpl_at(q, 0)] * d[0] + (double)B[hpl_at(q, 1)] * d[1] + (double)B[hpl_at(q, 2)] * d[2];
   }
   __shared__ double red[THREADS / 32][6];
   block_sum_array<double, 6, THREADS>(acc, &red[0][0]);
@@ -901,7 +1054,7 @@ __global__ void ba_backsub(const int* hb_ptr, const int* hpl_row, int Pf, const 
     for (int c = 0; c < 3; ++c) {
       double s = 0.0;
 #pragma unroll
-      for (int r = 0; r < 6; ++r) s += (double)B[r * 3 + c] * xp[r];
+      for (int r = 0; r < 6; ++r) s += (double)B[hpl_at(r, c)] * xp[r];
       cl[c] -= s;
     }
   }
@@ -936,7 +1089,7 @@ __global__ void ba_backsub_warp(const int* e_hpl, const int* hpl_row, const int*
       for (int c = 0; c < 3; ++c) {
         double t = 0.0;
 #pragma unroll
-        for (int r = 0; r < 6; ++r) t += (double)B[r * 3 + c] * xp[r];
+        for (int r = 0; r < 6; ++r) t += (double)B[hpl_at(r, c)] * xp[r];
         acc[c] = t;
       }
     }

@@ -183,7 +183,7 @@ struct g2oc_ctx {
   g2oc::DBuf<double4> e_om, c_om;
   g2oc::DBuf<double4> e_z3, e_oa3, c_z3, c_oa3;  // stereo edges (stereo_kernels.cuh)
   g2oc::DBuf<double2> e_ob3, c_ob3;
-  g2oc::DBuf<int> e_hpl, e_lm, lm_chunk_ptr, l_ptr, c_ptr, hb_ptr, hpl_row, hpl_col, hc_ptr, hc_blk, hc_col, hc_index, s_pair_ptr, s_hpp;
+  g2oc::DBuf<int> e_hpl, e_lm, lm_chunk_ptr, l_ptr, c_ptr, hb_ptr, hpl_row, hpl_col, hc_ptr, hc_blk, hc_col, s_pair_ptr, s_hpp;
   g2oc::DBuf<int2> s_pairs;
   // pose-graph edges
   g2oc::DBuf<int2> pe_v;
@@ -506,39 +506,6 @@ static int pcg_mode() {
 }
 static bool kernels_pcg() { return pcg_mode() == PCG_KERNELS; }
 
-// order of the Schur rows in their launches: 0 by pair work (longest
-// first), 1 by camera index
-static int schur_row_order() {
-  static const int v = [] {
-    const char* e = getenv("G2OC_SCHUR_ROW_ORDER");
-    return e ? atoi(e) : 0;
-  }();
-  return v;
-}
-
-// entries between the staged BD blocks of a Schur row: 18 (packed, the
-// default) or 24 (G2OC_SCHUR_BD_STRIDE=24: 16-byte aligned halves; measured
-// slower, 417 vs 238 us per launch on the BA configuration, from 4-way bank
-// conflicts of the staging stores)
-static int schur_bd_stride() {
-  static const int v = [] {
-    const char* e = getenv("G2OC_SCHUR_BD_STRIDE");
-    return e ? atoi(e) : 18;
-  }();
-  return v;
-}
-
-// FP32 Schur rows: gather each Hpl block with five aligned vector loads
-// instead of nine 8-byte loads (the default: 229 vs 243 us per launch on the
-// BA configuration; G2OC_SCHUR_VEC=0 for the 8-byte loads)
-static bool schur_vec_loads() {
-  static const int v = [] {
-    const char* e = getenv("G2OC_SCHUR_VEC");
-    return e ? atoi(e) : 1;
-  }();
-  return v != 0;
-}
-
 // tensor-core Cholesky substitutions: one cooperative launch per direction
 // (the default) or two launches per tile step (G2OC_TC_SOLVE=launches)
 static bool tc_solve_coop_on() {
@@ -547,19 +514,6 @@ static bool tc_solve_coop_on() {
     return e && strcmp(e, "launches") == 0 ? 0 : 1;
   }();
   return v != 0;
-}
-
-// order of a Schur row's off-diagonal blocks over its lane groups: 0
-// storage order (the default), 1 by pair count dealt in alternating rounds
-// (measured slower: 249 vs 229 us per launch on the BA configuration, the
-// scattered block order costing more in the stores than it saves in lane
-// balance)
-static int schur_block_order() {
-  static const int v = [] {
-    const char* e = getenv("G2OC_SCHUR_BLOCK_ORDER");
-    return e ? atoi(e) : 0;
-  }();
-  return v;
 }
 
 // LinearSolverPCG::_maxIter (the system dimension when unset); an FP32-stored
@@ -743,16 +697,13 @@ struct Engine final : EngineBase {
   DBuf<Real> hpp, hll, hpl, bdc, dinv, Sval, sysval;
   DBuf<double> minv, r, s, d0, d1, q, qrow, tbuf, cpart, tpart;
   DBuf<Real> tiles;  // dense-tile copy of the system (nearly full 6x6-block matrices), allocated on first use
-  // Schur rows by lanes per off-diagonal block (2 / 8 / 16), from the row's
-  // mean pair-list length (<= 12, <= 40, longer): a structural choice, so a
-  // row gets the same arithmetic whatever else is in the graph
-  DBuf<int> row_list[3];
-  DBuf<int> block_order;  // per row: its off-diagonal blocks in processing order (empty: j order)
-  int row_n[3] = {0, 0, 0};
+  // camera rows of the Schur launches, the ones with the most pairs first:
+  // schur_rows, and in FP32 the rows with short pair lists (schur_rows_short)
+  DBuf<int> row_list[2];
+  int row_n[2] = {0, 0};
   bool tiles_fresh = false;  // tiles hold the matrix of the current solve
   bool tiles_from_schur = false;  // the last Schur pass wrote the tiles, not the row-SoA values
   bool stage_in_smem = true;  // schur_rows: camera blocks staged in shared memory
-  int bd_stride = 18;         // schur_rows: entries between staged BD blocks
   size_t schur_smem = 0;
   DBuf<Real> hcontrib;
   DBuf<double> bcontrib;
@@ -771,67 +722,30 @@ struct Engine final : EngineBase {
       G2OC_TRY(dinv.alloc((size_t)S.Pf * 9 + 1));
       G2OC_TRY(Sval.alloc((size_t)S.schur_rc.size() / 2 * 36 + 1));
       {
-        // Schur rows by mean pair count, longest first (no Schur complement
-        // when every landmark is fixed: the lists stay empty)
-        std::vector<int> lists[3];
+        // rows with the most pair products first: the long rows start in the
+        // first wave of CTAs (a row's result does not depend on when it runs)
         std::vector<double> work(S.Cf);
+        std::vector<int> lists[2];
         for (int r = 0; r < (S.schur ? S.Cf : 0); ++r) {
           const int k0 = S.sys_rptr[r], k1 = S.sys_rptr[r + 1];
           const double pairs = (double)(S.s_pair_ptr[k1] - S.s_pair_ptr[k0]);
-          const double mean = k1 - k0 > 1 ? pairs / (k1 - k0 - 1) : 0.0;
-          lists[mean <= 12.0 ? 0 : mean <= 40.0 ? 1 : 2].push_back(r);
           work[r] = pairs + 2.0 * (S.hc_ptr[r + 1] - S.hc_ptr[r]);
+          // by the row alone, so a row gets the same arithmetic whatever else
+          // is in the graph: FP32 lists of 12 pairs on average, and enough
+          // blocks for two lanes each to fill a CTA
+          const bool brief = sizeof(Real) == 4 && k1 - k0 > 96 && pairs <= 12.0 * (k1 - k0 - 1);
+          lists[brief].push_back(r);
         }
-        // rows with the most pair products first: the long rows start in
-        // the first wave of CTAs (a row's result does not depend on when it
-        // runs); G2OC_SCHUR_ROW_ORDER=1 keeps camera order instead, so the
-        // rows in flight together are neighbours whose co-observed landmarks
-        // (and so the gathered Hpl blocks) largely coincide
-        const bool by_work = schur_row_order() == 0;
-        for (int gi = 0; gi < 3; ++gi) {
-          if (by_work)
-            std::stable_sort(lists[gi].begin(), lists[gi].end(), [&](int a, int b) { return work[a] > work[b]; });
-          row_n[gi] = (int)lists[gi].size();
-          G2OC_TRY(row_list[gi].upload(lists[gi].empty() ? std::vector<int>{0} : lists[gi], c->stream));
-        }
-        // the order in which a row's off-diagonal blocks go to its lane
-        // groups: by pair count, most first, dealt in rounds of one block per
-        // group with the direction reversed every round, so the blocks a warp
-        // runs side by side have nearly equal pair counts (a warp takes as
-        // long as its longest block) and the groups' totals even out
-        if (schur_block_order() != 0 && S.schur) {
-          std::vector<int> ord(S.schur_rc.size() / 2 + 1, 0);
-          std::vector<int> js;
-          for (int gi = 0; gi < 3; ++gi) {
-            const int groups = (sizeof(Real) == 4 ? 384 : 512) / (gi == 0 ? 2 : gi == 1 ? 8 : 16);
-            for (int r : lists[gi]) {
-              const int rb = S.sys_rptr[r], nb = S.sys_rptr[r + 1] - rb;
-              js.resize(std::max(nb - 1, 0));
-              for (int j = 1; j < nb; ++j) js[j - 1] = j;
-              std::stable_sort(js.begin(), js.end(), [&](int a, int b) {
-                return S.s_pair_ptr[rb + a + 1] - S.s_pair_ptr[rb + a] > S.s_pair_ptr[rb + b + 1] - S.s_pair_ptr[rb + b];
-              });
-              for (int q0 = 0; q0 < nb - 1; q0 += groups) {
-                const int q1 = std::min(nb - 1, q0 + groups);
-                if ((q0 / groups) & 1) std::reverse(js.begin() + q0, js.begin() + q1);
-              }
-              for (int q = 0; q < nb - 1; ++q) ord[rb + 1 + q] = js[q];
-            }
-          }
-          G2OC_TRY(block_order.upload(ord, c->stream));
-        } else {
-          block_order.release();
+        for (int q = 0; q < 2; ++q) {
+          std::stable_sort(lists[q].begin(), lists[q].end(), [&](int a, int b) { return work[a] > work[b]; });
+          row_n[q] = (int)lists[q].size();
+          G2OC_TRY(row_list[q].upload(lists[q].empty() ? std::vector<int>{0} : lists[q], c->stream));
         }
       }
-      // FP32: BD blocks 24 floats apart when two CTAs of the row kernel still
-      // fit on an SM (their halves then start on 16-byte boundaries): 228 KB
-      // of shared memory per SM, 1 KB reserved and ~3 KB static per CTA
-      bd_stride = schur_bd_stride() == 24 && sizeof(Real) == 4 &&
-                          (size_t)S.max_blocks_per_cam * 24 * 4 <= 110 * 1024 ? 24 : 18;
-      schur_smem = (size_t)S.max_blocks_per_cam * bd_stride * sizeof(Real);
+      schur_smem = (size_t)S.max_blocks_per_cam * 18 * sizeof(Real);
       stage_in_smem = schur_smem <= 190 * 1024;
       if (!stage_in_smem) schur_smem = 0;
-      if (!stage_in_smem) G2OC_TRY(bdc.alloc((size_t)S.hpl_rc.size() / 2 * 18 + 1));
+      if (!stage_in_smem) G2OC_TRY(bdc.alloc(S.hpl_rc.size() / 2 * 18 + 1));
       G2OC_TRY(c->db.alloc((size_t)S.Pf * 3 + 1));
       if (c->pose_edges()) {
         const size_t npa = S.pact.size();
@@ -1038,7 +952,7 @@ struct Engine final : EngineBase {
     if (to_tiles) tiles_fresh = true;
     if (S.Pf > 0) {
       G2OC_K(K_SCHUR_LANDMARK) schur_landmark<Real><<<cdiv(S.Pf, 128), 128, 0, st>>>(
-          hll.p, hpl.p, c->hb_ptr.p, c->hc_index.p, S.Pf, lambda, lam_l, dinv.p, nullptr, c->flag.p);
+          hll.p, S.Pf, lambda, lam_l, dinv.p, c->flag.p);
       G2OC_LAUNCH_CHECK();
     }
     if (S.Cf == 0) return G2OC_OK;
@@ -1047,14 +961,7 @@ struct Engine final : EngineBase {
     // sharded: the camera diagonal's lambda is added by rank 0 only (the
     // ranks' rows are summed); the landmarks' above is every rank's own
     lambda = (c->shard_world > 1 && c->shard_rank != 0) ? 0.0 : lambda;
-    for (int gi = 0; gi < 3; ++gi) {
-      if (row_n[gi] == 0) continue;
-      const int* rows = row_list[gi].p;
-      if (gi == 0) G2OC_TRY(launch_schur_rows<2>(rows, row_n[gi], lambda, lam_c, bp, bl, bs, to_tiles, to_windows));
-      else if (gi == 1) G2OC_TRY(launch_schur_rows<8>(rows, row_n[gi], lambda, lam_c, bp, bl, bs, to_tiles, to_windows));
-      else G2OC_TRY(launch_schur_rows<16>(rows, row_n[gi], lambda, lam_c, bp, bl, bs, to_tiles, to_windows));
-    }
-    return G2OC_OK;
+    return launch_schur_rows(lambda, lam_c, bp, bl, bs, to_tiles, to_windows);
   }
 
   // the PCG of a 6x6-block system runs on dense tiles (nearly full pattern,
@@ -1075,31 +982,27 @@ struct Engine final : EngineBase {
     return G2OC_OK;
   }
 
-  // schur_rows over a list of camera rows with G lanes per off-diagonal block
-  // (FP32 storage: 384 threads, two CTAs per SM; FP64: 512 threads, one)
-  template <int G>
-  int launch_schur_rows(const int* rows, int nrows, double lambda, const double* lam_c, const double* bp,
-                        const double* bl, double* bs, bool to_tiles, bool to_windows) {
+  // all camera rows (FP32 storage: 384 threads, two CTAs per SM; FP64: 512
+  // threads, one)
+  int launch_schur_rows(double lambda, const double* lam_c, const double* bp, const double* bl, double* bs,
+                        bool to_tiles, bool to_windows) {
     constexpr int T = sizeof(Real) == 4 ? 384 : 512;
     cudaStream_t st = c->stream;
-    Real* tl = to_tiles ? tiles.p : nullptr;
-    const int* toff = to_tiles ? c->tile_off.p : nullptr;
-    DenseOut dn{c->win_of_cam.p, c->win_cam.p, c->win_mat.p, to_windows ? c->win_scratch.p : nullptr};
-    if (stage_in_smem) {
-      auto kern = schur_vec_loads() ? schur_rows<Real, T, true, G, true> : schur_rows<Real, T, true, G, false>;
+    const SchurOut<Real> out{
+        Sval.p, to_tiles ? tiles.p : nullptr, to_tiles ? c->tile_off.p : nullptr,
+        DenseOut{c->win_of_cam.p, c->win_cam.p, c->win_mat.p, to_windows ? c->win_scratch.p : nullptr}};
+    auto launch = [&](auto kern, int q) -> int {
+      if (row_n[q] == 0) return G2OC_OK;
       G2OC_TRY(raise_dyn_smem((const void*)kern, schur_smem));
-      G2OC_K(K_SCHUR_BLOCKS) kern<<<nrows, T, schur_smem, st>>>(
-          rows, c->hc_ptr.p, c->hc_blk.p, c->hc_col.p, hpl.p, dinv.p, bdc.p, c->sys_rptr.p, c->sys_rcol.p,
-          c->s_pair_ptr.p, c->s_pairs.p, block_order.p, c->s_hpp.p, hpp.p, lambda, lam_c, Sval.p, tl, toff, dn, bp,
-          bl, bs, bd_stride);
-    } else {
-      G2OC_K(K_SCHUR_BLOCKS) schur_rows<Real, T, false, G><<<nrows, T, 0, st>>>(
-          rows, c->hc_ptr.p, c->hc_blk.p, c->hc_col.p, hpl.p, dinv.p, bdc.p, c->sys_rptr.p, c->sys_rcol.p,
-          c->s_pair_ptr.p, c->s_pairs.p, block_order.p, c->s_hpp.p, hpp.p, lambda, lam_c, Sval.p, tl, toff, dn, bp,
-          bl, bs, bd_stride);
-    }
-    G2OC_LAUNCH_CHECK();
-    return G2OC_OK;
+      G2OC_K(K_SCHUR_BLOCKS) kern<<<row_n[q], T, schur_smem, st>>>(
+          row_list[q].p, c->hc_ptr.p, c->hc_blk.p, c->hc_col.p, hpl.p, dinv.p, bdc.p, c->sys_rptr.p, c->sys_rcol.p,
+          c->s_pair_ptr.p, c->s_pairs.p, c->s_hpp.p, hpp.p, lambda, lam_c, out, bp, bl, bs, c->S.npp > 0);
+      G2OC_LAUNCH_CHECK();
+      return G2OC_OK;
+    };
+    if constexpr (sizeof(Real) == 4)
+      G2OC_TRY(launch(stage_in_smem ? schur_rows_short<T, true> : schur_rows_short<T, false>, 1));
+    return launch(stage_in_smem ? schur_rows<Real, T, true> : schur_rows<Real, T, false>, 0);
   }
 
   int schur_rhs_from(const double* rp, const double* rl, double* bs) {
@@ -1295,7 +1198,7 @@ struct Engine final : EngineBase {
       if (S.ba && S.Pf > 0) {
         if (S.schur) {
           G2OC_K(K_SCHUR_LANDMARK) schur_landmark<Real><<<cdiv(S.Pf, 128), 128, 0, st>>>(
-              hll.p, hpl.p, c->hb_ptr.p, c->hc_index.p, S.Pf, lambda, nullptr, dinv.p, nullptr, c->flag.p);
+              hll.p, S.Pf, lambda, nullptr, dinv.p, c->flag.p);
           G2OC_LAUNCH_CHECK();
           G2OC_TRY(backsub(c->b.p, c->xs.p, c->x.p));
         }
@@ -1539,7 +1442,9 @@ struct Engine final : EngineBase {
     if (S.ba && hpl_out && !S.hpl_rc.empty()) {
       std::vector<Real> h(S.hpl_rc.size() / 2 * 18);
       G2OC_CUDA_TRY(cudaMemcpy(h.data(), hpl.p, h.size() * sizeof(Real), cudaMemcpyDeviceToHost));
-      to_double(h, hpl_out);
+      for (size_t a = 0; a < h.size(); a += 18)
+        for (int r = 0; r < 6; ++r)
+          for (int cc = 0; cc < 3; ++cc) hpl_out[a + r * 3 + cc] = (double)h[a + hpl_at(r, cc)];
     }
     return G2OC_OK;
   }
@@ -2769,12 +2674,8 @@ static int upload_topology(g2oc_ctx* c, const g2oc_graph* g) {
     G2OC_TRY(c->hpl_col.upload(hcl, st));
     G2OC_TRY(c->hc_ptr.upload(S.hc_ptr, st));
     G2OC_TRY(c->hc_blk.upload(S.hc_blk, st));
-    std::vector<int> hcidx(S.hc_blk.size()), hccol(S.hc_blk.size());
-    for (size_t p = 0; p < S.hc_blk.size(); ++p) {
-      hcidx[S.hc_blk[p]] = (int)p;
-      hccol[p] = S.hpl_rc[2 * (size_t)S.hc_blk[p] + 1];
-    }
-    G2OC_TRY(c->hc_index.upload(hcidx, st));
+    std::vector<int> hccol(S.hc_blk.size());
+    for (size_t p = 0; p < S.hc_blk.size(); ++p) hccol[p] = S.hpl_rc[2 * (size_t)S.hc_blk[p] + 1];
     G2OC_TRY(c->hc_col.upload(hccol, st));
     G2OC_TRY(c->s_pair_ptr.upload(S.s_pair_ptr, st));
     std::vector<int2> ab(S.s_pairs.size() / 2);

@@ -203,7 +203,7 @@ __global__ void st_landmark_pass(BAEdges E, BAVertices V, const int* l_ptr, int 
       for (int r = 0; r < 6; ++r)
 #pragma unroll
         for (int c = 0; c < 3; ++c)
-          B[r * 3 + c] += L.Jc[r] * L.A[c] + L.Jc[6 + r] * L.A[3 + c] + L.Jc[12 + r] * L.A[6 + c];
+          B[hpl_at(r, c)] += L.Jc[r] * L.A[c] + L.Jc[6 + r] * L.A[3 + c] + L.Jc[12 + r] * L.A[6 + c];
     }
   }
   if (cur >= 0) {
