@@ -20,6 +20,7 @@
 #include "chol_plan.h"
 #include "g2oc_internal.h"
 #include "pcg_kernels.cuh"
+#include "reduce.cuh"
 #include "tile_potrf.cuh"
 
 namespace g2oc {
@@ -43,12 +44,12 @@ struct CholState {
   CholTickets factor, forward, backward;
   int info;  // a pivot was not positive
   int err;   // a wait ran out
-  double floor;  // smallest accepted pivot of the current factorization
+  unsigned long long max_diag;  // bits of the largest |diagonal entry| (chol_floor), back to 0 after a factorization
 };
 
 // device side of the plan
 struct CholDev {
-  int nt, ns;
+  int nt, ns, ntask;  // tile columns, slots, tasks of the factorization
   const int *col_ptr, *row, *col, *width, *orig;
   const int* asm_ptr;
   const int4* asm_ent;  // offset (low, high) and stride of the block's entries, packed place
@@ -59,6 +60,7 @@ struct CholDev {
   double *y, *x;   // nt * kTile: forward and backward substituted vectors
   unsigned *flag, *yflag, *xflag;
   CholState* st;
+  double floor;    // smallest accepted pivot over the largest diagonal entry: 4 n eps
 };
 
 // int arrays of a plan, laid end to end (16-byte aligned) so that a plan is
@@ -121,16 +123,17 @@ static int chol_plan_build(CholPlan& P, int nb, int bs, const std::vector<int>& 
   G2OC_TRY(P.vals.alloc((ns + nt) * kTileElems + 2 * nt * kTile));
   G2OC_TRY(P.flags.alloc(ns + 2 * nt));
   G2OC_TRY(P.state.alloc(1));
+  G2OC_CUDA_TRY(cudaMemsetAsync(P.vals.p, 0, P.vals.bytes(), st));  // the parts without unknowns stay zero
   G2OC_CUDA_TRY(cudaMemsetAsync(P.flags.p, 0, P.flags.bytes(), st));
   G2OC_CUDA_TRY(cudaMemsetAsync(P.state.p, 0, P.state.bytes(), st));
   const int* q = P.ints.p;
   double* L = P.vals.p;
   double* W = L + ns * kTileElems;
   double* y = W + nt * kTileElems;
-  P.d = CholDev{S.nt, (int)ns, q + o[0], q + o[1], q + o[2], q + o[3], q + o[4], q + o[5],
+  P.d = CholDev{S.nt, (int)ns, (int)S.task.size(), q + o[0], q + o[1], q + o[2], q + o[3], q + o[4], q + o[5],
                 reinterpret_cast<const int4*>(q + o[6]), q + o[7], reinterpret_cast<const int2*>(q + o[8]), q + o[9],
                 q + o[10], q + o[11], q + o[12], L, W, y, y + nt * kTile, P.flags.p, P.flags.p + ns,
-                P.flags.p + ns + nt, P.state.p};
+                P.flags.p + ns + nt, P.state.p, 4.0 * (double)S.n * 2.220446049250313e-16};
   P.pos = q + o[13];
   int dev = 0;
   G2OC_CUDA_TRY(cudaGetDevice(&dev));
@@ -176,93 +179,215 @@ __device__ __forceinline__ int chol_ticket(CholTickets* t, int* sh) {
   __syncthreads();
   return *sh;
 }
-__device__ __forceinline__ void chol_leave(CholTickets* t) {
+// the last CTA to leave also runs `end`
+template <typename F>
+__device__ __forceinline__ void chol_leave(CholTickets* t, F&& end) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     if (atomicInc(&t->left, gridDim.x - 1) == gridDim.x - 1) {  // the last one; left is back at 0
       t->next = 0;
       t->epoch += 1;
+      end();
       __threadfence();
     }
   }
 }
 
-// The pivot floor of a factorization: 4 n eps times the largest diagonal
-// entry of the matrix, and the info flag cleared. One CTA of 1024 threads
-// (fixed tree).
-template <typename Real>
-__global__ void __launch_bounds__(1024) chol_begin(SysDev<Real> S, int bs, CholState* st) {
+// The largest |diagonal entry| of the matrix (the pivot floor is a multiple
+// of it) and the outcome of the last factorization cleared: one thread per
+// diagonal entry, a maximum has no order. m: this thread's entry
+__device__ __forceinline__ void chol_floor_max(double m, CholState* st) {
   __shared__ double red[32];
-  const int n = S.nb * bs;
-  double m = 0.0;
-  for (int t = threadIdx.x; t < n; t += blockDim.x) {
-    const int i = t / bs, a = t % bs;
-    const int rb = S.rptr[i], nblk = S.rptr[i + 1] - rb;
-    m = fmax(m, fabs((double)S.val[(size_t)rb * bs * bs + (size_t)a * (bs + 1) * nblk + (S.diag[i] - rb)]));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double r = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r = fmax(r, red[w]);
-    st->floor = 4.0 * (double)n * 2.220446049250313e-16 * r;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->info = 0;
     st->err = 0;
   }
+  block_max(m, red);
+  if (threadIdx.x == 0 && red[0] > 0.0) atomicMax(&st->max_diag, (unsigned long long)__double_as_longlong(red[0]));
 }
 
-// One tile product: acc += X Y^T over k < K (a multiple of 4), X and Y tiles
-// in shared memory (row-major, kLd, k contiguous); the fragments as
-// tile_dmma64 deals them to the eight warps.
-template <bool XK, bool YK>
-__device__ __forceinline__ void chol_mma(const double* Xs, const double* Ys, int K, double (&acc)[2][4][2]) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int i0 = 16 * (w & 3), j0 = 32 * (w >> 2);
+template <typename Real>
+__global__ void chol_floor(SysDev<Real> S, int bs, CholState* st) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  double m = 0.0;
+  if (t < S.nb * bs) {
+    const int i = t / bs, a = t % bs;
+    const int rb = S.rptr[i], nblk = S.rptr[i + 1] - rb;
+    m = fabs((double)S.val[(size_t)rb * bs * bs + (size_t)a * (bs + 1) * nblk + (S.diag[i] - rb)]);
+  }
+  chol_floor_max(m, st);
+}
+
+// sys_gather_damped and chol_floor in one pass: the damped pose-graph system
+// and its largest diagonal entry
+template <typename Real, int BS>
+__global__ void chol_gather_damped(const Real* src, const int* perm, const int* brow, const int* rptr,
+                                   const int* rcol, int nnzb, double lambda, Real* dst, CholState* st) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  double m = 0.0;
+  if (t < (long long)nnzb * BS * BS) {
+    const int k = (int)(t / (BS * BS)), e = (int)(t % (BS * BS));
+    const int r = brow[k], rb = rptr[r], nblk = rptr[r + 1] - rb;
+    double v = (double)src[(size_t)perm[k] * BS * BS + e];
+    const bool diag = rcol[k] == r && e % (BS + 1) == 0;
+    if (diag) v += lambda;
+    const Real d = (Real)v;
+    dst[sys_offset<BS>(rb, nblk, k - rb, e)] = d;
+    if (diag) m = fabs((double)d);
+  }
+  chol_floor_max(m, st);
+}
+
+// Products of tiles in 16 x 16 blocks: only the blocks of the tiles' leading
+// parts that hold unknowns are formed (the groups of a dissection seldom fill
+// their last tile), of a symmetric product only the lower ones. Block b of
+// the nblk blocks goes to warp b % 8; a warp's (at most two) blocks are in
+// acc[b / 8], as 2 x 2 fragments of 8 x 8.
+struct CholBlocks {
+  int mb, n;   // block rows, blocks
+  bool lower;  // only bi >= bj
+  __device__ __forceinline__ CholBlocks(int rows, int cols, bool low) : mb((rows + 15) >> 4), lower(low) {
+    const int nb = (cols + 15) >> 4;
+    n = low ? mb * (mb + 1) / 2 : mb * nb;
+  }
+  __device__ __forceinline__ bool at(int q, int& bi, int& bj) const {
+    int b = (threadIdx.x >> 5) + 8 * q;
+    if (b >= n) return false;
+    if (lower) {
+      bj = 0;
+      while (b >= mb - bj) b -= mb - bj++;
+      bi = bj + b;
+    } else {
+      bj = b / mb;
+      bi = b - bj * mb;
+    }
+    return true;
+  }
+};
+using CholAcc = double[2][2][2][2];  // [block][fragment row][fragment column][element]
+
+// acc += X Y^T over k < K (a multiple of 4); X(i, k) at X[i * kLd + k] or, with
+// XK, at X[k * kLd + i], likewise Y. TRI: Y(j, k) is zero for k > j.
+template <bool XK, bool YK, bool TRI = false>
+__device__ __forceinline__ void chol_mma(const CholBlocks& B, const double* X, const double* Y, int K, CholAcc& acc) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    int bi, bj;
+    if (!B.at(q, bi, bj)) continue;
+    const double* x = XK ? X + t * kLd + 16 * bi + g : X + (16 * bi + g) * kLd + t;
+    const double* y = YK ? Y + t * kLd + 16 * bj + g : Y + (16 * bj + g) * kLd + t;
+    const int k1 = TRI ? min(K, 16 * bj + 16) : K;
 #pragma unroll 4
-  for (int k0 = 0; k0 < K; k0 += 4) {
-    double fa[2], fb[4];
+    for (int k0 = 0; k0 < k1; k0 += 4) {
+      const int kx = XK ? k0 * kLd : k0, ky = YK ? k0 * kLd : k0;
+      double fa[2], fb[2];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) fa[u] = XK ? Xs[(k0 + t) * kLd + i0 + 8 * u + g] : Xs[(i0 + 8 * u + g) * kLd + k0 + t];
+      for (int u = 0; u < 2; ++u) {
+        fa[u] = x[kx + (XK ? 8 * u : 8 * u * kLd)];
+        fb[u] = y[ky + (YK ? 8 * u : 8 * u * kLd)];
+      }
 #pragma unroll
-    for (int v = 0; v < 4; ++v) fb[v] = YK ? Ys[(k0 + t) * kLd + j0 + 8 * v + g] : Ys[(j0 + 8 * v + g) * kLd + k0 + t];
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int v = 0; v < 2; ++v)
+          asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                       : "+d"(acc[q][u][v][0]), "+d"(acc[q][u][v][1])
+                       : "d"(fa[u]), "d"(fb[v]));
+    }
+  }
+}
+
+// f(row, column, the two accumulators of row and column, column + 1)
+template <typename F>
+__device__ __forceinline__ void chol_each_frag(const CholBlocks& B, CholAcc& acc, F&& f) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    int bi, bj;
+    if (!B.at(q, bi, bj)) continue;
 #pragma unroll
     for (int u = 0; u < 2; ++u)
 #pragma unroll
-      for (int v = 0; v < 4; ++v)
-        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                     : "+d"(acc[u][v][0]), "+d"(acc[u][v][1])
-                     : "d"(fa[u]), "d"(fb[v]));
+      for (int v = 0; v < 2; ++v) f(16 * bi + 8 * u + g, 16 * bj + 8 * v + 2 * t, acc[q][u][v]);
   }
 }
-
-// f(row, column, value pair) over this thread's fragment elements
-template <typename F>
-__device__ __forceinline__ void chol_each_frag(F&& f) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int i0 = 16 * (w & 3), j0 = 32 * (w >> 2);
+__device__ __forceinline__ void chol_clear(CholAcc& acc) {
 #pragma unroll
-  for (int u = 0; u < 2; ++u)
+  for (int q = 0; q < 2; ++q)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) f(i0 + 8 * u + g, j0 + 8 * v + 2 * t, u, v);
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int v = 0; v < 2; ++v) acc[q][u][v][0] = acc[q][u][v][1] = 0.0;
 }
 
-// a tile of global memory (row-major) into shared memory
-__device__ __forceinline__ void chol_load_tile(const double* src, double* dst) {
-#pragma unroll
-  for (int q = 0; q < kTileElems / 2 / 256; ++q) {
-    const int e = 2 * (threadIdx.x + 256 * q);
-    cp_async16(dst + (e >> 6) * kLd + (e & 63), src + e);
+// the leading rows x cols (rounded up to 16, and to 16, 32 or 64) of a tile of
+// global memory (row-major) into shared memory
+__device__ __forceinline__ void chol_load_tile(const double* src, double* dst, int rows, int cols) {
+  const int sh = cols <= 16 ? 3 : cols <= 32 ? 4 : 5;  // 16-byte pieces per row
+  const int n = ((rows + 15) & ~15) << sh;
+  for (int i = threadIdx.x; i < n; i += 256) {
+    const int r = i >> sh, c = 2 * (i & ((1 << sh) - 1));
+    cp_async16(dst + r * kLd + c, src + r * kTile + c);
   }
 }
+__device__ __forceinline__ void chol_load_tile(const double* src, double* dst) { chol_load_tile(src, dst, kTile, kTile); }
 
-// shared memory of chol_factor_dag: two stages of two operand tiles, a
+// shared memory of chol_factor_dag: three stages of two operand tiles, a
 // vector per stage and the right-hand side
-constexpr int kFactorSmem = (4 * kTileBuf + 3 * kTile) * (int)sizeof(double);
+constexpr int kFactorStages = 3;
+constexpr int kFactorSmem = kFactorStages * (2 * kTileBuf + kTile) * (int)sizeof(double) + kTile * (int)sizeof(double);
+
+// How many of the products from u on (at most 16, in list order) have both
+// operand tiles ready: one round trip for all of them. One warp.
+__device__ __forceinline__ int chol_ready(const CholDev& P, const int2* upd, int u, int nu, unsigned want) {
+  const int lane = threadIdx.x & 31, q = u + (lane >> 1);
+  bool ok = false;
+  if (q < nu) {
+    const int2 ab = upd[q];
+    ok = chol_load_flag(P.flag + ((lane & 1) ? ab.y : ab.x)) == want;
+  }
+  const unsigned m = __ballot_sync(0xffffffffu, ok), missing = ~(m & (m >> 1)) & 0x55555555u;
+  return missing ? (__ffs(missing) - 1) >> 1 : 16;
+}
+
+// The blocks of a slot into a tile of shared memory (256 threads; identity on
+// the padding of a diagonal tile); a barrier is needed before and after.
+template <typename Real>
+__device__ __forceinline__ void chol_assemble(const SysDev<Real>& S, int bs, const CholDev& P, int s, double* As) {
+  const int k = P.col[s];
+  const bool diag = P.row[s] == k;
+  for (int e = threadIdx.x; e < kTileElems; e += 256) {
+    const int r = e >> 6, c = e & 63;
+    As[r * kLd + c] = diag && r == c && P.orig[(size_t)k * kTile + r] < 0 ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  const int bs2 = bs * bs, e0 = P.asm_ptr[s], ne = (P.asm_ptr[s + 1] - e0) * bs2;
+  for (int q = threadIdx.x; q < ne; q += 256) {
+    const int b = q / bs2, e = q - b * bs2;
+    const int4 en = P.asm_ent[e0 + b];
+    const size_t off = ((size_t)(unsigned)en.x | ((size_t)(unsigned)en.y << 32)) + (size_t)e * en.z;
+    const int bi = e / bs, bj = e - bi * bs;
+    const bool tr = (en.w >> 16) != 0;
+    const int r = (en.w & 255) - kTile + (tr ? bj : bi), c = ((en.w >> 8) & 255) - kTile + (tr ? bi : bj);
+    if ((unsigned)r < (unsigned)kTile && (unsigned)c < (unsigned)kTile) As[r * kLd + c] = (double)S.val[off];
+  }
+}
+
+// fragments <- -tile and tile <- -fragments
+__device__ __forceinline__ void chol_frags_from(const CholBlocks& B, const double* T, CholAcc& acc) {
+  chol_each_frag(B, acc, [&](int r, int c, double (&a)[2]) {
+    a[0] = -T[r * kLd + c];
+    a[1] = -T[r * kLd + c + 1];
+  });
+}
+__device__ __forceinline__ void chol_frags_to(const CholBlocks& B, double* T, CholAcc& acc) {
+  chol_each_frag(B, acc, [&](int r, int c, double (&a)[2]) {
+    T[r * kLd + c] = -a[0];
+    T[r * kLd + c + 1] = -a[1];
+  });
+}
 
 // The whole factorization, one persistent CTA of 256 threads per SM. Tiles
 // are handed out by ticket in the plan's order (estimated start times, always
@@ -281,110 +406,119 @@ constexpr int kFactorSmem = (4 * kTileBuf + 3 * kTile) * (int)sizeof(double);
 // and 1,600 products, which 148 SMs pass in some 20 us, but a chain of 11
 // diagonal tiles. What counts is the time of a tile of that chain: the
 // diagonal factorization (tile_potrf_inv64) and the hand-over through L2.
-// Measured on a 3,500-pose 2D graph (n = 10,497, 11 levels): factorization and
-// both substitutions 0.28 ms per solve, against 10.1 ms for the reverse
-// Cuthill-McKee band (165 strictly sequential tile steps in one CTA); on a
-// 2,500-pose 3D graph (n = 14,994) 0.35 ms against 19.7 ms.
+// A task near the root has up to 40 products in its list, nearly all of them
+// long ready when it starts: the flags of 16 products are read in one round
+// trip and the operands of two are on their way while one is multiplied.
+// Measured per solve, factorization and both substitutions: a 3,500-pose 2D
+// graph (n = 10,497, 11 levels) 0.20 ms, against 10.1 ms for a reverse
+// Cuthill-McKee band (165 strictly sequential tile steps in one CTA); a
+// 2,500-pose 3D graph (n = 14,994) 0.27 ms, against 19.7 ms. With one flag
+// per round trip, one product's operands ahead and whole 64 x 64 products
+// they took 0.27 and 0.34 ms. Computing the tile below the diagonal in the
+// diagonal's task (W(k) then need not travel) gained 4% where that task had
+// few products and lost 15% where it had many.
 template <typename Real>
-__global__ void __launch_bounds__(256) chol_factor_dag(SysDev<Real> S, int bs, CholDev P, const double* rhs,
-                                                       unsigned extra) {
+__global__ void __launch_bounds__(256, 1) chol_factor_dag(SysDev<Real> S, int bs, CholDev P, const double* rhs,
+                                                          unsigned extra) {
   extern __shared__ __align__(16) double sm_chol[];
-  __shared__ int sh_ticket, sh_ok;
-  double* buf[2][2] = {{sm_chol, sm_chol + kTileBuf}, {sm_chol + 2 * kTileBuf, sm_chol + 3 * kTileBuf}};
-  double* yb = sm_chol + 4 * kTileBuf;
-  double* vb = yb + 2 * kTile;
+  __shared__ int sh_ticket, sh_ready;
+  // stage q: operand tiles at 2 q and 2 q + 1
+  auto buf = [&](int q) { return sm_chol + q * kTileBuf; };
+  double* yb = sm_chol + 2 * kFactorStages * kTileBuf;
+  double* vb = yb + kFactorStages * kTile;
   const int tid = threadIdx.x;
   const unsigned want = P.st->factor.epoch + 1;  // the flag value of this launch
   const unsigned wait_for = want + extra;
-  const double floor = P.st->floor;
+  const double floor = P.floor * __longlong_as_double((long long)P.st->max_diag);
   int* err = &P.st->err;
   for (;;) {
     const int tk = chol_ticket(&P.st->factor, &sh_ticket);
-    if (tk >= P.ns) break;
+    if (tk >= P.ntask) break;
     const int s = P.task[tk];
-    const int i = P.row[s], k = P.col[s];
-    const bool diag = i == k;
-    // A(i, k)
-    double* As = buf[0][0];
-    for (int e = tid; e < kTileElems; e += 256) {
-      const int r = e >> 6, c = e & 63;
-      As[r * kLd + c] = diag && r == c && P.orig[(size_t)k * kTile + r] < 0 ? 1.0 : 0.0;
+    const int k = P.col[s];
+    const bool diag = P.row[s] == k;
+    const int wk = P.width[k], wi = P.width[P.row[s]];
+    const CholBlocks B(wi, wk, diag);
+    CholAcc acc;
+    chol_clear(acc);
+    const int2* upd = P.upd + P.upd_ptr[s];
+    const int nu = P.upd_ptr[s + 1] - P.upd_ptr[s];
+    if (tid < 32) {
+      const int n = chol_ready(P, upd, 0, nu, wait_for);
+      if (tid == 0) sh_ready = n;
     }
+    chol_assemble(S, bs, P, s, buf(0));
     if (diag && tid < kTile) {
       const int o = rhs ? P.orig[(size_t)k * kTile + tid] : -1;
       vb[tid] = o >= 0 ? rhs[o] : 0.0;
     }
     __syncthreads();
-    const int bs2 = bs * bs, e0 = P.asm_ptr[s], ne = (P.asm_ptr[s + 1] - e0) * bs2;
-    for (int q = tid; q < ne; q += 256) {
-      const int b = q / bs2, e = q - b * bs2;
-      const int4 en = P.asm_ent[e0 + b];
-      const size_t off = ((size_t)(unsigned)en.x | ((size_t)(unsigned)en.y << 32)) + (size_t)e * en.z;
-      const int bi = e / bs, bj = e - bi * bs;
-      const bool tr = (en.w >> 16) != 0;
-      const int r = (en.w & 255) - kTile + (tr ? bj : bi), c = ((en.w >> 8) & 255) - kTile + (tr ? bi : bj);
-      if ((unsigned)r < (unsigned)kTile && (unsigned)c < (unsigned)kTile) As[r * kLd + c] = (double)S.val[off];
-    }
+    int ready = sh_ready;  // products below are known to have their operands
+    chol_frags_from(B, buf(0), acc);
     __syncthreads();
-    double acc[2][4][2];
-    chol_each_frag([&](int r, int c, int u, int v) {
-      acc[u][v][0] = -As[r * kLd + c];
-      acc[u][v][1] = -As[r * kLd + c + 1];
-    });
-    __syncthreads();
-    // updates
-    const int u0 = P.upd_ptr[s], nu = P.upd_ptr[s + 1] - u0;
+    // updates L(i, j) L(k, j)^T: the operands of the next two are fetched while
+    // one is multiplied, as far as they are known to be ready
     double ysum = 0.0;
-    auto issue = [&](int2 ab, int stage) {
-      chol_load_tile(P.L + (size_t)ab.x * kTileElems, buf[stage][0]);
-      if (ab.y != ab.x) chol_load_tile(P.L + (size_t)ab.y * kTileElems, buf[stage][1]);
+    auto issue = [&](int u) {
+      const int2 ab = upd[u];
+      const int q = u % kFactorStages, K = P.width[P.col[ab.x]];
+      chol_load_tile(P.L + (size_t)ab.x * kTileElems, buf(2 * q), wi, K);
+      if (!diag) chol_load_tile(P.L + (size_t)ab.y * kTileElems, buf(2 * q + 1), wk, K);
       if (diag && tid < kTile / 2)
-        cp_async16(yb + stage * kTile + 2 * tid, P.y + (size_t)P.col[ab.x] * kTile + 2 * tid);
+        cp_async16(yb + q * kTile + 2 * tid, P.y + (size_t)P.col[ab.x] * kTile + 2 * tid);
+      asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    bool issued = false, ok = true;
-    int2 ab = nu > 0 ? P.upd[u0] : make_int2(0, 0);
+    int issued = 0;
+    bool ok = true;
     for (int u = 0; u < nu; ++u) {
-      const int stage = u & 1;
-      const int2 nx = u + 1 < nu ? P.upd[u0 + u + 1] : make_int2(0, 0);
-      if (!issued) {
-        if (tid == 0)
-          sh_ok = chol_wait(P.flag + ab.x, wait_for, err) && (ab.y == ab.x || chol_wait(P.flag + ab.y, wait_for, err));
+      if (u >= ready) {
+        __syncthreads();  // sh_ready has been read
+        if (tid < 32) {
+          int n = 0;
+          unsigned spins = 0;
+          while ((n = chol_ready(P, upd, u, nu, wait_for)) == 0) {
+            if ((spins & 255u) == 255u && __any_sync(0xffffffffu, *(volatile int*)err != 0)) break;
+            if (spins++ >= kCholSpinLimit) {
+              if (tid == 0) atomicExch(err, 1);
+              break;
+            }
+          }
+          if (tid == 0) sh_ready = u + n;
+        }
         __syncthreads();
-        ok = sh_ok != 0;
+        ready = sh_ready;
+        ok = ready > u;
         if (!ok) break;
-        issue(ab, stage);
       }
-      cp_async_wait_all();
-      int ready = 0;
-      if (tid == 0 && u + 1 < nu) ready = chol_load_flag(P.flag + nx.x) == wait_for && chol_load_flag(P.flag + nx.y) == wait_for;
-      issued = __syncthreads_or(ready) != 0;
-      if (issued) issue(nx, stage ^ 1);
-      const double* X = buf[stage][0];
-      const double* Y = ab.y == ab.x ? X : buf[stage][1];
+      if (issued <= u) {
+        issue(u);
+        issued = u + 1;
+      }
+      if (issued - u == 1) asm volatile("cp.async.wait_group 0;" ::: "memory");
+      else asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncthreads();
+      while (issued < nu && issued < ready && issued < u + kFactorStages) issue(issued++);
+      const int2 ab = upd[u];
+      const int q = u % kFactorStages;
+      const double *X = buf(2 * q), *Y = diag ? X : buf(2 * q + 1);
       const int K = (P.width[P.col[ab.x]] + 3) & ~3;
-      chol_mma<false, false>(X, Y, K, acc);
+      chol_mma<false, false>(B, X, Y, K, acc);
       if (diag) {
-        const int r = tid >> 2, q = tid & 3;
-        const double* yv = yb + stage * kTile;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) ysum += X[r * kLd + 4 * c + q] * yv[4 * c + q];
+        const int r = tid >> 2;
+        const double* yv = yb + q * kTile;
+        if (r < wk)
+          for (int c = tid & 3; c < K; c += 4) ysum += X[r * kLd + c] * yv[c];
       }
-      ab = nx;
     }
     if (!ok) break;
     __syncthreads();
-    const int wk = P.width[k];
+    double *T = buf(0), *Ws = buf(1);  // the tile after its updates; W(k)
+    chol_frags_to(B, T, acc);
     if (diag) {
-      double* T = buf[0][0];
-      double* Ws = buf[0][1];
-      chol_each_frag([&](int r, int c, int u, int v) {
-        T[r * kLd + c] = -acc[u][v][0];
-        T[r * kLd + c + 1] = -acc[u][v][1];
-      });
       ysum += __shfl_xor_sync(0xffffffffu, ysum, 1);
       ysum += __shfl_xor_sync(0xffffffffu, ysum, 2);
       if ((tid & 3) == 0) vb[tid >> 2] -= ysum;
-      tile_potrf_inv64(T, Ws, buf[1][0], wk, floor, &P.st->info);
+      tile_potrf_inv64(T, Ws, buf(2), wk, floor, &P.st->info);
       double* Wg = P.W + (size_t)k * kTileElems;
 #pragma unroll
       for (int q = 0; q < kTileElems / 2 / 256; ++q) {
@@ -399,23 +533,17 @@ __global__ void __launch_bounds__(256) chol_factor_dag(SysDev<Real> S, int bs, C
       yv += __shfl_xor_sync(0xffffffffu, yv, 2);
       if (q == 0) P.y[(size_t)k * kTile + r] = yv;
     } else {
-      double* X = buf[0][0];
-      double* Ws = buf[1][0];
-      chol_each_frag([&](int r, int c, int u, int v) {
-        X[r * kLd + c] = -acc[u][v][0];
-        X[r * kLd + c + 1] = -acc[u][v][1];
-        acc[u][v][0] = acc[u][v][1] = 0.0;
-      });
-      if (tid == 0) sh_ok = chol_wait(P.flag + P.col_ptr[k], wait_for, err);
+      if (tid == 0) sh_ready = chol_wait(P.flag + P.col_ptr[k], wait_for, err);
       __syncthreads();
-      if (sh_ok == 0) break;
-      chol_load_tile(P.W + (size_t)k * kTileElems, Ws);
+      if (sh_ready == 0) break;
+      chol_load_tile(P.W + (size_t)k * kTileElems, Ws, wk, wk);
       cp_async_wait_all();
       __syncthreads();
-      chol_mma<false, false>(X, Ws, (wk + 3) & ~3, acc);  // Y(j, t) = W(j, t)
+      chol_clear(acc);
+      chol_mma<false, false, true>(B, T, Ws, (wk + 3) & ~3, acc);  // W(j, t): lower triangular
       double* Lg = P.L + (size_t)s * kTileElems;
-      chol_each_frag([&](int r, int c, int u, int v) {
-        *reinterpret_cast<double2*>(Lg + r * kTile + c) = make_double2(acc[u][v][0], acc[u][v][1]);
+      chol_each_frag(B, acc, [&](int r, int c, double (&a)[2]) {
+        *reinterpret_cast<double2*>(Lg + r * kTile + c) = make_double2(a[0], a[1]);
       });
     }
     __syncthreads();
@@ -424,7 +552,7 @@ __global__ void __launch_bounds__(256) chol_factor_dag(SysDev<Real> S, int bs, C
       chol_store_flag(P.flag + s, want);
     }
   }
-  chol_leave(&P.st->factor);
+  chol_leave(&P.st->factor, [&]() { P.st->max_diag = 0; });
 }
 
 // Substitutions: tile columns handed out by ticket, one CTA of 256 threads
@@ -489,11 +617,13 @@ static __global__ void __launch_bounds__(256) chol_forward_dag(CholDev P, const 
       chol_store_flag(P.yflag + k, want);
     }
   }
-  chol_leave(&P.st->forward);
+  chol_leave(&P.st->forward, []() {});
 }
 
-// x(k) = W(k)^T (y(k) - sum_i L(i, k)^T x(i)), written in the caller's order
-static __global__ void __launch_bounds__(256) chol_backward_dag(CholDev P, double* xout, unsigned extra) {
+// x(k) = W(k)^T (y(k) - sum_i L(i, k)^T x(i)), written in the caller's order;
+// sc != nullptr gets the outcome of the solve
+static __global__ void __launch_bounds__(256) chol_backward_dag(CholDev P, double* xout, DevScalars* sc,
+                                                                unsigned extra) {
   __shared__ int sh_ticket, sh_ok;
   __shared__ double v[kTile], part[4][kTile];
   const int tid = threadIdx.x, c = tid & 63, q = tid >> 6;
@@ -548,7 +678,11 @@ static __global__ void __launch_bounds__(256) chol_backward_dag(CholDev P, doubl
       chol_store_flag(P.xflag + k, want);
     }
   }
-  chol_leave(&P.st->backward);
+  chol_leave(&P.st->backward, [&]() {
+    if (!sc) return;
+    sc->solve_ok = P.st->info == 0;
+    if (P.st->err) sc->chol_error = 1;
+  });
 }
 
 static int chol_launch_check(const char* what) {
@@ -561,21 +695,26 @@ static int chol_launch_check(const char* what) {
 }
 
 // factor S: the plan holds L (tiles below the diagonal), W, the pivot flag
-// and, for rhs != nullptr, the forward-substituted vector
+// and, for rhs != nullptr, the forward-substituted vector. have_floor: the
+// largest diagonal entry is in the state already (chol_gather_damped)
 template <typename Real>
-static int chol_factor(CholPlan& P, cudaStream_t st, const SysDev<Real>& S, const double* rhs, long long* nl) {
-  const int ns = (int)P.S.row.size();
+static int chol_factor(CholPlan& P, cudaStream_t st, const SysDev<Real>& S, const double* rhs, long long* nl,
+                       bool have_floor = false) {
+  const int ntask = (int)P.S.task.size();
   G2OC_CUDA_TRY(
       cudaFuncSetAttribute(chol_factor_dag<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFactorSmem));
-  chol_begin<Real><<<1, 1024, 0, st>>>(S, P.S.bs, P.state.p);
-  chol_factor_dag<Real><<<std::min(P.sms, ns), 256, kFactorSmem, st>>>(S, P.S.bs, P.dev(), rhs, P.extra);
-  *nl += 2;
+  if (!have_floor) {
+    chol_floor<Real><<<(P.S.n + 255) / 256, 256, 0, st>>>(S, P.S.bs, P.state.p);
+    *nl += 1;
+  }
+  chol_factor_dag<Real><<<std::min(P.sms, ntask), 256, kFactorSmem, st>>>(S, P.S.bs, P.dev(), rhs, P.extra);
+  *nl += 1;
   return chol_launch_check("cholesky");
 }
 
 // backward substitution of the vector the plan holds
-static int chol_backward(CholPlan& P, cudaStream_t st, double* xout, long long* nl) {
-  chol_backward_dag<<<std::min(2 * P.sms, P.S.nt), 256, 0, st>>>(P.dev(), xout, P.extra);
+static int chol_backward(CholPlan& P, cudaStream_t st, double* xout, long long* nl, DevScalars* sc = nullptr) {
+  chol_backward_dag<<<std::min(2 * P.sms, P.S.nt), 256, 0, st>>>(P.dev(), xout, sc, P.extra);
   *nl += 1;
   return chol_launch_check("cholesky solve");
 }
@@ -592,12 +731,13 @@ static int chol_resolve(CholPlan& P, cudaStream_t st, const double* rhs, double*
 }
 
 // factor and solve, all queued on the stream; the outcome stays in P.state
+// and, for sc != nullptr, goes to sc->solve_ok / chol_error
 template <typename Real>
 static int chol_solve_async(CholPlan& P, cudaStream_t st, const SysDev<Real>& S, const double* rhs, double* xout,
-                            long long* nlaunch) {
+                            long long* nlaunch, DevScalars* sc = nullptr, bool have_floor = false) {
   long long nl = 0;
-  G2OC_TRY(chol_factor<Real>(P, st, S, rhs, &nl));
-  G2OC_TRY(chol_backward(P, st, xout, &nl));
+  G2OC_TRY(chol_factor<Real>(P, st, S, rhs, &nl, have_floor));
+  G2OC_TRY(chol_backward(P, st, xout, &nl, sc));
   if (nlaunch) *nlaunch += nl;
   return G2OC_OK;
 }
@@ -650,10 +790,12 @@ static __global__ void __launch_bounds__(256) selinv_panel(CholDev P) {
   chol_load_tile(P.W + (size_t)J * kTileElems, Y);
   cp_async_wait_all();
   __syncthreads();
-  double acc[2][4][2] = {};
-  chol_mma<false, true>(X, Y, (P.width[J] + 3) & ~3, acc);
-  chol_each_frag([&](int r, int c, int u, int v) {
-    *reinterpret_cast<double2*>(Lg + r * kTile + c) = make_double2(acc[u][v][0], acc[u][v][1]);
+  const CholBlocks B(P.width[P.row[s]], P.width[J], false);
+  CholAcc acc;
+  chol_clear(acc);
+  chol_mma<false, true>(B, X, Y, (P.width[J] + 3) & ~3, acc);
+  chol_each_frag(B, acc, [&](int r, int c, double (&a)[2]) {
+    *reinterpret_cast<double2*>(Lg + r * kTile + c) = make_double2(a[0], a[1]);
   });
 }
 
@@ -680,16 +822,18 @@ static __global__ void __launch_bounds__(256) selinv_dag(CholDev P, SelinvDev Q,
     if (tk >= P.ns) break;
     const int s = Q.task[tk], J = P.col[s];
     const bool diag = P.row[s] == J;
-    double acc[2][4][2] = {};
+    const CholBlocks B(P.width[P.row[s]], P.width[J], false);
+    CholAcc acc;
+    chol_clear(acc);
     if (diag) {
       chol_load_tile(P.W + (size_t)J * kTileElems, buf[0][0]);
       cp_async_wait_all();
       __syncthreads();
-      chol_mma<true, true>(buf[0][0], buf[0][0], kTile, acc);  // W is zero above the diagonal and beyond the width
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v][0] = -acc[u][v][0], acc[u][v][1] = -acc[u][v][1];
+      chol_mma<true, true>(B, buf[0][0], buf[0][0], kTile, acc);  // W is zero above the diagonal and beyond the width
+      chol_each_frag(B, acc, [](int, int, double (&a)[2]) {
+        a[0] = -a[0];
+        a[1] = -a[1];
+      });
       __syncthreads();
     }
     const int q0 = Q.ptr[s], nq = Q.ptr[s + 1] - q0;
@@ -714,9 +858,9 @@ static __global__ void __launch_bounds__(256) selinv_dag(CholDev P, SelinvDev Q,
       if (tid == 0 && q + 1 < nq) ready = chol_load_flag(Q.flag + nx.x) == wait_for;
       issued = __syncthreads_or(ready) != 0;
       if (issued) issue(nx, stage ^ 1);
-      if (diag) chol_mma<true, true>(buf[stage][1], buf[stage][0], en.w, acc);
-      else if (en.z) chol_mma<true, true>(buf[stage][0], buf[stage][1], en.w, acc);
-      else chol_mma<false, true>(buf[stage][0], buf[stage][1], en.w, acc);
+      if (diag) chol_mma<true, true>(B, buf[stage][1], buf[stage][0], en.w, acc);
+      else if (en.z) chol_mma<true, true>(B, buf[stage][0], buf[stage][1], en.w, acc);
+      else chol_mma<false, true>(B, buf[stage][0], buf[stage][1], en.w, acc);
       en = nx;
     }
     if (!ok) break;
@@ -724,18 +868,16 @@ static __global__ void __launch_bounds__(256) selinv_dag(CholDev P, SelinvDev Q,
     if (diag) {
       double* T = buf[0][0];
       __syncthreads();
-      chol_each_frag([&](int r, int c, int u, int v) {
-        T[r * kLd + c] = -acc[u][v][0];
-        T[r * kLd + c + 1] = -acc[u][v][1];
-      });
+      chol_frags_to(B, T, acc);
       __syncthreads();
+      const int w = 16 * B.mb;
       for (int e = tid; e < kTileElems; e += 256) {
         const int r = e >> 6, c = e & 63;
-        Sg[e] = 0.5 * (T[r * kLd + c] + T[c * kLd + r]);
+        if (r < w && c < w) Sg[e] = 0.5 * (T[r * kLd + c] + T[c * kLd + r]);
       }
     } else {
-      chol_each_frag([&](int r, int c, int u, int v) {
-        *reinterpret_cast<double2*>(Sg + r * kTile + c) = make_double2(-acc[u][v][0], -acc[u][v][1]);
+      chol_each_frag(B, acc, [&](int r, int c, double (&a)[2]) {
+        *reinterpret_cast<double2*>(Sg + r * kTile + c) = make_double2(-a[0], -a[1]);
       });
     }
     __syncthreads();
@@ -744,7 +886,7 @@ static __global__ void __launch_bounds__(256) selinv_dag(CholDev P, SelinvDev Q,
       chol_store_flag(Q.flag + s, want);
     }
   }
-  chol_leave(&P.st->forward);
+  chol_leave(&P.st->forward, []() {});
 }
 
 // requested blocks (row, col) of H^-1, row-major bs x bs each
@@ -814,6 +956,7 @@ static int chol_selected_inverse(CholPlan& P, cudaStream_t st, const SysDev<Real
   G2OC_TRY(flag.alloc(ns));
   G2OC_TRY(sigma.alloc((size_t)ns * kTileElems));
   G2OC_CUDA_TRY(cudaMemsetAsync(flag.p, 0, flag.bytes(), st));
+  G2OC_CUDA_TRY(cudaMemsetAsync(sigma.p, 0, sigma.bytes(), st));  // the parts without unknowns are not written
   G2OC_TRY(chol_outcome(P, st, ok));
   if (!*ok) return G2OC_OK;
   const SelinvDev Q{ints.p + o[0], reinterpret_cast<const int4*>(ints.p + o[2]), ints.p + o[1], flag.p, sigma.p};

@@ -1179,17 +1179,18 @@ struct Engine final : EngineBase {
     return G2OC_OK;
   }
 
-  // the outcome (positive definite or not) stays on the device, c->chol->state
-  int chol_solve(const Real* val, const double* rhs, double* xout) {
+  // the outcome (positive definite or not) goes to sc.solve_ok on the device
+  int chol_solve(const Real* val, const double* rhs, double* xout, bool have_floor = false) {
     G2OC_TRY(ensure_chol());
-    return chol_solve_async<Real>(*c->chol, c->stream, sys(val), rhs, xout, &c->kcount[K_CHOLESKY]);
+    return chol_solve_async<Real>(*c->chol, c->stream, sys(val), rhs, xout, &c->kcount[K_CHOLESKY], c->sc.p,
+                                  have_floor);
   }
 
   int solve(double lambda) override {
     const Structure& S = c->S;
     cudaStream_t st = c->stream;
     int ok = 1;
-    const CholState* outcome = nullptr;
+    bool decided = false;  // the Cholesky sets sc.solve_ok itself
     const bool use_chol = c->prm.linear_solver == G2OC_LINEAR_CHOLESKY ||
                           (c->prm.linear_solver == 2 && !S.ba);
     if (S.Cf == 0) {
@@ -1228,7 +1229,7 @@ struct Engine final : EngineBase {
         G2OC_TRY(tc_resolve(c->rhs.p, c->xs.p));
       } else if (use_chol) {
         G2OC_TRY(chol_solve(Sval.p, c->rhs.p, c->xs.p));
-        outcome = c->chol->state.p;
+        decided = true;
       } else {
         G2OC_TRY(pcg_solve(Sval.p, c->rhs.p, c->xs.p, false));
       }
@@ -1316,26 +1317,38 @@ struct Engine final : EngineBase {
     } else {
       const int nnzb = S.sys_nnzb;
       const long long nel = (long long)nnzb * S.pd * S.pd;
-      if (S.pd == 3)
-        G2OC_K(K_DAMP) sys_gather_damped<Real, 3><<<cdiv(nel, 256), 256, 0, st>>>(
-            hpp.p, c->sys_perm.p, c->sys_brow.p, c->sys_rptr.p, c->sys_rcol.p, nnzb, lambda, sysval.p);
-      else
-        G2OC_K(K_DAMP) sys_gather_damped<Real, 6><<<cdiv(nel, 256), 256, 0, st>>>(
-            hpp.p, c->sys_perm.p, c->sys_brow.p, c->sys_rptr.p, c->sys_rcol.p, nnzb, lambda, sysval.p);
-      G2OC_LAUNCH_CHECK();
       if (use_chol) {
-        G2OC_TRY(chol_solve(sysval.p, c->b.p, c->x.p));
-        outcome = c->chol->state.p;
+        G2OC_TRY(ensure_chol());
+        if (S.pd == 3)
+          G2OC_K(K_DAMP) chol_gather_damped<Real, 3><<<cdiv(nel, 256), 256, 0, st>>>(
+              hpp.p, c->sys_perm.p, c->sys_brow.p, c->sys_rptr.p, c->sys_rcol.p, nnzb, lambda, sysval.p,
+              c->chol->state.p);
+        else
+          G2OC_K(K_DAMP) chol_gather_damped<Real, 6><<<cdiv(nel, 256), 256, 0, st>>>(
+              hpp.p, c->sys_perm.p, c->sys_brow.p, c->sys_rptr.p, c->sys_rcol.p, nnzb, lambda, sysval.p,
+              c->chol->state.p);
+        G2OC_LAUNCH_CHECK();
+        G2OC_TRY(chol_solve(sysval.p, c->b.p, c->x.p, true));
+        decided = true;
         if (sizeof(Real) == 4 && !S.ba && c->prm.refine_max_iterations >= 0) {
           G2OC_TRY(chol_outcome(*c->chol, st, &ok));
           if (ok) G2OC_TRY(refine_pose_graph(lambda));
         }
       } else {
+        if (S.pd == 3)
+          G2OC_K(K_DAMP) sys_gather_damped<Real, 3><<<cdiv(nel, 256), 256, 0, st>>>(
+              hpp.p, c->sys_perm.p, c->sys_brow.p, c->sys_rptr.p, c->sys_rcol.p, nnzb, lambda, sysval.p);
+        else
+          G2OC_K(K_DAMP) sys_gather_damped<Real, 6><<<cdiv(nel, 256), 256, 0, st>>>(
+              hpp.p, c->sys_perm.p, c->sys_brow.p, c->sys_rptr.p, c->sys_rcol.p, nnzb, lambda, sysval.p);
+        G2OC_LAUNCH_CHECK();
         G2OC_TRY(pcg_solve(sysval.p, c->b.p, c->x.p, false));
       }
     }
-    G2OC_K(K_LM_CONTROL) set_solve_ok<<<1, 32, 0, st>>>(c->sc.p, ok, outcome);
-    G2OC_LAUNCH_CHECK();
+    if (!decided) {
+      G2OC_K(K_LM_CONTROL) set_solve_ok<<<1, 32, 0, st>>>(c->sc.p, ok);
+      G2OC_LAUNCH_CHECK();
+    }
     return G2OC_OK;
   }
 
@@ -1811,7 +1824,7 @@ struct BalEngine final : EngineBase {
   int solve(double lambda) override {
     const Structure& S = c->S;
     cudaStream_t st = c->stream;
-    const CholState* outcome = nullptr;
+    bool decided = false;
     const double* bl = c->b.p + (size_t)S.Cf * 9;
     if (S.Cf == 0) {
       // every camera fixed: x_l = (H_ll + lambda I)^-1 b_l
@@ -1830,8 +1843,8 @@ struct BalEngine final : EngineBase {
           P->extra = c->barrier_extra;
           c->chol = std::move(P);
         }
-        G2OC_TRY(chol_solve_async<double>(*c->chol, st, A, c->rhs.p, c->xs.p, &c->kcount[K_CHOLESKY]));
-        outcome = c->chol->state.p;
+        G2OC_TRY(chol_solve_async<double>(*c->chol, st, A, c->rhs.p, c->xs.p, &c->kcount[K_CHOLESKY], c->sc.p));
+        decided = true;
       } else {
         G2OC_K(K_PCG_DIAG_INV) pcg_diag_inv_lanes<double, 9><<<cdiv(A.nb, 3 * 4), 128, 0, st>>>(A, minv.p,
                                                                                              c->flag.p);
@@ -1844,8 +1857,10 @@ struct BalEngine final : EngineBase {
                                     st));
       G2OC_TRY(backsub(bl, c->xs.p, c->x.p + (size_t)S.Cf * 9));
     }
-    G2OC_K(K_LM_CONTROL) set_solve_ok<<<1, 32, 0, st>>>(c->sc.p, 1, outcome);
-    G2OC_LAUNCH_CHECK();
+    if (!decided) {
+      G2OC_K(K_LM_CONTROL) set_solve_ok<<<1, 32, 0, st>>>(c->sc.p, 1);
+      G2OC_LAUNCH_CHECK();
+    }
     return G2OC_OK;
   }
 

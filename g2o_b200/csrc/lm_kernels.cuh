@@ -4,7 +4,6 @@
 // kernels shared by the paths.
 #pragma once
 
-#include "cholesky.cuh"
 #include "g2oc_internal.h"
 #include "pcg_kernels.cuh"
 #include "reduce.cuh"
@@ -47,11 +46,8 @@ static __global__ void lm_decide(DevScalars* sc) {
   sc->rho = rho;
 }
 
-// outcome: the queued Cholesky's state (nullptr: no Cholesky)
-static __global__ void set_solve_ok(DevScalars* sc, int ok, const CholState* outcome) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  sc->solve_ok = ok && !(outcome && outcome->info);
-  if (outcome && outcome->err) sc->chol_error = 1;
+static __global__ void set_solve_ok(DevScalars* sc, int ok) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) sc->solve_ok = ok;
 }
 
 // partial sums of x (lambda x + b) (computeScale)

@@ -244,10 +244,19 @@ __device__ __forceinline__ void tile_trail_frag(double* T, int o, int fi, int fj
 // columns 8 f .. of the sums L_p,: W (W is lower triangular: k from 8 f on)
 __device__ __forceinline__ void tile_w_sum(const double* T, const double* Ws, double* S, int p, int f) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
-  double c[2];
-  dmma_frag<false, true>(T + 8 * p * kLd + 8 * f, kLd, Ws + 8 * f * kLd + 8 * f, kLd, 0, 0, 8 * (p - f), c);
-  S[g * kLd + 8 * f + 2 * t4] = c[0];
-  S[g * kLd + 8 * f + 2 * t4 + 1] = c[1];
+  const double* X = T + (8 * p + g) * kLd + 8 * f + t4;
+  const double* Y = Ws + (8 * f + t4) * kLd + 8 * f + g;
+  double c[2][2] = {{0.0, 0.0}, {0.0, 0.0}};  // two chains of products
+#pragma unroll 2
+  for (int k0 = 0; k0 < 8 * (p - f); k0 += 8) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                   : "+d"(c[h][0]), "+d"(c[h][1])
+                   : "d"(X[k0 + 4 * h]), "d"(Y[(k0 + 4 * h) * kLd]));
+  }
+  S[g * kLd + 8 * f + 2 * t4] = c[0][0] + c[1][0];
+  S[g * kLd + 8 * f + 2 * t4 + 1] = c[0][1] + c[1][1];
 }
 __device__ __forceinline__ void tile_w_row(double* Ws, const double* S, int p, int f) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
@@ -260,7 +269,6 @@ __device__ __forceinline__ void tile_w_row(double* Ws, const double* S, int p, i
 __device__ __forceinline__ void tile_potrf_inv64(double* T, double* Ws, double* S, int width, double floor,
                                                  int* info) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int e = tid; e < 64 * 64; e += 256) Ws[(e >> 6) * kLd + (e & 63)] = 0.0;
   __syncthreads();
   const int nst = (width + 7) >> 3;
   for (int p = 0; p < nst; ++p) {
@@ -270,13 +278,19 @@ __device__ __forceinline__ void tile_potrf_inv64(double* T, double* Ws, double* 
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j <= i; ++j) d[i][j] = T[(o + i) * kLd + o + j];
+        for (int j = 0; j <= i; j += 2) {
+          const double2 v = *reinterpret_cast<const double2*>(T + (o + i) * kLd + o + j);
+          d[i][j] = v.x;
+          if (j < i) d[i][j + 1] = v.y;
+        }
+      // what this lane solves against the factor: a row of the panel below, or
+      // (warp 2) a unit vector, which gives a column of W_pp. Its steps fill the
+      // waits of the chain of pivots.
       const int row = o + 8 + tid;
       const bool mine = warp < 2 && row < 8 * nst;
       double x[8];
-      if (mine)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) x[c] = T[row * kLd + o + c];
+      for (int c = 0; c < 8; ++c) x[c] = mine ? T[row * kLd + o + c] : (c == lane ? 1.0 : 0.0);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         double v = d[j][j];
@@ -287,35 +301,29 @@ __device__ __forceinline__ void tile_potrf_inv64(double* T, double* Ws, double* 
         rs[j] = rsqrt(v);
 #pragma unroll
         for (int i = j + 1; i < 8; ++i) d[i][j] *= rs[j];
+        x[j] *= rs[j];
 #pragma unroll
         for (int c = j + 1; c < 8; ++c)
 #pragma unroll
           for (int i = c; i < 8; ++i) d[i][c] -= d[i][j] * d[c][j];
+#pragma unroll
+        for (int q = j + 1; q < 8; ++q) x[q] -= x[j] * d[q][j];
       }
       if (mine) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          x[c] *= rs[c];
-#pragma unroll
-          for (int q = c + 1; q < 8; ++q) x[q] -= x[c] * d[q][c];
-        }
-#pragma unroll
         for (int c = 0; c < 8; ++c) T[row * kLd + o + c] = x[c];
       } else if (warp == 2 && lane < 8) {
-        // column `lane` of W_pp
-        double w[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) w[i] = i == lane ? 1.0 : 0.0;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          w[c] *= rs[c];
-#pragma unroll
-          for (int q = c + 1; q < 8; ++q) w[q] -= w[c] * d[q][c];
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) Ws[(o + i) * kLd + o + lane] = w[i];
+        for (int i = 0; i < 8; ++i) Ws[(o + i) * kLd + o + lane] = x[i];
       }
-    } else if (p > 0) {
+    } else if (p == 0) {
+      // W's blocks above the diagonal and beyond the width (the others are
+      // written whole)
+      for (int e = tid - 96; e < 64 * 64; e += 160) {
+        const int r = e >> 6, c = e & 63;
+        if ((c >> 3) > (r >> 3) || r >= 8 * nst) Ws[r * kLd + c] = 0.0;
+      }
+    } else {
       const int nw = p - 1, nf = nst - 1 - p, n = nw + nf * (nf + 1) / 2;
       for (int f = warp - 3; f < n; f += 5) {
         if (f < nw) {

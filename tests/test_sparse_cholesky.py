@@ -69,10 +69,11 @@ def system(kind, nb, bs, seed):
 
 
 # n = nb * bs around one and two tiles of 64, and wide enough for several
-# separators; the full pattern keeps the given order in one group
+# separators; the full pattern keeps the given order in one group (its largest
+# here has more products per tile than are looked up at a time)
 CASES = [("chain", 1, 3), ("chain", 21, 3), ("chain", 22, 3), ("chain", 10, 6), ("chain", 11, 6), ("chain", 400, 3),
-         ("star", 43, 3), ("star", 150, 6), ("full", 11, 6), ("full", 43, 3), ("full", 60, 6), ("grid", 64, 3),
-         ("grid", 199, 6), ("islands", 90, 3), ("islands", 33, 6), ("random", 130, 3), ("random", 77, 6)]
+         ("star", 43, 3), ("star", 150, 6), ("full", 11, 6), ("full", 43, 3), ("full", 60, 6), ("full", 190, 6),
+         ("grid", 64, 3), ("grid", 199, 6), ("islands", 90, 3), ("islands", 33, 6), ("random", 130, 3), ("random", 77, 6)]
 
 
 @pytest.mark.gpu
