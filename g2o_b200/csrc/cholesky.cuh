@@ -60,7 +60,6 @@ struct CholDev {
   double *y, *x;   // nt * kTile: forward and backward substituted vectors
   unsigned *flag, *yflag, *xflag;
   CholState* st;
-  double floor;    // smallest accepted pivot over the largest diagonal entry: 4 n eps
 };
 
 // int arrays of a plan, laid end to end (16-byte aligned) so that a plan is
@@ -83,6 +82,7 @@ struct CholPlan {
   DBuf<unsigned> flags;
   DBuf<CholState> state;
   CholDev d{};
+  bool smem_raised = false;  // the factorization may use its shared memory (a plan is factored in one type)
   const int* pos = nullptr;  // device copy of S.pos
   int sms = 0;
   unsigned extra = 0;  // the bounded-wait test: flags are compared with a number that is never reached
@@ -133,7 +133,7 @@ static int chol_plan_build(CholPlan& P, int nb, int bs, const std::vector<int>& 
   P.d = CholDev{S.nt, (int)ns, (int)S.task.size(), q + o[0], q + o[1], q + o[2], q + o[3], q + o[4], q + o[5],
                 reinterpret_cast<const int4*>(q + o[6]), q + o[7], reinterpret_cast<const int2*>(q + o[8]), q + o[9],
                 q + o[10], q + o[11], q + o[12], L, W, y, y + nt * kTile, P.flags.p, P.flags.p + ns,
-                P.flags.p + ns + nt, P.state.p, 4.0 * (double)S.n * 2.220446049250313e-16};
+                P.flags.p + ns + nt, P.state.p};
   P.pos = q + o[13];
   int dev = 0;
   G2OC_CUDA_TRY(cudaGetDevice(&dev));
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(256, 1) chol_factor_dag(SysDev<Real> S, int bs
   const int tid = threadIdx.x;
   const unsigned want = P.st->factor.epoch + 1;  // the flag value of this launch
   const unsigned wait_for = want + extra;
-  const double floor = P.floor * __longlong_as_double((long long)P.st->max_diag);
+  const double max_diag = __longlong_as_double((long long)P.st->max_diag);
   int* err = &P.st->err;
   for (;;) {
     const int tk = chol_ticket(&P.st->factor, &sh_ticket);
@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(256, 1) chol_factor_dag(SysDev<Real> S, int bs
         cp_async16(yb + q * kTile + 2 * tid, P.y + (size_t)P.col[ab.x] * kTile + 2 * tid);
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    int issued = 0;
+    int issued = 0, terms = wk;  // terms: a bound on the entries of L in a row of the tile
     bool ok = true;
     for (int u = 0; u < nu; ++u) {
       if (u >= ready) {
@@ -501,7 +501,8 @@ __global__ void __launch_bounds__(256, 1) chol_factor_dag(SysDev<Real> S, int bs
       const int2 ab = upd[u];
       const int q = u % kFactorStages;
       const double *X = buf(2 * q), *Y = diag ? X : buf(2 * q + 1);
-      const int K = (P.width[P.col[ab.x]] + 3) & ~3;
+      const int wj = P.width[P.col[ab.x]], K = (wj + 3) & ~3;
+      terms += wj;
       chol_mma<false, false>(B, X, Y, K, acc);
       if (diag) {
         const int r = tid >> 2;
@@ -518,6 +519,12 @@ __global__ void __launch_bounds__(256, 1) chol_factor_dag(SysDev<Real> S, int bs
       ysum += __shfl_xor_sync(0xffffffffu, ysum, 1);
       ysum += __shfl_xor_sync(0xffffffffu, ysum, 2);
       if ((tid & 3) == 0) vb[tid >> 2] -= ysum;
+      // a pivot is a diagonal entry less the squares of its row of L: with m
+      // entries its rounding is at most some m eps of the largest entry, and
+      // what does not exceed that is taken for zero. The rows of a dissected
+      // factor are short; n in the place of m refuses definite systems whose
+      // root is only weakly tied to the fixed vertices (a 40,000-pose chain)
+      const double floor = 4.0 * terms * 2.220446049250313e-16 * max_diag;
       tile_potrf_inv64(T, Ws, buf(2), wk, floor, &P.st->info);
       double* Wg = P.W + (size_t)k * kTileElems;
 #pragma unroll
@@ -701,8 +708,11 @@ template <typename Real>
 static int chol_factor(CholPlan& P, cudaStream_t st, const SysDev<Real>& S, const double* rhs, long long* nl,
                        bool have_floor = false) {
   const int ntask = (int)P.S.task.size();
-  G2OC_CUDA_TRY(
-      cudaFuncSetAttribute(chol_factor_dag<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFactorSmem));
+  if (!P.smem_raised) {
+    G2OC_CUDA_TRY(
+        cudaFuncSetAttribute(chol_factor_dag<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFactorSmem));
+    P.smem_raised = true;
+  }
   if (!have_floor) {
     chol_floor<Real><<<(P.S.n + 255) / 256, 256, 0, st>>>(S, P.S.bs, P.state.p);
     *nl += 1;

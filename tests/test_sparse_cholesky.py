@@ -133,3 +133,17 @@ def test_wait_that_runs_out_is_an_error(monkeypatch):
     good = backend.CudaProblem(g, prm)
     done, st = good.optimize(3)
     assert done == 3 and np.isfinite(st[-1]["chi2"])
+
+
+# a chain's root is tied to the fixed pose by a pivot far below n eps of the
+# largest entry; without the fixed pose the root's pivot is rounding alone
+@pytest.mark.gpu
+@pytest.mark.parametrize("poses,fixed,status", [(3400, True, 0), (40_000, True, 0), (60, False, 4), (3400, False, 4)])
+def test_pivot_floor(poses, fixed, status):
+    from g2o_b200 import backend, synth
+    g = synth.pose_graph_2d(poses, poses // 3, seed=5)
+    if not fixed:
+        g.pose_fixed = np.zeros_like(g.pose_fixed)
+    p = backend.CudaProblem(g, backend.OptimizationAlgorithmFactory.instance().construct("gn_cuda"))
+    p.build_system()
+    assert p.solve(0.0)[0] == status
