@@ -94,7 +94,7 @@ __device__ __forceinline__ void ba_edge_error(const BAVertices& V, int2 v, doubl
 
 // computeActiveErrors + activeChi2 / activeRobustChi2
 // (g2o/core/sparse_optimizer.cpp:78-130): partials[2*block] = (chi2, robust)
-static __global__ void ba_chi2_kernel(BAEdges E, BAVertices V, double* partials) {
+static __global__ void ba_chi2_kernel(BAEdges E, BAVertices V, double* partials, GridSum G) {
   double c = 0.0, r = 0.0;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < E.n; k += gridDim.x * blockDim.x) {
     double e[2], Xc[3], chi2, w;
@@ -110,6 +110,7 @@ static __global__ void ba_chi2_kernel(BAEdges E, BAVertices V, double* partials)
     }
   }
   block_sum2(c, r, partials + 2 * blockIdx.x);
+  grid_sum2(partials, G);
 }
 
 // ------------------------------------------------------- structure only
@@ -1253,7 +1254,9 @@ __global__ void __launch_bounds__(THREADS) ba_resid64_camera(BACamEdges CE, BAVe
 // SparseOptimizer::update (sparse_optimizer.cpp:457-468) with
 // VertexSE3Expmap::oplusImpl (g2o/types/sba/vertex_se3_expmap.cpp:48-51):
 // T <- exp(dx) * T; VertexPointXYZ: p <- p + dx (vertex_pointxyz.h:47-50)
-static __global__ void ba_oplus(BAVertices V, int Cf, int Pf, const double* x, int* nonfinite) {
+// cam_bak / pt_bak (nullptr: none): the estimates before the update
+static __global__ void ba_oplus(BAVertices V, int Cf, int Pf, const double* x, int* nonfinite, double* cam_bak,
+                                double* pt_bak) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < Cf) {
     double u[6];
@@ -1265,6 +1268,11 @@ static __global__ void ba_oplus(BAVertices V, int Cf, int Pf, const double* x, i
     }
     if (bad) *nonfinite = 1;
     double* cam = V.cam + (size_t)V.free_pose[t] * 8;
+    if (cam_bak) {
+      double* s = cam_bak + (size_t)V.free_pose[t] * 8;
+#pragma unroll
+      for (int i = 0; i < 7; ++i) s[i] = cam[i];
+    }
     SE3Q<double> T;
     T.q = Q4<double>{cam[0], cam[1], cam[2], cam[3]};
     T.t[0] = cam[4]; T.t[1] = cam[5]; T.t[2] = cam[6];
@@ -1276,6 +1284,12 @@ static __global__ void ba_oplus(BAVertices V, int Cf, int Pf, const double* x, i
     double* p = V.pt + (size_t)V.free_point[l] * 4;
     const double* u = x + (size_t)Cf * 6 + (size_t)l * 3;
     if (!isfinite(u[0]) || !isfinite(u[1]) || !isfinite(u[2])) *nonfinite = 1;
+    if (pt_bak) {
+      double* s = pt_bak + (size_t)V.free_point[l] * 4;
+      s[0] = p[0];
+      s[1] = p[1];
+      s[2] = p[2];
+    }
     p[0] += u[0];
     p[1] += u[1];
     p[2] += u[2];

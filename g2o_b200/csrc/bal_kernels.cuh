@@ -163,7 +163,7 @@ __device__ __forceinline__ void bal_edge(const BAVertices& V, int2 v, double2 z,
 
 // computeActiveErrors + activeChi2 / activeRobustChi2
 // (g2o/core/sparse_optimizer.cpp:78-130): partials[2*block] = (chi2, robust)
-static __global__ void bal_chi2_kernel(BAEdges E, BAVertices V, double* partials) {
+static __global__ void bal_chi2_kernel(BAEdges E, BAVertices V, double* partials, GridSum G) {
   double c = 0.0, r = 0.0;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < E.n; k += gridDim.x * blockDim.x) {
     double e[2], chi2, w;
@@ -179,6 +179,7 @@ static __global__ void bal_chi2_kernel(BAEdges E, BAVertices V, double* partials
     }
   }
   block_sum2(c, r, partials + 2 * blockIdx.x);
+  grid_sum2(partials, G);
 }
 
 // per-edge errors (parity hook)
@@ -927,18 +928,26 @@ static __global__ void bal_backsub_warp(const int* e_hpl, const int* hpl_row, co
 
 // VertexCameraBAL::oplusImpl / VertexPointBAL::oplusImpl
 // (bal_example.cpp:88-91, 116-119): estimate += update
-static __global__ void bal_oplus(BAVertices V, int Cf, int Pf, const double* x, int* nonfinite) {
+// cam_bak / pt_bak (nullptr: none): the estimates before the update
+static __global__ void bal_oplus(BAVertices V, int Cf, int Pf, const double* x, int* nonfinite, double* cam_bak,
+                                 double* pt_bak) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < Cf * 9) {
     const int h = t / 9, d = t % 9;
     const double u = x[t];
     if (!isfinite(u)) *nonfinite = 1;
-    V.cam[(size_t)V.free_pose[h] * kBalCam + d] += u;
+    const size_t o = (size_t)V.free_pose[h] * kBalCam + d;
+    const double v = V.cam[o];
+    if (cam_bak) cam_bak[o] = v;
+    V.cam[o] = v + u;
   } else if (t < Cf * 9 + Pf * 3) {
     const int q = t - Cf * 9, l = q / 3, d = q % 3;
     const double u = x[t];
     if (!isfinite(u)) *nonfinite = 1;
-    V.pt[(size_t)V.free_point[l] * 4 + d] += u;
+    const size_t o = (size_t)V.free_point[l] * 4 + d;
+    const double v = V.pt[o];
+    if (pt_bak) pt_bak[o] = v;
+    V.pt[o] = v + u;
   }
 }
 

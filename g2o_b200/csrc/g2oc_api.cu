@@ -5,6 +5,7 @@
 // kernels of ba_kernels.cuh, pg_kernels.cuh, pcg_kernels.cuh,
 // lm_kernels.cuh and cholesky.cuh.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdlib>
@@ -89,7 +90,7 @@ struct EngineBase {
   // dst = Hpp src over the Hessian-order vector (landmark part of dst zero):
   // BlockSolver::multiplyHessian (g2o/core/block_solver.h:96)
   virtual int multiply_hessian(const double* src, double* dst) = 0;
-  virtual int solve(double lambda) = 0;  // -> x, sc.solve_ok (PCG iterations: PcgState::total_iterations)
+  virtual int solve(double lambda) = 0;  // -> x, g2oc_ctx::solve_ok (PCG iterations: PcgState::total_iterations)
   virtual int get_hessian(double* hpp, double* hll, double* hpl) = 0;
   virtual int schur_export(double lambda, double* S, double* bs) = 0;
   // Gauss-Newton solve H x = rhs (lambda 0) with a given device right-hand
@@ -108,16 +109,27 @@ struct EngineBase {
 enum KernelId {
   K_CHI2, K_ERRORS, K_JACOBIANS, K_LANDMARK_PASS, K_CAMERA_PASS, K_SCHUR_LANDMARK, K_SCHUR_BLOCKS, K_SCHUR_RHS,
   K_BACKSUB, K_RESID_CAM, K_RESID_LM, K_OPLUS, K_MAX_DIAG, K_PCG_DIAG_INV, K_PCG_INIT, K_PCG_SPMV, K_PCG_UPDATE,
-  K_PCG_CHECK, K_PG_LINEARIZE, K_PG_ASSEMBLE_H, K_PG_ASSEMBLE_B, K_DAMP, K_LM_CONTROL, K_REDUCE, K_AXPY,
+  K_PCG_CHECK, K_PG_LINEARIZE, K_PG_ASSEMBLE, K_DAMP, K_LM_CONTROL, K_REDUCE, K_AXPY,
   K_CHOLESKY, K_PCG_COLPASS, K_SCHUR_DB, K_IO, K_PCG_SOLVE, K_PCG_TILES, K_TILE_COPY, K_BACKWARD, K_PG_RESID,
   K_TC_EXPAND, K_TC_POTRF, K_TC_TILES, K_TC_SOLVE, K_COUNT
 };
 static const char* kKernelNames[K_COUNT] = {
   "chi2", "errors", "jacobians", "ba_landmark_pass", "ba_camera_pass", "schur_landmark", "schur_blocks",
   "schur_rhs", "ba_backsub", "ba_resid_cam", "ba_resid_lm", "oplus", "max_diag", "pcg_diag_inv", "pcg_init",
-  "pcg_spmv", "pcg_update", "pcg_check_dn", "pg_linearize", "pg_assemble_h", "pg_assemble_b", "damp_diag",
+  "pcg_spmv", "pcg_update", "pcg_check_dn", "pg_linearize", "pg_assemble", "damp_diag",
   "lm_control", "reduce", "axpy", "cholesky", "pcg_colpass", "schur_db", "io_reorder", "pcg_solve", "pcg_solve_tiles",
   "sys_to_tiles", "ba_backward", "pg_resid64", "tc_expand", "tc_potrf", "tc_tiles", "tc_solve"};
+
+// control state of both kinds in one allocation: one read-back for both
+struct DevState {
+  DevScalars sc;
+  PcgState pcg;
+};
+static_assert(sizeof(DevState) % 8 == 0, "published in 8-byte words");
+struct HostState {
+  DevState s;
+  unsigned seq;
+};
 
 struct PendingTiming {
   int kid;
@@ -176,6 +188,7 @@ struct g2oc_ctx {
   double4 om_const = {0.0, 0.0, 0.0, 0.0};
   // vertex state
   g2oc::DBuf<double> pose, point, pose_bak, point_bak, pose_init, point_init;
+  bool bak_fixed = false;  // the backups hold the vertices that no step changes
   g2oc::DBuf<int> oplus_count, free_pose, free_point, pose_h, point_l;
   // BA edges
   g2oc::DBuf<int2> e_v, c_v;
@@ -214,8 +227,8 @@ struct g2oc_ctx {
   g2oc::PinnedVec<int32_t> pk_ev;
   // the LM / PCG state read once per trial: page-locked, so the copy is a DMA
   // the host can poll for
-  g2oc::PinnedVec<g2oc::DevScalars> h_sc;
-  g2oc::PinnedVec<g2oc::PcgState> h_pcg;
+  g2oc::PinnedVec<g2oc::HostState> h_dev;
+  unsigned seq = 0;  // publications asked for
   cudaEvent_t ev_read = nullptr;
   cudaEvent_t coop_done = nullptr;  // completion of this context's last grid-barrier launch
   // Dogleg state (OptimizationAlgorithmDogleg's members) and its vectors
@@ -245,8 +258,9 @@ struct g2oc_ctx {
   g2oc::WinDev windev() const {
     return g2oc::WinDev{nw, win_cam.p, win_lm.p, win_edge.p, win_pose.p, win_point.p, win_mat.p};
   }
-  g2oc::DBuf<g2oc::DevScalars> sc;
-  g2oc::DBuf<g2oc::PcgState> pcg;
+  g2oc::DBuf<g2oc::DevState> dev;
+  struct { g2oc::DevScalars* p = nullptr; } sc;  // its parts
+  struct { g2oc::PcgState* p = nullptr; } pcg;
   g2oc::DBuf<int> flag;  // nonfinite flag
   // the caller's arrays as copied (g2oc_graph layout), reordered on the device
   g2oc::DBuf<double> raw_meas, raw_info, raw_delta, raw_pose, raw_point;
@@ -265,6 +279,7 @@ struct g2oc_ctx {
   std::unique_ptr<g2oc::CholPlan> chol;
   long long pcg_seen = 0;        // PcgState::total_iterations at the last read
   double lambda_host = 0.0;      // the device's LM lambda as of the last read
+  int solve_ok = 1;              // outcome of the last solve; -1: it is in sc.solve_ok on the device
   bool chi2_carry = false;       // chi2_current / chi2_plain hold the current estimates' values
   g2oc_iteration_stats* cur_stats = nullptr;  // stats of the iteration in progress
   double last_refine_dn = 0.0;
@@ -297,6 +312,7 @@ struct g2oc_ctx {
     cudaEvent_t a, b;
     double* out;
     double* out2;
+    bool own_b;  // b is not the start of the next span
   };
   std::vector<Span> spans;
   cudaEvent_t mark() {
@@ -304,30 +320,41 @@ struct g2oc_ctx {
     cudaEventRecord(e, stream);
     return e;
   }
-  void span(cudaEvent_t a, double* out, double* out2 = nullptr) { spans.push_back({a, mark(), out, out2}); }
+  void span(cudaEvent_t a, double* out, double* out2 = nullptr) { spans.push_back({a, mark(), out, out2, true}); }
+  // a span whose end is the start of the next one
+  cudaEvent_t lap(cudaEvent_t a, double* out) {
+    cudaEvent_t b = mark();
+    spans.push_back({a, b, out, nullptr, false});
+    return b;
+  }
   // forget the recorded spans without writing their times: after a call that
   // failed half-way their targets (the call's own stats) no longer exist
   void drop_spans() {
     for (auto& sp : spans) {
       event_pool.push_back(sp.a);
-      event_pool.push_back(sp.b);
+      if (sp.own_b) event_pool.push_back(sp.b);
     }
     spans.clear();
+    spans_ended = 0;
     cur_stats = nullptr;
   }
-  void resolve_spans() {
-    if (spans.empty()) return;
-    cudaEventSynchronize(spans.back().b);
-    for (auto& sp : spans) {
+  size_t spans_ended = 0;  // the spans of iterations that are over
+  void resolve_spans(size_t count) {
+    if (count == 0) return;
+    cudaEventSynchronize(spans[count - 1].b);
+    for (size_t i = 0; i < count; ++i) {
+      const Span& sp = spans[i];
       float ms = 0.f;
       cudaEventElapsedTime(&ms, sp.a, sp.b);
       if (sp.out) *sp.out += ms * 1e-3;
       if (sp.out2) *sp.out2 -= ms * 1e-3;
       event_pool.push_back(sp.a);
-      event_pool.push_back(sp.b);
+      if (sp.own_b) event_pool.push_back(sp.b);
     }
-    spans.clear();
+    spans.erase(spans.begin(), spans.begin() + count);
+    spans_ended = 0;
   }
+  void resolve_spans() { resolve_spans(spans.size()); }
   void flush_timing() {
     if (pending.empty()) return;
     cudaEventSynchronize(pending.back().b);
@@ -826,10 +853,7 @@ struct Engine final : EngineBase {
                                                                         hcontrib.p, bcontrib.p);
         G2OC_LAUNCH_CHECK();
         const int nnzb = (int)S.hpp_rc.size() / 2;
-        G2OC_K(K_PG_ASSEMBLE_H) pg_assemble_h<Real, 3><<<cdiv((long long)nnzb * 3, 128), 128, 0, st>>>(nnzb, c->hb_src_ptr.p, c->hb_src.p,
-                                                                               hcontrib.p, hpp.p);
-        G2OC_K(K_PG_ASSEMBLE_B) pg_assemble_b<3><<<cdiv((long long)S.Cf * 3, 128), 128, 0, st>>>(S.Cf, c->bv_src_ptr.p, c->bv_src.p,
-                                                                       bcontrib.p, c->b.p);
+        assemble<3>(nnzb, hpp.p, c->b.p);
       } else {
         if (S.pose_type == G2OC_POSE_SE3EXPMAP)
           G2OC_K(K_PG_LINEARIZE) pg_linearize<Real, G2OC_POSE_SE3EXPMAP><<<cdiv(n, 64), 64, 0, st>>>(
@@ -839,15 +863,20 @@ struct Engine final : EngineBase {
               c->pose.p, c->pg_edges(), c->pe_trans.p, hcontrib.p, bcontrib.p);
         G2OC_LAUNCH_CHECK();
         const int nnzb = (int)S.hpp_rc.size() / 2;
-        G2OC_K(K_PG_ASSEMBLE_H) pg_assemble_h<Real, 6><<<cdiv((long long)nnzb * 6, 128), 128, 0, st>>>(nnzb, c->hb_src_ptr.p, c->hb_src.p,
-                                                                               hcontrib.p, hpp.p);
-        G2OC_K(K_PG_ASSEMBLE_B) pg_assemble_b<6><<<cdiv((long long)S.Cf * 6, 128), 128, 0, st>>>(S.Cf, c->bv_src_ptr.p, c->bv_src.p,
-                                                                       bcontrib.p, c->b.p);
+        assemble<6>(nnzb, hpp.p, c->b.p);
       }
       G2OC_LAUNCH_CHECK();
     }
     if (S.ba && c->pose_edges()) G2OC_TRY(pose_edge_system());
     return G2OC_OK;
+  }
+
+  // the edge contributions summed per block and per vertex
+  template <int D>
+  void assemble(int nblk, Real* h, double* b) {
+    const int hb = cdiv((long long)nblk * D, 128), bb = cdiv((long long)c->S.Cf * D, 128);
+    G2OC_K(K_PG_ASSEMBLE) pg_assemble<Real, D><<<hb + bb, 128, 0, c->stream>>>(
+        hb, nblk, c->hb_src_ptr.p, c->hb_src.p, hcontrib.p, h, c->S.Cf, c->bv_src_ptr.p, c->bv_src.p, bcontrib.p, b);
   }
 
   // The pose edge set's part of buildSystem: the pose-graph kernels' edge
@@ -864,12 +893,9 @@ struct Engine final : EngineBase {
         c->pgpose.p, c->ba_pose_edges(), c->pe_trans.p, hcontrib.p, bcontrib.p);
     G2OC_LAUNCH_CHECK();
     const int nblk = S.Cf + S.npp;
-    G2OC_K(K_PG_ASSEMBLE_H) pg_assemble_h<Real, 6><<<cdiv((long long)nblk * 6, 128), 128, 0, st>>>(
-        nblk, c->hb_src_ptr.p, c->hb_src.p, hcontrib.p, phpp.p);
-    G2OC_K(K_PG_ASSEMBLE_B) pg_assemble_b<6><<<cdiv((long long)S.Cf * 6, 128), 128, 0, st>>>(
-        S.Cf, c->bv_src_ptr.p, c->bv_src.p, bcontrib.p, pb.p);
+    assemble<6>(nblk, phpp.p, pb.p);
     const long long tot = (long long)nblk * 36 + (long long)S.Cf * 6;
-    G2OC_K(K_PG_ASSEMBLE_H) ba_add_pose_system<Real><<<cdiv(tot, 256), 256, 0, st>>>(S.Cf, S.npp, phpp.p, hpp.p,
+    G2OC_K(K_PG_ASSEMBLE) ba_add_pose_system<Real><<<cdiv(tot, 256), 256, 0, st>>>(S.Cf, S.npp, phpp.p, hpp.p,
                                                                                       pb.p, c->b.p);
     G2OC_LAUNCH_CHECK();
     return G2OC_OK;
@@ -1190,7 +1216,7 @@ struct Engine final : EngineBase {
     const Structure& S = c->S;
     cudaStream_t st = c->stream;
     int ok = 1;
-    bool decided = false;  // the Cholesky sets sc.solve_ok itself
+    bool decided = false;  // the Cholesky leaves its outcome in sc.solve_ok
     const bool use_chol = c->prm.linear_solver == G2OC_LINEAR_CHOLESKY ||
                           (c->prm.linear_solver == 2 && !S.ba);
     if (S.Cf == 0) {
@@ -1226,15 +1252,14 @@ struct Engine final : EngineBase {
       const bool tc_chol = use_chol && tc_chol_used();
       if (tc_chol) {
         G2OC_TRY(tc_factor(&ok));
-        G2OC_TRY(tc_resolve(c->rhs.p, c->xs.p));
+        G2OC_TRY(tc_resolve(c->rhs.p, c->x.p));
       } else if (use_chol) {
-        G2OC_TRY(chol_solve(Sval.p, c->rhs.p, c->xs.p));
+        G2OC_TRY(chol_solve(Sval.p, c->rhs.p, c->x.p));
         decided = true;
       } else {
-        G2OC_TRY(pcg_solve(Sval.p, c->rhs.p, c->xs.p, false));
+        G2OC_TRY(pcg_solve(Sval.p, c->rhs.p, c->x.p, false));
       }
-      G2OC_CUDA_TRY(cudaMemcpyAsync(c->x.p, c->xs.p, (size_t)S.Cf * 6 * sizeof(double), cudaMemcpyDeviceToDevice, st));
-      G2OC_TRY(backsub(bl, c->xs.p, c->x.p + (size_t)S.Cf * 6));
+      G2OC_TRY(backsub(bl, c->x.p, c->x.p + (size_t)S.Cf * 6));
       // mixed precision: FP64 iterative refinement on the true residual of
       // the damped normal equations, r = b - (J^T Om' J + lambda I) x, formed
       // matrix-free from the edges in FP64. A correction is solved (FP32
@@ -1345,10 +1370,7 @@ struct Engine final : EngineBase {
         G2OC_TRY(pcg_solve(sysval.p, c->b.p, c->x.p, false));
       }
     }
-    if (!decided) {
-      G2OC_K(K_LM_CONTROL) set_solve_ok<<<1, 32, 0, st>>>(c->sc.p, ok);
-      G2OC_LAUNCH_CHECK();
-    }
+    c->solve_ok = decided ? -1 : ok;
     return G2OC_OK;
   }
 
@@ -1843,24 +1865,19 @@ struct BalEngine final : EngineBase {
           P->extra = c->barrier_extra;
           c->chol = std::move(P);
         }
-        G2OC_TRY(chol_solve_async<double>(*c->chol, st, A, c->rhs.p, c->xs.p, &c->kcount[K_CHOLESKY], c->sc.p));
+        G2OC_TRY(chol_solve_async<double>(*c->chol, st, A, c->rhs.p, c->x.p, &c->kcount[K_CHOLESKY], c->sc.p));
         decided = true;
       } else {
         G2OC_K(K_PCG_DIAG_INV) pcg_diag_inv_lanes<double, 9><<<cdiv(A.nb, 3 * 4), 128, 0, st>>>(A, minv.p,
                                                                                              c->flag.p);
         G2OC_LAUNCH_CHECK();
-        const int rc = run_pcg_persistent<double, 9>(c, A, minv.p, c->rhs.p, c->xs.p, r.p, s.p, d.p, tbuf.p,
+        const int rc = run_pcg_persistent<double, 9>(c, A, minv.p, c->rhs.p, c->x.p, r.p, s.p, d.p, tbuf.p,
                                                      cpart.p, false);
         if (rc != G2OC_OK) return rc;
       }
-      G2OC_CUDA_TRY(cudaMemcpyAsync(c->x.p, c->xs.p, (size_t)S.Cf * 9 * sizeof(double), cudaMemcpyDeviceToDevice,
-                                    st));
-      G2OC_TRY(backsub(bl, c->xs.p, c->x.p + (size_t)S.Cf * 9));
+      G2OC_TRY(backsub(bl, c->x.p, c->x.p + (size_t)S.Cf * 9));
     }
-    if (!decided) {
-      G2OC_K(K_LM_CONTROL) set_solve_ok<<<1, 32, 0, st>>>(c->sc.p, 1);
-      G2OC_LAUNCH_CHECK();
-    }
+    c->solve_ok = decided ? -1 : 1;
     return G2OC_OK;
   }
 
@@ -1926,49 +1943,100 @@ struct BalEngine final : EngineBase {
 };
 
 // ------------------------------------------------------------ driver ops
-static int chi2_to(g2oc_ctx* c, double* out_plain, double* out_robust) {
+static int ensure_read(g2oc_ctx* c) {
+  if (c->ev_read) return G2OC_OK;
+  G2OC_TRY(c->h_dev.resize(1));
+  memset(c->h_dev.data(), 0, sizeof(HostState));
+  c->seq = 0;
+  G2OC_CUDA_TRY(cudaEventCreateWithFlags(&c->ev_read, cudaEventDisableTiming));
+  return G2OC_OK;
+}
+
+// the record of a kernel that ends by sending the control state to the host
+static int next_publish(g2oc_ctx* c, Publish* p) {
+  G2OC_TRY(ensure_read(c));
+  HostState* h = c->h_dev.data();
+  *p = Publish{reinterpret_cast<const unsigned long long*>(c->dev.p), reinterpret_cast<unsigned long long*>(&h->s),
+               (int)(sizeof(DevState) / 8), ++c->seq, &h->seq};
+  return G2OC_OK;
+}
+
+// chi2 and robust chi2 of the estimates, one partial per block; finish: also
+// their sums, into out_plain and out_robust, and over the ranks; published:
+// the kernel is to send the control state to the host too, set to whether it
+// does. Returns the number of partials in *nparts
+static int chi2_pass(g2oc_ctx* c, bool finish, double* out_plain, double* out_robust, int* nparts, bool* published) {
   const Structure& S = c->S;
   cudaStream_t st = c->stream;
+  const bool extra = S.ba && c->pose_edges();  // a second kernel's partials follow
+  GridSum G{finish && !extra ? &c->sc.p->ticket : nullptr, out_plain, out_robust, Publish{}};
+  if (published) {
+    *published = G.ticket && c->shard_world <= 1;
+    if (*published) G2OC_TRY(next_publish(c, &G.publish));
+  }
+  // a block per 256 edges (128 threads where the edge takes more registers),
+  // up to the grids that fill the GPU; the edges of a thread do not depend on it
+  const int threads = S.ba || S.pose_type == G2OC_POSE_SE2 ? 256 : 128;
+  const int grid = std::max(1, std::min(S.ba ? kChi2Blocks : kRedBlocks, cdiv((long long)S.act.size(), threads)));
   if (S.bal)
-    G2OC_K(K_CHI2) bal_chi2_kernel<<<kChi2Blocks, 256, 0, st>>>(c->ba_edges(), c->ba_vertices(), c->partials.p);
+    G2OC_K(K_CHI2) bal_chi2_kernel<<<grid, threads, 0, st>>>(c->ba_edges(), c->ba_vertices(), c->partials.p, G);
   else if (S.ba && S.D == 3)
-    G2OC_K(K_CHI2) st_chi2_kernel<<<kChi2Blocks, 256, 0, st>>>(c->ba_edges(), c->ba_vertices(), c->partials.p);
-  else if (S.ba) G2OC_K(K_CHI2) ba_chi2_kernel<<<kChi2Blocks, 256, 0, st>>>(c->ba_edges(), c->ba_vertices(), c->partials.p);
+    G2OC_K(K_CHI2) st_chi2_kernel<<<grid, threads, 0, st>>>(c->ba_edges(), c->ba_vertices(), c->partials.p, G);
+  else if (S.ba)
+    G2OC_K(K_CHI2) ba_chi2_kernel<<<grid, threads, 0, st>>>(c->ba_edges(), c->ba_vertices(), c->partials.p, G);
   else if (S.pose_type == G2OC_POSE_SE2)
-    G2OC_K(K_CHI2) pg_chi2_kernel<G2OC_POSE_SE2><<<kRedBlocks, 256, 0, st>>>(c->pose.p, c->pg_edges(), c->partials.p);
+    G2OC_K(K_CHI2) pg_chi2_kernel<G2OC_POSE_SE2><<<grid, threads, 0, st>>>(c->pose.p, c->pg_edges(), c->partials.p, G);
   else if (S.pose_type == G2OC_POSE_SE3EXPMAP)
-    G2OC_K(K_CHI2) pg_chi2_kernel<G2OC_POSE_SE3EXPMAP><<<kRedBlocks, 128, 0, st>>>(c->pose.p, c->pg_edges(), c->partials.p);
-  else G2OC_K(K_CHI2) pg_chi2_kernel<G2OC_POSE_SE3><<<kRedBlocks, 128, 0, st>>>(c->pose.p, c->pg_edges(), c->partials.p);
+    G2OC_K(K_CHI2) pg_chi2_kernel<G2OC_POSE_SE3EXPMAP><<<grid, threads, 0, st>>>(c->pose.p, c->pg_edges(),
+                                                                                c->partials.p, G);
+  else
+    G2OC_K(K_CHI2) pg_chi2_kernel<G2OC_POSE_SE3><<<grid, threads, 0, st>>>(c->pose.p, c->pg_edges(), c->partials.p, G);
   G2OC_LAUNCH_CHECK();
-  int nparts = S.ba ? kChi2Blocks : kRedBlocks;
-  if (S.ba && c->pose_edges()) {
+  *nparts = grid;
+  if (extra) {
     // the pose edge set's chi2 in the partials after the projection edges'
     G2OC_K(K_CHI2) ba_unpack_poses<<<cdiv((long long)S.C * 7, 256), 256, 0, st>>>(S.C, c->pose.p, c->pgpose.p);
-    G2OC_K(K_CHI2) pg_chi2_kernel<G2OC_POSE_SE3EXPMAP><<<kRedBlocks, 128, 0, st>>>(c->pgpose.p, c->ba_pose_edges(),
-                                                                                 c->partials.p + 2 * nparts);
+    G2OC_K(K_CHI2) pg_chi2_kernel<G2OC_POSE_SE3EXPMAP><<<kRedBlocks, 128, 0, st>>>(
+        c->pgpose.p, c->ba_pose_edges(), c->partials.p + 2 * grid, GridSum{});
     G2OC_LAUNCH_CHECK();
-    nparts += kRedBlocks;
+    *nparts += kRedBlocks;
   }
-  G2OC_TRY(finalize_sum(c, nparts, 2, out_plain, out_robust));
+  if (!finish) return G2OC_OK;
+  if (extra) G2OC_TRY(finalize_sum(c, *nparts, 2, out_plain, out_robust));
   G2OC_TRY(shard_reduce(c, out_plain, 1, G2OC_DT_F64, G2OC_RED_SUM));
   return shard_reduce(c, out_robust, 1, G2OC_DT_F64, G2OC_RED_SUM);
 }
 
-static int oplus(g2oc_ctx* c) {
+static int chi2_to(g2oc_ctx* c, double* out_plain, double* out_robust) {
+  int nparts = 0;
+  return chi2_pass(c, true, out_plain, out_robust, &nparts, nullptr);
+}
+
+static bool solve_succeeded(const g2oc_ctx* c, const DevScalars& h) {
+  return c->solve_ok < 0 ? h.solve_ok != 0 : c->solve_ok != 0;
+}
+
+// x <- x [+] dx; backup: the free vertices' estimates before it go to the
+// backups, with which those hold what pop() restores
+static int oplus(g2oc_ctx* c, bool backup) {
   const Structure& S = c->S;
   cudaStream_t st = c->stream;
+  double* pose_bak = backup ? c->pose_bak.p : nullptr;
+  double* point_bak = backup ? c->point_bak.p : nullptr;
   if (S.bal)
     G2OC_K(K_OPLUS) bal_oplus<<<cdiv((long long)S.Cf * 9 + (long long)S.Pf * 3, 256), 256, 0, st>>>(
-        c->ba_vertices(), S.Cf, S.Pf, c->x.p, c->flag.p);
-  else if (S.ba) G2OC_K(K_OPLUS) ba_oplus<<<cdiv(S.Cf + S.Pf, 256), 256, 0, st>>>(c->ba_vertices(), S.Cf, S.Pf, c->x.p, c->flag.p);
+        c->ba_vertices(), S.Cf, S.Pf, c->x.p, c->flag.p, pose_bak, point_bak);
+  else if (S.ba)
+    G2OC_K(K_OPLUS) ba_oplus<<<cdiv(S.Cf + S.Pf, 256), 256, 0, st>>>(c->ba_vertices(), S.Cf, S.Pf, c->x.p, c->flag.p,
+                                                                     pose_bak, point_bak);
   else if (S.pose_type == G2OC_POSE_SE2)
     G2OC_K(K_OPLUS) pg_oplus<G2OC_POSE_SE2><<<cdiv(S.Cf, 128), 128, 0, st>>>(c->pose.p, c->free_pose.p, S.Cf, c->x.p,
-                                                             c->oplus_count.p, c->flag.p);
+                                                             c->oplus_count.p, c->flag.p, pose_bak);
   else if (S.pose_type == G2OC_POSE_SE3EXPMAP)
     G2OC_K(K_OPLUS) pg_oplus<G2OC_POSE_SE3EXPMAP><<<cdiv(S.Cf, 128), 128, 0, st>>>(c->pose.p, c->free_pose.p, S.Cf,
-                                                                                  c->x.p, c->oplus_count.p, c->flag.p);
+                                                                                  c->x.p, c->oplus_count.p, c->flag.p, pose_bak);
   else G2OC_K(K_OPLUS) pg_oplus<G2OC_POSE_SE3><<<cdiv(S.Cf, 128), 128, 0, st>>>(c->pose.p, c->free_pose.p, S.Cf, c->x.p,
-                                                                c->oplus_count.p, c->flag.p);
+                                                                c->oplus_count.p, c->flag.p, pose_bak);
   G2OC_LAUNCH_CHECK();
   return G2OC_OK;
 }
@@ -1977,6 +2045,7 @@ static int push(g2oc_ctx* c) {
   G2OC_CUDA_TRY(cudaMemcpyAsync(c->pose_bak.p, c->pose.p, c->pose.bytes(), cudaMemcpyDeviceToDevice, c->stream));
   if (c->point.n)
     G2OC_CUDA_TRY(cudaMemcpyAsync(c->point_bak.p, c->point.p, c->point.bytes(), cudaMemcpyDeviceToDevice, c->stream));
+  c->bak_fixed = true;
   return G2OC_OK;
 }
 
@@ -1990,25 +2059,43 @@ static int pop(g2oc_ctx* c) {
 static int reset_pcg(g2oc_ctx* c);
 
 // DevScalars and PcgState after the queued work (the one wait of an LM
-// trial): PCG iterations since the last read go to stv
-static int read_state(g2oc_ctx* c, DevScalars* h, g2oc_iteration_stats* stv) {
-  if (!c->ev_read) {
-    G2OC_TRY(c->h_sc.resize(1));
-    G2OC_TRY(c->h_pcg.resize(1));
-    G2OC_CUDA_TRY(cudaEventCreateWithFlags(&c->ev_read, cudaEventDisableTiming));
+// trial): PCG iterations since the last read go to stv. published: the last
+// kernel queued sends them (next_publish), else they are copied. The phase
+// times of the iteration before are taken while the GPU works.
+static int read_state(g2oc_ctx* c, DevScalars* h, g2oc_iteration_stats* stv, bool published = false) {
+  G2OC_TRY(ensure_read(c));
+  if (!published) {
+    G2OC_CUDA_TRY(
+        cudaMemcpyAsync(&c->h_dev.data()->s, c->dev.p, sizeof(DevState), cudaMemcpyDeviceToHost, c->stream));
+    G2OC_CUDA_TRY(cudaEventRecord(c->ev_read, c->stream));
   }
-  G2OC_CUDA_TRY(cudaMemcpyAsync(c->h_sc.data(), c->sc.p, sizeof(DevScalars), cudaMemcpyDeviceToHost, c->stream));
-  G2OC_CUDA_TRY(cudaMemcpyAsync(c->h_pcg.data(), c->pcg.p, sizeof(PcgState), cudaMemcpyDeviceToHost, c->stream));
-  G2OC_CUDA_TRY(cudaEventRecord(c->ev_read, c->stream));
+  c->resolve_spans(c->spans_ended);
   // the host polls (the trial's work is a few hundred microseconds at most;
   // a blocking wait would add its wake-up latency to every trial)
-  cudaError_t q;
-  while ((q = cudaEventQuery(c->ev_read)) == cudaErrorNotReady) {
+  if (published) {
+    volatile unsigned* seq = &c->h_dev.data()->seq;
+    for (unsigned n = 1; *seq != c->seq; ++n) {
+      if (n & 4095u) continue;
+      const cudaError_t q = cudaStreamQuery(c->stream);
+      if (q == cudaErrorNotReady) {
+        cudaGetLastError();  // not an error of later launches
+        continue;
+      }
+      G2OC_CUDA_TRY(q);
+      if (*seq == c->seq) break;
+      set_error("the control state did not arrive");
+      return G2OC_ERR_CUDA;
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+  } else {
+    cudaError_t q;
+    while ((q = cudaEventQuery(c->ev_read)) == cudaErrorNotReady) {
+    }
+    G2OC_CUDA_TRY(q);
+    cudaGetLastError();  // the not-ready answers are not errors of later launches
   }
-  G2OC_CUDA_TRY(q);
-  cudaGetLastError();  // the not-ready answers are not errors of later launches
-  *h = *c->h_sc.data();
-  const PcgState ps = *c->h_pcg.data();
+  *h = c->h_dev.data()->s.sc;
+  const PcgState ps = c->h_dev.data()->s.pcg;
   if (ps.sync_error) {
     G2OC_TRY(reset_pcg(c));
     set_error("PCG: a grid barrier wait ran out");
@@ -2035,8 +2122,8 @@ static int lm_iteration(g2oc_ctx* c, int iteration, g2oc_iteration_stats* stv, i
   c->cur_stats = stv;
   cudaEvent_t t0 = c->mark();
   if (!c->chi2_carry) G2OC_TRY(chi2_to(c, &sc->chi2_plain, &sc->chi2_current));
-  c->span(t0, &stv->time_residuals);
-  t0 = c->mark();
+  c->chi2_carry = false;
+  t0 = c->lap(t0, &stv->time_residuals);
   G2OC_TRY(c->eng->build_system());
   c->system_built = true;
   c->span(t0, &stv->time_quadratic_form);
@@ -2052,28 +2139,35 @@ static int lm_iteration(g2oc_ctx* c, int iteration, g2oc_iteration_stats* stv, i
   int qmax = 0;
   bool accepted = false;
   do {
-    G2OC_TRY(push(c));
+    if (!c->bak_fixed) G2OC_TRY(push(c));
     t0 = c->mark();
     G2OC_TRY(c->eng->solve(c->lambda_host));
-    c->span(t0, &stv->time_linear_solver);
-    t0 = c->mark();
-    G2OC_TRY(oplus(c));
+    t0 = c->lap(t0, &stv->time_linear_solver);
+    G2OC_TRY(oplus(c, true));
     c->span(t0, &stv->time_update);
-    G2OC_TRY(chi2_to(c, &sc->chi2_temp_plain, &sc->chi2_temp));
-    {
+    if (c->shard_world <= 1) {
+      int nchi = 0;
+      Publish P;
+      G2OC_TRY(chi2_pass(c, false, nullptr, nullptr, &nchi, nullptr));
+      G2OC_TRY(next_publish(c, &P));
+      G2OC_K(K_LM_CONTROL) lm_finish<<<std::max(1, std::min(kRedBlocks, cdiv(n, 256))), 256, 0, st>>>(
+          c->x.p, c->b.p, n, sc, c->partials.p, nchi, c->partials.p + 2 * nchi, c->solve_ok, P);
+      G2OC_LAUNCH_CHECK();
+    } else {
+      G2OC_TRY(chi2_to(c, &sc->chi2_temp_plain, &sc->chi2_temp));
       // sharded: the camera entries are the same on every rank, their lambda
       // term (and the 1e-3) counted on rank 0 only; b's camera part is each
       // rank's share
-      const bool other = c->shard_world > 1 && c->shard_rank != 0;
+      const bool other = c->shard_rank != 0;
       G2OC_K(K_LM_CONTROL) lm_scale_partials<<<kRedBlocks, 256, 0, st>>>(c->x.p, c->b.p, n, sc, c->partials.p,
                                                                          other ? c->S.Cf * 6 : 0);
       G2OC_LAUNCH_CHECK();
       G2OC_TRY(finalize_sum(c, kRedBlocks, 1, &sc->scale, nullptr, other ? 0.0 : 1e-3));
       G2OC_TRY(shard_reduce(c, &sc->scale, 1, G2OC_DT_F64, G2OC_RED_SUM));
+      G2OC_K(K_LM_CONTROL) lm_decide<<<1, 32, 0, st>>>(sc, c->solve_ok);
+      G2OC_LAUNCH_CHECK();
     }
-    G2OC_K(K_LM_CONTROL) lm_decide<<<1, 32, 0, st>>>(sc);
-    G2OC_LAUNCH_CHECK();
-    G2OC_TRY(read_state(c, &h, stv));
+    G2OC_TRY(read_state(c, &h, stv, c->shard_world <= 1));
     rho = h.rho;
     accepted = h.accept != 0;
     if (!accepted) {
@@ -2090,7 +2184,6 @@ static int lm_iteration(g2oc_ctx* c, int iteration, g2oc_iteration_stats* stv, i
   c->chi2_carry = accepted;
   stv->lambda = h.lambda;
   stv->chi2 = h.chi2_current;  // activeRobustChi2 of the state the iteration ends in (G2OBatchStatistics::chi2)
-  c->resolve_spans();
   c->cur_stats = nullptr;
   if (qmax == c->prm.max_trials_after_failure || rho == 0 || !std::isfinite(h.lambda)) *result = G2OC_RESULT_TERMINATE;
   else *result = G2OC_RESULT_OK;
@@ -2101,27 +2194,27 @@ static int lm_iteration(g2oc_ctx* c, int iteration, g2oc_iteration_stats* stv, i
 static int gn_iteration(g2oc_ctx* c, int iteration, g2oc_iteration_stats* stv, int* result) {
   (void)iteration;
   c->cur_stats = stv;
-  c->chi2_carry = false;
+  DevScalars* sc = c->sc.p;
   cudaEvent_t t0 = c->mark();
-  G2OC_TRY(chi2_to(c, &c->sc.p->chi2_plain, &c->sc.p->chi2_current));
-  c->span(t0, &stv->time_residuals);
-  t0 = c->mark();
+  if (!c->chi2_carry) G2OC_TRY(chi2_to(c, &sc->chi2_plain, &sc->chi2_current));
+  c->chi2_carry = false;
+  t0 = c->lap(t0, &stv->time_residuals);
   G2OC_TRY(c->eng->build_system());
   c->system_built = true;
-  c->span(t0, &stv->time_quadratic_form);
-  t0 = c->mark();
+  t0 = c->lap(t0, &stv->time_quadratic_form);
   G2OC_TRY(c->eng->solve(0.0));
-  c->span(t0, &stv->time_linear_solver);
-  t0 = c->mark();
-  G2OC_TRY(oplus(c));
+  t0 = c->lap(t0, &stv->time_linear_solver);
+  G2OC_TRY(oplus(c, false));
   c->span(t0, &stv->time_update);
-  G2OC_TRY(chi2_to(c, nullptr, &c->sc.p->chi2_temp));
+  int nparts = 0;
+  bool published = false;
+  G2OC_TRY(chi2_pass(c, true, &sc->chi2_plain, &sc->chi2_current, &nparts, &published));
   DevScalars h;
-  G2OC_TRY(read_state(c, &h, stv));
-  stv->chi2 = h.chi2_temp;  // activeRobustChi2 after the update (G2OBatchStatistics::chi2)
-  c->resolve_spans();
+  G2OC_TRY(read_state(c, &h, stv, published));
+  c->chi2_carry = true;  // the next iteration starts from these errors
+  stv->chi2 = h.chi2_current;  // activeRobustChi2 after the update (G2OBatchStatistics::chi2)
   c->cur_stats = nullptr;
-  *result = h.solve_ok ? G2OC_RESULT_OK : G2OC_RESULT_FAIL;
+  *result = solve_succeeded(c, h) ? G2OC_RESULT_OK : G2OC_RESULT_FAIL;
   return G2OC_OK;
 }
 
@@ -2198,7 +2291,7 @@ static int dl_iteration(g2oc_ctx* c, int iteration, g2oc_iteration_stats* stv, i
         G2OC_TRY(c->eng->solve(c->dl_was_pd ? 0.0 : c->dl_lambda));
         c->span(t0, &stv->time_linear_solver);
         G2OC_TRY(read_state(c, &h, stv));
-        ok = h.solve_ok != 0;
+        ok = solve_succeeded(c, h);
         c->dl_was_pd = c->dl_was_pd && ok;
         if (!c->dl_was_pd) {
           if (ok) {
@@ -2250,7 +2343,7 @@ static int dl_iteration(g2oc_ctx* c, int iteration, g2oc_iteration_stats* stv, i
     double linear_gain = -1 * hh + 2 * bh;
     G2OC_TRY(push(c));
     t0 = c->mark();
-    G2OC_TRY(oplus(c));
+    G2OC_TRY(oplus(c, false));
     c->span(t0, &stv->time_update);
     G2OC_TRY(chi2_to(c, &sc->chi2_temp_plain, &sc->chi2_temp));
     G2OC_TRY(read_state(c, &h, stv));
@@ -2485,8 +2578,9 @@ int g2oc_create(int device, g2oc_ctx** out) {
   if (const char* e = getenv("G2OC_TEST_BARRIER_EXTRA")) c->barrier_extra = atoi(e) > 0 ? 1u : 0u;
   G2OC_CUDA_TRY(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   g2oc_default_params(&c->prm);
-  G2OC_TRY(c->sc.alloc(1));
-  G2OC_TRY(c->pcg.alloc(1));
+  G2OC_TRY(c->dev.alloc(1));
+  c->sc.p = &c->dev.p->sc;
+  c->pcg.p = &c->dev.p->pcg;
   G2OC_TRY(c->flag.alloc(1));
   G2OC_TRY(c->partials.alloc(2 * 8192));
   G2OC_CUDA_TRY(cudaMemsetAsync(c->sc.p, 0, sizeof(DevScalars), c->stream));
@@ -2883,7 +2977,7 @@ static void drop_windows(g2oc_ctx* c) {
 
 int g2oc_upload(g2oc_ctx* c, const g2oc_graph* g) {
   G2OC_TRY(check_ctx(c, false));
-  c->chi2_carry = false;
+  c->chi2_carry = c->bak_fixed = false;
   drop_windows(c);
   if (!g) {
     set_error("graph is NULL");
@@ -2929,7 +3023,7 @@ int g2oc_get_hessian_info(g2oc_ctx* c, g2oc_hessian_info* info) {
 
 int g2oc_set_estimates(g2oc_ctx* c, const double* pose, const double* point) {
   G2OC_TRY(check_ctx(c, true));
-  c->chi2_carry = false;
+  c->chi2_carry = c->bak_fixed = false;
   const Structure& S = c->S;
   if (S.ba) {
     G2OC_TRY(upload_ba_estimates(c, pose, point));
@@ -3008,22 +3102,23 @@ static int optimize_impl(g2oc_ctx* c, int iterations, g2oc_iteration_stats* stat
   G2OC_TRY(reset_pcg(c));  // LinearSolverPCG::init via BlockSolver::init
   int result = G2OC_RESULT_OK;
   int it = 0;
+  g2oc_iteration_stats scratch;  // the phase times are written to stats[] an iteration late
   for (int i = 0; i < iterations && result == G2OC_RESULT_OK; ++i) {
-    g2oc_iteration_stats stv;
-    memset(&stv, 0, sizeof(stv));
+    g2oc_iteration_stats* stv = stats ? stats + i : &scratch;
+    memset(stv, 0, sizeof(*stv));
     cudaEvent_t t0 = c->mark();
-    if (c->prm.algorithm == G2OC_ALGO_LEVENBERG) G2OC_TRY(lm_iteration(c, i, &stv, &result));
-    else if (c->prm.algorithm == G2OC_ALGO_DOGLEG) G2OC_TRY(dl_iteration(c, i, &stv, &result));
-    else if (c->prm.algorithm == G2OC_ALGO_STRUCTURE_ONLY) G2OC_TRY(so_iteration(c, &stv, &result));
-    else G2OC_TRY(gn_iteration(c, i, &stv, &result));
-    stv.iteration = i;
-    stv.result = result;
-    c->span(t0, &stv.time_iteration);
-    c->resolve_spans();
-    if (stats) stats[i] = stv;
+    if (c->prm.algorithm == G2OC_ALGO_LEVENBERG) G2OC_TRY(lm_iteration(c, i, stv, &result));
+    else if (c->prm.algorithm == G2OC_ALGO_DOGLEG) G2OC_TRY(dl_iteration(c, i, stv, &result));
+    else if (c->prm.algorithm == G2OC_ALGO_STRUCTURE_ONLY) G2OC_TRY(so_iteration(c, stv, &result));
+    else G2OC_TRY(gn_iteration(c, i, stv, &result));
+    stv->iteration = i;
+    stv->result = result;
+    c->span(t0, &stv->time_iteration);
+    c->spans_ended = c->spans.size();
     ++it;
   }
   G2OC_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  c->resolve_spans();
   if (done) *done = (result == G2OC_RESULT_FAIL) ? 0 : it;
   return G2OC_OK;
 }
@@ -3055,7 +3150,10 @@ static int iterate_impl(g2oc_ctx* c, int iteration, g2oc_iteration_stats* stats,
 int g2oc_optimize(g2oc_ctx* c, int iterations, g2oc_iteration_stats* stats, int* done) {
   G2OC_TRY(check_ctx(c, true));
   const int st = optimize_impl(c, iterations, stats, done);
-  if (st != G2OC_OK) c->drop_spans();
+  if (st != G2OC_OK) {
+    c->resolve_spans(c->spans_ended);  // the iterations before the one that failed
+    c->drop_spans();
+  }
   return st;
 }
 
@@ -3210,7 +3308,7 @@ int g2oc_solve(g2oc_ctx* c, double lambda, double* x, int32_t* iters) {
   G2OC_TRY(read_state(c, &h, &stv));
   if (iters) *iters = stv.iterations_linear_solver;
   if (x) G2OC_CUDA_TRY(cudaMemcpy(x, c->x.p, c->x.bytes(), cudaMemcpyDeviceToHost));
-  return h.solve_ok ? G2OC_OK : G2OC_ERR_NOT_PD;
+  return solve_succeeded(c, h) ? G2OC_OK : G2OC_ERR_NOT_PD;
 }
 
 int g2oc_solver_init(g2oc_ctx* c) {
@@ -3677,7 +3775,7 @@ static int window_round(g2oc_ctx* c, bool autotune) {
   G2OC_K(K_LM_CONTROL) win_mask_step<<<cdiv(n, 256), 256, 0, st>>>(c->win_of_cam.p, S.Cf, c->win_of_lm.p, S.Pf,
                                                                     c->win_state.p, c->x.p);
   G2OC_LAUNCH_CHECK();
-  G2OC_TRY(oplus(c));
+  G2OC_TRY(oplus(c, false));
   G2OC_TRY(window_chi2(c, 1));
   G2OC_K(K_LM_CONTROL) win_scale<256><<<c->nw, 256, 0, st>>>(c->x.p, c->b.p, S.Cf, W, c->win_state.p);
   G2OC_K(K_LM_CONTROL) win_decide<<<cdiv(c->nw, 128), 128, 0, st>>>(c->win_state.p, c->nw,
@@ -3988,7 +4086,7 @@ int g2oc_get_stream(g2oc_ctx* c, void** stream) {
 
 int g2oc_restore_initial_estimates(g2oc_ctx* c) {
   G2OC_TRY(check_ctx(c, true));
-  c->chi2_carry = false;
+  c->chi2_carry = c->bak_fixed = false;
   G2OC_CUDA_TRY(cudaMemcpyAsync(c->pose.p, c->pose_init.p, c->pose.bytes(), cudaMemcpyDeviceToDevice, c->stream));
   if (c->point.n)
     G2OC_CUDA_TRY(cudaMemcpyAsync(c->point.p, c->point_init.p, c->point.bytes(), cudaMemcpyDeviceToDevice, c->stream));

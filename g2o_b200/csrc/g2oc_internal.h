@@ -180,7 +180,8 @@ struct DevScalars {
   int accept;            // last trial accepted
   int nonfinite;         // a non-finite value was met
   int chol_error;        // a wait of the tiled Cholesky ran out
-  int pad[2];
+  unsigned ticket;       // blocks that have left a grid-wide sum (zero between launches)
+  int pad;
 };
 
 }  // namespace g2oc

@@ -21,8 +21,7 @@ static __global__ void lm_init_lambda(DevScalars* sc, double user_lambda, double
 // One trial's decision. rho = (chi_current - chi_temp) / (scale + 1e-3);
 // accept: lambda *= max(1/3, min(2/3, 1 - (2 rho - 1)^3)), ni = 2;
 // reject: lambda *= ni, ni *= 2 (estimates restored by the host).
-static __global__ void lm_decide(DevScalars* sc) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__device__ __forceinline__ void lm_decide_trial(DevScalars* sc) {
   const bool ok2 = sc->solve_ok != 0;
   double tempChi = sc->chi2_temp;
   if (!ok2) tempChi = 1.79769313486231570815e+308;
@@ -46,8 +45,10 @@ static __global__ void lm_decide(DevScalars* sc) {
   sc->rho = rho;
 }
 
-static __global__ void set_solve_ok(DevScalars* sc, int ok) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) sc->solve_ok = ok;
+static __global__ void lm_decide(DevScalars* sc, int ok) {
+  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  if (ok >= 0) sc->solve_ok = ok;
+  lm_decide_trial(sc);
 }
 
 // partial sums of x (lambda x + b) (computeScale)
@@ -62,6 +63,37 @@ static __global__ void lm_scale_partials(const double* x, const double* b, int n
     s += x[i] * ((i >= lam_from ? lambda : 0.0) * x[i] + b[i]);
   s = block_sum1(s);
   if (threadIdx.x == 0) partials[blockIdx.x] = s;
+}
+
+// The end of a trial in one launch: computeScale's sum over the grid, then, in
+// the block that comes last, the chi2 partials' sums (the order of
+// finalize_sum_kernel) and the decision. ok < 0: the solve left its outcome in
+// sc->solve_ok. Where it took five launches (the sum and its end, the chi2's
+// end, solve_ok, the decision) a trial spent 19 us on them and the gaps
+// between them. 256 threads.
+static __global__ void lm_finish(const double* x, const double* b, int n, DevScalars* sc, const double* chi2, int nchi,
+                                 double* partials, int ok, Publish P) {
+  const double lambda = sc->lambda;
+  double s = 0.0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    s += x[i] * (lambda * x[i] + b[i]);
+  s = block_sum1(s);
+  if (threadIdx.x == 0) partials[blockIdx.x] = s;
+  if (!grid_last(&sc->ticket)) return;
+  double plain, robust;
+  sum_partials2(chi2, nchi, plain, robust);
+  s = 0.0;
+  for (int j = threadIdx.x; j < (int)gridDim.x; j += blockDim.x) s += __ldcg(partials + j);
+  s = block_sum1(s);
+  if (threadIdx.x == 0) {
+    sc->chi2_temp_plain = plain;
+    sc->chi2_temp = robust;
+    sc->scale = s + 1e-3;
+    if (ok >= 0) sc->solve_ok = ok;
+    lm_decide_trial(sc);
+    __threadfence();
+  }
+  publish_state(P);
 }
 
 // sum of squares partials (refinement residual norms)

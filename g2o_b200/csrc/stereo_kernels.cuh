@@ -99,7 +99,7 @@ __device__ __forceinline__ void st_jacobians(const double* cam, const double Xc[
 }
 
 // computeActiveErrors + activeChi2 / activeRobustChi2
-static __global__ void st_chi2_kernel(BAEdges E, BAVertices V, double* partials) {
+static __global__ void st_chi2_kernel(BAEdges E, BAVertices V, double* partials, GridSum G) {
   double c = 0.0, r = 0.0;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < E.n; k += gridDim.x * blockDim.x) {
     const StereoObs o = st_load(E.z3, E.oa3, E.ob3, k);
@@ -115,6 +115,7 @@ static __global__ void st_chi2_kernel(BAEdges E, BAVertices V, double* partials)
     }
   }
   block_sum2(c, r, partials + 2 * blockIdx.x);
+  grid_sum2(partials, G);
 }
 
 // per-edge errors and Jacobians in FP64 (parity hooks)
