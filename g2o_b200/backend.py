@@ -313,6 +313,12 @@ class CudaProblem:
         _check(library().g2oc_get_pattern(self._h, _p(hpp, C.c_int32), _p(hpl, C.c_int32), _p(sch, C.c_int32)))
         return hpp, hpl[: i.hpl_nnzb], sch[: i.schur_nnzb]
 
+    def gradient(self):
+        """b of the system built last (the Hessian stays on the device)."""
+        b = np.empty(self.info.vector_size)
+        _check(library().g2oc_get_hessian(self._h, None, None, None, _p(b)))
+        return b
+
     def hessian(self):
         i = self.info
         pd = i.pose_dim
@@ -456,7 +462,7 @@ class BlockSolverCuda:
     def build_system(self, pose_estimate, point_estimate=None) -> bool:
         self._prob.set_estimates(pose_estimate, point_estimate)
         self._prob.build_system()
-        self._b = self._prob.hessian()[3]
+        self._b = self._prob.gradient()
         return True
 
     # Solver::setLambda / solve / restoreDiagonal

@@ -82,9 +82,14 @@ struct CholPlan {
   DBuf<unsigned> flags;
   DBuf<CholState> state;
   CholDev d{};
-  bool smem_raised = false;  // the factorization may use its shared memory (a plan is factored in one type)
+  bool smem_raised = false;  // the kernels may use their shared memory
   const int* pos = nullptr;  // device copy of S.pos
   int sms = 0;
+  // the selected inverse: its lists (device; made on first use) and tiles
+  DBuf<int> inv_ints;
+  DBuf<unsigned> inv_flag;
+  DBuf<double> inv_sigma;
+  size_t inv_at[3] = {0, 0, 0};
   unsigned extra = 0;  // the bounded-wait test: flags are compared with a number that is never reached
   const CholDev& dev() const { return d; }
 };
@@ -710,7 +715,9 @@ static int chol_factor(CholPlan& P, cudaStream_t st, const SysDev<Real>& S, cons
   const int ntask = (int)P.S.task.size();
   if (!P.smem_raised) {
     G2OC_CUDA_TRY(
-        cudaFuncSetAttribute(chol_factor_dag<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFactorSmem));
+        cudaFuncSetAttribute(chol_factor_dag<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFactorSmem));
+    G2OC_CUDA_TRY(
+        cudaFuncSetAttribute(chol_factor_dag<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFactorSmem));
     P.smem_raised = true;
   }
   if (!have_floor) {
@@ -922,13 +929,9 @@ static __global__ void selinv_gather(CholDev P, const double* sigma, const int* 
   out[t] = sigma[(size_t)lo * kTileElems + (i % kTile) * kTile + j % kTile];
 }
 
-// the requested blocks of S^-1 (pairs (row, col) of block indices, covered by
-// the plan's extra pairs) into out (device, nreq * bs * bs)
-template <typename Real>
-static int chol_selected_inverse(CholPlan& P, cudaStream_t st, const SysDev<Real>& S, const int2* d_req, int nreq,
-                                 double* d_out, int* ok, long long* nlaunch) {
-  long long nl = 0;
-  G2OC_TRY(chol_factor<Real>(P, st, S, nullptr, &nl));
+// the lists of the selected inverse, which are the plan's alone
+static int chol_inverse_plan(CholPlan& P, cudaStream_t st) {
+  if (P.inv_ints.p) return G2OC_OK;
   const CholSymbolic& Y = P.S;
   const int ns = (int)Y.row.size(), nt = Y.nt;
   auto slot = [&](int i, int k) {
@@ -957,35 +960,57 @@ static int chol_selected_inverse(CholPlan& P, cudaStream_t st, const SysDev<Real
     return ka < kb;
   });
   CholInts I;
-  const size_t o[] = {I.add(ptr), I.add(task), I.add(reinterpret_cast<const int*>(ent.data()), 4 * ent.size())};
+  P.inv_at[0] = I.add(ptr);
+  P.inv_at[1] = I.add(task);
+  P.inv_at[2] = I.add(reinterpret_cast<const int*>(ent.data()), 4 * ent.size());
   I.v.resize(I.v.size() + 4, 0);
-  DBuf<int> ints;
-  DBuf<unsigned> flag;
-  DBuf<double> sigma;
-  G2OC_TRY(ints.upload(I.v, st));
-  G2OC_TRY(flag.alloc(ns));
-  G2OC_TRY(sigma.alloc((size_t)ns * kTileElems));
-  G2OC_CUDA_TRY(cudaMemsetAsync(flag.p, 0, flag.bytes(), st));
-  G2OC_CUDA_TRY(cudaMemsetAsync(sigma.p, 0, sigma.bytes(), st));  // the parts without unknowns are not written
-  G2OC_TRY(chol_outcome(P, st, ok));
-  if (!*ok) return G2OC_OK;
-  const SelinvDev Q{ints.p + o[0], reinterpret_cast<const int4*>(ints.p + o[2]), ints.p + o[1], flag.p, sigma.p};
+  G2OC_TRY(P.inv_flag.alloc(ns));
+  G2OC_TRY(P.inv_sigma.alloc((size_t)ns * kTileElems));
+  G2OC_CUDA_TRY(cudaMemsetAsync(P.inv_sigma.p, 0, P.inv_sigma.bytes(), st));  // the parts without unknowns stay zero
+  G2OC_TRY(P.inv_ints.upload(I.v, st));
+  G2OC_CUDA_TRY(cudaStreamSynchronize(st));  // the copied host array goes out of scope
+  return G2OC_OK;
+}
+
+// whether the plan's pattern holds the block (r, c)
+static bool chol_covers(const CholPlan& P, int r, int c) {
+  const CholSymbolic& Y = P.S;
+  const int i0 = Y.pos[r], j0 = Y.pos[c];
+  for (int a = 0; a < Y.bs; a += Y.bs - 1)
+    for (int b = 0; b < Y.bs; b += Y.bs - 1) {
+      const int i = std::max(i0 + a, j0 + b) / kTile, j = std::min(i0 + a, j0 + b) / kTile;
+      if (!std::binary_search(Y.row.begin() + Y.col_ptr[j], Y.row.begin() + Y.col_ptr[j + 1], i)) return false;
+    }
+  return true;
+}
+
+// the requested blocks of S^-1 (pairs (row, col) of block indices, covered by
+// the plan's extra pairs) into out (device, nreq * bs * bs)
+template <typename Real>
+static int chol_selected_inverse(CholPlan& P, cudaStream_t st, const SysDev<Real>& S, const int2* d_req, int nreq,
+                                 double* d_out, int* ok, long long* nlaunch) {
+  long long nl = 0;
+  G2OC_TRY(chol_factor<Real>(P, st, S, nullptr, &nl));
+  G2OC_TRY(chol_inverse_plan(P, st));
+  const int ns = (int)P.S.row.size(), bs = P.S.bs;
+  G2OC_CUDA_TRY(cudaMemsetAsync(P.inv_flag.p, 0, P.inv_flag.bytes(), st));
+  const int* q = P.inv_ints.p;
+  const SelinvDev Q{q + P.inv_at[0], reinterpret_cast<const int4*>(q + P.inv_at[2]), q + P.inv_at[1], P.inv_flag.p,
+                    P.inv_sigma.p};
   constexpr int kSmem = 4 * kTileBuf * (int)sizeof(double);
   G2OC_CUDA_TRY(cudaFuncSetAttribute(selinv_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem / 2));
   G2OC_CUDA_TRY(cudaFuncSetAttribute(selinv_dag, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
   selinv_panel<<<ns, 256, kSmem / 2, st>>>(P.dev());
   selinv_dag<<<std::min(P.sms, ns), 256, kSmem, st>>>(P.dev(), Q, P.extra);
   nl += 2;
-  const long long work = (long long)nreq * Y.bs * Y.bs;
+  const long long work = (long long)nreq * bs * bs;
   if (work > 0) {
-    selinv_gather<<<(int)((work + 255) / 256), 256, 0, st>>>(P.dev(), sigma.p, P.pos, Y.bs, d_req, nreq, d_out);
+    selinv_gather<<<(int)((work + 255) / 256), 256, 0, st>>>(P.dev(), P.inv_sigma.p, P.pos, bs, d_req, nreq, d_out);
     nl += 1;
   }
   G2OC_TRY(chol_launch_check("selected inverse"));
-  int fine = 0;
-  G2OC_TRY(chol_outcome(P, st, &fine));
   if (nlaunch) *nlaunch += nl;
-  return G2OC_OK;
+  return chol_outcome(P, st, ok);
 }
 
 }  // namespace g2oc

@@ -81,6 +81,100 @@ constexpr int kAdjointMaxSteps = 100;
 constexpr double kAdjointTolerance = 1e-12;
 constexpr double kAdjointAcceptance = 1e-6;
 
+// ---------------------------------------------------- device buffer cache
+// Released buffers of up to 64 MB, at most 256 MB a device, kept by size class
+// (four per power of two: at most a quarter is lost) until they are taken
+// again, until 4096 buffers were taken and released since, or until an
+// allocation fails. The stream a buffer was last used on is not known here, so
+// before a buffer is taken again the device is waited for once after its
+// release, as cudaFree would have done for each; the wait serves all buffers
+// released before it. One lock per device: contexts may be on several threads.
+namespace {
+struct DevCache {
+  struct Block {
+    void* p;
+    bool idle;  // the device was waited for since the release
+    unsigned long long tick;
+  };
+  static constexpr size_t kMaxBlock = 64u << 20, kMaxTotal = 256u << 20;
+  static constexpr unsigned long long kMaxAge = 4096;
+  std::mutex m;
+  std::multimap<size_t, Block> blocks;
+  size_t total = 0;
+  unsigned long long tick = 0;
+  void drop(std::multimap<size_t, Block>::iterator it) {
+    cudaFree(it->second.p);
+    total -= it->first;
+    blocks.erase(it);
+  }
+};
+constexpr int kMaxDevices = 64;
+DevCache& dev_cache(int device) {
+  static DevCache* c = new DevCache[kMaxDevices];  // outlives every context; the driver frees at exit
+  return c[device];
+}
+size_t size_class(size_t bytes) {
+  size_t b = std::max<size_t>(bytes, 512), p = 512;
+  while (p * 2 <= b) p *= 2;
+  const size_t step = p / 4;
+  return (b + step - 1) / step * step;
+}
+}  // namespace
+
+cudaError_t dev_alloc(void** p, size_t* bytes, int* device) {
+  cudaError_t e = cudaGetDevice(device);
+  if (e != cudaSuccess) return e;
+  if (*device >= kMaxDevices) return cudaMalloc(p, *bytes);
+  DevCache& C = dev_cache(*device);
+  std::lock_guard<std::mutex> lk(C.m);
+  ++C.tick;
+  if (*bytes <= DevCache::kMaxBlock) {
+    *bytes = size_class(*bytes);
+    const auto r = C.blocks.equal_range(*bytes);
+    if (r.first != r.second) {
+      auto it = r.first;
+      while (it != r.second && !it->second.idle) ++it;
+      if (it == r.second) {
+        it = r.first;
+        e = cudaDeviceSynchronize();
+        if (e != cudaSuccess) return e;
+        for (auto& b : C.blocks) b.second.idle = true;
+      }
+      *p = it->second.p;
+      C.total -= it->first;
+      C.blocks.erase(it);
+      return cudaSuccess;
+    }
+  }
+  e = cudaMalloc(p, *bytes);
+  if (e == cudaErrorMemoryAllocation && !C.blocks.empty()) {
+    cudaGetLastError();
+    while (!C.blocks.empty()) C.drop(C.blocks.begin());
+    e = cudaMalloc(p, *bytes);
+  }
+  return e;
+}
+
+void dev_free(void* p, size_t bytes, int device) {
+  if (device >= kMaxDevices || bytes > DevCache::kMaxBlock) {
+    cudaFree(p);
+    return;
+  }
+  DevCache& C = dev_cache(device);
+  std::lock_guard<std::mutex> lk(C.m);
+  ++C.tick;
+  for (auto it = C.blocks.begin(); it != C.blocks.end();) {
+    const auto b = it++;
+    if (b->second.tick + DevCache::kMaxAge < C.tick) C.drop(b);
+  }
+  if (C.total + bytes > DevCache::kMaxTotal) {
+    cudaFree(p);
+    return;
+  }
+  C.blocks.emplace(bytes, DevCache::Block{p, false, C.tick});
+  C.total += bytes;
+}
+
 // --------------------------------------------------------------- engine
 struct EngineBase {
   virtual ~EngineBase() = default;
@@ -92,6 +186,12 @@ struct EngineBase {
   virtual int multiply_hessian(const double* src, double* dst) = 0;
   virtual int solve(double lambda) = 0;  // -> x, g2oc_ctx::solve_ok (PCG iterations: PcgState::total_iterations)
   virtual int get_hessian(double* hpp, double* hll, double* hpl) = 0;
+  // blocks of Hpp^-1 from the context's own factor plan; *done = false: it
+  // does not hold them (or the graph has no such plan), nothing was computed
+  virtual int hpp_inverse(const std::vector<int2>&, double*, int*, bool* done) {
+    *done = false;
+    return G2OC_OK;
+  }
   virtual int schur_export(double lambda, double* S, double* bs) = 0;
   // Gauss-Newton solve H x = rhs (lambda 0) with a given device right-hand
   // side in Hessian order, through the same Schur + PCG / Cholesky path (BA)
@@ -1202,6 +1302,34 @@ struct Engine final : EngineBase {
     G2OC_TRY(chol_plan_build(*P, S.sys_nb, S.pd, S.sys_brow, S.sys_rcol, !S.ba, c->stream));
     P->extra = c->barrier_extra;
     c->chol = std::move(P);
+    return G2OC_OK;
+  }
+
+  int hpp_inverse(const std::vector<int2>& req, double* out, int* ok, bool* done) override {
+    const Structure& S = c->S;
+    cudaStream_t st = c->stream;
+    *done = false;
+    if (S.ba) return G2OC_OK;
+    G2OC_TRY(ensure_chol());
+    for (const int2& q : req)
+      if (!chol_covers(*c->chol, q.x, q.y)) return G2OC_OK;
+    *done = true;
+    const long long nel = (long long)S.sys_nnzb * S.pd * S.pd;
+    if (S.pd == 3)
+      G2OC_K(K_DAMP) sys_gather_damped<Real, 3><<<cdiv(nel, 256), 256, 0, st>>>(
+          hpp.p, c->sys_perm.p, c->sys_brow.p, c->sys_rptr.p, c->sys_rcol.p, S.sys_nnzb, 0.0, sysval.p);
+    else
+      G2OC_K(K_DAMP) sys_gather_damped<Real, 6><<<cdiv(nel, 256), 256, 0, st>>>(
+          hpp.p, c->sys_perm.p, c->sys_brow.p, c->sys_rptr.p, c->sys_rcol.p, S.sys_nnzb, 0.0, sysval.p);
+    G2OC_LAUNCH_CHECK();
+    DBuf<int2> d_req;
+    DBuf<double> d_out;
+    const size_t n = req.size() * S.pd * S.pd;
+    G2OC_TRY(d_req.upload(req, st));
+    G2OC_TRY(d_out.alloc(n));
+    G2OC_TRY(chol_selected_inverse<Real>(*c->chol, st, sys(sysval.p), d_req.p, (int)req.size(), d_out.p, ok,
+                                         &c->kcount[K_CHOLESKY]));
+    if (*ok && n > 0) G2OC_CUDA_TRY(cudaMemcpy(out, d_out.p, n * sizeof(double), cudaMemcpyDeviceToHost));
     return G2OC_OK;
   }
 
@@ -2566,10 +2694,11 @@ int g2oc_create(int device, g2oc_ctx** out) {
     set_error("device %d out of range (%d devices)", device, n);
     return G2OC_ERR_INVALID_ARGUMENT;
   }
-  cudaDeviceProp prop;
-  G2OC_CUDA_TRY(cudaGetDeviceProperties(&prop, device));
-  if (prop.major != 10) {
-    set_error("device %d is sm_%d%d; this library is built for sm_100a", device, prop.major, prop.minor);
+  int major = 0, minor = 0;  // (cudaGetDeviceProperties takes milliseconds)
+  G2OC_CUDA_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+  G2OC_CUDA_TRY(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+  if (major != 10) {
+    set_error("device %d is sm_%d%d; this library is built for sm_100a", device, major, minor);
     return G2OC_ERR_NO_DEVICE;
   }
   G2OC_CUDA_TRY(cudaSetDevice(device));
@@ -4006,14 +4135,12 @@ int g2oc_solve_block_system(g2oc_ctx* c, int32_t linear_solver, int32_t nb, cons
   return ok ? G2OC_OK : G2OC_ERR_NOT_PD;
 }
 
-// blocks of the inverse of a caller system (LinearSolver::solvePattern)
-static int solve_pattern(g2oc_ctx* c, CallerSystem& cs, int32_t nb, int32_t nreq, const int32_t* req, double* out) {
+static int block_requests(int nb, int32_t nreq, const int32_t* req, const double* out, std::vector<int2>& pairs) {
   if (nreq < 0 || (nreq > 0 && (!req || !out))) {
     set_error("invalid block index arguments");
     return G2OC_ERR_INVALID_ARGUMENT;
   }
-  std::vector<int32_t> extra(req, req + 2 * (size_t)nreq);
-  std::vector<int2> pairs(nreq > 0 ? nreq : 1, make_int2(0, 0));
+  pairs.resize(nreq);
   for (int q = 0; q < nreq; ++q) {
     const int r = req[2 * q], cc = req[2 * q + 1];
     if (r < 0 || cc < 0 || r >= nb || cc >= nb) {
@@ -4022,6 +4149,15 @@ static int solve_pattern(g2oc_ctx* c, CallerSystem& cs, int32_t nb, int32_t nreq
     }
     pairs[q] = make_int2(r, cc);
   }
+  return G2OC_OK;
+}
+
+// blocks of the inverse of a caller system (LinearSolver::solvePattern)
+static int solve_pattern(g2oc_ctx* c, CallerSystem& cs, int32_t nb, int32_t nreq, const int32_t* req, double* out) {
+  std::vector<int2> pairs;
+  G2OC_TRY(block_requests(nb, nreq, req, out, pairs));
+  const std::vector<int32_t> extra(req, req + 2 * (size_t)nreq);
+  if (pairs.empty()) pairs.push_back(make_int2(0, 0));
   cudaStream_t st = c->stream;
   CholPlan P;
   G2OC_TRY(chol_plan_build(P, nb, cs.bs, cs.tmp.sys_brow, cs.tmp.sys_rcol, true, st, &extra));
@@ -4063,6 +4199,19 @@ int g2oc_compute_marginals(g2oc_ctx* c, int32_t num_blocks, const int32_t* block
   }
   // H at the current estimates, then its pose part Hpp
   G2OC_TRY(g2oc_build_system(c));
+  std::vector<int2> req;
+  G2OC_TRY(block_requests(nb, num_blocks, block_indices, out, req));
+  // the blocks that the factor of Hpp itself covers (all diagonal ones) come
+  // from the plan the context keeps, with Hpp read where it is; others need a
+  // plan whose pattern has them
+  int ok = 1;
+  bool done = false;
+  G2OC_TRY(c->eng->hpp_inverse(req, out, &ok, &done));
+  if (done) {
+    if (ok) return G2OC_OK;
+    set_error("the matrix is not positive definite");
+    return G2OC_ERR_NOT_PD;
+  }
   const int pd = S.pd;
   const size_t nnzb = S.hpp_rc.size() / 2;
   std::vector<double> hpp(nnzb * pd * pd);

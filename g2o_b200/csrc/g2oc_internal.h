@@ -31,7 +31,14 @@ void set_error(const char* fmt, ...);
     if (_s != G2OC_OK) return _s; \
   } while (0)
 
-// Device allocation owned by the context (cudaMalloc at upload, cudaFree at
+// Device memory from a per-device cache of released buffers, by size classes
+// (g2oc_api.cu): a context of a small graph makes some 75 buffers, and making
+// and freeing them took a third of a call that builds its graph, optimizes it
+// and lets it go. *bytes is the size asked for, then that of the class.
+cudaError_t dev_alloc(void** p, size_t* bytes, int* device);
+void dev_free(void* p, size_t bytes, int device);
+
+// Device allocation owned by the context (made at upload, released at
 // re-upload or destroy).
 template <typename T>
 struct DBuf {
@@ -42,7 +49,7 @@ struct DBuf {
   DBuf& operator=(const DBuf&) = delete;
   ~DBuf() { release(); }
   void release() {
-    if (p) cudaFree(p);
+    if (p) dev_free(p, size_, device_);
     p = nullptr;
     n = 0;
   }
@@ -50,7 +57,8 @@ struct DBuf {
     if (count == n && p) return G2OC_OK;
     release();
     if (count == 0) return G2OC_OK;
-    cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+    size_ = count * sizeof(T);
+    cudaError_t e = dev_alloc(reinterpret_cast<void**>(&p), &size_, &device_);
     if (e != cudaSuccess) {
       set_error("cudaMalloc of %zu bytes failed: %s", count * sizeof(T), cudaGetErrorString(e));
       p = nullptr;
@@ -65,6 +73,10 @@ struct DBuf {
     return G2OC_OK;
   }
   size_t bytes() const { return n * sizeof(T); }
+
+ private:
+  size_t size_ = 0;
+  int device_ = 0;
 };
 
 // ------------------------------------------------------------------ structure
