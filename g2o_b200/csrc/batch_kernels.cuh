@@ -7,11 +7,12 @@
 // trial with its own lambda, accepts or rejects it (restoring only its own
 // vertices) and advances its own iteration count. Each window's reduced
 // camera system is solved by a dense FP64 Cholesky (LinearSolverDense,
-// g2o/solvers/dense/linear_solver_dense.h:57-105), one CTA per window.
+// g2o/solvers/dense/linear_solver_dense.h:57-105), tile by tile over all windows.
 #pragma once
 
 #include "../../include/g2o_cuda.h"
 #include "ba_kernels.cuh"
+#include "cholesky.cuh"
 #include "pcg_kernels.cuh"
 #include "reduce.cuh"
 
@@ -33,7 +34,7 @@ struct WinState {
   int accept;         // the last trial was accepted
   int result;         // G2OC_RESULT_* of the last iteration
   int solve_ok;       // the last factorization succeeded
-  int pad;
+  int not_pd;         // a pivot of the factorization under way was not positive
 };
 
 // ranges of window w: free cameras [cam[w], cam[w+1]) and landmarks
@@ -137,231 +138,61 @@ static __global__ void win_spread_lambda(const int* win_of_cam, int Cf, const in
   else if (t < Cf + Pf) lam_l[t - Cf] = ws[win_of_lm[t - Cf]].lambda;
 }
 
-constexpr int kWinNB = 32;      // panel width of the window Cholesky (one warp)
-constexpr int kWinGroups = 16;  // fixed partial-sum groups of the backward solve
+// Largest number of free camera unknowns of a window.
+constexpr int kWinMaxUnknowns = 837;
 
-// shared memory of win_chol_solve for windows of at most nmax unknowns: the
-// panel (kWinNB x win_ldt(nmax), column-major), x (nmax), the group sums and
-// the reciprocal pivots (nmax)
-__host__ __device__ inline int win_ldt(int n) { return (n + 2) & ~1; }
-inline size_t win_chol_smem(int nmax) {
-  return ((size_t)kWinNB * win_ldt(nmax) + 2 * nmax + kWinGroups * kWinNB) * sizeof(double);
-}
-
-// Dense Cholesky solve of one window's reduced camera system, one CTA per
-// window from the list (LinearSolverDense: LLT of the damped Schur complement,
-// then the two triangular solves). The matrix is the window's (n + 1) x n
-// block of the scratch, written by the Schur rows (lower triangle; row n =
-// the right-hand side), factored in place, right-looking, by panels of
-// kWinNB columns:
-//   - the panel (rows p0..n, the right-hand side row included) is staged in
-//     shared memory column-major;
-//   - warp 0 factors its diagonal block with the block's rows in registers
-//     (lane i = row i; L_jk broadcast by shuffles, no CTA barrier per column);
-//   - every thread solves one panel row against the diagonal block (the
-//     right-hand-side row gives y = L^-1 b on the way);
-//   - the trailing lower triangle takes the panel's update in 16 x 16 tiles,
-//     one warp each, as FP64 tensor-core products (mma.sync m8n8k4) fed from
-//     the column-major panel.
-// Then x = L^-T y backwards by blocks of kWinNB: the sums over the rows below
-// a block in kWinGroups fixed row groups, the block's triangle on warp 0.
-// Every sum runs in an order fixed by n alone (not by the CTA size). The
-// pivots' reciprocals 1/L_kk = rsqrt(d_k) are kept, so the long dependent
-// chains (the diagonal block, each panel row, the backward block solves)
-// multiply instead of divide. A non-positive pivot sets solve_ok = 0 for the
-// window and x = 0.
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS, 512 / THREADS) win_chol_solve(const int* wlist, int nlist, WinDev W, const double* bs,
-                                                           double* xp, double* scratch, WinState* ws) {
-  constexpr int WARPS = THREADS / 32;
-  constexpr unsigned FULL = 0xffffffffu;
-  extern __shared__ __align__(16) double sm[];
-  __shared__ int s_ok;
-  if ((int)blockIdx.x >= nlist) return;
-  const int w = wlist[blockIdx.x];
-  const int h0 = W.cam[w], n = 6 * (W.cam[w + 1] - h0);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (ws[w].done || n == 0) {
-    for (int i = tid; i < n; i += THREADS) xp[(size_t)h0 * 6 + i] = 0.0;
-    return;
+// The windows' dense reduced camera systems as one batch for the tiled
+// Cholesky (LinearSolverDense: LLT of the damped Schur complement, then the
+// two triangular solves): the tiles of all windows are tasks of one launch, so
+// a large window is worked on by several SMs and small ones fill the rest.
+// With a CTA per window the launch took as long as its largest window: 96
+// windows of 8 to 58 free cameras (n = 48 to 348) 480 us a round, against
+// 122 us for both launches here.
+// The matrices (n x n, row-major, lower triangle) are as the Schur rows wrote
+// them and stay so. Any positive pivot passes; a window with another one gets
+// solve_ok = 0 and x = 0. Finished windows are left out.
+struct CholWindows {
+  const double* M;
+  const long long* mat;
+  const int* cam;
+  const int2* tile;  // per tile column: window, place in it
+  WinState* ws;
+  __device__ __forceinline__ double scale(const CholDev&) const { return 0.0; }
+  __device__ __forceinline__ bool skip(const CholDev&, int k) const { return ws[tile[k].x].done != 0; }
+  __device__ __forceinline__ void begin(const CholDev&, int k) const {
+    if (tile[k].y == 0) ws[tile[k].x].not_pd = 0;
   }
-  const int ldt = win_ldt(n);
-  double* PT = sm;                          // PT[k * ldt + i]: panel column k, row p0 + i
-  double* vec = sm + (size_t)kWinNB * ldt;  // x
-  double* grp = vec + n;                    // kWinGroups x kWinNB
-  double* invd = grp + kWinGroups * kWinNB; // 1 / L_kk
-  double* M = scratch + W.mat[w];
-  for (int i = tid; i < n; i += THREADS) M[(size_t)n * n + i] = bs[(size_t)h0 * 6 + i];
-  if (tid == 0) s_ok = 1;
-  __syncthreads();
-  for (int p0 = 0; p0 < n; p0 += kWinNB) {
-    const int pb = min(kWinNB, n - p0);  // panel width
-    const int m = n + 1 - p0;            // panel rows, the right-hand side row last
-    // stage: row-major global reads (coalesced), entries above the diagonal
-    // and columns past pb as zeros
-    for (int t = tid; t < m * kWinNB; t += THREADS) {
-      const int i = t / kWinNB, k = t % kWinNB;
-      PT[k * ldt + i] = (k < pb && k <= i) ? M[(size_t)(p0 + i) * n + p0 + k] : 0.0;
-    }
-    __syncthreads();
-    // diagonal block on warp 0
-    if (warp == 0) {
-      double a[kWinNB];
-#pragma unroll
-      for (int j = 0; j < kWinNB; ++j) a[j] = PT[j * ldt + lane];
-      bool ok = true;
-#pragma unroll
-      for (int k = 0; k < kWinNB; ++k) {
-        if (k < pb && ok) {
-          const double d = __shfl_sync(FULL, a[k], k);
-          if (!(d > 0.0)) {
-            ok = false;  // uniform: every lane read the same pivot
-          } else {
-            const double inv = rsqrt(d);
-            if (lane == k) {
-              a[k] = d * inv;
-              invd[p0 + k] = inv;
-            } else if (lane > k) {
-              a[k] *= inv;
-            }
-#pragma unroll
-            for (int j = k + 1; j < kWinNB; ++j) {
-              const double ljk = __shfl_sync(FULL, a[k], j);
-              if (lane >= j) a[j] -= a[k] * ljk;
-            }
-          }
-        }
+  __device__ __forceinline__ int* info(const CholDev&, int k) const { return &ws[tile[k].x].not_pd; }
+  __device__ __forceinline__ void assemble(const CholDev& P, int s, double* As) const {
+    const int k = P.col[s], i = P.row[s], wk = P.width[k], wi = P.width[i];
+    const int2 t = tile[k];
+    const int n = 6 * (cam[t.x + 1] - cam[t.x]);  // even: rows and columns start on 16 bytes
+    const double* src = M + mat[t.x] + (size_t)(t.y + i - k) * kTile * n + t.y * kTile;
+    for (int e = threadIdx.x; e < kTileElems / 2; e += 256) {
+      const int r = e >> 5, c = 2 * (e & 31);
+      double2 v = make_double2(0.0, 0.0);
+      if (r < wi && c < wk) v = *reinterpret_cast<const double2*>(src + (size_t)r * n + c);
+      if (i == k) {
+        if (c > r) v.x = 0.0;
+        if (c + 1 > r) v.y = 0.0;
+        if (r >= wk && c == r) v.x = 1.0;
+        if (r >= wk && c + 1 == r) v.y = 1.0;
       }
-      if (lane < pb) {
-#pragma unroll
-        for (int j = 0; j < kWinNB; ++j)
-          if (j <= lane) PT[j * ldt + lane] = a[j];
-      }
-      if (!ok && lane == 0) s_ok = 0;
+      *reinterpret_cast<double2*>(As + r * kLd + c) = v;
     }
-    __syncthreads();
-    if (!s_ok) break;  // uniform
-    // panel rows below the diagonal block: x L_JJ^T = a
-    for (int i = pb + tid; i < m; i += THREADS) {
-      double x[kWinNB];
-#pragma unroll
-      for (int j = 0; j < kWinNB; ++j) x[j] = PT[j * ldt + i];
-#pragma unroll
-      for (int k = 0; k < kWinNB; ++k) {
-        if (k < pb) {
-          x[k] *= invd[p0 + k];
-#pragma unroll
-          for (int j = k + 1; j < kWinNB; ++j) x[j] -= x[k] * PT[k * ldt + j];
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kWinNB; ++j) PT[j * ldt + i] = x[j];
-    }
-    __syncthreads();
-    // the factored panel back (lower part and the right-hand side row)
-    for (int t = tid; t < m * kWinNB; t += THREADS) {
-      const int i = t / kWinNB, k = t % kWinNB;
-      if (k < pb && k <= i) M[(size_t)(p0 + i) * n + p0 + k] = PT[k * ldt + i];
-    }
-    // trailing update: rows pb..m-1 (local), columns pb..m-2, lower part, in
-    // 16 x 16 tiles (a, b), b <= a, numbered row-block by row-block, one warp
-    // per tile: 2 x 2 FP64 tensor-core products (mma m8n8k4) per 4 columns of
-    // the panel, operands straight from the column-major panel
-    const int nc = m - 1 - pb;
-    if (nc > 0) {
-      const int nbc = (nc + 15) / 16, nbr = (m - pb + 15) / 16;
-      const int tri = nbc * (nbc + 1) / 2;
-      const int ntile = tri + (nbr > nbc ? nbc : 0);  // the last row block holds the right-hand side row only
-      const int gi = lane >> 2, ti = lane & 3;
-      for (int t = warp; t < ntile; t += WARPS) {
-        int a, b;
-        if (t < tri) {
-          a = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
-          while ((a + 1) * (a + 2) / 2 <= t) ++a;
-          while (a * (a + 1) / 2 > t) --a;
-          b = t - a * (a + 1) / 2;
-        } else {
-          a = nbc;
-          b = t - tri;
-        }
-        const int i0 = pb + 16 * a, j0 = pb + 16 * b;
-        double acc[2][2][2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-          for (int v = 0; v < 2; ++v) acc[u][v][0] = acc[u][v][1] = 0.0;
-        for (int k0 = 0; k0 < pb; k0 += 4) {
-          const double* col = PT + (k0 + ti) * ldt;
-          const double fa0 = col[i0 + gi], fa1 = col[i0 + 8 + gi];
-          const double fb0 = col[j0 + gi], fb1 = col[j0 + 8 + gi];
-          const double fa[2] = {fa0, fa1}, fb[2] = {fb0, fb1};
-#pragma unroll
-          for (int u = 0; u < 2; ++u)
-#pragma unroll
-            for (int v = 0; v < 2; ++v)
-              asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                           : "+d"(acc[u][v][0]), "+d"(acc[u][v][1])
-                           : "d"(fa[u]), "d"(fb[v]));
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-          for (int v = 0; v < 2; ++v)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int i = i0 + 8 * u + gi, j = j0 + 8 * v + 2 * ti + e;
-              if (i < m && j <= m - 2 && j <= i) {
-                double* pm = M + (size_t)(p0 + i) * n + p0 + j;
-                *pm = *pm - acc[u][v][e];
-              }
-            }
-      }
-    }
-    __syncthreads();
   }
-  if (!s_ok) {
-    if (tid == 0) ws[w].solve_ok = 0;
-    for (int i = tid; i < n; i += THREADS) xp[(size_t)h0 * 6 + i] = 0.0;
-    return;
+  __device__ __forceinline__ bool dead(const CholDev&, int k) const {
+    const WinState& s = ws[tile[k].x];
+    return s.done || s.not_pd;
   }
-  // x = L^-T y, y = row n; blocks from the last
-  const double* y = M + (size_t)n * n;
-  const int nblk = (n + kWinNB - 1) / kWinNB;
-  for (int J = nblk - 1; J >= 0; --J) {
-    const int q0 = J * kWinNB, qb = min(kWinNB, n - q0), r0 = q0 + qb;
-    // group sums: g covers rows r0 + g, r0 + g + kWinGroups, ...
-    for (int g = warp; g < kWinGroups; g += WARPS) {
-      double acc = 0.0;
-      if (lane < qb)
-        for (int i = r0 + g; i < n; i += kWinGroups) acc += M[(size_t)i * n + q0 + lane] * vec[i];
-      grp[g * kWinNB + lane] = acc;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      double sj = 0.0;
-      if (lane < qb) {
-        sj = y[q0 + lane];
-        for (int g = 0; g < kWinGroups; ++g) sj -= grp[g * kWinNB + lane];
-      }
-      double lc[kWinNB];  // column lane of the block: lc[k] = L(q0 + k, q0 + lane)
-#pragma unroll
-      for (int k = 0; k < kWinNB; ++k)
-        lc[k] = (k < qb && lane <= k) ? M[(size_t)(q0 + k) * n + q0 + lane] : 0.0;
-#pragma unroll
-      for (int k = kWinNB - 1; k >= 0; --k) {
-        if (k < qb) {
-          const double xk = __shfl_sync(FULL, sj * invd[q0 + k], k);  // lane k: s_k / L_kk
-          if (lane == k) sj = xk;
-          else if (lane < k) sj -= lc[k] * xk;
-        }
-      }
-      if (lane < qb) vec[q0 + lane] = sj;
-    }
-    __syncthreads();
+  __device__ __forceinline__ void solved(const CholDev&, int k) const {
+    WinState& s = ws[tile[k].x];
+    if (tile[k].y == 0 && !s.done) s.solve_ok = !s.not_pd;
   }
-  for (int i = tid; i < n; i += THREADS) xp[(size_t)h0 * 6 + i] = vec[i];
-  if (tid == 0) ws[w].solve_ok = 1;
-}
+  __device__ __forceinline__ void end(const CholDev& P, DevScalars* sc) const {
+    if (P.st->err) sc->chol_error = 1;
+  }
+};
 
 // zero the step of finished windows (their vertices stay as they are)
 static __global__ void win_mask_step(const int* win_of_cam, int Cf, const int* win_of_lm, int Pf, const WinState* ws,

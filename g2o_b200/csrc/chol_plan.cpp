@@ -286,67 +286,9 @@ struct Dissector {
 
 }  // namespace
 
-void chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow, const std::vector<int>& bcol,
-                   bool reorder, const std::vector<int32_t>* extra) {
-  P = CholSymbolic();
-  P.nb = nb;
-  P.bs = bs;
-  P.n = nb * bs;
-  const int nnzb = (int)brow.size();
-  // positions: the groups of the elimination order start on tile boundaries
-  P.pos.assign(nb, 0);
-  if (reorder) {
-    std::vector<int> ptr(nb + 1, 0), adj;
-    for (int k = 0; k < nnzb; ++k)
-      if (brow[k] != bcol[k]) ++ptr[brow[k] + 1], ++ptr[bcol[k] + 1];
-    for (int i = 0; i < nb; ++i) ptr[i + 1] += ptr[i];
-    adj.resize(ptr[nb]);
-    std::vector<int> at(ptr.begin(), ptr.end() - 1);
-    for (int k = 0; k < nnzb; ++k)
-      if (brow[k] != bcol[k]) {
-        adj[at[brow[k]]++] = bcol[k];
-        adj[at[bcol[k]]++] = brow[k];
-      }
-    Dissector D(ptr, adj, nb, std::max(1, kTile / bs));
-    std::vector<int> all(nb);
-    std::iota(all.begin(), all.end(), 0);
-    D.components(all);
-    int p = 0;
-    for (auto& g : D.groups) {
-      for (int v : g) {
-        P.pos[v] = p;
-        p += bs;
-      }
-      p = (p + kTile - 1) / kTile * kTile;
-    }
-    P.nt = p / kTile;
-  } else {
-    for (int i = 0; i < nb; ++i) P.pos[i] = i * bs;
-    P.nt = (P.n + kTile - 1) / kTile;
-  }
+// the fill of the pattern below the diagonal (tile rows by column) and its slots
+static void plan_slots(CholSymbolic& P, std::vector<std::vector<int>>& col) {
   const int nt = P.nt;
-  P.orig.assign((size_t)nt * kTile, -1);
-  for (int i = 0; i < nb; ++i)
-    for (int a = 0; a < bs; ++a) P.orig[P.pos[i] + a] = i * bs + a;
-  P.width.assign(nt, 0);
-  for (int t = 0; t < nt; ++t)
-    for (int a = 0; a < kTile; ++a)
-      if (P.orig[(size_t)t * kTile + a] >= 0) P.width[t] = a + 1;
-  // pattern of the tiles below the diagonal, by column
-  std::vector<std::vector<int>> col(nt);
-  auto mark = [&](int r, int c) {
-    const int a0 = P.pos[r], b0 = P.pos[c];
-    for (int ti = a0 / kTile; ti <= (a0 + bs - 1) / kTile; ++ti)
-      for (int tj = b0 / kTile; tj <= (b0 + bs - 1) / kTile; ++tj)
-        if (ti != tj) {
-          std::vector<int>& l = col[std::min(ti, tj)];
-          const int i = std::max(ti, tj);
-          if (l.empty() || l.back() != i) l.push_back(i);
-        }
-  };
-  for (int k = 0; k < nnzb; ++k) mark(brow[k], bcol[k]);
-  if (extra)
-    for (size_t k = 0; k < extra->size() / 2; ++k) mark((*extra)[2 * k], (*extra)[2 * k + 1]);
   // fill: the rows of a column join its parent's (the first row below it)
   P.col_ptr.assign(nt + 1, 0);
   for (int k = 0; k < nt; ++k) {
@@ -371,37 +313,11 @@ void chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow
       P.col[s++] = k;
     }
   }
-  auto slot = [&](int i, int k) {
-    if (i == k) return P.col_ptr[k];
-    const auto b = P.row.begin() + P.col_ptr[k] + 1, e = P.row.begin() + P.col_ptr[k + 1];
-    return (int)(std::lower_bound(b, e, i) - P.row.begin());
-  };
-  // assembly
-  {
-    std::vector<int> sl, ent;
-    P.asm_ptr.assign(ns + 1, 0);
-    for (int k = 0; k < nnzb; ++k) {
-      // the entry as stored: rows of block row brow, columns of block row
-      // bcol; the tile holds it with the larger position as the row
-      const bool tr = P.pos[brow[k]] < P.pos[bcol[k]];
-      const int a0 = P.pos[tr ? bcol[k] : brow[k]], b0 = P.pos[tr ? brow[k] : bcol[k]];
-      for (int ti = a0 / kTile; ti <= (a0 + bs - 1) / kTile; ++ti)
-        for (int tj = b0 / kTile; tj <= (b0 + bs - 1) / kTile; ++tj) {
-          if (ti < tj) continue;
-          const int s = slot(ti, tj);
-          sl.push_back(s);
-          ent.insert(ent.end(), {k, a0 - ti * kTile, b0 - tj * kTile, tr ? 1 : 0});
-          ++P.asm_ptr[s + 1];
-        }
-    }
-    for (int s = 0; s < ns; ++s) P.asm_ptr[s + 1] += P.asm_ptr[s];
-    P.asm_ent.resize(ent.size());
-    std::vector<int> at(P.asm_ptr.begin(), P.asm_ptr.end() - 1);
-    for (size_t q = 0; q < sl.size(); ++q) {
-      const int o = at[sl[q]]++;
-      std::copy(ent.begin() + 4 * q, ent.begin() + 4 * q + 4, P.asm_ent.begin() + 4 * (size_t)o);
-    }
-  }
+}
+
+// update lists, hand-out order and substitution lists of the slots
+static void plan_lists(CholSymbolic& P) {
+  const int nt = P.nt, ns = P.col_ptr[nt];
   // updates, by target slot (columns ascending within a target)
   P.upd_ptr.assign(ns + 1, 0);
   auto each_update = [&](auto&& f) {
@@ -490,6 +406,132 @@ void chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow
   P.solve_order.resize(nt);
   std::iota(P.solve_order.begin(), P.solve_order.end(), 0);
   std::stable_sort(P.solve_order.begin(), P.solve_order.end(), [&](int a, int b) { return depth[a] < depth[b]; });
+}
+
+void chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow, const std::vector<int>& bcol,
+                   bool reorder, const std::vector<int32_t>* extra) {
+  P = CholSymbolic();
+  P.nb = nb;
+  P.bs = bs;
+  P.n = nb * bs;
+  const int nnzb = (int)brow.size();
+  // positions: the groups of the elimination order start on tile boundaries
+  P.pos.assign(nb, 0);
+  if (reorder) {
+    std::vector<int> ptr(nb + 1, 0), adj;
+    for (int k = 0; k < nnzb; ++k)
+      if (brow[k] != bcol[k]) ++ptr[brow[k] + 1], ++ptr[bcol[k] + 1];
+    for (int i = 0; i < nb; ++i) ptr[i + 1] += ptr[i];
+    adj.resize(ptr[nb]);
+    std::vector<int> at(ptr.begin(), ptr.end() - 1);
+    for (int k = 0; k < nnzb; ++k)
+      if (brow[k] != bcol[k]) {
+        adj[at[brow[k]]++] = bcol[k];
+        adj[at[bcol[k]]++] = brow[k];
+      }
+    Dissector D(ptr, adj, nb, std::max(1, kTile / bs));
+    std::vector<int> all(nb);
+    std::iota(all.begin(), all.end(), 0);
+    D.components(all);
+    int p = 0;
+    for (auto& g : D.groups) {
+      for (int v : g) {
+        P.pos[v] = p;
+        p += bs;
+      }
+      p = (p + kTile - 1) / kTile * kTile;
+    }
+    P.nt = p / kTile;
+  } else {
+    for (int i = 0; i < nb; ++i) P.pos[i] = i * bs;
+    P.nt = (P.n + kTile - 1) / kTile;
+  }
+  const int nt = P.nt;
+  P.orig.assign((size_t)nt * kTile, -1);
+  for (int i = 0; i < nb; ++i)
+    for (int a = 0; a < bs; ++a) P.orig[P.pos[i] + a] = i * bs + a;
+  P.width.assign(nt, 0);
+  for (int t = 0; t < nt; ++t)
+    for (int a = 0; a < kTile; ++a)
+      if (P.orig[(size_t)t * kTile + a] >= 0) P.width[t] = a + 1;
+  // pattern of the tiles below the diagonal, by column
+  std::vector<std::vector<int>> col(nt);
+  auto mark = [&](int r, int c) {
+    const int a0 = P.pos[r], b0 = P.pos[c];
+    for (int ti = a0 / kTile; ti <= (a0 + bs - 1) / kTile; ++ti)
+      for (int tj = b0 / kTile; tj <= (b0 + bs - 1) / kTile; ++tj)
+        if (ti != tj) {
+          std::vector<int>& l = col[std::min(ti, tj)];
+          const int i = std::max(ti, tj);
+          if (l.empty() || l.back() != i) l.push_back(i);
+        }
+  };
+  for (int k = 0; k < nnzb; ++k) mark(brow[k], bcol[k]);
+  if (extra)
+    for (size_t k = 0; k < extra->size() / 2; ++k) mark((*extra)[2 * k], (*extra)[2 * k + 1]);
+  plan_slots(P, col);
+  const int ns = P.col_ptr[nt];
+  auto slot = [&](int i, int k) {
+    if (i == k) return P.col_ptr[k];
+    const auto b = P.row.begin() + P.col_ptr[k] + 1, e = P.row.begin() + P.col_ptr[k + 1];
+    return (int)(std::lower_bound(b, e, i) - P.row.begin());
+  };
+  // assembly
+  {
+    std::vector<int> sl, ent;
+    P.asm_ptr.assign(ns + 1, 0);
+    for (int k = 0; k < nnzb; ++k) {
+      // the entry as stored: rows of block row brow, columns of block row
+      // bcol; the tile holds it with the larger position as the row
+      const bool tr = P.pos[brow[k]] < P.pos[bcol[k]];
+      const int a0 = P.pos[tr ? bcol[k] : brow[k]], b0 = P.pos[tr ? brow[k] : bcol[k]];
+      for (int ti = a0 / kTile; ti <= (a0 + bs - 1) / kTile; ++ti)
+        for (int tj = b0 / kTile; tj <= (b0 + bs - 1) / kTile; ++tj) {
+          if (ti < tj) continue;
+          const int s = slot(ti, tj);
+          sl.push_back(s);
+          ent.insert(ent.end(), {k, a0 - ti * kTile, b0 - tj * kTile, tr ? 1 : 0});
+          ++P.asm_ptr[s + 1];
+        }
+    }
+    for (int s = 0; s < ns; ++s) P.asm_ptr[s + 1] += P.asm_ptr[s];
+    P.asm_ent.resize(ent.size());
+    std::vector<int> at(P.asm_ptr.begin(), P.asm_ptr.end() - 1);
+    for (size_t q = 0; q < sl.size(); ++q) {
+      const int o = at[sl[q]]++;
+      std::copy(ent.begin() + 4 * q, ent.begin() + 4 * q + 4, P.asm_ent.begin() + 4 * (size_t)o);
+    }
+  }
+  plan_lists(P);
+}
+
+void chol_dense_batch(CholSymbolic& P, const std::vector<int>& first, std::vector<int>& window,
+                      std::vector<int>& index) {
+  P = CholSymbolic();
+  const int nw = (int)first.size() - 1;
+  P.n = first[nw];
+  std::vector<int> order(nw);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int a, int b) { return first[a + 1] - first[a] > first[b + 1] - first[b]; });
+  window.clear();
+  index.clear();
+  std::vector<std::vector<int>> col;
+  for (int w : order) {
+    const int n = first[w + 1] - first[w], t = (n + kTile - 1) / kTile, k0 = (int)col.size();
+    for (int k = 0; k < t; ++k) {
+      window.push_back(w);
+      index.push_back(k);
+      col.emplace_back();
+      for (int i = k + 1; i < t; ++i) col.back().push_back(k0 + i);
+      P.width.push_back(std::min(kTile, n - k * kTile));
+      for (int a = 0; a < kTile; ++a) P.orig.push_back(k * kTile + a < n ? first[w] + k * kTile + a : -1);
+    }
+  }
+  P.nt = (int)col.size();
+  plan_slots(P, col);
+  P.asm_ptr.assign(P.row.size() + 1, 0);
+  plan_lists(P);
 }
 
 }  // namespace g2oc

@@ -44,4 +44,12 @@ struct CholSymbolic {
 void chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow, const std::vector<int>& bcol,
                    bool reorder, const std::vector<int32_t>* extra);
 
+// The plan of a batch of dense matrices: matrix w has the unknowns first[w] ..
+// first[w + 1] - 1. The largest come first, so that their chains start first.
+// window, index: per tile column its matrix and its place in it. No assembly
+// lists: the tiles are read from the matrices. The order of a matrix's sums
+// does not depend on the others.
+void chol_dense_batch(CholSymbolic& P, const std::vector<int>& first, std::vector<int>& window,
+                      std::vector<int>& index);
+
 }  // namespace g2oc

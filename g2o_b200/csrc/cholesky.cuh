@@ -94,29 +94,10 @@ struct CholPlan {
   const CholDev& dev() const { return d; }
 };
 
-// brow, bcol: the blocks of the matrix, row by row; extra: further (row,
-// col) block pairs whose entries the plan must hold (the blocks a selected
-// inverse is asked for), treated as structural nonzeros of the matrix so that
-// the symbolic fill covers them
-static int chol_plan_build(CholPlan& P, int nb, int bs, const std::vector<int>& brow, const std::vector<int>& bcol,
-                           bool reorder, cudaStream_t st, const std::vector<int32_t>* extra = nullptr) {
+// device arrays of the plan whose symbolic part is made
+static int chol_plan_alloc(CholPlan& P, cudaStream_t st) {
   CholSymbolic& S = P.S;
-  chol_symbolic(S, nb, bs, brow, bcol, reorder, extra);
   const size_t ns = S.row.size(), nt = (size_t)S.nt;
-  // entries of block p of row r at rptr[r] * bs^2 + e * nblk + (p - rptr[r])
-  std::vector<int> rptr(nb + 1, 0);
-  for (int r : brow) ++rptr[r + 1];
-  for (int i = 0; i < nb; ++i) rptr[i + 1] += rptr[i];
-  for (size_t q = 0; q < S.asm_ent.size() / 4; ++q) {
-    int* a = S.asm_ent.data() + 4 * q;
-    const int r = brow[a[0]];
-    const long long off = (long long)rptr[r] * bs * bs + (a[0] - rptr[r]);
-    const int place = (a[1] + kTile) | ((a[2] + kTile) << 8) | (a[3] << 16);
-    a[0] = (int)(off & 0xffffffffll);
-    a[1] = (int)(off >> 32);
-    a[2] = rptr[r + 1] - rptr[r];
-    a[3] = place;
-  }
   CholInts I;
   const size_t o[] = {I.add(S.col_ptr), I.add(S.row), I.add(S.col), I.add(S.width), I.add(S.orig), I.add(S.asm_ptr),
                       I.add(S.asm_ent), I.add(S.upd_ptr), I.add(S.upd), I.add(S.task), I.add(S.solve_order),
@@ -145,6 +126,31 @@ static int chol_plan_build(CholPlan& P, int nb, int bs, const std::vector<int>& 
   G2OC_CUDA_TRY(cudaDeviceGetAttribute(&P.sms, cudaDevAttrMultiProcessorCount, dev));
   G2OC_CUDA_TRY(cudaStreamSynchronize(st));  // the copied host array goes out of scope
   return G2OC_OK;
+}
+
+// brow, bcol: the blocks of the matrix, row by row; extra: further (row,
+// col) block pairs whose entries the plan must hold (the blocks a selected
+// inverse is asked for), treated as structural nonzeros of the matrix so that
+// the symbolic fill covers them
+static int chol_plan_build(CholPlan& P, int nb, int bs, const std::vector<int>& brow, const std::vector<int>& bcol,
+                           bool reorder, cudaStream_t st, const std::vector<int32_t>* extra = nullptr) {
+  CholSymbolic& S = P.S;
+  chol_symbolic(S, nb, bs, brow, bcol, reorder, extra);
+  // entries of block p of row r at rptr[r] * bs^2 + e * nblk + (p - rptr[r])
+  std::vector<int> rptr(nb + 1, 0);
+  for (int r : brow) ++rptr[r + 1];
+  for (int i = 0; i < nb; ++i) rptr[i + 1] += rptr[i];
+  for (size_t q = 0; q < S.asm_ent.size() / 4; ++q) {
+    int* a = S.asm_ent.data() + 4 * q;
+    const int r = brow[a[0]];
+    const long long off = (long long)rptr[r] * bs * bs + (a[0] - rptr[r]);
+    const int place = (a[1] + kTile) | ((a[2] + kTile) << 8) | (a[3] << 16);
+    a[0] = (int)(off & 0xffffffffll);
+    a[1] = (int)(off >> 32);
+    a[2] = rptr[r + 1] - rptr[r];
+    a[3] = place;
+  }
+  return chol_plan_alloc(P, st);
 }
 
 // asynchronous 16-byte global -> shared copies past L1 (tiles written by
@@ -394,6 +400,28 @@ __device__ __forceinline__ void chol_frags_to(const CholBlocks& B, double* T, Ch
   });
 }
 
+// What chol_factor_dag factors: a block-sparse matrix (the tiles' entries by
+// the plan's assembly lists). A source has
+//   scale    the magnitude that the pivot floor is relative to (0: any
+//            positive pivot passes)
+//   skip     whether the tile column k is left out of this launch
+//   begin    called by thread 0 before the first pivot of a tile column
+//   info     where a pivot that is too small is noted
+template <typename Real>
+struct CholSystem {
+  SysDev<Real> S;
+  int bs;
+  __device__ __forceinline__ double scale(const CholDev& P) const {
+    return __longlong_as_double((long long)P.st->max_diag);
+  }
+  __device__ __forceinline__ bool skip(const CholDev&, int) const { return false; }
+  __device__ __forceinline__ void begin(const CholDev&, int) const {}
+  __device__ __forceinline__ int* info(const CholDev& P, int) const { return &P.st->info; }
+  __device__ __forceinline__ void assemble(const CholDev& P, int s, double* As) const {
+    chol_assemble(S, bs, P, s, As);
+  }
+};
+
 // The whole factorization, one persistent CTA of 256 threads per SM. Tiles
 // are handed out by ticket in the plan's order (estimated start times, always
 // after every tile they need), so a wait is for a tile that some CTA is
@@ -422,9 +450,8 @@ __device__ __forceinline__ void chol_frags_to(const CholBlocks& B, double* T, Ch
 // they took 0.27 and 0.34 ms. Computing the tile below the diagonal in the
 // diagonal's task (W(k) then need not travel) gained 4% where that task had
 // few products and lost 15% where it had many.
-template <typename Real>
-__global__ void __launch_bounds__(256, 1) chol_factor_dag(SysDev<Real> S, int bs, CholDev P, const double* rhs,
-                                                          unsigned extra) {
+template <typename Source>
+__global__ void __launch_bounds__(256, 1) chol_factor_dag(Source A, CholDev P, const double* rhs, unsigned extra) {
   extern __shared__ __align__(16) double sm_chol[];
   __shared__ int sh_ticket, sh_ready;
   // stage q: operand tiles at 2 q and 2 q + 1
@@ -434,7 +461,7 @@ __global__ void __launch_bounds__(256, 1) chol_factor_dag(SysDev<Real> S, int bs
   const int tid = threadIdx.x;
   const unsigned want = P.st->factor.epoch + 1;  // the flag value of this launch
   const unsigned wait_for = want + extra;
-  const double max_diag = __longlong_as_double((long long)P.st->max_diag);
+  const double scale = A.scale(P);
   int* err = &P.st->err;
   for (;;) {
     const int tk = chol_ticket(&P.st->factor, &sh_ticket);
@@ -442,6 +469,10 @@ __global__ void __launch_bounds__(256, 1) chol_factor_dag(SysDev<Real> S, int bs
     const int s = P.task[tk];
     const int k = P.col[s];
     const bool diag = P.row[s] == k;
+    if (A.skip(P, k)) {
+      if (tid == 0) chol_store_flag(P.flag + s, want);
+      continue;
+    }
     const int wk = P.width[k], wi = P.width[P.row[s]];
     const CholBlocks B(wi, wk, diag);
     CholAcc acc;
@@ -452,7 +483,8 @@ __global__ void __launch_bounds__(256, 1) chol_factor_dag(SysDev<Real> S, int bs
       const int n = chol_ready(P, upd, 0, nu, wait_for);
       if (tid == 0) sh_ready = n;
     }
-    chol_assemble(S, bs, P, s, buf(0));
+    A.assemble(P, s, buf(0));
+    if (diag && tid == 0) A.begin(P, k);
     if (diag && tid < kTile) {
       const int o = rhs ? P.orig[(size_t)k * kTile + tid] : -1;
       vb[tid] = o >= 0 ? rhs[o] : 0.0;
@@ -529,8 +561,8 @@ __global__ void __launch_bounds__(256, 1) chol_factor_dag(SysDev<Real> S, int bs
       // what does not exceed that is taken for zero. The rows of a dissected
       // factor are short; n in the place of m refuses definite systems whose
       // root is only weakly tied to the fixed vertices (a 40,000-pose chain)
-      const double floor = 4.0 * terms * 2.220446049250313e-16 * max_diag;
-      tile_potrf_inv64(T, Ws, buf(2), wk, floor, &P.st->info);
+      const double floor = 4.0 * terms * 2.220446049250313e-16 * scale;
+      tile_potrf_inv64(T, Ws, buf(2), wk, floor, A.info(P, k));
       double* Wg = P.W + (size_t)k * kTileElems;
 #pragma unroll
       for (int q = 0; q < kTileElems / 2 / 256; ++q) {
@@ -633,9 +665,20 @@ static __global__ void __launch_bounds__(256) chol_forward_dag(CholDev P, const 
 }
 
 // x(k) = W(k)^T (y(k) - sum_i L(i, k)^T x(i)), written in the caller's order;
-// sc != nullptr gets the outcome of the solve
-static __global__ void __launch_bounds__(256) chol_backward_dag(CholDev P, double* xout, DevScalars* sc,
-                                                                unsigned extra) {
+// sc != nullptr gets the outcome of the solve. A source's columns may have no
+// solution (dead: x is zero there); solved is called by thread 0 per column.
+struct CholAlive {
+  __device__ __forceinline__ bool dead(const CholDev&, int) const { return false; }
+  __device__ __forceinline__ void solved(const CholDev&, int) const {}
+  __device__ __forceinline__ void end(const CholDev& P, DevScalars* sc) const {
+    if (!sc) return;
+    sc->solve_ok = P.st->info == 0;
+    if (P.st->err) sc->chol_error = 1;
+  }
+};
+template <typename Source>
+__global__ void __launch_bounds__(256) chol_backward_dag(Source A, CholDev P, double* xout, DevScalars* sc,
+                                                         unsigned extra) {
   __shared__ int sh_ticket, sh_ok;
   __shared__ double v[kTile], part[4][kTile];
   const int tid = threadIdx.x, c = tid & 63, q = tid >> 6;
@@ -645,6 +688,15 @@ static __global__ void __launch_bounds__(256) chol_backward_dag(CholDev P, doubl
     const int tk = chol_ticket(&P.st->backward, &sh_ticket);
     if (tk >= P.nt) break;
     const int k = P.solve_order[P.nt - 1 - tk];
+    if (tid == 0) A.solved(P, k);
+    if (A.dead(P, k)) {
+      if (tid < kTile) {
+        const int o = P.orig[(size_t)k * kTile + tid];
+        if (o >= 0) xout[o] = 0.0;
+      }
+      if (tid == 0) chol_store_flag(P.xflag + k, want);
+      continue;
+    }
     double w[16], t[16];
     auto fetch = [&](const double* tile, double (&d)[16]) {
 #pragma unroll
@@ -690,11 +742,7 @@ static __global__ void __launch_bounds__(256) chol_backward_dag(CholDev P, doubl
       chol_store_flag(P.xflag + k, want);
     }
   }
-  chol_leave(&P.st->backward, [&]() {
-    if (!sc) return;
-    sc->solve_ok = P.st->info == 0;
-    if (P.st->err) sc->chol_error = 1;
-  });
+  chol_leave(&P.st->backward, [&]() { A.end(P, sc); });
 }
 
 static int chol_launch_check(const char* what) {
@@ -715,23 +763,23 @@ static int chol_factor(CholPlan& P, cudaStream_t st, const SysDev<Real>& S, cons
   const int ntask = (int)P.S.task.size();
   if (!P.smem_raised) {
     G2OC_CUDA_TRY(
-        cudaFuncSetAttribute(chol_factor_dag<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFactorSmem));
+        cudaFuncSetAttribute(chol_factor_dag<CholSystem<double>>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFactorSmem));
     G2OC_CUDA_TRY(
-        cudaFuncSetAttribute(chol_factor_dag<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFactorSmem));
+        cudaFuncSetAttribute(chol_factor_dag<CholSystem<float>>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFactorSmem));
     P.smem_raised = true;
   }
   if (!have_floor) {
     chol_floor<Real><<<(P.S.n + 255) / 256, 256, 0, st>>>(S, P.S.bs, P.state.p);
     *nl += 1;
   }
-  chol_factor_dag<Real><<<std::min(P.sms, ntask), 256, kFactorSmem, st>>>(S, P.S.bs, P.dev(), rhs, P.extra);
+  chol_factor_dag<<<std::min(P.sms, ntask), 256, kFactorSmem, st>>>(CholSystem<Real>{S, P.S.bs}, P.dev(), rhs, P.extra);
   *nl += 1;
   return chol_launch_check("cholesky");
 }
 
 // backward substitution of the vector the plan holds
 static int chol_backward(CholPlan& P, cudaStream_t st, double* xout, long long* nl, DevScalars* sc = nullptr) {
-  chol_backward_dag<<<std::min(2 * P.sms, P.S.nt), 256, 0, st>>>(P.dev(), xout, sc, P.extra);
+  chol_backward_dag<<<std::min(2 * P.sms, P.S.nt), 256, 0, st>>>(CholAlive{}, P.dev(), xout, sc, P.extra);
   *nl += 1;
   return chol_launch_check("cholesky solve");
 }

@@ -201,7 +201,7 @@ struct EngineBase {
   // batched windows: per-window lambda initialisation, and the trial's solve
   // (Schur with per-vertex damping, dense Cholesky per window, back-substitution)
   virtual int batch_lambda_init(double user_lambda, double tau) = 0;
-  virtual int batch_solve(bool autotune) = 0;
+  virtual int batch_solve() = 0;
 };
 
 // kernel identifiers for the launch counters and the optional per-launch
@@ -344,16 +344,10 @@ struct g2oc_ctx {
   g2oc::DBuf<double> win_scratch, lam_c, lam_l;
   g2oc::DBuf<g2oc::WinState> win_state;
   g2oc::DBuf<int> win_active;
-  g2oc::DBuf<int> win_list[3];       // windows factored with 128 / 256 / 512 threads
-  int win_list_n[3] = {0, 0, 0};
-  int win_list_nmax[3] = {0, 0, 0};  // largest window of each list (its shared memory)
-  int win_threads_of_class[3] = {0, 0, 0};  // autotuned, per size class (n < 96, < 192, >= 192)
-  std::vector<int> win_threads;      // per window, for the statistics
-  int win_nmax = 0;
+  std::unique_ptr<g2oc::CholPlan> win_chol;  // the dense systems of all windows
+  g2oc::DBuf<int2> win_tile;                 // per tile column: window, place in it
   int win_iterations = 0;
   int win_rounds = 0;
-  bool win_tuned = false;
-  bool win_sparse = false;  // some window's reduced system has blocks outside its pattern (zeroed each round)
   cudaGraphExec_t win_graph = nullptr;
   g2oc::WinDev windev() const {
     return g2oc::WinDev{nw, win_cam.p, win_lm.p, win_edge.p, win_pose.p, win_point.p, win_mat.p};
@@ -473,6 +467,7 @@ struct g2oc_ctx {
     if (win_graph) cudaGraphExecDestroy(win_graph);
     eng.reset();
     chol.reset();
+    win_chol.reset();
     flush_timing();
     drop_spans();
     for (cudaEvent_t e : event_pool) cudaEventDestroy(e);
@@ -1619,112 +1614,21 @@ struct Engine final : EngineBase {
     return G2OC_OK;
   }
 
-  // one launch of the dense per-window solve with THREADS threads per window
-  template <int T>
-  int launch_win_chol(const int* list, int nlist, int nmax) {
-    if (nlist == 0) return G2OC_OK;
-    const size_t smem = win_chol_smem(nmax);
-    if (smem > 48 * 1024) G2OC_TRY(raise_dyn_smem((const void*)win_chol_solve<T>, smem));
-    G2OC_K(K_CHOLESKY) win_chol_solve<T><<<nlist, T, smem, c->stream>>>(list, nlist, c->windev(), c->rhs.p, c->xs.p,
-                                                                          c->win_scratch.p, c->win_state.p);
-    G2OC_LAUNCH_CHECK();
-    return G2OC_OK;
-  }
-  int launch_win_chol_t(int t, const int* list, int nlist, int nmax) {
-    if (t == 0) return launch_win_chol<128>(list, nlist, nmax);
-    if (t == 1) return launch_win_chol<256>(list, nlist, nmax);
-    return launch_win_chol<512>(list, nlist, nmax);
-  }
-
-  // Times the dense solve with 128 / 256 / 512 threads per window on each
-  // window-size class (n < 96, < 192, >= 192 unknowns) and keeps the fastest;
-  // the windows are then solved in three launches, one per thread count.
-  int batch_autotune() {
-    const Structure& S = c->S;
-    (void)S;
-    cudaStream_t st = c->stream;
-    // windows largest first within a launch (the long factorizations start
-    // in the first wave)
-    auto wn = [&](int w) { return 6 * (c->win_cam_h[w + 1] - c->win_cam_h[w]); };
-    auto by_size = [&](std::vector<int>& v) {
-      std::stable_sort(v.begin(), v.end(), [&](int a, int b) { return wn(a) > wn(b); });
-    };
-    std::vector<int> cls[3];
-    int cls_nmax[3] = {0, 0, 0};
-    for (int w = 0; w < c->nw; ++w) {
-      const int n = wn(w);
-      const int k = n < 96 ? 0 : n < 192 ? 1 : 2;
-      cls[k].push_back(w);
-      cls_nmax[k] = std::max(cls_nmax[k], n);
-    }
-    for (auto& v : cls) by_size(v);
-    DBuf<int> tmp;
-    // the solve factors the windows' matrices in place: every trial starts
-    // from a copy of them, and the copy is put back for the real solve
-    DBuf<double> saved;
-    const size_t mbytes = c->win_scratch.bytes();
-    G2OC_TRY(saved.alloc(c->win_scratch.n));
-    G2OC_CUDA_TRY(cudaMemcpyAsync(saved.p, c->win_scratch.p, mbytes, cudaMemcpyDeviceToDevice, st));
-    auto restore = [&]() -> int {
-      G2OC_CUDA_TRY(cudaMemcpyAsync(c->win_scratch.p, saved.p, mbytes, cudaMemcpyDeviceToDevice, st));
-      return G2OC_OK;
-    };
-    cudaEvent_t a, b;
-    G2OC_CUDA_TRY(cudaEventCreate(&a));
-    G2OC_CUDA_TRY(cudaEventCreate(&b));
-    std::vector<int> lists[3];
-    c->win_threads.assign(c->nw, 0);
-    for (int k = 0; k < 3; ++k) {
-      if (cls[k].empty()) continue;
-      G2OC_TRY(tmp.upload(cls[k], st));
-      int best = 1;
-      float best_ms = 1e30f;
-      for (int t = 0; t < 3; ++t) {
-        G2OC_TRY(restore());
-        G2OC_TRY(launch_win_chol_t(t, tmp.p, (int)cls[k].size(), cls_nmax[k]));  // warm
-        G2OC_TRY(restore());
-        G2OC_CUDA_TRY(cudaEventRecord(a, st));
-        G2OC_TRY(launch_win_chol_t(t, tmp.p, (int)cls[k].size(), cls_nmax[k]));
-        G2OC_CUDA_TRY(cudaEventRecord(b, st));
-        G2OC_CUDA_TRY(cudaEventSynchronize(b));
-        float ms = 0.f;
-        G2OC_CUDA_TRY(cudaEventElapsedTime(&ms, a, b));
-        if (ms < best_ms) {
-          best_ms = ms;
-          best = t;
-        }
-      }
-      c->win_threads_of_class[k] = 128 << best;
-      for (int w : cls[k]) {
-        lists[best].push_back(w);
-        c->win_threads[w] = 128 << best;
-      }
-    }
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-    G2OC_TRY(restore());
-    for (int t = 0; t < 3; ++t) {
-      by_size(lists[t]);
-      c->win_list_n[t] = (int)lists[t].size();
-      c->win_list_nmax[t] = lists[t].empty() ? 0 : wn(lists[t][0]);
-      G2OC_TRY(c->win_list[t].upload(lists[t].empty() ? std::vector<int>{0} : lists[t], st));
-    }
-    G2OC_CUDA_TRY(cudaStreamSynchronize(st));
-    c->win_tuned = true;
-    return G2OC_OK;
-  }
-
-  int batch_solve(bool autotune) override {
+  int batch_solve() override {
     const Structure& S = c->S;
     cudaStream_t st = c->stream;
-    if (c->win_sparse)
-      G2OC_CUDA_TRY(cudaMemsetAsync(c->win_scratch.p, 0, c->win_scratch.bytes(), st));
     G2OC_TRY(schur(0.0, c->rhs.p, c->lam_c.p, c->lam_l.p, false, true));
-    if (autotune && !c->win_tuned) G2OC_TRY(batch_autotune());
-    for (int t = 0; t < 3; ++t)
-      G2OC_TRY(launch_win_chol_t(t, c->win_list[t].p, c->win_list_n[t], c->win_list_nmax[t]));
-    G2OC_CUDA_TRY(cudaMemcpyAsync(c->x.p, c->xs.p, (size_t)S.Cf * 6 * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    return backsub(c->b.p + (size_t)S.Cf * 6, c->xs.p, c->x.p + (size_t)S.Cf * 6);
+    CholPlan& P = *c->win_chol;
+    if (P.S.nt > 0) {
+      const CholWindows A{c->win_scratch.p, c->win_mat.p, c->win_cam.p, c->win_tile.p, c->win_state.p};
+      G2OC_TRY(raise_dyn_smem((const void*)chol_factor_dag<CholWindows>, kFactorSmem));
+      G2OC_K(K_CHOLESKY) chol_factor_dag<<<std::min(P.sms, (int)P.S.task.size()), 256, kFactorSmem, st>>>(
+          A, P.dev(), c->rhs.p, P.extra);
+      G2OC_K(K_CHOLESKY) chol_backward_dag<<<std::min(2 * P.sms, P.S.nt), 256, 0, st>>>(A, P.dev(), c->x.p, c->sc.p,
+                                                                                        P.extra);
+      G2OC_LAUNCH_CHECK();
+    }
+    return backsub(c->b.p + (size_t)S.Cf * 6, c->x.p, c->x.p + (size_t)S.Cf * 6);
   }
 
   int solve_rhs(const double* rhs, double* out, bool reuse_schur = false) override {
@@ -2064,7 +1968,7 @@ struct BalEngine final : EngineBase {
     set_error("batched windows take SE3 bundle adjustments");
     return G2OC_ERR_NOT_SUPPORTED;
   }
-  int batch_solve(bool) override {
+  int batch_solve() override {
     set_error("batched windows take SE3 bundle adjustments");
     return G2OC_ERR_NOT_SUPPORTED;
   }
@@ -3097,7 +3001,6 @@ static int upload_data(g2oc_ctx* c, const g2oc_graph* g) {
 static void drop_windows(g2oc_ctx* c) {
   c->batch = false;
   c->nw = 0;
-  c->win_tuned = false;
   if (c->win_graph) {
     cudaGraphExecDestroy(c->win_graph);
     c->win_graph = nullptr;
@@ -3737,7 +3640,7 @@ int g2oc_upload_windows(g2oc_ctx* c, int32_t num_windows, const g2oc_graph* w) {
   packed.principal_point[0] = w[0].principal_point[0];
   packed.principal_point[1] = w[0].principal_point[1];
   // a re-upload of the same windows (same topology, same window ranges) keeps
-  // the tuned dense-solve schedule and the captured LM round: every device
+  // the plan of the dense solve and the captured LM round: every device
   // buffer they use keeps its size and address
   struct Kept {
     cudaGraphExec_t graph = nullptr;
@@ -3747,7 +3650,7 @@ int g2oc_upload_windows(g2oc_ctx* c, int32_t num_windows, const g2oc_graph* w) {
   } kept;
   kept.graph = c->win_graph;
   c->win_graph = nullptr;
-  const bool was_batch = c->batch, was_tuned = c->win_tuned;
+  const bool was_batch = c->batch;
   const int old_nw = c->nw;
   const std::vector<int> old_pose = c->win_pose_h, old_point = c->win_point_h;
   G2OC_TRY(g2oc_upload(c, &packed));
@@ -3793,20 +3696,19 @@ int g2oc_upload_windows(g2oc_ctx* c, int32_t num_windows, const g2oc_graph* w) {
     prev = wi;
   }
   for (int j = prev + 1; j <= nw; ++j) we[j] = na;
-  // each window's dense (n + 1) x n matrix: the reduced system's lower
-  // triangle, then the right-hand side row
+  // each window's dense n x n matrix: the reduced system's lower triangle
   std::vector<long long> mat(nw);
   long long off = 0;
   int nmax = 0;
   for (int i = 0; i < nw; ++i) {
     const int n = 6 * (wc[i + 1] - wc[i]);
     mat[i] = off;
-    off += (long long)n * (n + 1);
+    off += (long long)n * n;
     nmax = std::max(nmax, n);
   }
-  if (win_chol_smem(nmax) > 227 * 1024) {
+  if (nmax > kWinMaxUnknowns) {
     set_error("a window has %d free camera unknowns; the dense window solve takes at most %d", nmax,
-              (int)((227 * 1024 / sizeof(double) - kWinGroups * kWinNB - 2 * kWinNB) / (kWinNB + 2)));
+              kWinMaxUnknowns);
     return G2OC_ERR_NOT_SUPPORTED;
   }
   cudaStream_t st = c->stream;
@@ -3815,15 +3717,6 @@ int g2oc_upload_windows(g2oc_ctx* c, int32_t num_windows, const g2oc_graph* w) {
   c->win_lm_h = wl;
   c->win_pose_h = pose_off;
   c->win_point_h = point_off;
-  c->win_nmax = nmax;
-  // a window whose cameras do not all co-observe has zero blocks in its dense
-  // matrix, which the Schur rows do not write
-  c->win_sparse = false;
-  for (int i = 0; i < nw; ++i) {
-    const int nb = wc[i + 1] - wc[i];
-    const long long blocks = nb > 0 ? (long long)S.sys_rptr[wc[i + 1]] - S.sys_rptr[wc[i]] : 0;
-    if (blocks != (long long)nb * (nb + 1) / 2) c->win_sparse = true;
-  }
   G2OC_TRY(c->win_cam.upload(wc, st));
   G2OC_TRY(c->win_lm.upload(wl, st));
   G2OC_TRY(c->win_edge.upload(we, st));
@@ -3854,6 +3747,20 @@ int g2oc_upload_windows(g2oc_ctx* c, int32_t num_windows, const g2oc_graph* w) {
   G2OC_TRY(c->win_of_point.upload(ofq, st));
   G2OC_TRY(c->win_mat.upload(mat, st));
   G2OC_TRY(c->win_scratch.alloc((size_t)std::max(off, 1LL)));
+  // blocks of cameras that do not co-observe are not written by the Schur rows
+  G2OC_CUDA_TRY(cudaMemsetAsync(c->win_scratch.p, 0, c->win_scratch.bytes(), st));
+  if (!same_windows) {
+    std::vector<int> first(nw + 1), window, index;
+    for (int i = 0; i <= nw; ++i) first[i] = 6 * wc[i];
+    std::unique_ptr<CholPlan> P(new CholPlan());
+    chol_dense_batch(P->S, first, window, index);
+    std::vector<int2> tile(std::max<size_t>(window.size(), 1), make_int2(0, 0));
+    for (size_t k = 0; k < window.size(); ++k) tile[k] = make_int2(window[k], index[k]);
+    G2OC_TRY(c->win_tile.upload(tile, st));
+    if (!window.empty()) G2OC_TRY(chol_plan_alloc(*P, st));
+    P->extra = c->barrier_extra;
+    c->win_chol = std::move(P);
+  }
   G2OC_TRY(c->lam_c.alloc(std::max(S.Cf, 1)));
   G2OC_TRY(c->lam_l.alloc(std::max(S.Pf, 1)));
   G2OC_TRY(c->win_state.alloc(nw));
@@ -3861,7 +3768,6 @@ int g2oc_upload_windows(g2oc_ctx* c, int32_t num_windows, const g2oc_graph* w) {
   G2OC_CUDA_TRY(cudaStreamSynchronize(st));
   c->batch = true;
   if (same_windows) {
-    c->win_tuned = was_tuned;
     c->win_graph = kept.graph;
     kept.graph = nullptr;
   }
@@ -3886,7 +3792,7 @@ static int window_chi2(g2oc_ctx* c, int which) {
 
 // one LM round of every unfinished window (only stream-ordered work: this is
 // what the CUDA graph captures)
-static int window_round(g2oc_ctx* c, bool autotune) {
+static int window_round(g2oc_ctx* c) {
   const Structure& S = c->S;
   cudaStream_t st = c->stream;
   const WinDev W = c->windev();
@@ -3900,7 +3806,7 @@ static int window_round(g2oc_ctx* c, bool autotune) {
       c->win_of_cam.p, S.Cf, c->win_of_lm.p, S.Pf, c->win_state.p, c->lam_c.p, c->lam_l.p);
   G2OC_LAUNCH_CHECK();
   G2OC_TRY(push(c));
-  G2OC_TRY(c->eng->batch_solve(autotune));
+  G2OC_TRY(c->eng->batch_solve());
   G2OC_K(K_LM_CONTROL) win_mask_step<<<cdiv(n, 256), 256, 0, st>>>(c->win_of_cam.p, S.Cf, c->win_of_lm.p, S.Pf,
                                                                     c->win_state.p, c->x.p);
   G2OC_LAUNCH_CHECK();
@@ -3953,9 +3859,9 @@ int g2oc_optimize_windows(g2oc_ctx* c, int32_t iterations, g2oc_window_stats* st
   c->win_iterations = iterations;
   const int max_rounds = iterations * std::max(c->prm.max_trials_after_failure, 1);
   int rounds = 0, active = 1;
-  // first round eagerly (it also tunes the dense solve), then a captured round
+  // first round eagerly, then a captured round
   if (max_rounds > 0) {
-    G2OC_TRY(window_round(c, true));
+    G2OC_TRY(window_round(c));
     ++rounds;
     G2OC_CUDA_TRY(cudaMemcpyAsync(&active, c->win_active.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     G2OC_CUDA_TRY(cudaStreamSynchronize(st));
@@ -3964,7 +3870,7 @@ int g2oc_optimize_windows(g2oc_ctx* c, int32_t iterations, g2oc_window_stats* st
     c->timing = false;  // no per-launch events inside the graph
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-    int rs = e == cudaSuccess ? window_round(c, false) : G2OC_ERR_CUDA;
+    int rs = e == cudaSuccess ? window_round(c) : G2OC_ERR_CUDA;
     cudaError_t e2 = cudaStreamEndCapture(st, &graph);
     c->timing = timing;
     if (e != cudaSuccess || rs != G2OC_OK || e2 != cudaSuccess) {
@@ -3989,9 +3895,18 @@ int g2oc_optimize_windows(g2oc_ctx* c, int32_t iterations, g2oc_window_stats* st
     G2OC_CUDA_TRY(cudaMemcpyAsync(&active, c->win_active.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     G2OC_CUDA_TRY(cudaStreamSynchronize(st));
   }
+  int bad = 0;
+  G2OC_CUDA_TRY(cudaMemcpyAsync(&bad, &c->sc.p->chol_error, sizeof(int), cudaMemcpyDeviceToHost, st));
+  G2OC_CUDA_TRY(cudaStreamSynchronize(st));
   c->system_built = false;
   c->chi2_carry = false;
   c->win_rounds = rounds;
+  if (bad) {
+    G2OC_CUDA_TRY(cudaMemsetAsync(&c->sc.p->chol_error, 0, sizeof(int), st));
+    G2OC_CUDA_TRY(cudaMemsetAsync(&c->win_chol->state.p->err, 0, sizeof(int), st));
+    set_error("cholesky: a wait for a tile ran out");
+    return G2OC_ERR_TIMEOUT;
+  }
   if (stats) {
     std::vector<WinState> ws(c->nw);
     G2OC_CUDA_TRY(cudaMemcpy(ws.data(), c->win_state.p, ws.size() * sizeof(WinState), cudaMemcpyDeviceToHost));
@@ -4001,7 +3916,7 @@ int g2oc_optimize_windows(g2oc_ctx* c, int32_t iterations, g2oc_window_stats* st
       o.trials = ws[i].trials;
       o.result = ws[i].result;
       o.solve_ok = ws[i].solve_ok;
-      o.cholesky_threads = c->win_threads.empty() ? 0 : c->win_threads[i];
+      o.cholesky_threads = 256;  // per tile
       o.rounds = rounds;
       o.chi2_initial = ws[i].chi2_init;
       o.chi2 = ws[i].chi2_cur;
