@@ -721,10 +721,42 @@ static int run_pcg(g2oc_ctx* c, const SysDev<Real>& A, const double* minv, const
 
 // The whole PCG solve as one cooperative launch (pcg_solve_persistent), one
 // CTA pair per SM; the host reads the state once at the end.
+// one cluster for the whole solve (at most pcg_cluster_rows block rows)
+template <typename Real, int BS, int NB>
+static int run_pcg_cluster(g2oc_ctx* c, const SysDev<Real>& A, const double* minv, const double* rhs, double* xout,
+                           bool fixed_d0) {
+  int ranks = 1;
+  while (ranks * kPcgWarps < A.nb) ranks *= 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ranks);
+  cfg.blockDim = dim3(kPcgThreads);
+  cfg.stream = c->stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = ranks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const int max_iter = pcg_max_iter<Real>(c, A.nb * BS);
+  G2OC_K(K_PCG_SOLVE) {
+    G2OC_CUDA_TRY(cudaLaunchKernelEx(&cfg, pcg_solve_cluster<Real, BS, NB>, A, minv, rhs, xout, c->pcg.p,
+                                     (double)c->prm.pcg_tolerance, max_iter, (int)c->prm.pcg_absolute_tolerance,
+                                     fixed_d0 ? 1 : 0));
+  }
+  return G2OC_OK;
+}
+
 template <typename Real, int BS>
 static int run_pcg_persistent(g2oc_ctx* c, const SysDev<Real>& A, const double* minv, const double* rhs,
                               double* xout, double* r, double* s, double* d, double* tbuf, double* cpart,
                               bool fixed_d0) {
+  // the bounded waits (and their test) belong to the grid barrier; a cluster's
+  // CTAs always run together
+  if (A.nb <= pcg_cluster_rows(BS) && c->barrier_extra == 0) {
+    if constexpr (BS != 9)
+      if (A.nb > 32) return run_pcg_cluster<Real, BS, 2>(c, A, minv, rhs, xout, fixed_d0);
+    return run_pcg_cluster<Real, BS, 1>(c, A, minv, rhs, xout, fixed_d0);
+  }
   int& grid = c->pcg_grid[(sizeof(Real) == 4 ? 3 : 0) + (BS == 9 ? 2 : BS == 6 ? 1 : 0)];
   if (grid == 0) {
     int per_sm = 0, sms = 0;
@@ -753,7 +785,9 @@ static int run_pcg_persistent(g2oc_ctx* c, const SysDev<Real>& A, const double* 
   void* args[] = {&a,    &chunk_ptr, &chunk_row, &nchunks, &minv,    &rhs,    &xout, &r,       &s,
                   &d,    &tbuf,      &cpart,     &part_dq, &part_rs, &stp,    &tol,  &max_iter, &abs_tol,
                   &fixed, &extra};
-  G2OC_K(K_PCG_SOLVE) { G2OC_TRY(coop_launch(c, (const void*)pcg_solve_persistent<Real, BS>, grid, kPcgThreads, args)); }
+  // no more CTAs than have a chunk or a row: the barriers cost by the CTA
+  const int used = std::min(grid, cdiv(std::max(nchunks, A.nb), kPcgWarps));
+  G2OC_K(K_PCG_SOLVE) { G2OC_TRY(coop_launch(c, (const void*)pcg_solve_persistent<Real, BS>, used, kPcgThreads, args)); }
   return G2OC_OK;
 }
 
@@ -787,7 +821,8 @@ static int run_pcg_tiles(g2oc_ctx* c, const Real* tiles, int nb, const double* m
   unsigned extra = c->barrier_extra;
   void* args[] = {&tiles, &tij,  &ntiles, &nbt,  &nb,      &minv,    &rhs, &xout,     &r,       &s,
                   &dbuf0, &dbuf1, &part,  &part_dq, &part_rs, &stp, &tol, &max_iter, &abs_tol, &fixed, &extra};
-  G2OC_K(K_PCG_TILES) { G2OC_TRY(coop_launch(c, (const void*)pcg_solve_tiles<Real>, grid, kTileThreads, args)); }
+  const int used = std::min(grid, std::max(ntiles, cdiv(nb, kTileWarps)));  // see run_pcg_persistent
+  G2OC_K(K_PCG_TILES) { G2OC_TRY(coop_launch(c, (const void*)pcg_solve_tiles<Real>, used, kTileThreads, args)); }
   return G2OC_OK;
 }
 
