@@ -896,6 +896,120 @@ __global__ void __launch_bounds__(THREADS, sizeof(Real) == 4 ? 2 : 1)
   }
 }
 
+// The two parts of schur_rows as two launches, for graphs with a camera whose
+// blocks do not fit in shared memory: the BD_a go through global memory anyway,
+// and the blocks no longer wait for their camera's part nor a camera for the
+// blocks of the one before it.
+template <typename Real, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+    schur_cameras(const int* rows, const int* hc_ptr, const int* hc_blk, const int* hc_col, const Real* hpl,
+                  const Real* dinv, Real* bdc, const int* rptr, const int* s_hpp, const Real* hpp, double lambda_all,
+                  const double* lambda_of, SchurOut<Real> out, const double* b_p, const double* b_l, double* bs) {
+  __shared__ double red[THREADS / 32][36];
+  const int r = rows[blockIdx.x];
+  schur_camera<Real, THREADS>(r, hc_ptr, hc_blk, hc_col, hpl, dinv, bdc + (size_t)hc_ptr[r] * 18, rptr, s_hpp, hpp,
+                              lambda_of ? lambda_of[r] : lambda_all, out, b_p, b_l, bs, red);
+}
+
+// One warp per off-diagonal block, its pairs as in schur_rows. Bound by the
+// gathers of both operands. 96 windows of 10 to 60 cameras (2 M edges, Hpl
+// 290 MB in FP64): schur_cameras 132 us (580 MB), schur_blocks 130 us, against
+// 335 us for schur_rows, which has 16 warps per SM to hide the gathers with and
+// none during a camera's part.
+template <typename Real>
+__global__ void __launch_bounds__(256, 3)
+    schur_blocks(int nnzb, const int* brow, const int* hc_ptr, const Real* hpl,
+                 const Real* bdc, const int* rptr, const int* rcol, const int* pair_ptr, const int2* pairs,
+                 const int* s_hpp, const Real* hpp, SchurOut<Real> out, bool pose_blocks) {
+  constexpr int TS = kTileBlocks * 6;
+  using R2 = typename Vec2<Real>::T;
+  const int lane = threadIdx.x & 31, k = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (k >= nnzb) return;
+  const int r = brow[k], rb = rptr[r], nblk = rptr[r + 1] - rb, j = k - rb;
+  if (j == 0) return;  // the diagonal: schur_cameras
+  const int p1 = pair_ptr[k + 1];
+  const Real* const BD = bdc + (size_t)hc_ptr[r] * 18;
+  const int g = lane >> 2, t = lane & 3;
+  const bool in = g < 6;
+  auto index = [&](int p) { return p + t < p1 ? __ldcs(pairs + p + t) : make_int2(-1, -1); };
+  auto gather = [&](const Real* base, int blk, Real (&b)[3]) {
+    R2 u;
+    u.x = u.y = Real(0);
+    b[2] = Real(0);
+    if (blk >= 0 && in) {
+      const Real* B = base + (size_t)blk * 18;
+      u = __ldg(reinterpret_cast<const R2*>(B) + g);
+      b[2] = __ldg(B + 12 + g);
+    }
+    b[0] = u.x;
+    b[1] = u.y;
+  };
+  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+  int p = pair_ptr[k];
+  int2 i0[2] = {index(p), index(p + 4)}, i1[2] = {index(p + 8), index(p + 12)};
+  Real x[2][3], b[2][3];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    gather(BD, i0[h].x, x[h]);
+    gather(hpl, i0[h].y, b[h]);
+  }
+  for (; p < p1; p += 8) {
+    const int2 i2[2] = {index(p + 16), index(p + 20)};
+    Real xn[2][3], bn[2][3];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      gather(BD, i1[h].x, xn[h]);
+      gather(hpl, i1[h].y, bn[h]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int m = 2; m >= 0; --m)
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                     : "+d"(acc[h][0]), "+d"(acc[h][1])
+                     : "d"((double)x[h][m]), "d"((double)b[h][m]));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      i1[h] = i2[h];
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        x[h][m] = xn[h][m];
+        b[h][m] = bn[h][m];
+      }
+    }
+  }
+  if (!in || t > 2) return;
+  const int hb = pose_blocks ? s_hpp[k] : -1;
+  double w0 = -(acc[0][0] + acc[1][0]), w1 = -(acc[0][1] + acc[1][1]);
+  if (hb >= 0) {
+    w0 += (double)hpp[(size_t)hb * 36 + g * 6 + 2 * t];
+    w1 += (double)hpp[(size_t)hb * 36 + g * 6 + 2 * t + 1];
+  }
+  const int cc = rcol[k], off = out.tiles ? out.tile_off[k] : 0;
+  if (out.tiles) {
+    R2 pr;
+    pr.x = (Real)w0;
+    pr.y = (Real)w1;
+    __stcs(reinterpret_cast<R2*>(out.tiles + off + g * TS + 2 * t), pr);
+    if (r / kTileBlocks == cc / kTileBlocks) {
+      Real* base = out.tiles + (size_t)(off / (TS * TS)) * (TS * TS);
+      Real* m = base + ((cc % kTileBlocks) * 6 + 2 * t) * TS + (r % kTileBlocks) * 6 + g;
+      __stcs(m, pr.x);
+      __stcs(m + TS, pr.y);
+    }
+  } else if (out.dn.M) {
+    // block (r, cc) transposed into the lower triangle of the window's matrix
+    const int wi = out.dn.win_of_cam[r], h0 = out.dn.cam[wi], n = 6 * (out.dn.cam[wi + 1] - h0);
+    double* D = out.dn.M + out.dn.mat[wi] + ((size_t)(cc - h0) * 6 + 2 * t) * n + (r - h0) * 6 + g;
+    D[0] = (double)(Real)w0;
+    D[n] = (double)(Real)w1;
+  } else {
+    Real* Sr = out.S + (size_t)rb * 36;
+    __stcs(Sr + (size_t)(g * 6 + 2 * t) * nblk + j, (Real)w0);
+    __stcs(Sr + (size_t)(g * 6 + 2 * t + 1) * nblk + j, (Real)w1);
+  }
+}
+
 // FP32 rows with short pair lists: the off-diagonal blocks by two lanes each
 // (lane parity = rows 0-2 or 3-5, 18 FP32 accumulators each) over their pairs
 // in landmark order, two gathers in flight per lane. FP32 FMAs need no

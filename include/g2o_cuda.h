@@ -383,7 +383,7 @@ typedef struct g2oc_window_stats {
   int32_t trials;            /* LM trials in all */
   int32_t result;            /* G2OC_RESULT_* of the last iteration */
   int32_t solve_ok;          /* the last dense factorization succeeded */
-  int32_t cholesky_threads;  /* threads per window of the dense solve (autotuned) */
+  int32_t cholesky_threads;  /* threads per CTA of the dense solve */
   int32_t rounds;            /* rounds the batch ran */
   double chi2_initial;       /* robust chi2 before the first iteration */
   double chi2;               /* robust chi2 at the end */
