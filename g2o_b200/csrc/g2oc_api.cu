@@ -949,7 +949,13 @@ struct Engine final : EngineBase {
     const Structure& S = c->S;
     cudaStream_t st = c->stream;
     if (S.ba && S.D == 3) {
-      if (S.Pf > 0) {
+      if (S.Pf > 0 && S.lm_warp_ok) {
+        const int nch = (int)S.lm_chunk_ptr.size() - 1;
+        G2OC_K(K_LANDMARK_PASS) st_landmark_warp<Real><<<cdiv(nch, 4), 128, 0, st>>>(
+            c->ba_edges(), c->ba_vertices(), c->lm_chunk_ptr.p, nch, c->e_lm.p, hll.p, hpl.p,
+            c->b.p + (size_t)S.Cf * 6);
+        G2OC_LAUNCH_CHECK();
+      } else if (S.Pf > 0) {
         G2OC_K(K_LANDMARK_PASS) st_landmark_pass<Real><<<cdiv(S.Pf, 128), 128, 0, st>>>(
             c->ba_edges(), c->ba_vertices(), c->l_ptr.p, S.Pf, hll.p, hpl.p, c->b.p + (size_t)S.Cf * 6);
         G2OC_LAUNCH_CHECK();
