@@ -110,7 +110,7 @@ struct DevCache {
 };
 constexpr int kMaxDevices = 64;
 DevCache& dev_cache(int device) {
-  static DevCache* c = new DevCache[kMaxDevices];  // outlives every context; the driver frees at exit
+  static DevCache* c = new DevCache[kMaxDevices];  // outlives every context; its memory goes with the process
   return c[device];
 }
 size_t size_class(size_t bytes) {
