@@ -158,6 +158,7 @@ struct CholWindows {
   const int2* tile;  // per tile column: window, place in it
   WinState* ws;
   __device__ __forceinline__ double scale(const CholDev&) const { return 0.0; }
+  __device__ __forceinline__ bool ranked(const CholDev&) const { return false; }
   __device__ __forceinline__ bool skip(const CholDev&, int k) const { return ws[tile[k].x].done != 0; }
   __device__ __forceinline__ void begin(const CholDev&, int k) const {
     if (tile[k].y == 0) ws[tile[k].x].not_pd = 0;

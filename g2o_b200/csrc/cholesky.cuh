@@ -10,8 +10,9 @@
 // Numeric (every solve, on the device): one launch computes every tile of L
 // (chol_factor_dag), handing the tiles out in an order in which each only
 // needs tiles handed out before it; a second one substitutes backward. A
-// non-positive pivot sets the info flag (G2OC_ERR_NOT_PD at the boundary);
-// nothing traps.
+// pivot that is zero to working precision, or a direction that is (see
+// kRankTol), sets the info flag (G2OC_ERR_NOT_PD at the boundary); nothing
+// traps.
 #pragma once
 
 #include <algorithm>
@@ -40,16 +41,35 @@ constexpr unsigned kCholSpinLimit = 1u << 22;
 struct CholTickets {
   unsigned next, left, epoch, pad;
 };
+
+// Rank of a matrix in a dissected order. A pivot there is what its unknown
+// has left when all others are known only through the separators above it:
+// for a pose in the middle of 40,000 it is 7e-11 of the largest diagonal entry
+// in a definite system, while the pivot of a part that may turn about its
+// hinge, zero but for rounding, is 1e-11 of it already at 10,000 poses. The
+// pivot's size does not tell them apart; its direction does. With u = L^-T e_k
+// (u'Au = 1), 1 / sum_i a_ii u_i^2 is the pivot's share of what rounding the
+// entries of A can change: at most 2 eps for systems with a free direction (2D
+// graphs of 4 to 20,000 poses: chains, grids, cliques, random loops, a hub),
+// at least 788 eps for definite ones (the least for a straight corridor of
+// 10,000 odometry edges). Pivots that kept less than kSuspect of their diagonal
+// entry are looked at together, u = L^-T (ones at them): the sum's inverse is
+// then no larger than the smallest share. The system is refused when it is
+// below kRankTol. u rides along in the backward pass, and only if a pivot is
+// suspect: none is in a graph of some thousand poses.
+constexpr double kSuspect = 1e-6, kRankTol = 4 * 2.220446049250313e-16;
+
 struct CholState {
   CholTickets factor, forward, backward;
   int info;  // a pivot was not positive
   int err;   // a wait ran out
+  int suspect, pad;  // a pivot is small beside its diagonal entry (kSuspect)
   unsigned long long max_diag;  // bits of the largest |diagonal entry| (chol_floor), back to 0 after a factorization
 };
 
 // device side of the plan
 struct CholDev {
-  int nt, ns, ntask;  // tile columns, slots, tasks of the factorization
+  int n, nt, ns, ntask;  // unknowns, tile columns, slots, tasks of the factorization
   const int *col_ptr, *row, *col, *width, *orig;
   const int* asm_ptr;
   const int4* asm_ent;  // offset (low, high) and stride of the block's entries, packed place
@@ -58,6 +78,9 @@ struct CholDev {
   const int *task, *solve_order, *fwd_ptr, *fwd;
   double *L, *W;   // tiles row-major, kTileElems each: per slot, per tile column (W(k) = L(k,k)^-1)
   double *y, *x;   // nt * kTile: forward and backward substituted vectors
+  bool dissected;  // the rank is decided by kRankTol, with the vectors below
+  double *adiag, *suspect, *u;  // nt * kTile: diagonal of the matrix, ones at the suspect pivots, L^-T of those
+  double* uu;      // per tile column its part of sum_i a_ii u_i^2
   unsigned *flag, *yflag, *xflag;
   CholState* st;
 };
@@ -95,7 +118,7 @@ struct CholPlan {
 };
 
 // device arrays of the plan whose symbolic part is made
-static int chol_plan_alloc(CholPlan& P, cudaStream_t st) {
+static int chol_plan_alloc(CholPlan& P, bool dissected, cudaStream_t st) {
   CholSymbolic& S = P.S;
   const size_t ns = S.row.size(), nt = (size_t)S.nt;
   CholInts I;
@@ -106,7 +129,8 @@ static int chol_plan_alloc(CholPlan& P, cudaStream_t st) {
   std::vector<int>().swap(S.upd);
   I.v.resize(I.v.size() + 4, 0);
   G2OC_TRY(P.ints.upload(I.v, st));
-  G2OC_TRY(P.vals.alloc((ns + nt) * kTileElems + 2 * nt * kTile));
+  const size_t vec = nt * kTile;
+  G2OC_TRY(P.vals.alloc((ns + nt) * kTileElems + 5 * vec + nt));
   G2OC_TRY(P.flags.alloc(ns + 2 * nt));
   G2OC_TRY(P.state.alloc(1));
   G2OC_CUDA_TRY(cudaMemsetAsync(P.vals.p, 0, P.vals.bytes(), st));  // the parts without unknowns stay zero
@@ -116,10 +140,10 @@ static int chol_plan_alloc(CholPlan& P, cudaStream_t st) {
   double* L = P.vals.p;
   double* W = L + ns * kTileElems;
   double* y = W + nt * kTileElems;
-  P.d = CholDev{S.nt, (int)ns, (int)S.task.size(), q + o[0], q + o[1], q + o[2], q + o[3], q + o[4], q + o[5],
+  P.d = CholDev{S.n, S.nt, (int)ns, (int)S.task.size(), q + o[0], q + o[1], q + o[2], q + o[3], q + o[4], q + o[5],
                 reinterpret_cast<const int4*>(q + o[6]), q + o[7], reinterpret_cast<const int2*>(q + o[8]), q + o[9],
-                q + o[10], q + o[11], q + o[12], L, W, y, y + nt * kTile, P.flags.p, P.flags.p + ns,
-                P.flags.p + ns + nt, P.state.p};
+                q + o[10], q + o[11], q + o[12], L, W, y, y + vec, dissected, y + 2 * vec, y + 3 * vec, y + 4 * vec, y + 5 * vec,
+                P.flags.p, P.flags.p + ns, P.flags.p + ns + nt, P.state.p};
   P.pos = q + o[13];
   int dev = 0;
   G2OC_CUDA_TRY(cudaGetDevice(&dev));
@@ -150,7 +174,7 @@ static int chol_plan_build(CholPlan& P, int nb, int bs, const std::vector<int>& 
     a[2] = rptr[r + 1] - rptr[r];
     a[3] = place;
   }
-  return chol_plan_alloc(P, st);
+  return chol_plan_alloc(P, reorder, st);
 }
 
 // asynchronous 16-byte global -> shared copies past L1 (tiles written by
@@ -213,6 +237,7 @@ __device__ __forceinline__ void chol_floor_max(double m, CholState* st) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->info = 0;
     st->err = 0;
+    st->suspect = 0;
   }
   block_max(m, red);
   if (threadIdx.x == 0 && red[0] > 0.0) atomicMax(&st->max_diag, (unsigned long long)__double_as_longlong(red[0]));
@@ -407,6 +432,7 @@ __device__ __forceinline__ void chol_frags_to(const CholBlocks& B, double* T, Ch
 //   skip     whether the tile column k is left out of this launch
 //   begin    called by thread 0 before the first pivot of a tile column
 //   info     where a pivot that is too small is noted
+//   ranked   whether the rank is decided by kRankTol
 template <typename Real>
 struct CholSystem {
   SysDev<Real> S;
@@ -417,6 +443,7 @@ struct CholSystem {
   __device__ __forceinline__ bool skip(const CholDev&, int) const { return false; }
   __device__ __forceinline__ void begin(const CholDev&, int) const {}
   __device__ __forceinline__ int* info(const CholDev& P, int) const { return &P.st->info; }
+  __device__ __forceinline__ bool ranked(const CholDev& P) const { return P.dissected; }
   __device__ __forceinline__ void assemble(const CholDev& P, int s, double* As) const {
     chol_assemble(S, bs, P, s, As);
   }
@@ -490,6 +517,7 @@ __global__ void __launch_bounds__(256, 1) chol_factor_dag(Source A, CholDev P, c
       vb[tid] = o >= 0 ? rhs[o] : 0.0;
     }
     __syncthreads();
+    const double akk = diag && tid < kTile ? buf(0)[tid * (kLd + 1)] : 0.0;
     int ready = sh_ready;  // products below are known to have their operands
     chol_frags_from(B, buf(0), acc);
     __syncthreads();
@@ -556,13 +584,21 @@ __global__ void __launch_bounds__(256, 1) chol_factor_dag(Source A, CholDev P, c
       ysum += __shfl_xor_sync(0xffffffffu, ysum, 1);
       ysum += __shfl_xor_sync(0xffffffffu, ysum, 2);
       if ((tid & 3) == 0) vb[tid >> 2] -= ysum;
-      // a pivot is a diagonal entry less the squares of its row of L: with m
-      // entries its rounding is at most some m eps of the largest entry, and
-      // what does not exceed that is taken for zero. The rows of a dissected
-      // factor are short; n in the place of m refuses definite systems whose
-      // root is only weakly tied to the fixed vertices (a 40,000-pose chain)
-      const double floor = 4.0 * terms * 2.220446049250313e-16 * scale;
+      // what does not exceed the rounding of the sums that a pivot is made of
+      // is taken for zero: n terms in the given order; in a dissected one the
+      // terms of the tile's rows, and the rank is decided by kRankTol (n in
+      // their place refuses definite systems whose root is weakly tied to the
+      // fixed vertices)
+      const bool ranked = A.ranked(P);
+      const double floor = 4.0 * (ranked ? terms : P.n) * 2.220446049250313e-16 * scale;
       tile_potrf_inv64(T, Ws, buf(2), wk, floor, A.info(P, k));
+      if (ranked && tid < kTile) {
+        const double w = Ws[tid * (kLd + 1)];  // 1 / sqrt(pivot)
+        const bool small = kSuspect * akk * w * w >= 1.0;
+        P.adiag[(size_t)k * kTile + tid] = akk;
+        P.suspect[(size_t)k * kTile + tid] = small ? 1.0 : 0.0;
+        if (small) P.st->suspect = 1;
+      }
       double* Wg = P.W + (size_t)k * kTileElems;
 #pragma unroll
       for (int q = 0; q < kTileElems / 2 / 256; ++q) {
@@ -667,7 +703,10 @@ static __global__ void __launch_bounds__(256) chol_forward_dag(CholDev P, const 
 // x(k) = W(k)^T (y(k) - sum_i L(i, k)^T x(i)), written in the caller's order;
 // sc != nullptr gets the outcome of the solve. A source's columns may have no
 // solution (dead: x is zero there); solved is called by thread 0 per column.
+// Decides the rank of a factorization with suspect pivots (kRankTol); xout ==
+// nullptr: does only that.
 struct CholAlive {
+  __device__ __forceinline__ bool ranked(const CholDev& P) const { return P.dissected; }
   __device__ __forceinline__ bool dead(const CholDev&, int) const { return false; }
   __device__ __forceinline__ void solved(const CholDev&, int) const {}
   __device__ __forceinline__ void end(const CholDev& P, DevScalars* sc) const {
@@ -680,8 +719,10 @@ template <typename Source>
 __global__ void __launch_bounds__(256) chol_backward_dag(Source A, CholDev P, double* xout, DevScalars* sc,
                                                          unsigned extra) {
   __shared__ int sh_ticket, sh_ok;
-  __shared__ double v[kTile], part[4][kTile];
+  __shared__ double v[kTile], vu[kTile], part[4][kTile];
   const int tid = threadIdx.x, c = tid & 63, q = tid >> 6;
+  const bool ranked = A.ranked(P) && P.st->suspect != 0;
+  if (!xout && !ranked) return;
   const unsigned want = P.st->backward.epoch + 1, wait_for = want + extra;
   int* err = &P.st->err;
   for (;;) {
@@ -702,15 +743,15 @@ __global__ void __launch_bounds__(256) chol_backward_dag(Source A, CholDev P, do
 #pragma unroll
       for (int a = 0; a < 16; ++a) d[a] = tile[(16 * q + a) * kTile + c];
     };
-    auto dot = [&](const double (&d)[16]) {
+    auto dot = [&](const double (&d)[16], const double* z) {
       double a = 0.0;
 #pragma unroll
-      for (int b = 0; b < 16; ++b) a += d[b] * v[16 * q + b];
+      for (int b = 0; b < 16; ++b) a += d[b] * z[16 * q + b];
       return a;
     };
     fetch(P.W + (size_t)k * kTileElems, w);
     const double yk = tid < kTile ? P.y[(size_t)k * kTile + tid] : 0.0;
-    double sum = 0.0;
+    double sum = 0.0, sumu = 0.0;
     bool ok = true;
     for (int s = P.col_ptr[k + 1] - 1; s > P.col_ptr[k]; --s) {
       const int i = P.row[s];
@@ -720,21 +761,42 @@ __global__ void __launch_bounds__(256) chol_backward_dag(Source A, CholDev P, do
       ok = sh_ok != 0;
       if (!ok) break;
       if (tid < kTile) v[tid] = __ldcg(P.x + (size_t)i * kTile + tid);
+      if (ranked && tid < kTile) vu[tid] = __ldcg(P.u + (size_t)i * kTile + tid);
       __syncthreads();
-      sum += dot(t);
+      sum += dot(t, v);
+      if (ranked) sumu += dot(t, vu);
     }
     if (!ok) break;
-    part[q][c] = sum;
-    __syncthreads();
-    if (tid < kTile) v[tid] = yk - (((part[0][tid] + part[1][tid]) + part[2][tid]) + part[3][tid]);
-    __syncthreads();
-    part[q][c] = dot(w);
-    __syncthreads();
+    // W(k)^T (y - sum), to thread tid < kTile
+    auto finish = [&](double s, double y, double* z) {
+      part[q][c] = s;
+      __syncthreads();
+      if (tid < kTile) z[tid] = y - (((part[0][tid] + part[1][tid]) + part[2][tid]) + part[3][tid]);
+      __syncthreads();
+      part[q][c] = dot(w, z);
+      __syncthreads();
+      return tid < kTile ? ((part[0][tid] + part[1][tid]) + part[2][tid]) + part[3][tid] : 0.0;
+    };
+    const double x = finish(sum, yk, v);
     if (tid < kTile) {
-      const double x = ((part[0][tid] + part[1][tid]) + part[2][tid]) + part[3][tid];
       P.x[(size_t)k * kTile + tid] = x;
       const int o = P.orig[(size_t)k * kTile + tid];
-      if (o >= 0) xout[o] = x;
+      if (o >= 0 && xout) xout[o] = x;
+    }
+    if (ranked) {
+      __syncthreads();  // part is read
+      const size_t at = (size_t)k * kTile + tid;
+      const double u = finish(sumu, tid < kTile ? P.suspect[at] : 0.0, vu);
+      double uu = 0.0;
+      if (tid < kTile) {
+        P.u[at] = u;
+        uu = P.adiag[at] * u * u;
+      }
+      uu = warp_sum(uu);
+      __syncthreads();
+      if (tid == 32) part[0][0] = uu;
+      __syncthreads();
+      if (tid == 0) P.uu[k] = uu + part[0][0];
     }
     __syncthreads();
     if (tid == 0) {
@@ -742,7 +804,15 @@ __global__ void __launch_bounds__(256) chol_backward_dag(Source A, CholDev P, do
       chol_store_flag(P.xflag + k, want);
     }
   }
-  chol_leave(&P.st->backward, [&]() { A.end(P, sc); });
+  chol_leave(&P.st->backward, [&]() {
+    if (ranked) {
+      double uu = 0.0;
+      for (int k = 0; k < P.nt; ++k) uu += __ldcg(P.uu + k);
+      if (!(kRankTol * uu < 1.0)) P.st->info = 1;
+      P.st->suspect = 0;  // decided: not again for a further right-hand side
+    }
+    A.end(P, sc);
+  });
 }
 
 static int chol_launch_check(const char* what) {
@@ -1039,6 +1109,7 @@ static int chol_selected_inverse(CholPlan& P, cudaStream_t st, const SysDev<Real
                                  double* d_out, int* ok, long long* nlaunch) {
   long long nl = 0;
   G2OC_TRY(chol_factor<Real>(P, st, S, nullptr, &nl));
+  G2OC_TRY(chol_backward(P, st, nullptr, &nl));  // the rank
   G2OC_TRY(chol_inverse_plan(P, st));
   const int ns = (int)P.S.row.size(), bs = P.S.bs;
   G2OC_CUDA_TRY(cudaMemsetAsync(P.inv_flag.p, 0, P.inv_flag.bytes(), st));

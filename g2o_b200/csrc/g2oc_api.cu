@@ -3808,7 +3808,7 @@ int g2oc_upload_windows(g2oc_ctx* c, int32_t num_windows, const g2oc_graph* w) {
     std::vector<int2> tile(std::max<size_t>(window.size(), 1), make_int2(0, 0));
     for (size_t k = 0; k < window.size(); ++k) tile[k] = make_int2(window[k], index[k]);
     G2OC_TRY(c->win_tile.upload(tile, st));
-    if (!window.empty()) G2OC_TRY(chol_plan_alloc(*P, st));
+    if (!window.empty()) G2OC_TRY(chol_plan_alloc(*P, false, st));
     P->extra = c->barrier_extra;
     c->win_chol = std::move(P);
   }
