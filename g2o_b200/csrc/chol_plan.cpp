@@ -172,7 +172,7 @@ struct Dissector {
       s = k == 0 ? mid : next;
     }
     if (best >= 1e299) {
-      groups.push_back(vs);
+      if (!hubs(vs, t)) groups.push_back(vs);
       return;
     }
     std::vector<int> part[3];
@@ -190,6 +190,32 @@ struct Dissector {
       if (!part[p].empty()) components(part[p]);
     std::sort(part[2].begin(), part[2].end());
     groups.push_back(part[2]);
+  }
+
+  // A region that no cut between levels shortens, since some vertices are
+  // next to a large part of it: those with eight times the median number of
+  // neighbours become its separator, and what is left is dissected by itself.
+  // A pose that 19,999 others are measured from (137 million tile products as
+  // one dense group) leaves a graph without edges.
+  bool hubs(const std::vector<int>& vs, int t) {
+    const int m = (int)vs.size();
+    if (m <= 2 * leaf) return false;
+    std::vector<int> deg(m, 0);
+    for (int i = 0; i < m; ++i)
+      for (int e = ptr[vs[i]]; e < ptr[vs[i] + 1]; ++e) deg[i] += tag[adj[e]] == t;
+    std::vector<int> sorted(deg);
+    std::nth_element(sorted.begin(), sorted.begin() + m / 2, sorted.end());
+    const int least = std::max(leaf, 8 * sorted[m / 2]);
+    std::vector<int> sep, rest;
+    for (int i = 0; i < m; ++i) (deg[i] >= least ? sep : rest).push_back(vs[i]);
+    if (sep.empty() || (int)sep.size() > m / 8) return false;
+    const int nt = ntags++;
+    for (int v : rest) tag[v] = nt;
+    for (int v : sep) tag[v] = -1;
+    components(rest);
+    std::sort(sep.begin(), sep.end());
+    groups.push_back(sep);
+    return true;
   }
 
   // tiles a set of k blocks fills
