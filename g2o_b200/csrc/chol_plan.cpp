@@ -24,10 +24,12 @@ struct Dissector {
   std::vector<std::vector<int>> groups;  // elimination order: children before their separator
   std::vector<int> tag;                  // region of a vertex in the recursion
   std::vector<int> dist, match, seen;
+  std::vector<int> place;                // of a vertex in the breadth-first order under way
   int ntags = 1, stamp = 0;
 
   Dissector(const std::vector<int>& p, const std::vector<int>& a, int nv, int leaf_blocks)
-      : ptr(p), adj(a), leaf(leaf_blocks), tag(nv, 0), dist(nv, -1), match(nv, -1), seen(nv, 0) {}
+      : ptr(p), adj(a), leaf(leaf_blocks), tag(nv, 0), dist(nv, -1), match(nv, -1), seen(nv, 0),
+        place(nv, 0) {}
 
   // breadth-first order of the region t from s; dist gets the levels
   void bfs(int s, int t, std::vector<int>& order) {
@@ -65,23 +67,28 @@ struct Dissector {
     return false;
   }
 
-  // Minimum vertex cover of the edges between level `cut` and level cut + 1:
-  // side[] (0 / 1 / 2 = separator) of the region's vertices
-  int cover(const std::vector<int>& order, int t, int cut, std::vector<signed char>& side) {
-    std::vector<int> left;
-    for (int u : order)
-      if (dist[u] == cut) left.push_back(u);
-    for (int u : left) {
+  // A cut of a region: side[] (0 / 1 / 2 = separator) of its vertices in
+  // breadth-first order, their numbers, and the range of the separator's places
+  struct Cut {
+    std::vector<signed char> side;
+    int cnt[3], lo, hi;
+  };
+
+  // Minimum vertex cover of the edges between level `cut` and level cut + 1;
+  // below: vertices below a level. Looks at the two levels only.
+  void cover(const std::vector<int>& order, const std::vector<int>& below, int t, int cut, Cut& C) {
+    const int a = below[cut], b = below[cut + 1], c = below[cut + 2], m = (int)order.size();
+    for (int i = a; i < b; ++i) {
       ++stamp;
-      augment(u, t, cut);
+      augment(order[i], t, cut);
     }
     // reached from the unmatched left vertices by alternating paths
     ++stamp;
     std::vector<int> q;
-    for (int u : left)
-      if (match[u] < 0) {
-        seen[u] = stamp;
-        q.push_back(u);
+    for (int i = a; i < b; ++i)
+      if (match[order[i]] < 0) {
+        seen[order[i]] = stamp;
+        q.push_back(order[i]);
       }
     for (size_t h = 0; h < q.size(); ++h)
       for (int e = ptr[q[h]]; e < ptr[q[h] + 1]; ++e) {
@@ -93,16 +100,26 @@ struct Dissector {
           q.push_back(match[v]);
         }
       }
-    int sep = 0;
-    for (size_t i = 0; i < order.size(); ++i) {
+    C.side.assign(m, 1);
+    std::fill(C.side.begin(), C.side.begin() + b, 0);
+    C.cnt[0] = b;
+    C.cnt[1] = m - b;
+    C.cnt[2] = 0;
+    C.lo = m;
+    C.hi = -1;
+    for (int i = a; i < c; ++i) {
       const int u = order[i];
-      side[i] = dist[u] <= cut ? 0 : 1;
       if (match[u] < 0) continue;
-      const bool in = dist[u] == cut ? seen[u] != stamp : seen[u] == stamp;
-      if (in) side[i] = 2, ++sep;
+      if (i < b ? seen[u] != stamp : seen[u] == stamp) {
+        --C.cnt[C.side[i]];
+        C.side[i] = 2;
+        ++C.cnt[2];
+        C.lo = std::min(C.lo, i);
+        C.hi = i;
+      }
+      match[u] = -1;
     }
-    for (int u : order) match[u] = -1;
-    return sep;
+    // (a matched vertex is in one of the two levels, and so is its mate)
   }
 
   // one region (connected): cut it or make it one group
@@ -112,10 +129,17 @@ struct Dissector {
       groups.push_back(vs);
       return;
     }
+    // Every look at a cut costs the edges of its separator and every
+    // breadth-first order those of the region. Where a vertex has more than 16
+    // neighbours fewer are tried: the plan of 4,000 poses with 200 neighbours
+    // each took 150 ms, as long as all else that a first solve does
+    long long edges = 0;
+    for (int v : vs) edges += ptr[v + 1] - ptr[v];
+    const bool thick = edges > 16ll * m;
     // pseudo-peripheral start
-    std::vector<int> order, best_order;
+    std::vector<int> order;
     int s = vs[0], ecc = -1;
-    for (int sweep = 0; sweep < 6; ++sweep) {
+    for (int sweep = 0; sweep < (thick ? 2 : 6); ++sweep) {
       bfs(s, t, order);
       const int e = dist[order.back()];
       // a vertex of the last level with the fewest neighbours
@@ -127,12 +151,21 @@ struct Dissector {
       ecc = e;
       s = far;
     }
-    const int tries = 3;
-    std::vector<signed char> side(m), best_side;
+    if (ecc <= 1) {  // every vertex next to every other
+      groups.push_back(vs);
+      return;
+    }
+    const int tries = thick ? 1 : 3;
+    std::vector<int> orders[3];
+    Cut C;
+    std::vector<signed char> best_side;
+    int best_try = -1;
     double best = 1e300;
     std::vector<int> cand;
     for (int k = 0; k < tries; ++k) {
+      std::vector<int>& order = orders[k];
       bfs(s, t, order);
+      for (int i = 0; i < m; ++i) place[order[i]] = i;
       const int e = dist[order.back()];
       std::vector<int> count(e + 2, 0), below(e + 2, 0);
       for (int u : order) ++count[dist[u]];
@@ -148,21 +181,26 @@ struct Dissector {
         while (l + 1 < e && below[l + 1] * 2 < m) ++l;
         if (e > 0 && std::min(count[l], count[l + 1]) <= m / 4 + leaf) cand.push_back(l);
       }
+      // the narrowest first; where few are looked at, for what the cut takes off
+      // the larger part
+      auto width = [&](int l) {
+        const int w = std::min(count[l], count[l + 1]);
+        return thick ? (double)w / std::min(below[l + 1], m - below[l + 1]) : (double)w;
+      };
       std::sort(cand.begin(), cand.end(), [&](int a, int b) {
-        const int ca = std::min(count[a], count[a + 1]), cb = std::min(count[b], count[b + 1]);
-        return ca < cb || (ca == cb && a < b);
+        const double wa = width(a), wb = width(b);
+        return wa < wb || (wa == wb && a < b);
       });
-      if (cand.size() > 8) cand.resize(8);
+      const size_t most = thick ? std::max(1ll, 128ll * m / edges) : 8;
+      if (cand.size() > most) cand.resize(most);
       for (int l : cand) {
-        cover(order, t, l, side);
-        thin(order, t, side);
-        int cnt[3] = {0, 0, 0};
-        for (int i = 0; i < m; ++i) ++cnt[side[i]];
-        const double sc = score(cnt);
+        cover(order, below, t, l, C);
+        thin(order, t, C);
+        const double sc = score(C.cnt);
         if (sc < best) {
           best = sc;
-          best_side = side;
-          best_order = order;
+          best_side = C.side;
+          best_try = k;
         }
       }
       // the next try starts from a vertex of the middle level
@@ -176,10 +214,10 @@ struct Dissector {
       return;
     }
     std::vector<int> part[3];
-    for (int i = 0; i < m; ++i) part[best_side[i]].push_back(best_order[i]);
-    std::vector<int>().swap(best_order);
+    for (int i = 0; i < m; ++i) part[best_side[i]].push_back(orders[best_try][i]);
     std::vector<signed char>().swap(best_side);
-    std::vector<int>().swap(order);
+    std::vector<signed char>().swap(C.side);
+    for (auto& o : orders) std::vector<int>().swap(o);
     for (int p = 0; p < 2; ++p) {
       const int nt = ntags++;
       for (int v : part[p]) tag[v] = nt;
@@ -235,20 +273,17 @@ struct Dissector {
 
   // thin the separator: vertices with neighbours on one side only join it;
   // then moves of one vertex to a side that bring in at most as many as leave
-  void thin(const std::vector<int>& order, int t, std::vector<signed char>& side) {
-    const int m = (int)order.size();
-    // local index of a vertex: kept in match while this runs
-    for (int i = 0; i < m; ++i) match[order[i]] = i;
-    int cnt[3] = {0, 0, 0};
-    for (int i = 0; i < m; ++i) ++cnt[side[i]];
+  void thin(const std::vector<int>& order, int t, Cut& C) {
+    std::vector<signed char>& side = C.side;
+    int(&cnt)[3] = C.cnt;
     for (int pass = 0; pass < 8; ++pass) {
       bool moved = false;
-      for (int i = 0; i < m; ++i) {
+      for (int i = C.lo; i <= C.hi; ++i) {
         if (side[i] != 2) continue;
         const int u = order[i];
         int nb[2] = {0, 0};
         for (int e = ptr[u]; e < ptr[u + 1]; ++e)
-          if (tag[adj[e]] == t && side[match[adj[e]]] != 2) ++nb[side[match[adj[e]]]];
+          if (tag[adj[e]] == t && side[place[adj[e]]] != 2) ++nb[side[place[adj[e]]]];
         // move u to side p: its neighbours on the other side enter
         for (int q = 0; q < 2; ++q) {
           const int p = cnt[0] <= cnt[1] ? q : 1 - q;
@@ -260,11 +295,13 @@ struct Dissector {
             --cnt[2];
             if (in)
               for (int e = ptr[u]; e < ptr[u + 1]; ++e) {
-                const int v = adj[e];
-                if (tag[v] == t && side[match[v]] == 1 - p) {
-                  side[match[v]] = 2;
+                const int v = place[adj[e]];
+                if (tag[adj[e]] == t && side[v] == 1 - p) {
+                  side[v] = 2;
                   --cnt[1 - p];
                   ++cnt[2];
+                  C.lo = std::min(C.lo, v);
+                  C.hi = std::max(C.hi, v);
                 }
               }
             moved = true;
@@ -274,7 +311,6 @@ struct Dissector {
       }
       if (!moved) break;
     }
-    for (int i = 0; i < m; ++i) match[order[i]] = -1;
   }
 
   // the connected components of a set that already has its own tag; small
@@ -389,15 +425,17 @@ static void plan_lists(CholSymbolic& P) {
       order.push_back({std::max(fin[a], fin[b]), u});
       kmin = std::max(kmin, std::max(key[a], key[b]) + kEps);
     }
-    std::sort(order.begin(), order.end());
-    tmp.clear();
     float t = 0.f;
-    for (auto& o : order) {
-      tmp.push_back(P.upd[2 * (size_t)o.second]);
-      tmp.push_back(P.upd[2 * (size_t)o.second + 1]);
-      t = std::max(t, o.first) + kGemm;
+    if (!std::is_sorted(order.begin(), order.end())) {  // it is where the columns form a chain
+      std::sort(order.begin(), order.end());
+      tmp.clear();
+      for (auto& o : order) {
+        tmp.push_back(P.upd[2 * (size_t)o.second]);
+        tmp.push_back(P.upd[2 * (size_t)o.second + 1]);
+      }
+      std::copy(tmp.begin(), tmp.end(), P.upd.begin() + 2 * (size_t)u0);
     }
-    std::copy(tmp.begin(), tmp.end(), P.upd.begin() + 2 * (size_t)u0);
+    for (auto& o : order) t = std::max(t, o.first) + kGemm;
     float start = order.empty() ? 0.f : order.back().first - kGemm * (order.size() - 1);
     if (s != P.col_ptr[P.col[s]]) {
       const int d = P.col_ptr[P.col[s]];
@@ -480,12 +518,18 @@ void chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow
   for (int t = 0; t < nt; ++t)
     for (int a = 0; a < kTile; ++a)
       if (P.orig[(size_t)t * kTile + a] >= 0) P.width[t] = a + 1;
+  // the first and the last tile that a block's unknowns are in
+  struct Tiles {
+    int first, last;
+  };
+  std::vector<Tiles> tiles(nb);
+  for (int i = 0; i < nb; ++i) tiles[i] = Tiles{P.pos[i] / kTile, (P.pos[i] + bs - 1) / kTile};
   // pattern of the tiles below the diagonal, by column
   std::vector<std::vector<int>> col(nt);
   auto mark = [&](int r, int c) {
-    const int a0 = P.pos[r], b0 = P.pos[c];
-    for (int ti = a0 / kTile; ti <= (a0 + bs - 1) / kTile; ++ti)
-      for (int tj = b0 / kTile; tj <= (b0 + bs - 1) / kTile; ++tj)
+    const Tiles a = tiles[r], b = tiles[c];
+    for (int ti = a.first; ti <= a.last; ++ti)
+      for (int tj = b.first; tj <= b.last; ++tj)
         if (ti != tj) {
           std::vector<int>& l = col[std::min(ti, tj)];
           const int i = std::max(ti, tj);
@@ -502,32 +546,35 @@ void chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow
     const auto b = P.row.begin() + P.col_ptr[k] + 1, e = P.row.begin() + P.col_ptr[k + 1];
     return (int)(std::lower_bound(b, e, i) - P.row.begin());
   };
-  // assembly
-  {
-    std::vector<int> sl, ent;
-    P.asm_ptr.assign(ns + 1, 0);
+  // assembly: a block's tiles in order; the blocks of a row follow one another,
+  // so a tile's slot mostly is that of the last one in its tile column (a row
+  // has at most two of those) or the next
+  P.asm_ptr.assign(ns + 1, 0);
+  struct Last {
+    int i, j, slot;
+  } lasts[2] = {{-1, -1, 0}, {-1, -1, 0}};
+  auto each_entry = [&](auto&& f) {
     for (int k = 0; k < nnzb; ++k) {
-      // the entry as stored: rows of block row brow, columns of block row
-      // bcol; the tile holds it with the larger position as the row
+      // the tile holds the block with the larger position as the row
       const bool tr = P.pos[brow[k]] < P.pos[bcol[k]];
-      const int a0 = P.pos[tr ? bcol[k] : brow[k]], b0 = P.pos[tr ? brow[k] : bcol[k]];
-      for (int ti = a0 / kTile; ti <= (a0 + bs - 1) / kTile; ++ti)
-        for (int tj = b0 / kTile; tj <= (b0 + bs - 1) / kTile; ++tj) {
+      const Tiles a = tiles[tr ? bcol[k] : brow[k]], b = tiles[tr ? brow[k] : bcol[k]];
+      for (int ti = a.first; ti <= a.last; ++ti)
+        for (int tj = b.first; tj <= b.last; ++tj) {
           if (ti < tj) continue;
-          const int s = slot(ti, tj);
-          sl.push_back(s);
-          ent.insert(ent.end(), {k, a0 - ti * kTile, b0 - tj * kTile, tr ? 1 : 0});
-          ++P.asm_ptr[s + 1];
+          Last& l = lasts[tj & 1];
+          if (tj != l.j || ti != l.i) {
+            const bool next = tj == l.j && l.slot + 1 < P.col_ptr[tj + 1] && P.row[l.slot + 1] == ti;
+            l = Last{ti, tj, next ? l.slot + 1 : slot(ti, tj)};
+          }
+          f(l.slot, k);
         }
     }
-    for (int s = 0; s < ns; ++s) P.asm_ptr[s + 1] += P.asm_ptr[s];
-    P.asm_ent.resize(ent.size());
-    std::vector<int> at(P.asm_ptr.begin(), P.asm_ptr.end() - 1);
-    for (size_t q = 0; q < sl.size(); ++q) {
-      const int o = at[sl[q]]++;
-      std::copy(ent.begin() + 4 * q, ent.begin() + 4 * q + 4, P.asm_ent.begin() + 4 * (size_t)o);
-    }
-  }
+  };
+  each_entry([&](int s, int) { ++P.asm_ptr[s + 1]; });
+  for (int s = 0; s < ns; ++s) P.asm_ptr[s + 1] += P.asm_ptr[s];
+  P.asm_ent.resize(P.asm_ptr[ns]);
+  std::vector<int> at(P.asm_ptr.begin(), P.asm_ptr.end() - 1);
+  each_entry([&](int s, int k) { P.asm_ent[at[s]++] = k; });
   plan_lists(P);
 }
 

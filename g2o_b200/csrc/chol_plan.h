@@ -22,11 +22,10 @@ struct CholSymbolic {
   std::vector<int> col_ptr;  // nt + 1
   std::vector<int> row;      // per slot: tile row
   std::vector<int> col;      // per slot: tile column
-  // blocks of the matrix in each slot: (block of the row-ordered list, row
-  // and column of its first entry in the tile -- negative or beyond the tile
-  // for a block that straddles tiles --, 1 if the block is stored transposed)
+  // blocks of the matrix (of the row-ordered list) in each slot; one that
+  // straddles tiles is in several
   std::vector<int> asm_ptr;  // slots + 1
-  std::vector<int> asm_ent;  // 4 per entry
+  std::vector<int> asm_ent;
   // updates of each slot (i, k): the slots (i, j), (k, j) of every earlier
   // column j that has both, the ones expected to be finished first in front
   std::vector<int> upd_ptr;  // slots + 1

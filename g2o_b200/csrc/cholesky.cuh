@@ -101,12 +101,13 @@ struct CholInts {
 struct CholPlan {
   CholSymbolic S;
   DBuf<int> ints;
+  DBuf<int4> places;
   DBuf<double> vals;    // L, W, y, x
   DBuf<unsigned> flags;
   DBuf<CholState> state;
   CholDev d{};
   bool smem_raised = false;  // the kernels may use their shared memory
-  const int* pos = nullptr;  // device copy of S.pos
+  const int *pos = nullptr, *asm_ent = nullptr;  // device copies of S.pos and S.asm_ent
   int sms = 0;
   // the selected inverse: its lists (device; made on first use) and tiles
   DBuf<int> inv_ints;
@@ -122,6 +123,7 @@ static int chol_plan_alloc(CholPlan& P, bool dissected, cudaStream_t st) {
   CholSymbolic& S = P.S;
   const size_t ns = S.row.size(), nt = (size_t)S.nt;
   CholInts I;
+  I.v.reserve(S.asm_ent.size() + S.upd.size() + 8 * (ns + nt) + nt * kTile + S.pos.size() + 64);
   const size_t o[] = {I.add(S.col_ptr), I.add(S.row), I.add(S.col), I.add(S.width), I.add(S.orig), I.add(S.asm_ptr),
                       I.add(S.asm_ent), I.add(S.upd_ptr), I.add(S.upd), I.add(S.task), I.add(S.solve_order),
                       I.add(S.fwd_ptr), I.add(S.fwd), I.add(S.pos)};
@@ -129,6 +131,7 @@ static int chol_plan_alloc(CholPlan& P, bool dissected, cudaStream_t st) {
   std::vector<int>().swap(S.upd);
   I.v.resize(I.v.size() + 4, 0);
   G2OC_TRY(P.ints.upload(I.v, st));
+  G2OC_TRY(P.places.alloc(S.asm_ptr.back()));
   const size_t vec = nt * kTile;
   G2OC_TRY(P.vals.alloc((ns + nt) * kTileElems + 5 * vec + nt));
   G2OC_TRY(P.flags.alloc(ns + 2 * nt));
@@ -141,10 +144,11 @@ static int chol_plan_alloc(CholPlan& P, bool dissected, cudaStream_t st) {
   double* W = L + ns * kTileElems;
   double* y = W + nt * kTileElems;
   P.d = CholDev{S.n, S.nt, (int)ns, (int)S.task.size(), q + o[0], q + o[1], q + o[2], q + o[3], q + o[4], q + o[5],
-                reinterpret_cast<const int4*>(q + o[6]), q + o[7], reinterpret_cast<const int2*>(q + o[8]), q + o[9],
+                P.places.p, q + o[7], reinterpret_cast<const int2*>(q + o[8]), q + o[9],
                 q + o[10], q + o[11], q + o[12], L, W, y, y + vec, dissected, y + 2 * vec, y + 3 * vec, y + 4 * vec, y + 5 * vec,
                 P.flags.p, P.flags.p + ns, P.flags.p + ns + nt, P.state.p};
   P.pos = q + o[13];
+  P.asm_ent = q + o[6];
   int dev = 0;
   G2OC_CUDA_TRY(cudaGetDevice(&dev));
   G2OC_CUDA_TRY(cudaDeviceGetAttribute(&P.sms, cudaDevAttrMultiProcessorCount, dev));
@@ -152,29 +156,40 @@ static int chol_plan_alloc(CholPlan& P, bool dissected, cudaStream_t st) {
   return G2OC_OK;
 }
 
-// brow, bcol: the blocks of the matrix, row by row; extra: further (row,
-// col) block pairs whose entries the plan must hold (the blocks a selected
-// inverse is asked for), treated as structural nonzeros of the matrix so that
-// the symbolic fill covers them
-static int chol_plan_build(CholPlan& P, int nb, int bs, const std::vector<int>& brow, const std::vector<int>& bcol,
-                           bool reorder, cudaStream_t st, const std::vector<int32_t>* extra = nullptr) {
-  CholSymbolic& S = P.S;
-  chol_symbolic(S, nb, bs, brow, bcol, reorder, extra);
-  // entries of block p of row r at rptr[r] * bs^2 + e * nblk + (p - rptr[r])
-  std::vector<int> rptr(nb + 1, 0);
-  for (int r : brow) ++rptr[r + 1];
-  for (int i = 0; i < nb; ++i) rptr[i + 1] += rptr[i];
-  for (size_t q = 0; q < S.asm_ent.size() / 4; ++q) {
-    int* a = S.asm_ent.data() + 4 * q;
-    const int r = brow[a[0]];
-    const long long off = (long long)rptr[r] * bs * bs + (a[0] - rptr[r]);
-    const int place = (a[1] + kTile) | ((a[2] + kTile) << 8) | (a[3] << 16);
-    a[0] = (int)(off & 0xffffffffll);
-    a[1] = (int)(off >> 32);
-    a[2] = rptr[r + 1] - rptr[r];
-    a[3] = place;
+// Where the entries of a slot's blocks are (values of block p of row r at
+// rptr[r] bs^2 + e nblk + (p - rptr[r])) and where they go: the row and column
+// of the block's first entry in the tile, negative or beyond the tile for a
+// block that straddles tiles. One CTA per slot, once per plan: the list of
+// blocks is a quarter of it, which is what the host makes and sends.
+static __global__ void chol_places(CholDev P, const int* asm_ent, const int* brow, const int* rcol, const int* rptr,
+                                   const int* pos, int bs, int4* places) {
+  const int s = blockIdx.x, i0 = P.row[s] * kTile, j0 = P.col[s] * kTile;
+  for (int q = P.asm_ptr[s] + threadIdx.x; q < P.asm_ptr[s + 1]; q += blockDim.x) {
+    const int k = asm_ent[q], r = brow[k], c = rcol[k], rb = rptr[r];
+    const bool tr = pos[r] < pos[c];  // the tile holds it with the larger position as the row
+    const long long off = (long long)rb * bs * bs + (k - rb);
+    const int i = pos[tr ? c : r] - i0 + kTile, j = pos[tr ? r : c] - j0 + kTile;
+    places[q] = make_int4((int)(off & 0xffffffffll), (int)(off >> 32), rptr[r + 1] - rb, i | (j << 8) | ((tr ? 1 : 0) << 16));
   }
-  return chol_plan_alloc(P, reorder, st);
+}
+
+// brow, bcol: the blocks of the matrix, row by row, and d_brow, d_rcol, d_rptr
+// its lists on the device (SysDev); extra: further (row, col) block pairs whose
+// entries the plan must hold (the blocks a selected inverse is asked for),
+// treated as structural nonzeros of the matrix so that the symbolic fill covers
+// them
+static int chol_plan_build(CholPlan& P, int nb, int bs, const std::vector<int>& brow, const std::vector<int>& bcol,
+                           const int* d_brow, const int* d_rcol, const int* d_rptr, bool reorder, cudaStream_t st,
+                           const std::vector<int32_t>* extra = nullptr) {
+  chol_symbolic(P.S, nb, bs, brow, bcol, reorder, extra);
+  G2OC_TRY(chol_plan_alloc(P, reorder, st));
+  chol_places<<<P.d.ns, 128, 0, st>>>(P.dev(), P.asm_ent, d_brow, d_rcol, d_rptr, P.pos, bs, P.places.p);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_error("cholesky plan launch: %s", cudaGetErrorString(e));
+    return G2OC_ERR_CUDA;
+  }
+  return G2OC_OK;
 }
 
 // asynchronous 16-byte global -> shared copies past L1 (tiles written by

@@ -1345,7 +1345,8 @@ struct Engine final : EngineBase {
     if (c->chol) return G2OC_OK;
     const Structure& S = c->S;
     std::unique_ptr<CholPlan> P(new CholPlan());
-    G2OC_TRY(chol_plan_build(*P, S.sys_nb, S.pd, S.sys_brow, S.sys_rcol, !S.ba, c->stream));
+    G2OC_TRY(chol_plan_build(*P, S.sys_nb, S.pd, S.sys_brow, S.sys_rcol, c->sys_brow.p, c->sys_rcol.p,
+                             c->sys_rptr.p, !S.ba, c->stream));
     P->extra = c->barrier_extra;
     c->chol = std::move(P);
     return G2OC_OK;
@@ -1944,7 +1945,8 @@ struct BalEngine final : EngineBase {
       if (c->prm.linear_solver == G2OC_LINEAR_CHOLESKY) {
         if (!c->chol) {
           std::unique_ptr<CholPlan> P(new CholPlan());
-          G2OC_TRY(chol_plan_build(*P, S.sys_nb, 9, S.sys_brow, S.sys_rcol, false, st));
+          G2OC_TRY(chol_plan_build(*P, S.sys_nb, 9, S.sys_brow, S.sys_rcol, c->sys_brow.p, c->sys_rcol.p,
+                                   c->sys_rptr.p, false, st));
           P->extra = c->barrier_extra;
           c->chol = std::move(P);
         }
@@ -4075,7 +4077,7 @@ int g2oc_solve_block_system(g2oc_ctx* c, int32_t linear_solver, int32_t nb, cons
   int it = 0, ok = 1;
   if (linear_solver == G2OC_LINEAR_CHOLESKY) {
     CholPlan P;
-    G2OC_TRY(chol_plan_build(P, nb, bs, cs.tmp.sys_brow, cs.tmp.sys_rcol, true, st));
+    G2OC_TRY(chol_plan_build(P, nb, bs, cs.tmp.sys_brow, cs.tmp.sys_rcol, A.brow, A.rcol, A.rptr, true, st));
     G2OC_TRY(chol_solve<double>(P, st, A, rhs.p, xo.p, &ok, &c->kcount[K_CHOLESKY]));
   } else {
     G2OC_TRY(mi.alloc((size_t)nb * bs * bs));
@@ -4126,7 +4128,8 @@ static int solve_pattern(g2oc_ctx* c, CallerSystem& cs, int32_t nb, int32_t nreq
   if (pairs.empty()) pairs.push_back(make_int2(0, 0));
   cudaStream_t st = c->stream;
   CholPlan P;
-  G2OC_TRY(chol_plan_build(P, nb, cs.bs, cs.tmp.sys_brow, cs.tmp.sys_rcol, true, st, &extra));
+  G2OC_TRY(chol_plan_build(P, nb, cs.bs, cs.tmp.sys_brow, cs.tmp.sys_rcol, cs.A.brow, cs.A.rcol, cs.A.rptr, true, st,
+                           &extra));
   DBuf<int2> d_req;
   DBuf<double> d_out;
   G2OC_TRY(d_req.upload(pairs, st));

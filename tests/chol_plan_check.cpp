@@ -106,13 +106,9 @@ int main(int argc, char** argv) {
     std::vector<std::vector<int>> where(brow.size());
     for (int s = 0; s < ns; ++s)
       for (int e = P.asm_ptr[s]; e < P.asm_ptr[s + 1]; ++e) {
-        const int* a = P.asm_ent.data() + 4 * (size_t)e;
-        const int r = brow[a[0]], c = bcol[a[0]];
-        const bool tr = P.pos[r] < P.pos[c];
-        if (a[3] != (tr ? 1 : 0) || a[1] + P.row[s] * kTile != P.pos[tr ? c : r] ||
-            a[2] + P.col[s] * kTile != P.pos[tr ? r : c])
-          return fail("assembly entry");
-        where[a[0]].push_back(s);
+        const int k = P.asm_ent[e];
+        if (k < 0 || k >= (int)brow.size()) return fail("assembly entry");
+        where[k].push_back(s);
       }
     for (size_t k = 0; k < brow.size(); ++k) {
       const int a = P.pos[brow[k]], b = P.pos[bcol[k]];
