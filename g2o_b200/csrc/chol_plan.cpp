@@ -2,6 +2,7 @@
 #include "chol_plan.h"
 
 #include <algorithm>
+#include <climits>
 #include <cstddef>
 #include <numeric>
 #include <utility>
@@ -348,9 +349,11 @@ struct Dissector {
 
 }  // namespace
 
-// the fill of the pattern below the diagonal (tile rows by column) and its slots
-static void plan_slots(CholSymbolic& P, std::vector<std::vector<int>>& col) {
+// the fill of the pattern below the diagonal (tile rows by column) and its
+// slots; false: more of them, or of the products, than the plan may have
+static bool plan_slots(CholSymbolic& P, std::vector<std::vector<int>>& col, long long max_tiles) {
   const int nt = P.nt;
+  long long tiles = nt, products = 0;
   // fill: the rows of a column join its parent's (the first row below it)
   P.col_ptr.assign(nt + 1, 0);
   for (int k = 0; k < nt; ++k) {
@@ -361,7 +364,11 @@ static void plan_slots(CholSymbolic& P, std::vector<std::vector<int>>& col) {
       std::vector<int>& p = col[l[0]];
       p.insert(p.end(), l.begin() + 1, l.end());
     }
-    P.col_ptr[k + 1] = P.col_ptr[k] + 1 + (int)l.size();
+    const long long rows = (long long)l.size();
+    tiles += 1 + rows;
+    products += rows * (rows + 1) / 2;
+    if (tiles > std::min<long long>(max_tiles, INT_MAX) || products > INT_MAX) return false;
+    P.col_ptr[k + 1] = P.col_ptr[k] + 1 + (int)rows;
   }
   const int ns = P.col_ptr[nt];
   P.row.resize(ns);
@@ -375,6 +382,7 @@ static void plan_slots(CholSymbolic& P, std::vector<std::vector<int>>& col) {
       P.col[s++] = k;
     }
   }
+  return true;
 }
 
 // update lists, hand-out order and substitution lists of the slots
@@ -472,8 +480,8 @@ static void plan_lists(CholSymbolic& P) {
   std::stable_sort(P.solve_order.begin(), P.solve_order.end(), [&](int a, int b) { return depth[a] < depth[b]; });
 }
 
-void chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow, const std::vector<int>& bcol,
-                   bool reorder, const std::vector<int32_t>* extra) {
+bool chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow, const std::vector<int>& bcol,
+                   bool reorder, const std::vector<int32_t>* extra, long long max_tiles) {
   P = CholSymbolic();
   P.nb = nb;
   P.bs = bs;
@@ -539,7 +547,7 @@ void chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow
   for (int k = 0; k < nnzb; ++k) mark(brow[k], bcol[k]);
   if (extra)
     for (size_t k = 0; k < extra->size() / 2; ++k) mark((*extra)[2 * k], (*extra)[2 * k + 1]);
-  plan_slots(P, col);
+  if (!plan_slots(P, col, max_tiles)) return false;
   const int ns = P.col_ptr[nt];
   auto slot = [&](int i, int k) {
     if (i == k) return P.col_ptr[k];
@@ -576,10 +584,11 @@ void chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow
   std::vector<int> at(P.asm_ptr.begin(), P.asm_ptr.end() - 1);
   each_entry([&](int s, int k) { P.asm_ent[at[s]++] = k; });
   plan_lists(P);
+  return true;
 }
 
-void chol_dense_batch(CholSymbolic& P, const std::vector<int>& first, std::vector<int>& window,
-                      std::vector<int>& index) {
+bool chol_dense_batch(CholSymbolic& P, const std::vector<int>& first, std::vector<int>& window,
+                      std::vector<int>& index, long long max_tiles) {
   P = CholSymbolic();
   const int nw = (int)first.size() - 1;
   P.n = first[nw];
@@ -602,9 +611,10 @@ void chol_dense_batch(CholSymbolic& P, const std::vector<int>& first, std::vecto
     }
   }
   P.nt = (int)col.size();
-  plan_slots(P, col);
+  if (!plan_slots(P, col, max_tiles)) return false;
   P.asm_ptr.assign(P.row.size() + 1, 0);
   plan_lists(P);
+  return true;
 }
 
 }  // namespace g2oc

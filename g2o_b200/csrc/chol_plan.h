@@ -39,16 +39,18 @@ struct CholSymbolic {
 
 // rc: (row, col) pairs of the upper blocks, row-ordered list index = position
 // in brow / bcol; extra: further block pairs the pattern has to hold.
-// reorder: nested dissection, else the given order.
-void chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow, const std::vector<int>& bcol,
-                   bool reorder, const std::vector<int32_t>* extra);
+// reorder: nested dissection, else the given order. False, before any list is
+// made, where the factor has more than max_tiles tiles or more tile products
+// than an int counts (dense, 150,000 unknowns).
+bool chol_symbolic(CholSymbolic& P, int nb, int bs, const std::vector<int>& brow, const std::vector<int>& bcol,
+                   bool reorder, const std::vector<int32_t>* extra, long long max_tiles = 1ll << 31);
 
 // The plan of a batch of dense matrices: matrix w has the unknowns first[w] ..
 // first[w + 1] - 1. The largest come first, so that their chains start first.
 // window, index: per tile column its matrix and its place in it. No assembly
 // lists: the tiles are read from the matrices. The order of a matrix's sums
 // does not depend on the others.
-void chol_dense_batch(CholSymbolic& P, const std::vector<int>& first, std::vector<int>& window,
-                      std::vector<int>& index);
+bool chol_dense_batch(CholSymbolic& P, const std::vector<int>& first, std::vector<int>& window,
+                      std::vector<int>& index, long long max_tiles = 1ll << 31);
 
 }  // namespace g2oc

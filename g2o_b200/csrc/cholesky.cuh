@@ -16,6 +16,8 @@
 #pragma once
 
 #include <algorithm>
+#include <climits>
+#include <exception>
 #include <vector>
 
 #include "chol_plan.h"
@@ -118,6 +120,23 @@ struct CholPlan {
   const CholDev& dev() const { return d; }
 };
 
+// The symbolic part of a plan by make(max_tiles), which says whether the plan
+// may be: no more tiles than fit on the device, so that what cannot be solved
+// costs no lists (up to 32,768 unknowns they are few, and the device is not
+// asked). No exception leaves it (its callers are C entries).
+template <typename F>
+static int chol_plan_symbolic(long long n, F&& make) {
+  size_t free_bytes = 0, total = (size_t)1 << 60;
+  if (n > 32768) G2OC_CUDA_TRY(cudaMemGetInfo(&free_bytes, &total));
+  try {
+    if (make((long long)(total / (kTileElems * sizeof(double))))) return G2OC_OK;
+    set_error("cholesky: the factor does not fit on the device, or has more than %d tile products", INT_MAX);
+  } catch (const std::exception& e) {
+    set_error("cholesky plan: %s", e.what());
+  }
+  return G2OC_ERR_NOT_SUPPORTED;
+}
+
 // device arrays of the plan whose symbolic part is made
 static int chol_plan_alloc(CholPlan& P, bool dissected, cudaStream_t st) {
   CholSymbolic& S = P.S;
@@ -181,7 +200,9 @@ static __global__ void chol_places(CholDev P, const int* asm_ent, const int* bro
 static int chol_plan_build(CholPlan& P, int nb, int bs, const std::vector<int>& brow, const std::vector<int>& bcol,
                            const int* d_brow, const int* d_rcol, const int* d_rptr, bool reorder, cudaStream_t st,
                            const std::vector<int32_t>* extra = nullptr) {
-  chol_symbolic(P.S, nb, bs, brow, bcol, reorder, extra);
+  G2OC_TRY(chol_plan_symbolic((long long)nb * bs, [&](long long max_tiles) {
+    return chol_symbolic(P.S, nb, bs, brow, bcol, reorder, extra, max_tiles);
+  }));
   G2OC_TRY(chol_plan_alloc(P, reorder, st));
   chol_places<<<P.d.ns, 128, 0, st>>>(P.dev(), P.asm_ent, d_brow, d_rcol, d_rptr, P.pos, bs, P.places.p);
   const cudaError_t e = cudaGetLastError();

@@ -3806,7 +3806,9 @@ int g2oc_upload_windows(g2oc_ctx* c, int32_t num_windows, const g2oc_graph* w) {
     std::vector<int> first(nw + 1), window, index;
     for (int i = 0; i <= nw; ++i) first[i] = 6 * wc[i];
     std::unique_ptr<CholPlan> P(new CholPlan());
-    chol_dense_batch(P->S, first, window, index);
+    G2OC_TRY(chol_plan_symbolic(first[nw], [&](long long max_tiles) {
+      return chol_dense_batch(P->S, first, window, index, max_tiles);
+    }));
     std::vector<int2> tile(std::max<size_t>(window.size(), 1), make_int2(0, 0));
     for (size_t k = 0; k < window.size(); ++k) tile[k] = make_int2(window[k], index[k]);
     G2OC_TRY(c->win_tile.upload(tile, st));

@@ -66,7 +66,10 @@ int main(int argc, char** argv) {
   std::vector<int> brow, bcol;
   for (auto& p : pattern(argv[1], nb)) brow.push_back(p.first), bcol.push_back(p.second);
   CholSymbolic P;
-  chol_symbolic(P, nb, bs, brow, bcol, reorder, nullptr);
+  if (!chol_symbolic(P, nb, bs, brow, bcol, reorder, nullptr)) {
+    std::printf("refused\n");
+    return 3;
+  }
   const int nt = P.nt, ns = (int)P.row.size();
   // positions: every unknown once
   std::vector<char> seen((size_t)nb * bs, 0);

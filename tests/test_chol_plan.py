@@ -16,9 +16,12 @@ def plan(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-O2", "-I", CSRC, "-o", exe, os.path.join(HERE, "chol_plan_check.cpp"),
                     os.path.join(CSRC, "chol_plan.cpp")], check=True)
 
-    def run(kind, nb, bs, reorder=True):
+    def run(kind, nb, bs, reorder=True, status=0):
         r = subprocess.run([exe, kind, str(nb), str(bs), str(int(reorder))], capture_output=True, text=True,
                            timeout=300)
+        if status:
+            assert r.returncode == status, (r.returncode, r.stderr)
+            return None
         assert r.returncode == 0, (r.returncode, r.stdout, r.stderr)
         return [int(v) for v in r.stdout.split()]
 
@@ -42,3 +45,9 @@ def test_hub_leaves_a_sparse_graph(plan, kind, nb, bs):
     nt, slots, products, chain = plan(kind, nb, bs)
     n = nb * bs
     assert slots <= 20 * n // 64 and products <= 100 * n // 64 and chain <= n // 64 // 3
+
+
+# 2,345 dense tile columns have 2^31 products
+@pytest.mark.parametrize("reorder", [False, True])
+def test_plan_with_too_many_products_is_refused(plan, reorder):
+    plan("full", 2345, 64, reorder, status=3)
