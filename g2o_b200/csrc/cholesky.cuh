@@ -116,7 +116,10 @@ struct CholPlan {
   DBuf<unsigned> inv_flag;
   DBuf<double> inv_sigma;
   size_t inv_at[3] = {0, 0, 0};
-  unsigned extra = 0;  // the bounded-wait test: flags are compared with a number that is never reached
+  // the bounded-wait tests: flags are compared with a number that is never
+  // reached, in every launch, in the next factorization and solve alone, or in
+  // the solves with a kept factor
+  unsigned extra = 0, extra_once = 0, extra_kept = 0;
   const CholDev& dev() const { return d; }
 };
 
@@ -884,19 +887,21 @@ static int chol_factor(CholPlan& P, cudaStream_t st, const SysDev<Real>& S, cons
 }
 
 // backward substitution of the vector the plan holds
-static int chol_backward(CholPlan& P, cudaStream_t st, double* xout, long long* nl, DevScalars* sc = nullptr) {
-  chol_backward_dag<<<std::min(2 * P.sms, P.S.nt), 256, 0, st>>>(CholAlive{}, P.dev(), xout, sc, P.extra);
+static int chol_backward(CholPlan& P, cudaStream_t st, double* xout, long long* nl, DevScalars* sc = nullptr,
+                         unsigned extra = 0) {
+  chol_backward_dag<<<std::min(2 * P.sms, P.S.nt), 256, 0, st>>>(CholAlive{}, P.dev(), xout, sc, P.extra + extra);
   *nl += 1;
   return chol_launch_check("cholesky solve");
 }
 
 // forward and backward substitution with the factor the plan holds (a
-// refinement's correction solve reuses it)
+// refinement's correction solve reuses it). Its waits are bounded too: the
+// caller reads P.state->err
 static int chol_resolve(CholPlan& P, cudaStream_t st, const double* rhs, double* xout, long long* nlaunch) {
   long long nl = 1;
-  chol_forward_dag<<<std::min(2 * P.sms, P.S.nt), 256, 0, st>>>(P.dev(), rhs, P.extra);
+  chol_forward_dag<<<std::min(2 * P.sms, P.S.nt), 256, 0, st>>>(P.dev(), rhs, P.extra + P.extra_kept);
   G2OC_TRY(chol_launch_check("cholesky solve"));
-  G2OC_TRY(chol_backward(P, st, xout, &nl));
+  G2OC_TRY(chol_backward(P, st, xout, &nl, nullptr, P.extra_kept));
   if (nlaunch) *nlaunch += nl;
   return G2OC_OK;
 }
@@ -907,8 +912,12 @@ template <typename Real>
 static int chol_solve_async(CholPlan& P, cudaStream_t st, const SysDev<Real>& S, const double* rhs, double* xout,
                             long long* nlaunch, DevScalars* sc = nullptr, bool have_floor = false) {
   long long nl = 0;
-  G2OC_TRY(chol_factor<Real>(P, st, S, rhs, &nl, have_floor));
-  G2OC_TRY(chol_backward(P, st, xout, &nl, sc));
+  P.extra += P.extra_once;
+  const int rc = chol_factor<Real>(P, st, S, rhs, &nl, have_floor);
+  const int rb = rc == G2OC_OK ? chol_backward(P, st, xout, &nl, sc) : rc;
+  P.extra -= P.extra_once;
+  P.extra_once = 0;
+  if (rb != G2OC_OK) return rb;
   if (nlaunch) *nlaunch += nl;
   return G2OC_OK;
 }

@@ -385,6 +385,7 @@ struct g2oc_ctx {
   // was created with G2OC_TEST_BARRIER_EXTRA set (every bounded barrier wait
   // of the persistent PCG then runs out: the test of that path)
   unsigned barrier_extra = 0;
+  unsigned chol_extra_once = 0, chol_extra_kept = 0;  // CholPlan::extra_once, extra_kept
   double ktime_ms[g2oc::K_COUNT] = {};
   long long chol_launches = 0;
   std::vector<cudaEvent_t> event_pool;
@@ -1348,8 +1349,18 @@ struct Engine final : EngineBase {
     G2OC_TRY(chol_plan_build(*P, S.sys_nb, S.pd, S.sys_brow, S.sys_rcol, c->sys_brow.p, c->sys_rcol.p,
                              c->sys_rptr.p, !S.ba, c->stream));
     P->extra = c->barrier_extra;
+    P->extra_once = c->chol_extra_once;
+    P->extra_kept = c->chol_extra_kept;
     c->chol = std::move(P);
     return G2OC_OK;
+  }
+
+  // the outcome of the Cholesky, where the host needs it before the end of the
+  // trial; a wait that ran out is reported here and not again there
+  int chol_result(int* ok) {
+    const int rc = chol_outcome(*c->chol, c->stream, ok);
+    if (rc == G2OC_ERR_TIMEOUT) cudaMemsetAsync(&c->sc.p->chol_error, 0, sizeof(int), c->stream);
+    return rc;
   }
 
   int hpp_inverse(const std::vector<int2>& req, double* out, int* ok, bool* done) override {
@@ -1531,7 +1542,7 @@ struct Engine final : EngineBase {
         G2OC_TRY(chol_solve(sysval.p, c->b.p, c->x.p, true));
         decided = true;
         if (sizeof(Real) == 4 && !S.ba && c->prm.refine_max_iterations >= 0) {
-          G2OC_TRY(chol_outcome(*c->chol, st, &ok));
+          G2OC_TRY(chol_result(&ok));
           if (ok) G2OC_TRY(refine_pose_graph(lambda));
         }
       } else {
@@ -1582,8 +1593,14 @@ struct Engine final : EngineBase {
       G2OC_LAUNCH_CHECK();
       G2OC_TRY(finalize_sum(c, kRedBlocks, 2, &c->sc.p->refine_rnorm, &c->sc.p->refine_bnorm));
       double rb[2];
+      int late = 0;  // a wait of the correction's solve ran out
       G2OC_CUDA_TRY(cudaMemcpyAsync(rb, &c->sc.p->refine_rnorm, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+      G2OC_CUDA_TRY(cudaMemcpyAsync(&late, &c->chol->state.p->err, sizeof(int), cudaMemcpyDeviceToHost, st));
       G2OC_CUDA_TRY(cudaStreamSynchronize(st));
+      if (late) {
+        set_error("cholesky: a wait for a tile ran out");
+        return G2OC_ERR_TIMEOUT;
+      }
       const double rel = rb[1] > 0.0 ? std::sqrt(rb[0] / rb[1]) : 0.0;
       c->last_refine_dn = rel;
       if (prev >= 0.0 && !(rel < prev)) {
@@ -1698,7 +1715,7 @@ struct Engine final : EngineBase {
     int ok = 1;
     if (use_chol) {
       G2OC_TRY(chol_solve(Sval.p, c->rhs.p, c->xs.p));
-      G2OC_TRY(chol_outcome(*c->chol, st, &ok));
+      G2OC_TRY(chol_result(&ok));
       if (!ok) {
         set_error("adjoint solve: the reduced system is not positive definite");
         return G2OC_ERR_NOT_PD;
@@ -2661,7 +2678,14 @@ int g2oc_create(int device, g2oc_ctx** out) {
   G2OC_CUDA_TRY(cudaSetDevice(device));
   std::unique_ptr<g2oc_ctx> c(new g2oc_ctx());
   c->device = device;
-  if (const char* e = getenv("G2OC_TEST_BARRIER_EXTRA")) c->barrier_extra = atoi(e) > 0 ? 1u : 0u;
+  // bounded-wait tests: 1 every wait, 2 the first Cholesky solve, 3 Cholesky
+  // solves with a kept factor
+  if (const char* e = getenv("G2OC_TEST_BARRIER_EXTRA")) {
+    const int kind = atoi(e);
+    c->barrier_extra = kind == 1 ? 1u : 0u;
+    c->chol_extra_once = kind == 2 ? 1u : 0u;
+    c->chol_extra_kept = kind == 3 ? 1u : 0u;
+  }
   G2OC_CUDA_TRY(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   g2oc_default_params(&c->prm);
   G2OC_TRY(c->dev.alloc(1));
