@@ -3202,7 +3202,11 @@ int g2oc_set_sharding(g2oc_ctx* c, int32_t rank, int32_t world, g2oc_allreduce_f
   return G2OC_OK;
 }
 
-static int optimize_impl(g2oc_ctx* c, int iterations, g2oc_iteration_stats* stats, int* done) {
+// scratch: the record of an iteration whose caller wants none (stats NULL). The
+// phase times are written to the records an iteration late, so it is the
+// caller's and not on the stack here
+static int optimize_impl(g2oc_ctx* c, int iterations, g2oc_iteration_stats* stats, g2oc_iteration_stats* scratch,
+                         int* done) {
   if (iterations < 0) {
     set_error("iterations < 0");
     return G2OC_ERR_INVALID_ARGUMENT;
@@ -3211,9 +3215,8 @@ static int optimize_impl(g2oc_ctx* c, int iterations, g2oc_iteration_stats* stat
   G2OC_TRY(reset_pcg(c));  // LinearSolverPCG::init via BlockSolver::init
   int result = G2OC_RESULT_OK;
   int it = 0;
-  g2oc_iteration_stats scratch;  // the phase times are written to stats[] an iteration late
   for (int i = 0; i < iterations && result == G2OC_RESULT_OK; ++i) {
-    g2oc_iteration_stats* stv = stats ? stats + i : &scratch;
+    g2oc_iteration_stats* stv = stats ? stats + i : scratch;
     memset(stv, 0, sizeof(*stv));
     cudaEvent_t t0 = c->mark();
     if (c->prm.algorithm == G2OC_ALGO_LEVENBERG) G2OC_TRY(lm_iteration(c, i, stv, &result));
@@ -3254,11 +3257,12 @@ static int iterate_impl(g2oc_ctx* c, int iteration, g2oc_iteration_stats* stats,
   return G2OC_OK;
 }
 
-// the iteration paths record phase-time spans aimed at a stats record on
-// their own stack; a failure half-way must not leave those behind
+// The iteration paths record phase-time spans aimed at the stats records of
+// the call; a failure half-way must not leave those behind
 int g2oc_optimize(g2oc_ctx* c, int iterations, g2oc_iteration_stats* stats, int* done) {
   G2OC_TRY(check_ctx(c, true));
-  const int st = optimize_impl(c, iterations, stats, done);
+  g2oc_iteration_stats scratch;
+  const int st = optimize_impl(c, iterations, stats, &scratch, done);
   if (st != G2OC_OK) {
     c->resolve_spans(c->spans_ended);  // the iterations before the one that failed
     c->drop_spans();
