@@ -63,6 +63,7 @@ def library() -> C.CDLL:
         "g2oc_construct": ([C.c_char_p, vp], C.c_int),
         "g2oc_create": ([C.c_int, C.POINTER(vp)], C.c_int),
         "g2oc_destroy": ([vp], None),
+        "g2oc_trim": ([C.c_int], C.c_int),
         "g2oc_set_params": ([vp, vp], C.c_int),
         "g2oc_upload": ([vp, vp], C.c_int),
         "g2oc_get_hessian_info": ([vp, vp], C.c_int),
@@ -164,6 +165,12 @@ class OptimizationAlgorithmFactory:
         if st != 0:
             return None
         return p
+
+
+def trim(device: int = 0):
+    """Give back the device memory that closed problems left for the next ones
+    (g2oc_trim)."""
+    _check(library().g2oc_trim(device))
 
 
 class CudaProblem:

@@ -84,16 +84,47 @@ constexpr double kAdjointAcceptance = 1e-6;
 // ---------------------------------------------------- device buffer cache
 // Released buffers of up to 64 MB, at most 256 MB a device, kept by size class
 // (four per power of two: at most a quarter is lost) until they are taken
-// again, until 4096 buffers were taken and released since, or until an
-// allocation fails. The stream a buffer was last used on is not known here, so
-// before a buffer is taken again the device is waited for once after its
-// release, as cudaFree would have done for each; the wait serves all buffers
-// released before it. One lock per device: contexts may be on several threads.
+// again, until 4096 buffers were taken and released since, until an allocation
+// fails or until g2oc_trim. A buffer enters once the stream of the context that
+// released it was waited for, as cudaFree would have done for the device, so
+// any thread may take it at once: no other stream is waited for, which might be
+// under capture or at work. Nothing is waited for under the lock. One lock per
+// device: contexts may be on several threads.
 namespace {
+// The calling thread's context: whose stream the buffers it releases were used
+// on. Set by every entry (check_ctx); idle: that stream has nothing queued and
+// gets nothing more (destruction).
+struct BufferOwner {
+  cudaStream_t stream = nullptr;
+  bool idle = false;
+};
+thread_local BufferOwner t_owner;
+
+// The number of the current CUDA context: memory of one that is gone
+// (cudaDeviceReset) must not be given out, nor freed. 0: none, or unknown, and
+// then nothing is kept.
+unsigned long long cuda_context() {
+  using GetCurrent = int (*)(void**);
+  using GetId = int (*)(void*, unsigned long long*);
+  static const std::pair<GetCurrent, GetId> f = [] {
+    void *a = nullptr, *b = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &a, cudaEnableDefault, &q) != cudaSuccess ||
+        cudaGetDriverEntryPoint("cuCtxGetId", &b, cudaEnableDefault, &q) != cudaSuccess) {
+      cudaGetLastError();
+      a = b = nullptr;
+    }
+    return std::make_pair(reinterpret_cast<GetCurrent>(a), reinterpret_cast<GetId>(b));
+  }();
+  void* ctx = nullptr;
+  unsigned long long id = 0;
+  if (!f.first || !f.second || f.first(&ctx) != 0 || !ctx || f.second(ctx, &id) != 0) return 0;
+  return id;
+}
+
 struct DevCache {
   struct Block {
     void* p;
-    bool idle;  // the device was waited for since the release
     unsigned long long tick;
   };
   static constexpr size_t kMaxBlock = 64u << 20, kMaxTotal = 256u << 20;
@@ -101,11 +132,27 @@ struct DevCache {
   std::mutex m;
   std::multimap<size_t, Block> blocks;
   size_t total = 0;
-  unsigned long long tick = 0;
-  void drop(std::multimap<size_t, Block>::iterator it) {
-    cudaFree(it->second.p);
-    total -= it->first;
-    blocks.erase(it);
+  unsigned long long tick = 0, context = 0;
+  // under the lock: forget the blocks of a context that is gone
+  void refresh() {
+    const unsigned long long now = cuda_context();
+    if (now != context) {
+      blocks.clear();
+      total = 0;
+      context = now;
+    }
+  }
+  // under the lock: the blocks released before `before` leave the cache
+  void drop(unsigned long long before, std::vector<void*>& out) {
+    for (auto it = blocks.begin(); it != blocks.end();) {
+      if (it->second.tick >= before) {
+        ++it;
+        continue;
+      }
+      out.push_back(it->second.p);
+      total -= it->first;
+      it = blocks.erase(it);
+    }
   }
 };
 constexpr int kMaxDevices = 64;
@@ -119,27 +166,31 @@ size_t size_class(size_t bytes) {
   const size_t step = p / 4;
   return (b + step - 1) / step * step;
 }
+// the current device's cache is given back
+void trim_cache(int device) {
+  std::vector<void*> out;
+  {
+    DevCache& C = dev_cache(device);
+    std::lock_guard<std::mutex> lk(C.m);
+    C.refresh();
+    C.drop(~0ull, out);
+  }
+  for (void* p : out) cudaFree(p);
+}
 }  // namespace
 
 cudaError_t dev_alloc(void** p, size_t* bytes, int* device) {
   cudaError_t e = cudaGetDevice(device);
   if (e != cudaSuccess) return e;
   if (*device >= kMaxDevices) return cudaMalloc(p, *bytes);
-  DevCache& C = dev_cache(*device);
-  std::lock_guard<std::mutex> lk(C.m);
-  ++C.tick;
   if (*bytes <= DevCache::kMaxBlock) {
     *bytes = size_class(*bytes);
-    const auto r = C.blocks.equal_range(*bytes);
-    if (r.first != r.second) {
-      auto it = r.first;
-      while (it != r.second && !it->second.idle) ++it;
-      if (it == r.second) {
-        it = r.first;
-        e = cudaDeviceSynchronize();
-        if (e != cudaSuccess) return e;
-        for (auto& b : C.blocks) b.second.idle = true;
-      }
+    DevCache& C = dev_cache(*device);
+    std::lock_guard<std::mutex> lk(C.m);
+    ++C.tick;
+    if (!C.blocks.empty()) C.refresh();
+    const auto it = C.blocks.find(*bytes);
+    if (it != C.blocks.end()) {
       *p = it->second.p;
       C.total -= it->first;
       C.blocks.erase(it);
@@ -147,32 +198,37 @@ cudaError_t dev_alloc(void** p, size_t* bytes, int* device) {
     }
   }
   e = cudaMalloc(p, *bytes);
-  if (e == cudaErrorMemoryAllocation && !C.blocks.empty()) {
+  if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    while (!C.blocks.empty()) C.drop(C.blocks.begin());
+    trim_cache(*device);
     e = cudaMalloc(p, *bytes);
   }
   return e;
 }
 
 void dev_free(void* p, size_t bytes, int device) {
-  if (device >= kMaxDevices || bytes > DevCache::kMaxBlock) {
+  int current = -1;
+  if (device >= kMaxDevices || bytes > DevCache::kMaxBlock || !t_owner.stream ||
+      cudaGetDevice(&current) != cudaSuccess || current != device ||
+      (!t_owner.idle && cudaStreamSynchronize(t_owner.stream) != cudaSuccess)) {
     cudaFree(p);
     return;
   }
-  DevCache& C = dev_cache(device);
-  std::lock_guard<std::mutex> lk(C.m);
-  ++C.tick;
-  for (auto it = C.blocks.begin(); it != C.blocks.end();) {
-    const auto b = it++;
-    if (b->second.tick + DevCache::kMaxAge < C.tick) C.drop(b);
+  std::vector<void*> out;
+  {
+    DevCache& C = dev_cache(device);
+    std::lock_guard<std::mutex> lk(C.m);
+    C.refresh();
+    ++C.tick;
+    if (C.tick > DevCache::kMaxAge) C.drop(C.tick - DevCache::kMaxAge, out);
+    if (C.context == 0 || C.total + bytes > DevCache::kMaxTotal) {
+      out.push_back(p);
+    } else {
+      C.blocks.emplace(bytes, DevCache::Block{p, C.tick});
+      C.total += bytes;
+    }
   }
-  if (C.total + bytes > DevCache::kMaxTotal) {
-    cudaFree(p);
-    return;
-  }
-  C.blocks.emplace(bytes, DevCache::Block{p, false, C.tick});
-  C.total += bytes;
+  for (void* q : out) cudaFree(q);
 }
 
 // --------------------------------------------------------------- engine
@@ -463,6 +519,8 @@ struct g2oc_ctx {
     pending.clear();
   }
   ~g2oc_ctx() {
+    if (stream) cudaStreamSynchronize(stream);
+    g2oc::t_owner = {stream, true};  // for the buffers below and the members after this body
     if (ev_read) cudaEventDestroy(ev_read);
     if (coop_done) cudaEventDestroy(coop_done);
     if (win_graph) cudaGraphExecDestroy(win_graph);
@@ -2526,6 +2584,7 @@ static int check_ctx(g2oc_ctx* c, bool need_upload) {
     return G2OC_ERR_STATE;
   }
   G2OC_CUDA_TRY(cudaSetDevice(c->device));
+  t_owner = {c->stream, false};
   return G2OC_OK;
 }
 
@@ -2708,6 +2767,20 @@ void g2oc_destroy(g2oc_ctx* c) {
   cudaStreamSynchronize(c->stream);
   coop_register(c, -1);
   delete c;
+  t_owner = {};
+}
+
+int g2oc_trim(int device) {
+  int n = 0;
+  if (cudaGetDeviceCount(&n) != cudaSuccess || device < 0 || device >= n) {
+    cudaGetLastError();
+    set_error("device %d out of range (%d devices)", device, n);
+    return G2OC_ERR_INVALID_ARGUMENT;
+  }
+  if (device >= kMaxDevices) return G2OC_OK;
+  G2OC_CUDA_TRY(cudaSetDevice(device));
+  trim_cache(device);
+  return G2OC_OK;
 }
 
 static int make_engine(g2oc_ctx* c) {

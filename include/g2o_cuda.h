@@ -248,6 +248,9 @@ int g2oc_construct(const char* name, g2oc_params* params);
 /* context */
 int g2oc_create(int device, g2oc_ctx** out);
 void g2oc_destroy(g2oc_ctx* ctx);
+/* gives back the device memory that released contexts left for the next ones
+   (at most 256 MB a device; an allocation that fails takes it back by itself) */
+int g2oc_trim(int device);
 int g2oc_set_params(g2oc_ctx* ctx, const g2oc_params* params);
 /* the context's CUDA stream (cudaStream_t), for callers that order their own
    work or CUDA events after the solver's */

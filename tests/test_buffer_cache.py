@@ -1,0 +1,113 @@
+"""The cache of released device buffers: contexts come and go on several threads
+while another one's round is being captured, the memory is given back, and
+nothing of it survives the CUDA context it belongs to."""
+
+import os
+import subprocess
+import sys
+import threading
+
+import numpy as np
+import pytest
+
+from g2o_b200 import synth
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def construct(name):
+    from g2o_b200 import backend
+    return backend.OptimizationAlgorithmFactory.instance().construct(name)
+
+
+@pytest.mark.gpu
+def test_contexts_come_and_go_beside_a_capture():
+    from g2o_b200 import backend
+    windows = [synth.bundle_adjustment(4 + i, 60 + 10 * i, seed=i) for i in range(4)]
+    graph = synth.pose_graph_2d(60, 20, seed=1)
+    stop = threading.Event()
+    errors = []
+
+    def run_windows():
+        w = backend.CudaWindows(windows)
+        stats = w.optimize(3)
+        assert stats[0]["rounds"] > 1  # the rounds after the first are captured
+        e = w.estimates_all()
+        w.close()
+        return e
+
+    def run_graph():
+        p = backend.CudaProblem(graph, construct("gn_cuda"))
+        p.optimize(1)
+        e = p.estimates()[0]
+        p.close()
+        return e
+
+    first_windows, first_graph = run_windows(), run_graph()
+
+    def worker():
+        try:
+            while not stop.is_set():
+                assert np.array_equal(run_graph(), first_graph)
+        except Exception as e:  # reported by the main thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=worker) for _ in range(3)]
+    for t in threads:
+        t.start()
+    try:
+        for _ in range(60):
+            for a, b in zip(run_windows(), first_windows):
+                assert all(np.array_equal(x, y) for x, y in zip(a, b))
+    finally:
+        stop.set()
+        for t in threads:
+            t.join()
+    assert not errors
+
+
+@pytest.mark.gpu
+def test_memory_is_given_back():
+    import torch
+    from g2o_b200 import backend
+    g = synth.bundle_adjustment(60, 20_000, seed=2)
+    p = backend.CudaProblem(g, construct("lm_cuda"))
+    p.optimize(1)
+    p.close()
+    kept = torch.cuda.mem_get_info()[0]
+    backend.trim()
+    given = torch.cuda.mem_get_info()[0]
+    assert given - kept >= 16 << 20
+    backend.trim()
+    assert torch.cuda.mem_get_info()[0] == given
+    p = backend.CudaProblem(g, construct("lm_cuda"))
+    assert p.optimize(2)[0] == 2
+    with pytest.raises(backend.G2ocError):
+        backend.trim(-1)
+
+
+CHILD = """
+import ctypes, numpy as np
+from g2o_b200 import backend, synth
+F = backend.OptimizationAlgorithmFactory.instance().construct
+def run():
+    p = backend.CudaProblem(synth.pose_graph_2d(200, 60, seed=1), F("gn_cuda"))
+    p.optimize(3)
+    e = p.estimates()[0]
+    p.close()
+    return e
+a = run()
+assert np.array_equal(a, run())
+rt = ctypes.CDLL("libcudart.so.12")
+assert rt.cudaDeviceReset() == 0
+assert np.array_equal(a, run())
+assert np.array_equal(a, run())
+backend.trim()
+print("same")
+"""
+
+
+@pytest.mark.gpu
+def test_nothing_survives_the_cuda_context():
+    r = subprocess.run([sys.executable, "-c", CHILD], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "same", r.stderr
