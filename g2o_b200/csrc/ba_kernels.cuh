@@ -546,9 +546,8 @@ __device__ __forceinline__ void ldg_block18(const double* hpl, int blk, double (
 }
 
 // Dense output of the Schur rows for batched windows: each camera row belongs
-// to one window, whose reduced system is a dense FP64 matrix (n + 1 rows of
-// n, row-major, at M + mat[w]; the last row holds the right-hand side). Only
-// the lower triangle is written: the diagonal blocks whole, each upper block
+// to one window, whose reduced system is a dense FP64 matrix (n x n,
+// row-major, at M + mat[w]). Only the lower triangle is written: the diagonal blocks whole, each upper block
 // (r, c) transposed into block (c, r).
 struct DenseOut {
   const int* win_of_cam;  // window of each camera row
@@ -556,7 +555,6 @@ struct DenseOut {
   const long long* mat;   // offset of each window's matrix in M
   double* M;              // nullptr: no dense output
 };
-
 
 // Where the Schur complement goes: the row-SoA layout of sys_offset (S);
 // tiles != nullptr: straight into the dense tiles of the tile PCG (block k at
@@ -575,11 +573,13 @@ struct SchurOut {
 // B_a Dinv_l of the camera's Hpl blocks, one thread per block, into BDw (shared
 // memory, or the camera's part of the scratch); with B_a still in registers,
 // its diagonal-block term BD_a B_a^T (upper 21 entries) and its
-// right-hand-side term BD_a b_l. The sums over the CTA (warp sums, then the
-// warps in order: a fixed order) give S(r, r) = Hpp(r) + lambda I -
-// sum_a BD_a B_a^T and, with bs != nullptr, bs_r = b_r - sum_a BD_a b_l(a).
-// Ends with a barrier that publishes BDw.
-template <typename Real, int THREADS>
+// right-hand-side term BD_a b_l. The sums over the blocks give S(r, r) =
+// Hpp(r) + lambda I - sum_a BD_a B_a^T and, with bs != nullptr, bs_r = b_r -
+// sum_a BD_a b_l(a). They are those of LANES threads (blocks LANES apart, warp
+// sums, the warps in order) however many the CTA has: a row has the same bits
+// whether it is formed here by schur_rows or by schur_cameras, which depends on
+// the other cameras of the graph. Ends with a barrier that publishes BDw.
+template <typename Real, int THREADS, int LANES = THREADS>
 __device__ __forceinline__ void schur_camera(int r, const int* hc_ptr, const int* hc_blk, const int* hc_col,
                                              const Real* hpl, const Real* dinv, Real* BDw, const int* rptr,
                                              const int* s_hpp, const Real* hpp, double lambda,
@@ -587,69 +587,68 @@ __device__ __forceinline__ void schur_camera(int r, const int* hc_ptr, const int
                                              double* bs, double (*red)[36]) {
   constexpr int TS = kTileBlocks * 6;  // scalar row stride of a tile
   const int a0 = hc_ptr[r], na = hc_ptr[r + 1] - a0;
-  Real dacc[21];
-  double racc[6] = {0, 0, 0, 0, 0, 0};
+  const int lane = threadIdx.x & 31;
+  for (int first = threadIdx.x; first < LANES; first += THREADS) {
+    Real dacc[21];
+    double racc[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
-  for (int u = 0; u < 21; ++u) dacc[u] = 0;
-  // the next block's indices are loaded while this one's Hpl and Dinv are
-  int a_next = 0, l_next = 0;
-  if ((int)threadIdx.x < na) {
-    a_next = hc_blk[a0 + threadIdx.x];
-    l_next = hc_col[a0 + threadIdx.x];
-  }
-  for (int t = threadIdx.x; t < na; t += THREADS) {
-    const int a = a_next, l = l_next;
-    if (t + THREADS < na) {
-      a_next = hc_blk[a0 + t + THREADS];
-      l_next = hc_col[a0 + t + THREADS];
+    for (int u = 0; u < 21; ++u) dacc[u] = 0;
+    // the next block's indices are loaded while this one's Hpl and Dinv are
+    int a_next = 0, l_next = 0;
+    if (first < na) {
+      a_next = hc_blk[a0 + first];
+      l_next = hc_col[a0 + first];
     }
-    const Real* Dl = dinv + (size_t)l * 9;
-    Real b[18], D[9], bd[18];
-    ldg_block18(hpl, a, b);
-#pragma unroll
-    for (int q = 0; q < 9; ++q) D[q] = Dl[q];
-    Real* o = BDw + (size_t)t * 18;
-#pragma unroll
-    for (int i = 0; i < 6; ++i)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        bd[hpl_at(i, c)] = b[hpl_at(i, 0)] * D[c] + b[hpl_at(i, 1)] * D[3 + c] + b[hpl_at(i, 2)] * D[6 + c];
-        o[hpl_at(i, c)] = bd[hpl_at(i, c)];
+    for (int t = first; t < na; t += LANES) {
+      const int a = a_next, l = l_next;
+      if (t + LANES < na) {
+        a_next = hc_blk[a0 + t + LANES];
+        l_next = hc_col[a0 + t + LANES];
       }
-    int u = 0;
+      const Real* Dl = dinv + (size_t)l * 9;
+      Real b[18], D[9], bd[18];
+      ldg_block18(hpl, a, b);
 #pragma unroll
-    for (int i = 0; i < 6; ++i)
+      for (int q = 0; q < 9; ++q) D[q] = Dl[q];
+      Real* o = BDw + (size_t)t * 18;
 #pragma unroll
-      for (int c = i; c < 6; ++c, ++u)
-        dacc[u] += bd[hpl_at(i, 0)] * b[hpl_at(c, 0)] + bd[hpl_at(i, 1)] * b[hpl_at(c, 1)] +
-                   bd[hpl_at(i, 2)] * b[hpl_at(c, 2)];
-    if (bs) {
-      const double* bl = b_l + (size_t)l * 3;
+      for (int i = 0; i < 6; ++i)
 #pragma unroll
-      for (int q = 0; q < 6; ++q)
-        racc[q] += (double)bd[hpl_at(q, 0)] * bl[0] + (double)bd[hpl_at(q, 1)] * bl[1] +
-                   (double)bd[hpl_at(q, 2)] * bl[2];
+        for (int c = 0; c < 3; ++c) {
+          bd[hpl_at(i, c)] = b[hpl_at(i, 0)] * D[c] + b[hpl_at(i, 1)] * D[3 + c] + b[hpl_at(i, 2)] * D[6 + c];
+          o[hpl_at(i, c)] = bd[hpl_at(i, c)];
+        }
+      int u = 0;
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int c = i; c < 6; ++c, ++u)
+          dacc[u] += bd[hpl_at(i, 0)] * b[hpl_at(c, 0)] + bd[hpl_at(i, 1)] * b[hpl_at(c, 1)] +
+                     bd[hpl_at(i, 2)] * b[hpl_at(c, 2)];
+      if (bs) {
+        const double* bl = b_l + (size_t)l * 3;
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+          racc[q] += (double)bd[hpl_at(q, 0)] * bl[0] + (double)bd[hpl_at(q, 1)] * bl[1] +
+                     (double)bd[hpl_at(q, 2)] * bl[2];
+      }
     }
+    double acc[32];
+#pragma unroll
+    for (int u = 0; u < 21; ++u) acc[u] = (double)dacc[u];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) acc[21 + q] = racc[q];
+#pragma unroll
+    for (int u = 27; u < 32; ++u) acc[u] = 0.0;
+    red[first >> 5][lane] = warp_sums32(acc);
   }
   __threadfence_block();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double acc[27];
-#pragma unroll
-  for (int u = 0; u < 21; ++u) acc[u] = (double)dacc[u];
-#pragma unroll
-  for (int q = 0; q < 6; ++q) acc[21 + q] = racc[q];
-#pragma unroll
-  for (int u = 0; u < 27; ++u) acc[u] = warp_sum(acc[u]);
-  if (lane == 0) {
-#pragma unroll
-    for (int u = 0; u < 27; ++u) red[warp][u] = acc[u];
-  }
   __syncthreads();
   const int u = threadIdx.x;
   if (u >= 27) return;
   double sum = red[0][u];
 #pragma unroll
-  for (int w = 1; w < THREADS / 32; ++w) sum += red[w][u];
+  for (int w = 1; w < LANES / 32; ++w) sum += red[w][u];
   if (u >= 21) {
     if (bs) bs[(size_t)r * 6 + (u - 21)] = b_p[(size_t)r * 6 + (u - 21)] - sum;
     return;
@@ -682,6 +681,45 @@ __device__ __forceinline__ void schur_camera(int r, const int* hc_ptr, const int
   }
 }
 
+// An off-diagonal block S(r, cc) = [Hpp(r, cc)] - sum BD_a B_b^T (block j of
+// row r), lane (g, t) = (lane / 4, lane % 4) holding the sum's entries (g, 2 t)
+// and (g, 2 t + 1)
+template <typename Real>
+__device__ __forceinline__ void schur_store(const SchurOut<Real>& out, int r, int rb, int nblk, int j, int cc, int off,
+                                            const Real* hpp, double acc0, double acc1) {
+  constexpr int TS = kTileBlocks * 6;
+  using R2 = typename Vec2<Real>::T;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  if (g >= 6 || t > 2) return;
+  double w0 = -acc0, w1 = -acc1;
+  if (hpp) {
+    w0 += (double)hpp[g * 6 + 2 * t];
+    w1 += (double)hpp[g * 6 + 2 * t + 1];
+  }
+  if (out.tiles) {
+    R2 pr;
+    pr.x = (Real)w0;
+    pr.y = (Real)w1;
+    __stcs(reinterpret_cast<R2*>(out.tiles + off + g * TS + 2 * t), pr);
+    if (r / kTileBlocks == cc / kTileBlocks) {
+      Real* base = out.tiles + (size_t)(off / (TS * TS)) * (TS * TS);
+      Real* m = base + ((cc % kTileBlocks) * 6 + 2 * t) * TS + (r % kTileBlocks) * 6 + g;
+      __stcs(m, pr.x);
+      __stcs(m + TS, pr.y);
+    }
+  } else if (out.dn.M) {
+    // block (r, cc) transposed into the lower triangle of the window's matrix
+    const int wi = out.dn.win_of_cam[r], h0 = out.dn.cam[wi], n = 6 * (out.dn.cam[wi + 1] - h0);
+    double* D = out.dn.M + out.dn.mat[wi] + ((size_t)(cc - h0) * 6 + 2 * t) * n + (r - h0) * 6 + g;
+    D[0] = (double)(Real)w0;
+    D[n] = (double)(Real)w1;
+  } else {
+    Real* Sr = out.S + (size_t)rb * 36;
+    __stcs(Sr + (size_t)(g * 6 + 2 * t) * nblk + j, (Real)w0);
+    __stcs(Sr + (size_t)(g * 6 + 2 * t + 1) * nblk + j, (Real)w1);
+  }
+}
+
 // Schur complement by camera rows (block_solver.hpp:343-433): one CTA per
 // free camera r of `rows` (the ones with the most pairs first). schur_camera
 // stages the camera's BD_a blocks and forms the diagonal block and the reduced
@@ -711,7 +749,6 @@ __global__ void __launch_bounds__(THREADS, sizeof(Real) == 4 ? 2 : 1)
                const Real* dinv, Real* bdc, const int* rptr, const int* rcol, const int* pair_ptr,
                const int2* pairs, const int* s_hpp, const Real* hpp, double lambda_all, const double* lambda_of,
                SchurOut<Real> out, const double* b_p, const double* b_l, double* bs, bool pose_blocks) {
-  constexpr int TS = kTileBlocks * 6;  // scalar row stride of a tile
   constexpr int WARPS = THREADS / 32;
   using R2 = typename Vec2<Real>::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -758,36 +795,8 @@ __global__ void __launch_bounds__(THREADS, sizeof(Real) == 4 ? 2 : 1)
                    : "+d"(acc[0]), "+d"(acc[1])
                    : "d"(x[m]), "d"((double)b[m]));
   };
-  // entries (g, 2 t) and (g, 2 t + 1) of block j (acc: the sum of its products)
   auto store = [&](int j, double acc0, double acc1, int hb, int off, int cc) {
-    if (!in || t > 2) return;
-    double w0 = -acc0, w1 = -acc1;
-    if (hb >= 0) {
-      w0 += (double)hpp[(size_t)hb * 36 + g * 6 + 2 * t];
-      w1 += (double)hpp[(size_t)hb * 36 + g * 6 + 2 * t + 1];
-    }
-    if (out.tiles) {
-      R2 pr;
-      pr.x = (Real)w0;
-      pr.y = (Real)w1;
-      __stcs(reinterpret_cast<R2*>(out.tiles + off + g * TS + 2 * t), pr);
-      if (r / kTileBlocks == cc / kTileBlocks) {
-        Real* base = out.tiles + (size_t)(off / (TS * TS)) * (TS * TS);
-        Real* m = base + ((cc % kTileBlocks) * 6 + 2 * t) * TS + (r % kTileBlocks) * 6 + g;
-        __stcs(m, pr.x);
-        __stcs(m + TS, pr.y);
-      }
-    } else if (out.dn.M) {
-      // block (r, cc) transposed into the lower triangle of the window's matrix
-      const int wi = out.dn.win_of_cam[r], h0 = out.dn.cam[wi], n = 6 * (out.dn.cam[wi + 1] - h0);
-      double* D = out.dn.M + out.dn.mat[wi] + ((size_t)(cc - h0) * 6 + 2 * t) * n + (r - h0) * 6 + g;
-      D[0] = (double)(Real)w0;
-      D[n] = (double)(Real)w1;
-    } else {
-      Real* Sr = out.S + (size_t)rb * 36;
-      __stcs(Sr + (size_t)(g * 6 + 2 * t) * nblk + j, (Real)w0);
-      __stcs(Sr + (size_t)(g * 6 + 2 * t + 1) * nblk + j, (Real)w1);
-    }
+    schur_store(out, r, rb, nblk, j, cc, off, hb >= 0 ? hpp + (size_t)hb * 36 : nullptr, acc0, acc1);
   };
   const int split = noff * 4 <= WARPS ? 4 : noff * 2 <= WARPS ? 2 : 1;
   if (split > 1) {
@@ -900,54 +909,55 @@ __global__ void __launch_bounds__(THREADS, sizeof(Real) == 4 ? 2 : 1)
 // blocks do not fit in shared memory: the BD_a go through global memory anyway,
 // and the blocks no longer wait for their camera's part nor a camera for the
 // blocks of the one before it.
-template <typename Real, int THREADS>
+// FP64. LANES: the threads of schur_rows there, whose sums these are.
+template <int THREADS, int LANES>
 __global__ void __launch_bounds__(THREADS)
-    schur_cameras(const int* rows, const int* hc_ptr, const int* hc_blk, const int* hc_col, const Real* hpl,
-                  const Real* dinv, Real* bdc, const int* rptr, const int* s_hpp, const Real* hpp, double lambda_all,
-                  const double* lambda_of, SchurOut<Real> out, const double* b_p, const double* b_l, double* bs) {
-  __shared__ double red[THREADS / 32][36];
+    schur_cameras(const int* rows, const int* hc_ptr, const int* hc_blk, const int* hc_col, const double* hpl,
+                  const double* dinv, double* bdc, const int* rptr, const int* s_hpp, const double* hpp, double lambda_all,
+                  const double* lambda_of, SchurOut<double> out, const double* b_p, const double* b_l, double* bs) {
+  __shared__ double red[LANES / 32][36];
   const int r = rows[blockIdx.x];
-  schur_camera<Real, THREADS>(r, hc_ptr, hc_blk, hc_col, hpl, dinv, bdc + (size_t)hc_ptr[r] * 18, rptr, s_hpp, hpp,
+  schur_camera<double, THREADS, LANES>(r, hc_ptr, hc_blk, hc_col, hpl, dinv, bdc + (size_t)hc_ptr[r] * 18, rptr, s_hpp, hpp,
                               lambda_of ? lambda_of[r] : lambda_all, out, b_p, b_l, bs, red);
 }
 
-// One warp per off-diagonal block, its pairs as in schur_rows. Bound by the
-// gathers of both operands. 96 windows of 10 to 60 cameras (2 M edges, Hpl
+// One warp per off-diagonal block. The sums are those of schur_rows with WARPS
+// warps: its fours of pairs go to two of them in turn, or to four in a row that
+// schur_rows cuts over four warps. Bound by the gathers of both operands. 96 windows of 10 to 60 cameras (2 M edges, Hpl
 // 290 MB in FP64): schur_cameras 132 us (580 MB), schur_blocks 130 us, against
 // 335 us for schur_rows, which has 16 warps per SM to hide the gathers with and
 // none during a camera's part.
-template <typename Real>
+template <int WARPS>
 __global__ void __launch_bounds__(256, 3)
-    schur_blocks(int nnzb, const int* brow, const int* hc_ptr, const Real* hpl,
-                 const Real* bdc, const int* rptr, const int* rcol, const int* pair_ptr, const int2* pairs,
-                 const int* s_hpp, const Real* hpp, SchurOut<Real> out, bool pose_blocks) {
-  constexpr int TS = kTileBlocks * 6;
-  using R2 = typename Vec2<Real>::T;
+    schur_blocks(int nnzb, const int* brow, const int* hc_ptr, const double* hpl,
+                 const double* bdc, const int* rptr, const int* rcol, const int* pair_ptr, const int2* pairs,
+                 const int* s_hpp, const double* hpp, SchurOut<double> out, bool pose_blocks) {
   const int lane = threadIdx.x & 31, k = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (k >= nnzb) return;
   const int r = brow[k], rb = rptr[r], nblk = rptr[r + 1] - rb, j = k - rb;
   if (j == 0) return;  // the diagonal: schur_cameras
   const int p1 = pair_ptr[k + 1];
-  const Real* const BD = bdc + (size_t)hc_ptr[r] * 18;
+  const bool four = (nblk - 1) * 4 <= WARPS;
+  const double* const BD = bdc + (size_t)hc_ptr[r] * 18;
   const int g = lane >> 2, t = lane & 3;
   const bool in = g < 6;
   auto index = [&](int p) { return p + t < p1 ? __ldcs(pairs + p + t) : make_int2(-1, -1); };
-  auto gather = [&](const Real* base, int blk, Real (&b)[3]) {
-    R2 u;
-    u.x = u.y = Real(0);
-    b[2] = Real(0);
+  auto gather = [&](const double* base, int blk, double (&b)[3]) {
+    double2 u = make_double2(0.0, 0.0);
+    b[2] = 0.0;
     if (blk >= 0 && in) {
-      const Real* B = base + (size_t)blk * 18;
-      u = __ldg(reinterpret_cast<const R2*>(B) + g);
+      const double* B = base + (size_t)blk * 18;
+      u = __ldg(reinterpret_cast<const double2*>(B) + g);
       b[2] = __ldg(B + 12 + g);
     }
     b[0] = u.x;
     b[1] = u.y;
   };
-  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, acc4[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+  bool odd = false;
   int p = pair_ptr[k];
   int2 i0[2] = {index(p), index(p + 4)}, i1[2] = {index(p + 8), index(p + 12)};
-  Real x[2][3], b[2][3];
+  double x[2][3], b[2][3];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     gather(BD, i0[h].x, x[h]);
@@ -955,19 +965,24 @@ __global__ void __launch_bounds__(256, 3)
   }
   for (; p < p1; p += 8) {
     const int2 i2[2] = {index(p + 16), index(p + 20)};
-    Real xn[2][3], bn[2][3];
+    double xn[2][3], bn[2][3];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       gather(BD, i1[h].x, xn[h]);
       gather(hpl, i1[h].y, bn[h]);
     }
+    auto products = [&](double (&c)[2][2]) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int m = 2; m >= 0; --m)
-        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                     : "+d"(acc[h][0]), "+d"(acc[h][1])
-                     : "d"((double)x[h][m]), "d"((double)b[h][m]));
+        for (int m = 2; m >= 0; --m)
+          asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                       : "+d"(c[h][0]), "+d"(c[h][1])
+                       : "d"(x[h][m]), "d"(b[h][m]));
+    };
+    if (four && odd) products(acc4);
+    else products(acc);
+    odd = !odd;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       i1[h] = i2[h];
@@ -978,36 +993,14 @@ __global__ void __launch_bounds__(256, 3)
       }
     }
   }
-  if (!in || t > 2) return;
+  double s0 = acc[0][0] + acc[1][0], s1 = acc[0][1] + acc[1][1];
+  if (four) {
+    s0 = (s0 + acc4[0][0]) + acc4[1][0];
+    s1 = (s1 + acc4[0][1]) + acc4[1][1];
+  }
   const int hb = pose_blocks ? s_hpp[k] : -1;
-  double w0 = -(acc[0][0] + acc[1][0]), w1 = -(acc[0][1] + acc[1][1]);
-  if (hb >= 0) {
-    w0 += (double)hpp[(size_t)hb * 36 + g * 6 + 2 * t];
-    w1 += (double)hpp[(size_t)hb * 36 + g * 6 + 2 * t + 1];
-  }
-  const int cc = rcol[k], off = out.tiles ? out.tile_off[k] : 0;
-  if (out.tiles) {
-    R2 pr;
-    pr.x = (Real)w0;
-    pr.y = (Real)w1;
-    __stcs(reinterpret_cast<R2*>(out.tiles + off + g * TS + 2 * t), pr);
-    if (r / kTileBlocks == cc / kTileBlocks) {
-      Real* base = out.tiles + (size_t)(off / (TS * TS)) * (TS * TS);
-      Real* m = base + ((cc % kTileBlocks) * 6 + 2 * t) * TS + (r % kTileBlocks) * 6 + g;
-      __stcs(m, pr.x);
-      __stcs(m + TS, pr.y);
-    }
-  } else if (out.dn.M) {
-    // block (r, cc) transposed into the lower triangle of the window's matrix
-    const int wi = out.dn.win_of_cam[r], h0 = out.dn.cam[wi], n = 6 * (out.dn.cam[wi + 1] - h0);
-    double* D = out.dn.M + out.dn.mat[wi] + ((size_t)(cc - h0) * 6 + 2 * t) * n + (r - h0) * 6 + g;
-    D[0] = (double)(Real)w0;
-    D[n] = (double)(Real)w1;
-  } else {
-    Real* Sr = out.S + (size_t)rb * 36;
-    __stcs(Sr + (size_t)(g * 6 + 2 * t) * nblk + j, (Real)w0);
-    __stcs(Sr + (size_t)(g * 6 + 2 * t + 1) * nblk + j, (Real)w1);
-  }
+  schur_store(out, r, rb, nblk, j, rcol[k], out.tiles ? out.tile_off[k] : 0,
+              hb >= 0 ? hpp + (size_t)hb * 36 : nullptr, s0, s1);
 }
 
 // FP32 rows with short pair lists: the off-diagonal blocks by two lanes each

@@ -1221,19 +1221,23 @@ struct Engine final : EngineBase {
       G2OC_LAUNCH_CHECK();
       return G2OC_OK;
     };
-    if constexpr (sizeof(Real) == 4)
+    if constexpr (sizeof(Real) == 4) {
       G2OC_TRY(launch(stage_in_smem ? schur_rows_short<T, true> : schur_rows_short<T, false>, 1));
-    if (stage_in_smem) return launch(schur_rows<Real, T, true>, 0);
-    if constexpr (sizeof(Real) == 4) return launch(schur_rows<Real, T, false>, 0);  // beside schur_rows_short
-    if (row_n[0] == 0) return G2OC_OK;
-    G2OC_K(K_SCHUR_BLOCKS) schur_cameras<Real, 128><<<row_n[0], 128, 0, st>>>(
-        row_list[0].p, c->hc_ptr.p, c->hc_blk.p, c->hc_col.p, hpl.p, dinv.p, bdc.p, c->sys_rptr.p, c->s_hpp.p, hpp.p,
-        lambda, lam_c, out, bp, bl, bs);
-    G2OC_K(K_SCHUR_BLOCKS) schur_blocks<Real><<<cdiv(c->S.sys_nnzb, 8), 256, 0, st>>>(
-        c->S.sys_nnzb, c->sys_brow.p, c->hc_ptr.p, hpl.p, bdc.p, c->sys_rptr.p, c->sys_rcol.p,
-        c->s_pair_ptr.p, c->s_pairs.p, c->s_hpp.p, hpp.p, out, c->S.npp > 0);
-    G2OC_LAUNCH_CHECK();
-    return G2OC_OK;
+      return launch(stage_in_smem ? schur_rows<Real, T, true> : schur_rows<Real, T, false>, 0);
+    } else {
+      // one camera whose blocks do not fit in shared memory: two launches for
+      // all rows, with the same sums
+      if (stage_in_smem) return launch(schur_rows<Real, T, true>, 0);
+      if (row_n[0] == 0) return G2OC_OK;
+      G2OC_K(K_SCHUR_BLOCKS) schur_cameras<128, T><<<row_n[0], 128, 0, st>>>(
+          row_list[0].p, c->hc_ptr.p, c->hc_blk.p, c->hc_col.p, hpl.p, dinv.p, bdc.p, c->sys_rptr.p, c->s_hpp.p,
+          hpp.p, lambda, lam_c, out, bp, bl, bs);
+      G2OC_K(K_SCHUR_BLOCKS) schur_blocks<T / 32><<<cdiv(c->S.sys_nnzb, 8), 256, 0, st>>>(
+          c->S.sys_nnzb, c->sys_brow.p, c->hc_ptr.p, hpl.p, bdc.p, c->sys_rptr.p, c->sys_rcol.p,
+          c->s_pair_ptr.p, c->s_pairs.p, c->s_hpp.p, hpp.p, out, c->S.npp > 0);
+      G2OC_LAUNCH_CHECK();
+      return G2OC_OK;
+    }
   }
 
   int schur_rhs_from(const double* rp, const double* rl, double* bs) {

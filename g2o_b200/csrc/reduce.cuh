@@ -14,6 +14,23 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
+// warp_sum of 32 values, value u to lane u: lanes that are 16 (8, 4, 2, 1) apart
+// exchange halves of what they still hold, 31 shuffles where one warp_sum each
+// takes 160. The same pairs are added, so the sums have the same bits.
+__device__ __forceinline__ double warp_sums32(double (&v)[32]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const double keep = up ? v[i + o] : v[i], send = up ? v[i] : v[i + o];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  return v[0];
+}
+
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
