@@ -1128,19 +1128,23 @@ static int chol_inverse_plan(CholPlan& P, cudaStream_t st) {
   P.inv_at[2] = I.add(reinterpret_cast<const int*>(ent.data()), 4 * ent.size());
   I.v.resize(I.v.size() + 4, 0);
   G2OC_TRY(P.inv_flag.alloc(ns));
-  G2OC_TRY(P.inv_sigma.alloc((size_t)ns * kTileElems));
-  G2OC_CUDA_TRY(cudaMemsetAsync(P.inv_sigma.p, 0, P.inv_sigma.bytes(), st));  // the parts without unknowns stay zero
   G2OC_TRY(P.inv_ints.upload(I.v, st));
   G2OC_CUDA_TRY(cudaStreamSynchronize(st));  // the copied host array goes out of scope
   return G2OC_OK;
 }
 
+// The tiles of the inverse stay with the plan up to this size (some 2,000 of
+// them, a 5,000-pose 2D graph), as making them anew is a good part of a small
+// call; larger ones, as large as the factor, would take the memory of whatever
+// the program does next.
+constexpr size_t kInverseKept = 64u << 20;
+
 // whether the plan's pattern holds the block (r, c)
 static bool chol_covers(const CholPlan& P, int r, int c) {
   const CholSymbolic& Y = P.S;
   const int i0 = Y.pos[r], j0 = Y.pos[c];
-  for (int a = 0; a < Y.bs; a += Y.bs - 1)
-    for (int b = 0; b < Y.bs; b += Y.bs - 1) {
+  for (int a = 0; a < Y.bs; a += std::max(Y.bs - 1, 1))
+    for (int b = 0; b < Y.bs; b += std::max(Y.bs - 1, 1)) {
       const int i = std::max(i0 + a, j0 + b) / kTile, j = std::min(i0 + a, j0 + b) / kTile;
       if (!std::binary_search(Y.row.begin() + Y.col_ptr[j], Y.row.begin() + Y.col_ptr[j + 1], i)) return false;
     }
@@ -1157,6 +1161,10 @@ static int chol_selected_inverse(CholPlan& P, cudaStream_t st, const SysDev<Real
   G2OC_TRY(chol_backward(P, st, nullptr, &nl));  // the rank
   G2OC_TRY(chol_inverse_plan(P, st));
   const int ns = (int)P.S.row.size(), bs = P.S.bs;
+  if (!P.inv_sigma.p) {
+    G2OC_TRY(P.inv_sigma.alloc((size_t)ns * kTileElems));
+    G2OC_CUDA_TRY(cudaMemsetAsync(P.inv_sigma.p, 0, P.inv_sigma.bytes(), st));  // the parts without unknowns stay zero
+  }
   G2OC_CUDA_TRY(cudaMemsetAsync(P.inv_flag.p, 0, P.inv_flag.bytes(), st));
   const int* q = P.inv_ints.p;
   const SelinvDev Q{q + P.inv_at[0], reinterpret_cast<const int4*>(q + P.inv_at[2]), q + P.inv_at[1], P.inv_flag.p,
@@ -1174,7 +1182,9 @@ static int chol_selected_inverse(CholPlan& P, cudaStream_t st, const SysDev<Real
   }
   G2OC_TRY(chol_launch_check("selected inverse"));
   if (nlaunch) *nlaunch += nl;
-  return chol_outcome(P, st, ok);
+  const int rc = chol_outcome(P, st, ok);
+  if (P.inv_sigma.bytes() > kInverseKept) P.inv_sigma.release();
+  return rc;
 }
 
 }  // namespace g2oc

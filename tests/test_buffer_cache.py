@@ -111,3 +111,18 @@ print("same")
 def test_nothing_survives_the_cuda_context():
     r = subprocess.run([sys.executable, "-c", CHILD], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "same", r.stderr
+
+
+@pytest.mark.gpu
+def test_marginals_of_a_large_graph_leave_no_tiles():
+    import torch
+    from g2o_b200 import backend
+    g = synth.pose_graph_2d(20_000, 6_000, seed=3)  # 7,500 tiles, 245 MB
+    p = backend.CudaProblem(g, construct("gn_cuda"))
+    p.build_system()
+    assert p.solve(0.0)[0] == 0  # the factor is there
+    block = np.array([[1, 1], [19_000, 19_000]], np.int32)
+    before = torch.cuda.mem_get_info()[0]
+    a = p.compute_marginals(block)
+    assert before - torch.cuda.mem_get_info()[0] <= 64 << 20
+    assert np.array_equal(a, p.compute_marginals(block))
