@@ -166,6 +166,15 @@ def algorithmic_bytes(kernel, info, E, real, num_pairs):
     return None
 
 
+def passes_per_launch(kernel, kstats):
+    """Passes that algorithmic_bytes counts for, per launch of a kernel: a Schur
+    pass (one landmark step each) can be several launches of the Schur rows."""
+    passes = kstats.get("schur_landmark", (0, 0.0))[0]
+    if kernel in ("schur_rows", "schur_blocks") and passes > 0:
+        return passes / kstats[kernel][0]
+    return 1.0
+
+
 def traffic_table():
     """dram__bytes_read.sum + dram__bytes_write.sum per launch from the
     committed ncu summary (profiles/dram_traffic.txt: kernel precision bytes)."""
@@ -1228,6 +1237,8 @@ def run_ours(args):
     if dname in ("pcg_solve", "pcg_solve_tiles") and dlaunch > 0:  # one launch = a whole solve
         per_it = "pcg_iteration" if dname == "pcg_solve" else "pcg_tile_iteration"
         algo = algorithmic_bytes(per_it, pm.info, 0, real, 0) * pcg_its / dlaunch
+    elif algo is not None:
+        algo *= passes_per_launch(dname, kstats)
     peak, peak_kind = measured_peaks()
     roof = None
     if algo is not None and dlaunch > 0:
