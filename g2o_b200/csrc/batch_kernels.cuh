@@ -138,7 +138,10 @@ static __global__ void win_spread_lambda(const int* win_of_cam, int Cf, const in
   else if (t < Cf + Pf) lam_l[t - Cf] = ws[win_of_lm[t - Cf]].lambda;
 }
 
-// Largest number of free camera unknowns of a window.
+// Largest number of free camera unknowns of a window: what the interface has
+// promised since one CTA held a panel of a window's matrix in shared memory.
+// The tiles below know no such limit; a larger window is a bundle adjustment of
+// its own (g2oc_optimize).
 constexpr int kWinMaxUnknowns = 837;
 
 // The windows' dense reduced camera systems as one batch for the tiled

@@ -778,9 +778,7 @@ static int run_pcg(g2oc_ctx* c, const SysDev<Real>& A, const double* minv, const
   return G2OC_OK;
 }
 
-// The whole PCG solve as one cooperative launch (pcg_solve_persistent), one
-// CTA pair per SM; the host reads the state once at the end.
-// one cluster for the whole solve (at most pcg_cluster_rows block rows)
+// The whole PCG solve in one cluster (at most pcg_cluster_rows block rows)
 template <typename Real, int BS, int NB>
 static int run_pcg_cluster(g2oc_ctx* c, const SysDev<Real>& A, const double* minv, const double* rhs, double* xout,
                            bool fixed_d0) {
@@ -805,6 +803,9 @@ static int run_pcg_cluster(g2oc_ctx* c, const SysDev<Real>& A, const double* min
   return G2OC_OK;
 }
 
+// The whole PCG solve as one launch: in one cluster where that takes it, else
+// cooperative (pcg_solve_persistent), one CTA pair per SM; the host reads the
+// state once at the end.
 template <typename Real, int BS>
 static int run_pcg_persistent(g2oc_ctx* c, const SysDev<Real>& A, const double* minv, const double* rhs,
                               double* xout, double* r, double* s, double* d, double* tbuf, double* cpart,

@@ -254,16 +254,6 @@ static __global__ void __launch_bounds__(128, 1)
   }
 }
 
-// ------------------------------------------------------------ diagonal tile
-// Factor the diagonal tile k in FP64 (lower), write L(k,k) back in FP32 and
-// W(k) = L(k,k)^-1 (FP32, column-major 128 x 128, zero above the diagonal)
-// to Wk. The 128 x 128 tile is taken as 2 x 2 blocks of 64 (256 threads):
-//   L11 W11 = chol(A11)                    tile_potrf_inv_blk64
-//   L21 = A21 W11^T                        FP64 tensor-core product
-//   L22 W22 = chol(A22 - L21 L21^T)        product, then tile_potrf_inv_blk64
-//   W21 = -W22 (L21 W11)                   two products
-// A non-positive pivot sets *info (the pivot is replaced by 1 so the
-// arithmetic stays finite).
 // the pivot floor of a factorization: 4 n eps (FP64) times the largest
 // diagonal entry of the expanded matrix, one CTA of 1024 threads (fixed tree)
 static __global__ void __launch_bounds__(1024) tc_pivot_floor(const float* A, int np, int n, double* floor) {
@@ -281,6 +271,16 @@ static __global__ void __launch_bounds__(1024) tc_pivot_floor(const float* A, in
   }
 }
 
+// ------------------------------------------------------------ diagonal tile
+// Factor the diagonal tile k in FP64 (lower), write L(k,k) back in FP32 and
+// W(k) = L(k,k)^-1 (FP32, column-major 128 x 128, zero above the diagonal)
+// to Wk. The 128 x 128 tile is taken as 2 x 2 blocks of 64 (256 threads):
+//   L11 W11 = chol(A11)                    tile_potrf_inv_blk64
+//   L21 = A21 W11^T                        FP64 tensor-core product
+//   L22 W22 = chol(A22 - L21 L21^T)        product, then tile_potrf_inv_blk64
+//   W21 = -W22 (L21 W11)                   two products
+// A non-positive pivot sets *info (the pivot is replaced by 1 so the
+// arithmetic stays finite).
 constexpr int kTcLd = 68;                    // operand blocks, as tile_dmma64 reads them
 constexpr int kTcBlk = 64 * kTcLd;           // doubles per operand block
 constexpr int kTcTri = 64 * 65;              // doubles per diagonal block (leading dimension 65)
