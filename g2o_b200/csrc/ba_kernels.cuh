@@ -589,6 +589,10 @@ __device__ __forceinline__ void schur_camera(int r, const int* hc_ptr, const int
   const int a0 = hc_ptr[r], na = hc_ptr[r + 1] - a0;
   const int lane = threadIdx.x & 31;
   for (int first = threadIdx.x; first < LANES; first += THREADS) {
+    if (THREADS < LANES && first - lane >= na) {  // no blocks for this warp: its sums are zero
+      red[first >> 5][lane] = 0.0;
+      continue;
+    }
     Real dacc[21];
     double racc[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll
@@ -911,78 +915,63 @@ __global__ void __launch_bounds__(THREADS, sizeof(Real) == 4 ? 2 : 1)
 // blocks of the one before it.
 // FP64. LANES: the threads of schur_rows there, whose sums these are.
 template <int THREADS, int LANES>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 512 / THREADS)
     schur_cameras(const int* rows, const int* hc_ptr, const int* hc_blk, const int* hc_col, const double* hpl,
                   const double* dinv, double* bdc, const int* rptr, const int* s_hpp, const double* hpp, double lambda_all,
                   const double* lambda_of, SchurOut<double> out, const double* b_p, const double* b_l, double* bs) {
   __shared__ double red[LANES / 32][36];
   const int r = rows[blockIdx.x];
-  schur_camera<double, THREADS, LANES>(r, hc_ptr, hc_blk, hc_col, hpl, dinv, bdc + (size_t)hc_ptr[r] * 18, rptr, s_hpp, hpp,
-                              lambda_of ? lambda_of[r] : lambda_all, out, b_p, b_l, bs, red);
+  schur_camera<double, THREADS, LANES>(r, hc_ptr, hc_blk, hc_col, hpl, dinv, bdc + (size_t)hc_ptr[r] * 18, rptr, s_hpp,
+                                       hpp, lambda_of ? lambda_of[r] : lambda_all, out, b_p, b_l, bs, red);
 }
 
-// One warp per off-diagonal block. The sums are those of schur_rows with WARPS
-// warps: its fours of pairs go to two of them in turn, or to four in a row that
-// schur_rows cuts over four warps. Bound by the gathers of both operands. 96 windows of 10 to 60 cameras (2 M edges, Hpl
-// 290 MB in FP64): schur_cameras 132 us (580 MB), schur_blocks 130 us, against
-// 335 us for schur_rows, which has 16 warps per SM to hide the gathers with and
-// none during a camera's part.
-template <int WARPS>
-__global__ void __launch_bounds__(256, 3)
-    schur_blocks(int nnzb, const int* brow, const int* hc_ptr, const double* hpl,
-                 const double* bdc, const int* rptr, const int* rcol, const int* pair_ptr, const int2* pairs,
-                 const int* s_hpp, const double* hpp, SchurOut<double> out, bool pose_blocks) {
-  const int lane = threadIdx.x & 31, k = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (k >= nnzb) return;
-  const int r = brow[k], rb = rptr[r], nblk = rptr[r + 1] - rb, j = k - rb;
-  if (j == 0) return;  // the diagonal: schur_cameras
-  const int p1 = pair_ptr[k + 1];
-  const bool four = (nblk - 1) * 4 <= WARPS;
-  const double* const BD = bdc + (size_t)hc_ptr[r] * 18;
-  const int g = lane >> 2, t = lane & 3;
-  const bool in = g < 6;
-  auto index = [&](int p) { return p + t < p1 ? __ldcs(pairs + p + t) : make_int2(-1, -1); };
-  auto gather = [&](const double* base, int blk, double (&b)[3]) {
-    double2 u = make_double2(0.0, 0.0);
-    b[2] = 0.0;
-    if (blk >= 0 && in) {
-      const double* B = base + (size_t)blk * 18;
-      u = __ldg(reinterpret_cast<const double2*>(B) + g);
-      b[2] = __ldg(B + 12 + g);
-    }
-    b[0] = u.x;
-    b[1] = u.y;
-  };
-  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, acc4[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-  bool odd = false;
-  int p = pair_ptr[k];
-  int2 i0[2] = {index(p), index(p + 4)}, i1[2] = {index(p + 8), index(p + 12)};
+// the three values of a Hpl or BD block that lane (g, t) has in a product, 0 for
+// blk < 0 and in the fragment's empty rows
+__device__ __forceinline__ void schur_operand(const double* base, int blk, double (&b)[3]) {
+  const int g = (threadIdx.x & 31) >> 2;
+  double2 u = make_double2(0.0, 0.0);
+  b[2] = 0.0;
+  if (blk >= 0 && g < 6) {
+    const double* B = base + (size_t)blk * 18;
+    u = __ldg(reinterpret_cast<const double2*>(B) + g);
+    b[2] = __ldg(B + 12 + g);
+  }
+  b[0] = u.x;
+  b[1] = u.y;
+}
+__device__ __forceinline__ void schur_product(const double (&x)[3], const double (&b)[3], double (&c)[2]) {
+#pragma unroll
+  for (int m = 2; m >= 0; --m)
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(x[m]), "d"(b[m]));
+}
+
+// The pairs p, p + 1, .. of a block by fours, two at a time, STEP apart: the
+// sums of the first and of the second ones. The indices of the step after next
+// and the operands of the next are on their way.
+template <int STEP>
+__device__ __forceinline__ void schur_two_sums(const int2* pairs, int p, int p1, const double* BD, const double* hpl,
+                                               double (&acc)[2][2]) {
+  const int t = threadIdx.x & 3;
+  auto index = [&](int q) { return q + t < p1 ? __ldcs(pairs + q + t) : make_int2(-1, -1); };
+  int2 i0[2] = {index(p), index(p + 4)}, i1[2] = {index(p + STEP), index(p + STEP + 4)};
   double x[2][3], b[2][3];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    gather(BD, i0[h].x, x[h]);
-    gather(hpl, i0[h].y, b[h]);
+    schur_operand(BD, i0[h].x, x[h]);
+    schur_operand(hpl, i0[h].y, b[h]);
   }
-  for (; p < p1; p += 8) {
-    const int2 i2[2] = {index(p + 16), index(p + 20)};
+  for (; p < p1; p += STEP) {
+    const int2 i2[2] = {index(p + 2 * STEP), index(p + 2 * STEP + 4)};
     double xn[2][3], bn[2][3];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      gather(BD, i1[h].x, xn[h]);
-      gather(hpl, i1[h].y, bn[h]);
+      schur_operand(BD, i1[h].x, xn[h]);
+      schur_operand(hpl, i1[h].y, bn[h]);
     }
-    auto products = [&](double (&c)[2][2]) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int m = 2; m >= 0; --m)
-          asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                       : "+d"(c[h][0]), "+d"(c[h][1])
-                       : "d"(x[h][m]), "d"(b[h][m]));
-    };
-    if (four && odd) products(acc4);
-    else products(acc);
-    odd = !odd;
+    for (int h = 0; h < 2; ++h) schur_product(x[h], b[h], acc[h]);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       i1[h] = i2[h];
@@ -993,14 +982,51 @@ __global__ void __launch_bounds__(256, 3)
       }
     }
   }
-  double s0 = acc[0][0] + acc[1][0], s1 = acc[0][1] + acc[1][1];
-  if (four) {
-    s0 = (s0 + acc4[0][0]) + acc4[1][0];
-    s1 = (s1 + acc4[0][1]) + acc4[1][1];
+}
+
+// the sum of a block that schur_rows cuts over four warps: the first and the
+// second two of them
+static __device__ __forceinline__ double2 schur_sum_of_four(const int2* pairs, int p, int p1, const double* BD,
+                                                         const double* hpl) {
+  double s0 = 0.0, s1 = 0.0;
+  for (int first = p; first < p + 16; first += 8) {
+    double acc[2][2] = {};
+    schur_two_sums<16>(pairs, first, p1, BD, hpl, acc);
+    s0 = (s0 + acc[0][0]) + acc[1][0];
+    s1 = (s1 + acc[0][1]) + acc[1][1];
+  }
+  return make_double2(s0, s1);
+}
+
+// One warp per off-diagonal block. The sums are those of schur_rows with WARPS
+// warps: its fours of pairs go to two sums in turn, or to four in a row that
+// schur_rows cuts over four warps (a loop of its own, as such rows are few: with
+// the choice in one loop all blocks took 4 to 9% longer, and behind a call 2%).
+// Bound by the gathers of both operands. 96 windows of 10 to 60 cameras (2 M
+// edges, Hpl 290 MB in FP64): schur_cameras 132 us (580 MB), schur_blocks 130
+// us, against 335 us for schur_rows, which has 16 warps per SM to hide the
+// gathers with and none during a camera's part.
+template <int WARPS>
+__global__ void __launch_bounds__(256, 3)
+    schur_blocks(int nnzb, const int* brow, const int* hc_ptr, const double* hpl,
+                 const double* bdc, const int* rptr, const int* rcol, const int* pair_ptr, const int2* pairs,
+                 const int* s_hpp, const double* hpp, SchurOut<double> out, bool pose_blocks) {
+  const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (k >= nnzb) return;
+  const int r = brow[k], rb = rptr[r], nblk = rptr[r + 1] - rb, j = k - rb;
+  if (j == 0) return;  // the diagonal: schur_cameras
+  const double* const BD = bdc + (size_t)hc_ptr[r] * 18;
+  double2 sum;
+  if ((nblk - 1) * 4 <= WARPS) {
+    sum = schur_sum_of_four(pairs, pair_ptr[k], pair_ptr[k + 1], BD, hpl);
+  } else {
+    double acc[2][2] = {};
+    schur_two_sums<8>(pairs, pair_ptr[k], pair_ptr[k + 1], BD, hpl, acc);
+    sum = make_double2(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1]);
   }
   const int hb = pose_blocks ? s_hpp[k] : -1;
   schur_store(out, r, rb, nblk, j, rcol[k], out.tiles ? out.tile_off[k] : 0,
-              hb >= 0 ? hpp + (size_t)hb * 36 : nullptr, s0, s1);
+              hb >= 0 ? hpp + (size_t)hb * 36 : nullptr, sum.x, sum.y);
 }
 
 // FP32 rows with short pair lists: the off-diagonal blocks by two lanes each
