@@ -909,124 +909,137 @@ __global__ void __launch_bounds__(THREADS, sizeof(Real) == 4 ? 2 : 1)
   }
 }
 
+// Warps of a CTA of schur_rows on FP64 values: the sums of the two launches
+// below are those of that many
+constexpr int kSchurWarps = 16;
+
 // The two parts of schur_rows as two launches, for graphs with a camera whose
 // blocks do not fit in shared memory: the BD_a go through global memory anyway,
 // and the blocks no longer wait for their camera's part nor a camera for the
 // blocks of the one before it.
-// FP64. LANES: the threads of schur_rows there, whose sums these are.
-template <int THREADS, int LANES>
+template <int THREADS>
 __global__ void __launch_bounds__(THREADS, 512 / THREADS)
     schur_cameras(const int* rows, const int* hc_ptr, const int* hc_blk, const int* hc_col, const double* hpl,
                   const double* dinv, double* bdc, const int* rptr, const int* s_hpp, const double* hpp, double lambda_all,
                   const double* lambda_of, SchurOut<double> out, const double* b_p, const double* b_l, double* bs) {
-  __shared__ double red[LANES / 32][36];
+  __shared__ double red[kSchurWarps][36];
   const int r = rows[blockIdx.x];
-  schur_camera<double, THREADS, LANES>(r, hc_ptr, hc_blk, hc_col, hpl, dinv, bdc + (size_t)hc_ptr[r] * 18, rptr, s_hpp,
+  schur_camera<double, THREADS, 32 * kSchurWarps>(r, hc_ptr, hc_blk, hc_col, hpl, dinv, bdc + (size_t)hc_ptr[r] * 18, rptr, s_hpp,
                                        hpp, lambda_of ? lambda_of[r] : lambda_all, out, b_p, b_l, bs, red);
 }
 
-// the three values of a Hpl or BD block that lane (g, t) has in a product, 0 for
-// blk < 0 and in the fragment's empty rows
-__device__ __forceinline__ void schur_operand(const double* base, int blk, double (&b)[3]) {
-  const int g = (threadIdx.x & 31) >> 2;
-  double2 u = make_double2(0.0, 0.0);
-  b[2] = 0.0;
-  if (blk >= 0 && g < 6) {
-    const double* B = base + (size_t)blk * 18;
-    u = __ldg(reinterpret_cast<const double2*>(B) + g);
-    b[2] = __ldg(B + 12 + g);
-  }
-  b[0] = u.x;
-  b[1] = u.y;
-}
-__device__ __forceinline__ void schur_product(const double (&x)[3], const double (&b)[3], double (&c)[2]) {
-#pragma unroll
-  for (int m = 2; m >= 0; --m)
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(x[m]), "d"(b[m]));
-}
-
-// The pairs p, p + 1, .. of a block by fours, two at a time, STEP apart: the
-// sums of the first and of the second ones. The indices of the step after next
-// and the operands of the next are on their way.
-template <int STEP>
-__device__ __forceinline__ void schur_two_sums(const int2* pairs, int p, int p1, const double* BD, const double* hpl,
-                                               double (&acc)[2][2]) {
-  const int t = threadIdx.x & 3;
-  auto index = [&](int q) { return q + t < p1 ? __ldcs(pairs + q + t) : make_int2(-1, -1); };
-  int2 i0[2] = {index(p), index(p + 4)}, i1[2] = {index(p + STEP), index(p + STEP + 4)};
-  double x[2][3], b[2][3];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    schur_operand(BD, i0[h].x, x[h]);
-    schur_operand(hpl, i0[h].y, b[h]);
-  }
-  for (; p < p1; p += STEP) {
-    const int2 i2[2] = {index(p + 2 * STEP), index(p + 2 * STEP + 4)};
-    double xn[2][3], bn[2][3];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      schur_operand(BD, i1[h].x, xn[h]);
-      schur_operand(hpl, i1[h].y, bn[h]);
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) schur_product(x[h], b[h], acc[h]);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      i1[h] = i2[h];
-#pragma unroll
-      for (int m = 0; m < 3; ++m) {
-        x[h][m] = xn[h][m];
-        b[h][m] = bn[h][m];
-      }
-    }
-  }
-}
-
-// the sum of a block that schur_rows cuts over four warps: the first and the
-// second two of them
-static __device__ __forceinline__ double2 schur_sum_of_four(const int2* pairs, int p, int p1, const double* BD,
-                                                         const double* hpl) {
-  double s0 = 0.0, s1 = 0.0;
-  for (int first = p; first < p + 16; first += 8) {
-    double acc[2][2] = {};
-    schur_two_sums<16>(pairs, first, p1, BD, hpl, acc);
-    s0 = (s0 + acc[0][0]) + acc[1][0];
-    s1 = (s1 + acc[0][1]) + acc[1][1];
-  }
-  return make_double2(s0, s1);
-}
-
-// One warp per off-diagonal block. The sums are those of schur_rows with WARPS
-// warps: its fours of pairs go to two sums in turn, or to four in a row that
-// schur_rows cuts over four warps (a loop of its own, as such rows are few: with
-// the choice in one loop all blocks took 4 to 9% longer, and behind a call 2%).
+// A warp per off-diagonal block, whose fours of pairs go to two sums in turn;
+// the blocks of rows that schur_rows cuts over four warps (quads, nquad of
+// them) take four warps here too, in CTAs of their own, the last ones (4% of
+// both launches less than as the first ones). The sums are those of schur_rows.
 // Bound by the gathers of both operands. 96 windows of 10 to 60 cameras (2 M
-// edges, Hpl 290 MB in FP64): schur_cameras 132 us (580 MB), schur_blocks 130
-// us, against 335 us for schur_rows, which has 16 warps per SM to hide the
-// gathers with and none during a camera's part.
-template <int WARPS>
-__global__ void __launch_bounds__(256, 3)
-    schur_blocks(int nnzb, const int* brow, const int* hc_ptr, const double* hpl,
+// edges, Hpl 290 MB in FP64): schur_cameras and schur_blocks 271 us together
+// (580 MB in the first), against 335 us for schur_rows, which has 16 warps per
+// SM to hide the gathers with and none during a camera's part.
+static __global__ void __launch_bounds__(256, 3)
+    schur_blocks(int nnzb, const int* quads, int nquad, const int* brow, const int* hc_ptr, const double* hpl,
                  const double* bdc, const int* rptr, const int* rcol, const int* pair_ptr, const int2* pairs,
                  const int* s_hpp, const double* hpp, SchurOut<double> out, bool pose_blocks) {
-  const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (k >= nnzb) return;
-  const int r = brow[k], rb = rptr[r], nblk = rptr[r + 1] - rb, j = k - rb;
-  if (j == 0) return;  // the diagonal: schur_cameras
-  const double* const BD = bdc + (size_t)hc_ptr[r] * 18;
-  double2 sum;
-  if ((nblk - 1) * 4 <= WARPS) {
-    sum = schur_sum_of_four(pairs, pair_ptr[k], pair_ptr[k + 1], BD, hpl);
+  __shared__ double red[8][36];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & 3, g = lane >> 2;
+  const bool in = g < 6;
+  const int plain_ctas = (nnzb + 7) / 8;
+  const bool quad = (int)blockIdx.x >= plain_ctas;
+  int k = (int)blockIdx.x * 8 + warp;
+  if (quad) {
+    const int q = ((int)blockIdx.x - plain_ctas) * 2 + (warp >> 2);
+    k = q < nquad ? quads[q] : nnzb;
+  }
+  if (!quad && k >= nnzb) return;
+  int r = 0, rb = 0, nblk = 0, j = 0, p = 0, p1 = 0;
+  const double* BD = bdc;
+  if (k < nnzb) {
+    r = brow[k];
+    rb = rptr[r];
+    nblk = rptr[r + 1] - rb;
+    j = k - rb;
+    p = pair_ptr[k];
+    p1 = pair_ptr[k + 1];
+    BD = bdc + (size_t)hc_ptr[r] * 18;
+  }
+  auto index = [&](int p) { return p + t < p1 ? __ldcs(pairs + p + t) : make_int2(-1, -1); };
+  auto gather = [&](const double* base, int blk, double (&b)[3]) {
+    double2 u = make_double2(0.0, 0.0);
+    b[2] = 0.0;
+    if (blk >= 0 && in) {
+      const double* B = base + (size_t)blk * 18;
+      u = __ldg(reinterpret_cast<const double2*>(B) + g);
+      b[2] = __ldg(B + 12 + g);
+    }
+    b[0] = u.x;
+    b[1] = u.y;
+  };
+  auto product = [&](const double (&x)[3], const double (&b)[3], double (&c)[2]) {
+#pragma unroll
+    for (int m = 2; m >= 0; --m)
+      asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                   : "+d"(c[0]), "+d"(c[1])
+                   : "d"(x[m]), "d"(b[m]));
+  };
+  // fours of pairs, two at a time, into one sum or two; the indices of the step
+  // after next and the operands of the next are on their way
+  auto sums = [&](auto second, auto step, auto& acc) {
+    constexpr int H = decltype(second)::value, STEP = decltype(step)::value, N = sizeof(acc) / sizeof(acc[0]);
+    int2 i0[2] = {index(p), index(p + H)}, i1[2] = {index(p + STEP), index(p + STEP + H)};
+    double x[2][3], b[2][3];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      gather(BD, i0[h].x, x[h]);
+      gather(hpl, i0[h].y, b[h]);
+    }
+    for (; p < p1; p += STEP) {
+      const int2 i2[2] = {index(p + 2 * STEP), index(p + 2 * STEP + H)};
+      double xn[2][3], bn[2][3];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        gather(BD, i1[h].x, xn[h]);
+        gather(hpl, i1[h].y, bn[h]);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) product(x[h], b[h], acc[h % N]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        i1[h] = i2[h];
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          x[h][m] = xn[h][m];
+          b[h][m] = bn[h][m];
+        }
+      }
+    }
+  };
+  double s0, s1;
+  if (quad) {
+    double acc[1][2] = {{0.0, 0.0}};
+    p += 4 * (warp & 3);
+    sums(std::integral_constant<int, 16>(), std::integral_constant<int, 32>(), acc);
+    if (in && t < 3) {
+      red[warp][g * 6 + 2 * t] = acc[0][0];
+      red[warp][g * 6 + 2 * t + 1] = acc[0][1];
+    }
+    __syncthreads();
+    if ((warp & 3) || k >= nnzb || !in || t > 2) return;
+    s0 = acc[0][0];
+    s1 = acc[0][1];
+    for (int w = 1; w < 4; ++w) {
+      s0 += red[warp + w][g * 6 + 2 * t];
+      s1 += red[warp + w][g * 6 + 2 * t + 1];
+    }
   } else {
-    double acc[2][2] = {};
-    schur_two_sums<8>(pairs, pair_ptr[k], pair_ptr[k + 1], BD, hpl, acc);
-    sum = make_double2(acc[0][0] + acc[1][0], acc[0][1] + acc[1][1]);
+    if (j == 0 || (nblk - 1) * 4 <= kSchurWarps) return;  // schur_cameras; the last CTAs
+    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+    sums(std::integral_constant<int, 4>(), std::integral_constant<int, 8>(), acc);
+    s0 = acc[0][0] + acc[1][0];
+    s1 = acc[0][1] + acc[1][1];
   }
   const int hb = pose_blocks ? s_hpp[k] : -1;
   schur_store(out, r, rb, nblk, j, rcol[k], out.tiles ? out.tile_off[k] : 0,
-              hb >= 0 ? hpp + (size_t)hb * 36 : nullptr, sum.x, sum.y);
+              hb >= 0 ? hpp + (size_t)hb * 36 : nullptr, s0, s1);
 }
 
 // FP32 rows with short pair lists: the off-diagonal blocks by two lanes each
@@ -1387,7 +1400,7 @@ __global__ void __launch_bounds__(THREADS) ba_resid64_camera(BACamEdges CE, BAVe
 // SparseOptimizer::update (sparse_optimizer.cpp:457-468) with
 // VertexSE3Expmap::oplusImpl (g2o/types/sba/vertex_se3_expmap.cpp:48-51):
 // T <- exp(dx) * T; VertexPointXYZ: p <- p + dx (vertex_pointxyz.h:47-50)
-// cam_bak / pt_bak (nullptr: none): the estimates before the update
+// cam_bak / pt_bak (nullptr: none): the estimates before the update.
 static __global__ void ba_oplus(BAVertices V, int Cf, int Pf, const double* x, int* nonfinite, double* cam_bak,
                                 double* pt_bak) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;

@@ -918,6 +918,8 @@ struct Engine final : EngineBase {
   // schur_rows, and in FP32 the rows with short pair lists (schur_rows_short)
   DBuf<int> row_list[2];
   int row_n[2] = {0, 0};
+  DBuf<int> quads;  // schur_blocks: the blocks that take four warps
+  int nquad = 0;
   bool tiles_fresh = false;  // tiles hold the matrix of the current solve
   bool tiles_from_schur = false;  // the last Schur pass wrote the tiles, not the row-SoA values
   bool stage_in_smem = true;  // schur_rows: camera blocks staged in shared memory
@@ -963,6 +965,15 @@ struct Engine final : EngineBase {
       stage_in_smem = schur_smem <= 190 * 1024;
       if (!stage_in_smem) schur_smem = 0;
       if (!stage_in_smem) G2OC_TRY(bdc.alloc(S.hpl_rc.size() / 2 * 18 + 1));
+      if (!stage_in_smem && sizeof(Real) == 8) {
+        std::vector<int> q;
+        for (int r = 0; r < (S.schur ? S.Cf : 0); ++r)
+          if ((S.sys_rptr[r + 1] - S.sys_rptr[r] - 1) * 4 <= kSchurWarps)
+            for (int k = S.sys_rptr[r] + 1; k < S.sys_rptr[r + 1]; ++k) q.push_back(k);
+        nquad = (int)q.size();
+        if (q.empty()) q.push_back(0);
+        G2OC_TRY(quads.upload(q, c->stream));
+      }
       G2OC_TRY(c->db.alloc((size_t)S.Pf * 3 + 1));
       if (c->pose_edges()) {
         const size_t npa = S.pact.size();
@@ -1230,11 +1241,12 @@ struct Engine final : EngineBase {
       // all rows, with the same sums
       if (stage_in_smem) return launch(schur_rows<Real, T, true>, 0);
       if (row_n[0] == 0) return G2OC_OK;
-      G2OC_K(K_SCHUR_BLOCKS) schur_cameras<128, T><<<row_n[0], 128, 0, st>>>(
+      static_assert(T == 32 * kSchurWarps, "the same sums");
+      G2OC_K(K_SCHUR_BLOCKS) schur_cameras<128><<<row_n[0], 128, 0, st>>>(
           row_list[0].p, c->hc_ptr.p, c->hc_blk.p, c->hc_col.p, hpl.p, dinv.p, bdc.p, c->sys_rptr.p, c->s_hpp.p,
           hpp.p, lambda, lam_c, out, bp, bl, bs);
-      G2OC_K(K_SCHUR_BLOCKS) schur_blocks<T / 32><<<cdiv(c->S.sys_nnzb, 8), 256, 0, st>>>(
-          c->S.sys_nnzb, c->sys_brow.p, c->hc_ptr.p, hpl.p, bdc.p, c->sys_rptr.p, c->sys_rcol.p,
+      G2OC_K(K_SCHUR_BLOCKS) schur_blocks<<<cdiv(nquad, 2) + cdiv(c->S.sys_nnzb, 8), 256, 0, st>>>(
+          c->S.sys_nnzb, quads.p, nquad, c->sys_brow.p, c->hc_ptr.p, hpl.p, bdc.p, c->sys_rptr.p, c->sys_rcol.p,
           c->s_pair_ptr.p, c->s_pairs.p, c->s_hpp.p, hpp.p, out, c->S.npp > 0);
       G2OC_LAUNCH_CHECK();
       return G2OC_OK;
