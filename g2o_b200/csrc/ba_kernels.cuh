@@ -1400,9 +1400,11 @@ __global__ void __launch_bounds__(THREADS) ba_resid64_camera(BACamEdges CE, BAVe
 // SparseOptimizer::update (sparse_optimizer.cpp:457-468) with
 // VertexSE3Expmap::oplusImpl (g2o/types/sba/vertex_se3_expmap.cpp:48-51):
 // T <- exp(dx) * T; VertexPointXYZ: p <- p + dx (vertex_pointxyz.h:47-50)
-// cam_bak / pt_bak (nullptr: none): the estimates before the update.
+// cam_bak / pt_bak (nullptr: none): the estimates before the update. still: a
+// camera whose step is zero keeps its bits (exp(0) T normalizes the quaternion):
+// a finished window of a batch, in the rounds that others need
 static __global__ void ba_oplus(BAVertices V, int Cf, int Pf, const double* x, int* nonfinite, double* cam_bak,
-                                double* pt_bak) {
+                                double* pt_bak, bool still) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < Cf) {
     double u[6];
@@ -1419,6 +1421,7 @@ static __global__ void ba_oplus(BAVertices V, int Cf, int Pf, const double* x, i
 #pragma unroll
       for (int i = 0; i < 7; ++i) s[i] = cam[i];
     }
+    if (still && u[0] == 0.0 && u[1] == 0.0 && u[2] == 0.0 && u[3] == 0.0 && u[4] == 0.0 && u[5] == 0.0) return;
     SE3Q<double> T;
     T.q = Q4<double>{cam[0], cam[1], cam[2], cam[3]};
     T.t[0] = cam[4]; T.t[1] = cam[5]; T.t[2] = cam[6];

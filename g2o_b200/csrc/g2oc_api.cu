@@ -2205,7 +2205,7 @@ static int oplus(g2oc_ctx* c, bool backup) {
         c->ba_vertices(), S.Cf, S.Pf, c->x.p, c->flag.p, pose_bak, point_bak);
   else if (S.ba)
     G2OC_K(K_OPLUS) ba_oplus<<<cdiv(S.Cf + S.Pf, 256), 256, 0, st>>>(c->ba_vertices(), S.Cf, S.Pf, c->x.p, c->flag.p,
-                                                                     pose_bak, point_bak);
+                                                                     pose_bak, point_bak, c->batch);
   else if (S.pose_type == G2OC_POSE_SE2)
     G2OC_K(K_OPLUS) pg_oplus<G2OC_POSE_SE2><<<cdiv(S.Cf, 128), 128, 0, st>>>(c->pose.p, c->free_pose.p, S.Cf, c->x.p,
                                                              c->oplus_count.p, c->flag.p, pose_bak);
