@@ -4060,9 +4060,13 @@ int g2oc_optimize_windows(g2oc_ctx* c, int32_t iterations, g2oc_window_stats* st
       return G2OC_ERR_CUDA;
     }
   }
-  // replay the round, checking the count of unfinished windows every few rounds
+  // replay the round, reading the count of unfinished windows every few rounds
+  // while no window can have made its iterations, then after each: finished
+  // windows still take their part of a round, so rounds that none needs cost
+  // what the others do (one window of 512 that rounding gave an 18th trial made
+  // it 21 rounds instead of 17: 53 instead of 49 ms)
   while (active > 0 && rounds < max_rounds) {
-    const int k = std::min(4, max_rounds - rounds);
+    const int k = std::min(rounds < iterations ? std::min(4, iterations - rounds) : 1, max_rounds - rounds);
     for (int i = 0; i < k; ++i) G2OC_CUDA_TRY(cudaGraphLaunch(c->win_graph, st));
     rounds += k;
     G2OC_CUDA_TRY(cudaMemcpyAsync(&active, c->win_active.p, sizeof(int), cudaMemcpyDeviceToHost, st));
