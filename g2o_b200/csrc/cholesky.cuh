@@ -895,13 +895,14 @@ static int chol_backward(CholPlan& P, cudaStream_t st, double* xout, long long* 
 }
 
 // forward and backward substitution with the factor the plan holds (a
-// refinement's correction solve reuses it). Its waits are bounded too: the
-// caller reads P.state->err
-static int chol_resolve(CholPlan& P, cudaStream_t st, const double* rhs, double* xout, long long* nlaunch) {
+// refinement's correction solve reuses it). Its waits are bounded too: one
+// that ran out goes to sc->chol_error, which the end of the trial reads
+static int chol_resolve(CholPlan& P, cudaStream_t st, const double* rhs, double* xout, long long* nlaunch,
+                        DevScalars* sc) {
   long long nl = 1;
   chol_forward_dag<<<std::min(2 * P.sms, P.S.nt), 256, 0, st>>>(P.dev(), rhs, P.extra + P.extra_kept);
   G2OC_TRY(chol_launch_check("cholesky solve"));
-  G2OC_TRY(chol_backward(P, st, xout, &nl, nullptr, P.extra_kept));
+  G2OC_TRY(chol_backward(P, st, xout, &nl, sc, P.extra_kept));
   if (nlaunch) *nlaunch += nl;
   return G2OC_OK;
 }

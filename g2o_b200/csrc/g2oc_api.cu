@@ -1668,14 +1668,8 @@ struct Engine final : EngineBase {
       G2OC_LAUNCH_CHECK();
       G2OC_TRY(finalize_sum(c, kRedBlocks, 2, &c->sc.p->refine_rnorm, &c->sc.p->refine_bnorm));
       double rb[2];
-      int late = 0;  // a wait of the correction's solve ran out
       G2OC_CUDA_TRY(cudaMemcpyAsync(rb, &c->sc.p->refine_rnorm, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
-      G2OC_CUDA_TRY(cudaMemcpyAsync(&late, &c->chol->state.p->err, sizeof(int), cudaMemcpyDeviceToHost, st));
       G2OC_CUDA_TRY(cudaStreamSynchronize(st));
-      if (late) {
-        set_error("cholesky: a wait for a tile ran out");
-        return G2OC_ERR_TIMEOUT;
-      }
       const double rel = rb[1] > 0.0 ? std::sqrt(rb[0] / rb[1]) : 0.0;
       c->last_refine_dn = rel;
       if (prev >= 0.0 && !(rel < prev)) {
@@ -1685,7 +1679,7 @@ struct Engine final : EngineBase {
       }
       if (!(rel > c->prm.refine_tolerance) || k == c->prm.refine_max_iterations) break;
       prev = rel;
-      G2OC_TRY(chol_resolve(*c->chol, st, c->resid.p, c->dx.p, &c->kcount[K_CHOLESKY]));
+      G2OC_TRY(chol_resolve(*c->chol, st, c->resid.p, c->dx.p, &c->kcount[K_CHOLESKY], c->sc.p));
       c->refine_steps++;
       G2OC_K(K_AXPY) axpy_kernel<<<cdiv(n, 256), 256, 0, st>>>(c->x.p, c->dx.p, 1.0, n);
       G2OC_LAUNCH_CHECK();
