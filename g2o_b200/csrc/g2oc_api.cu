@@ -100,6 +100,19 @@ struct BufferOwner {
 };
 thread_local BufferOwner t_owner;
 
+// For a function with buffers of its own, which wait for the stream one by one
+// at its end otherwise: a BufferScope before them and a BufferScope::Settle
+// after them. Settle, destroyed first, waits once; the scope, destroyed last,
+// ends that.
+struct BufferScope {
+  ~BufferScope() { t_owner.idle = false; }
+  struct Settle {
+    ~Settle() {
+      if (t_owner.stream && cudaStreamSynchronize(t_owner.stream) == cudaSuccess) t_owner.idle = true;
+    }
+  };
+};
+
 // The number of the current CUDA context: memory of one that is gone
 // (cudaDeviceReset) must not be given out, nor freed. 0: none, or unknown, and
 // then nothing is kept.
@@ -1455,8 +1468,10 @@ struct Engine final : EngineBase {
       G2OC_K(K_DAMP) sys_gather_damped<Real, 6><<<cdiv(nel, 256), 256, 0, st>>>(
           hpp.p, c->sys_perm.p, c->sys_brow.p, c->sys_rptr.p, c->sys_rcol.p, S.sys_nnzb, 0.0, sysval.p);
     G2OC_LAUNCH_CHECK();
+    BufferScope scope;
     DBuf<int2> d_req;
     DBuf<double> d_out;
+    BufferScope::Settle settle;
     const size_t n = req.size() * S.pd * S.pd;
     G2OC_TRY(d_req.upload(req, st));
     G2OC_TRY(d_out.alloc(n));
@@ -4184,17 +4199,21 @@ int g2oc_solve_block_system(g2oc_ctx* c, int32_t linear_solver, int32_t nb, cons
     return G2OC_ERR_INVALID_ARGUMENT;
   }
   cudaStream_t st = c->stream;
+  BufferScope scope;
   CallerSystem cs;
+  DBuf<double> rhs, xo, mi, r, s, d0, d1, q, qrow, tb;
+  BufferScope::Settle settle;
   G2OC_TRY(caller_system(st, nb, offs, nnzb, rc, values, cs));
   const int bs = cs.bs;
   const SysDev<double>& A = cs.A;
-  DBuf<double> rhs, xo, mi, r, s, d0, d1, q, qrow, tb;
   const int n = nb * bs;
   G2OC_TRY(rhs.upload(std::vector<double>(b, b + n), st));
   G2OC_TRY(xo.alloc(n));
   int it = 0, ok = 1;
   if (linear_solver == G2OC_LINEAR_CHOLESKY) {
+    BufferScope plan_scope;
     CholPlan P;
+    BufferScope::Settle plan_settle;
     G2OC_TRY(chol_plan_build(P, nb, bs, cs.tmp.sys_brow, cs.tmp.sys_rcol, A.brow, A.rcol, A.rptr, true, st));
     G2OC_TRY(chol_solve<double>(P, st, A, rhs.p, xo.p, &ok, &c->kcount[K_CHOLESKY]));
   } else {
@@ -4245,11 +4264,13 @@ static int solve_pattern(g2oc_ctx* c, CallerSystem& cs, int32_t nb, int32_t nreq
   const std::vector<int32_t> extra(req, req + 2 * (size_t)nreq);
   if (pairs.empty()) pairs.push_back(make_int2(0, 0));
   cudaStream_t st = c->stream;
+  BufferScope scope;
   CholPlan P;
-  G2OC_TRY(chol_plan_build(P, nb, cs.bs, cs.tmp.sys_brow, cs.tmp.sys_rcol, cs.A.brow, cs.A.rcol, cs.A.rptr, true, st,
-                           &extra));
   DBuf<int2> d_req;
   DBuf<double> d_out;
+  BufferScope::Settle settle;
+  G2OC_TRY(chol_plan_build(P, nb, cs.bs, cs.tmp.sys_brow, cs.tmp.sys_rcol, cs.A.brow, cs.A.rcol, cs.A.rptr, true, st,
+                           &extra));
   G2OC_TRY(d_req.upload(pairs, st));
   G2OC_TRY(d_out.alloc((size_t)(nreq > 0 ? nreq : 1) * cs.bs * cs.bs));
   int ok = 1;
@@ -4267,7 +4288,9 @@ int g2oc_solve_pattern_block_system(g2oc_ctx* c, int32_t nb, const int32_t* offs
                                     const double* values, int32_t num_blocks, const int32_t* block_indices,
                                     double* out) {
   G2OC_TRY(check_ctx(c, false));
+  BufferScope scope;
   CallerSystem cs;
+  BufferScope::Settle settle;
   G2OC_TRY(caller_system(c->stream, nb, offs, nnzb, rc, values, cs));
   return solve_pattern(c, cs, nb, num_blocks, block_indices, out);
 }
@@ -4305,7 +4328,9 @@ int g2oc_compute_marginals(g2oc_ctx* c, int32_t num_blocks, const int32_t* block
   G2OC_TRY(c->eng->get_hessian(hpp.data(), nullptr, nullptr));
   std::vector<int32_t> offs(nb + 1);
   for (int i = 0; i <= nb; ++i) offs[i] = i * pd;
+  BufferScope scope;
   CallerSystem cs;
+  BufferScope::Settle settle;
   G2OC_TRY(caller_system(c->stream, nb, offs.data(), (int32_t)nnzb, S.hpp_rc.data(), hpp.data(), cs));
   return solve_pattern(c, cs, nb, num_blocks, block_indices, out);
 }
