@@ -58,7 +58,8 @@ struct CholTickets {
 // entry are looked at together, u = L^-T (ones at them): the sum's inverse is
 // then no larger than the smallest share. The system is refused when it is
 // below kRankTol. u rides along in the backward pass, and only if a pivot is
-// suspect: none is in a graph of some thousand poses.
+// suspect: none is in a graph of some thousand poses; 20,000 odometry edges
+// without a closure pay 6% of a solve (520 to 550 us).
 constexpr double kSuspect = 1e-6, kRankTol = 4 * 2.220446049250313e-16;
 
 struct CholState {
@@ -253,19 +254,23 @@ __device__ __forceinline__ int chol_ticket(CholTickets* t, int* sh) {
   __syncthreads();
   return *sh;
 }
-// the last CTA to leave also runs `end`
+// the last CTA to leave also runs `end`, with all its threads
 template <typename F>
 __device__ __forceinline__ void chol_leave(CholTickets* t, F&& end) {
+  __shared__ bool last;
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    if (atomicInc(&t->left, gridDim.x - 1) == gridDim.x - 1) {  // the last one; left is back at 0
-      t->next = 0;
-      t->epoch += 1;
-      end();
-      __threadfence();
-    }
+    last = atomicInc(&t->left, gridDim.x - 1) == gridDim.x - 1;  // left is back at 0 then
+    __threadfence();
   }
+  __syncthreads();
+  if (!last) return;
+  if (threadIdx.x == 0) {
+    t->next = 0;
+    t->epoch += 1;
+  }
+  end();
 }
 
 // The largest |diagonal entry| of the matrix (the pivot floor is a multiple
@@ -671,7 +676,9 @@ __global__ void __launch_bounds__(256, 1) chol_factor_dag(Source A, CholDev P, c
       chol_store_flag(P.flag + s, want);
     }
   }
-  chol_leave(&P.st->factor, [&]() { P.st->max_diag = 0; });
+  chol_leave(&P.st->factor, [&]() {
+    if (tid == 0) P.st->max_diag = 0;
+  });
 }
 
 // Substitutions: tile columns handed out by ticket, one CTA of 256 threads
@@ -846,11 +853,17 @@ __global__ void __launch_bounds__(256) chol_backward_dag(Source A, CholDev P, do
   chol_leave(&P.st->backward, [&]() {
     if (ranked) {
       double uu = 0.0;
-      for (int k = 0; k < P.nt; ++k) uu += __ldcg(P.uu + k);
-      if (!(kRankTol * uu < 1.0)) P.st->info = 1;
-      P.st->suspect = 0;  // decided: not again for a further right-hand side
+      for (int k = tid; k < P.nt; k += 256) uu += __ldcg(P.uu + k);
+      uu = warp_sum(uu);
+      if ((tid & 31) == 0) part[0][tid >> 5] = uu;
+      __syncthreads();
+      if (tid == 0) {
+        for (int w = 1; w < 8; ++w) uu += part[0][w];
+        if (!(kRankTol * uu < 1.0)) P.st->info = 1;
+        P.st->suspect = 0;  // decided: not again for a further right-hand side
+      }
     }
-    A.end(P, sc);
+    if (tid == 0) A.end(P, sc);
   });
 }
 
